@@ -12,16 +12,16 @@
 // One iteration (src/LU/lu-node.jl:233-270 with ssor src/LU/ssor.jl:9-254):
 //   exch_qbc       k_lu_pack + k_lu_unpack (every face packed before any is
 //                  unpacked, as the reference's sends are)
-//   rsd *= dt      fused into the first touch of each point in k_lu_lower
+//   rsd *= dt      fused into the first touch of each point in the lower sweep
 //   Jacobians      k_lu_jac: jacld's and jacu's off-diagonal blocks and the
 //                  factors of d at every point, fully parallel
 //   flux prims     per-point quantities of the flux functions (1/u1, the
 //                  viscous u21.., the convective u21 and q), refreshed where
 //                  u changes: k_lu_unpack (ghost faces), k_lu_pointwise<1>
 //                  (update), uploads; read by the sweeps and rhs
-//   blts           k_lu_lower, one launch per hyperplane i+j+k = l, five
-//                  threads per point (one per row of the 5x5 blocks)
-//   buts           k_lu_upper, one launch per hyperplane, l descending
+//   blts           k_lu_sweep<false>, one launch per hyperplane i+j+k = l,
+//                  five threads per point (one per row of the 5x5 blocks)
+//   buts           k_lu_sweep<true>, one launch per hyperplane, l descending
 //   update         k_lu_pointwise<1>
 //   rhs            k_lu_rhs<false>, one thread per point
 // blts / buts make point (i,j,k) depend on (i-1,j,k), (i,j-1,k), (i,j,k-1)
@@ -72,6 +72,8 @@ struct npbmz_lu_handle {
   double* prim = nullptr;  // PR_COUNT planes (PR_RHO first: 1/u1 for the sweeps)
   double* fac = nullptr;  // FAC_COUNT planes per point: d's factors and the off-diagonal blocks
   int* hps_d = nullptr;   // per zone, hstride ints: interior points with i+j+k < l
+  std::vector<int> hps;   // the same on the host
+  int* pts_d = nullptr;   // per slot (hyperplane order): the point's index within its zone
   std::vector<char> jac_ok;  // per zone: fac holds the blocks of the current u
   int* ri_d = nullptr;       // per zone, l and k: slot of the first interior point of row k of hyperplane l
   int ri_ks = 0;
@@ -203,15 +205,28 @@ int launch_jac(npbmz_lu_t* h, int z0, int nzs) {
   return 0;
 }
 
-int launch_lower(npbmz_lu_t* h, bool scale, int z0, int nzs) {
-  for (int l = h->lmin; l <= h->lmax; ++l) {
-    int c = 0;
-    for (int z = z0; z < z0 + nzs; ++z) c = std::max(c, hp_count(h->zh[z], l));
-    if (!c) continue;
-    const dim3 g((c + HP - 1) / HP, nzs);
-    (h->fast ? lu_fast::lower : lu_exact::lower)(scale, dev(h), h->fac, h->hps_d, h->hstride, l, z0, g, h->stream);
+// Points of hyperplane l in the largest of zones z0 .. z0+nzs-1.
+int hp_max(const npbmz_lu_t* h, int z0, int nzs, int l) {
+  int c = 0;
+  for (int z = z0; z < z0 + nzs; ++z) {
+    const int* p = h->hps.data() + (size_t)z * h->hstride;
+    c = std::max(c, p[l + 1] - p[l]);
   }
-  LU_CK(h, cudaGetLastError());
+  return c;
+}
+
+// One sweep over the wavefront, one launch per hyperplane; every launch after
+// the first may start before the one it follows has ended (k_lu_sweep).
+int launch_sweep(npbmz_lu_t* h, bool up, bool scale, int z0, int nzs) {
+  const LuSweep S{h->fac, h->hps_d, h->pts_d, h->hstride};
+  bool follows = false;
+  for (int n = 0; n <= h->lmax - h->lmin; ++n) {
+    const int l = up ? h->lmax - n : h->lmin + n, c = hp_max(h, z0, nzs, l);
+    if (!c) continue;
+    LU_CK(h, (h->fast ? lu_fast::sweep : lu_exact::sweep)(up, scale, dev(h), S, l, z0, dim3((c + HP - 1) / HP, nzs),
+                                                          follows, h->stream));
+    follows = true;
+  }
   return 0;
 }
 
@@ -238,7 +253,7 @@ int launch_phase(npbmz_lu_t* h, int phase, int zone) {
     case NPBMZ_LU_PHASE_SSOR + 100: {  // lower with the scaling fused
       // the blocks and d's factors of every interior point, then the wavefront
       int rc = launch_jac(h, z0, nzs);
-      if (!rc) rc = launch_lower(h, phase != NPBMZ_LU_PHASE_LOWER, z0, nzs);
+      if (!rc) rc = launch_sweep(h, false, phase != NPBMZ_LU_PHASE_LOWER, z0, nzs);
       return rc;
     }
     case NPBMZ_LU_PHASE_UPPER: {
@@ -247,13 +262,7 @@ int launch_phase(npbmz_lu_t* h, int phase, int zone) {
       bool stale = false;
       for (int z = z0; z < z0 + nzs; ++z) stale = stale || !h->jac_ok[z];
       if (stale && launch_jac(h, z0, nzs)) return -1;
-      for (int l = h->lmax; l >= h->lmin; --l) {
-        int c = 0;
-        for (int z = z0; z < z0 + nzs; ++z) c = std::max(c, hp_count(h->zh[z], l));
-        if (!c) continue;
-        const dim3 g((c + HP - 1) / HP, nzs);
-        (h->fast ? lu_fast::upper : lu_exact::upper)(dev(h), h->fac, h->hps_d, h->hstride, l, z0, g, h->stream);
-      }
+      if (launch_sweep(h, true, false, z0, nzs)) return -1;
       break;
     }
     case NPBMZ_LU_PHASE_SSOR: {
@@ -364,7 +373,7 @@ void free_all(npbmz_lu_t* h) {
   for (void* p : {(void*)h->zones_d, (void*)h->nbr_d, (void*)h->u, (void*)h->rsd, (void*)h->frct, (void*)h->prim,
                   (void*)h->fac, (void*)h->work_d,
                   (void*)h->zblock_d, (void*)h->partial, (void*)h->norms_d, (void*)h->zone_out_d, (void*)h->stage,
-                  (void*)h->zoff_d, (void*)h->img, (void*)h->hps_d, (void*)h->ri_d, (void*)h->fb_d,
+                  (void*)h->zoff_d, (void*)h->img, (void*)h->hps_d, (void*)h->pts_d, (void*)h->ri_d, (void*)h->fb_d,
                   (void*)h->health_d})
     if (p) cudaFree(p);
   if (h->health_h) cudaFreeHost(h->health_h);
@@ -498,7 +507,7 @@ int npbmz_lu_create(int nzones, const int* nx, const int* ny, const int* nz, con
   {
     // u, rsd, frct, the flux quantities and the Jacobian planes, checked
     // before anything is allocated
-    const double need = (double)(15 + PR_COUNT + FAC_COUNT) * (double)off * sizeof(double);
+    const double need = ((double)(15 + PR_COUNT + FAC_COUNT) * sizeof(double) + sizeof(int)) * (double)off;
     size_t free_b = 0, total_b = 0;
     const cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
     if (e != cudaSuccess) {
@@ -593,7 +602,7 @@ int npbmz_lu_create(int nzones, const int* nx, const int* ny, const int* nz, con
       cudaMalloc(&h->partial, h->work_h.size() * 5 * sizeof(double)) ||
       cudaMalloc(&h->zone_out_d, (6 * (size_t)nzones + 16) * sizeof(double)) ||
       cudaMalloc(&h->stage, so * sizeof(double)) || cudaMalloc(&h->zoff_d, nzones * sizeof(long long)) ||
-      cudaMalloc(&h->hps_d, hps.size() * sizeof(int)) || cudaMalloc(&h->ri_d, ri.size() * sizeof(int)) ||
+      cudaMalloc(&h->hps_d, hps.size() * sizeof(int)) || cudaMalloc(&h->pts_d, h->NP * sizeof(int)) || cudaMalloc(&h->ri_d, ri.size() * sizeof(int)) ||
       cudaMalloc(&h->fb_d, fb.size() * sizeof(int)) || cudaMalloc(&h->health_d, 2 * sizeof(unsigned long long)) ||
       cudaMallocHost(&h->health_h, 2 * sizeof(unsigned long long)))
     return bail("device allocation failed");
@@ -609,6 +618,9 @@ int npbmz_lu_create(int nzones, const int* nx, const int* ny, const int* nz, con
       cudaMemset(h->prim, 0, (size_t)PR_COUNT * h->NP * sizeof(double)) ||
       cudaMemset(h->fac, 0, (size_t)FAC_COUNT * h->NP * sizeof(double)))
     return bail("device initialisation failed");
+  lu_exact::points(dev(h), h->ri_d, h->hstride, h->ri_ks, h->pts_d, h->work_d, (int)h->work_h.size(), nullptr);
+  if (cudaGetLastError() || cudaStreamSynchronize(nullptr)) return bail("device initialisation failed");
+  h->hps = std::move(hps);
   *out = h;
   return 0;
 }
@@ -776,11 +788,8 @@ int npbmz_lu_synchronize(npbmz_lu_t* h) {
 int npbmz_lu_launches_per_iteration(npbmz_lu_t* h) {
   if (!h) return fail(nullptr, "null handle");
   int n = 2 + 3;  // exch (pack, unpack) + jac + update + rhs
-  for (int l = h->lmin; l <= h->lmax; ++l) {
-    int c = 0;
-    for (const LuZone& Z : h->zh) c = std::max(c, hp_count(Z, l));
-    if (c) n += 2;
-  }
+  for (int l = h->lmin; l <= h->lmax; ++l)
+    if (hp_max(h, 0, h->nzones, l)) n += 2;
   return n;
 }
 
@@ -799,7 +808,7 @@ int npbmz_lu_profile(npbmz_lu_t* h, int niter, double* phase_ms) {
     cudaEventRecord(ev[1], h->stream);
     if (!rc) rc = launch_jac(h, 0, h->nzones);
     cudaEventRecord(ev[2], h->stream);
-    if (!rc) rc = launch_lower(h, true, 0, h->nzones);
+    if (!rc) rc = launch_sweep(h, false, true, 0, h->nzones);
     cudaEventRecord(ev[3], h->stream);
     if (!rc) rc = launch_phase(h, NPBMZ_LU_PHASE_UPPER, -1);
     cudaEventRecord(ev[4], h->stream);

@@ -584,26 +584,6 @@ __device__ __forceinline__ void jac_off(const JC& J, double r1, double u2, doubl
   }
 }
 
-// The t-th point (0-based) of hyperplane i + j + k = l of a zone's interior,
-// enumerated by k ascending, then j ascending.
-__device__ inline bool hyperplane_point(const LuZone& Z, int l, int t, int& i, int& j, int& k) {
-  const int klo = max(2, l - (Z.nx - 1) - (Z.ny - 1)), khi = min(Z.nz - 1, l - 4);
-  for (int kk = klo; kk <= khi; ++kk) {
-    const int s = l - kk;
-    const int jlo = max(2, s - (Z.nx - 1)), jhi = min(Z.ny - 1, s - 2);
-    const int c = jhi - jlo + 1;
-    if (c <= 0) continue;
-    if (t < c) {
-      k = kk;
-      j = jlo + t;
-      i = s - j;
-      return true;
-    }
-    t -= c;
-  }
-  return false;
-}
-
 __device__ __forceinline__ void load5(const double* f, long long NP, long long p, double v[5]) {
 #pragma unroll
   for (int m = 0; m < 5; ++m) v[m] = f[m * NP + p];
@@ -615,7 +595,7 @@ __device__ __forceinline__ void store_blk(double* jac, long long NP, long long h
   for (int r = 0; r < 5; ++r)
 #pragma unroll
     for (int c = 0; c < 5; ++c)
-      if (!off_zero(DIR, r, c)) jac[(FAC_BLK + (2 * DIR + S) * BLK_NZ + blk_idx(DIR, r, c)) * NP + h] = b[r][c];
+      if (off_stored(DIR, r, c)) jac[(FAC_BLK + (2 * DIR + S) * BLK_N + blk_idx(DIR, r, c)) * NP + h] = b[r][c];
 }
 
 // jacld's (SG = -1) and jacu's (SG = +1) blocks of direction DIR built from
@@ -638,6 +618,24 @@ __device__ __forceinline__ void jac_dir(const JC& J, double r1, const double u[5
     jac_off<DIR, 1>(J, r1, u[1], u[2], u[3], u[4], c);
     store_blk<DIR, 1>(jac, NP, slot_up, c);
   }
+}
+
+// Slot of interior point (i, j, k) in the zone's hyperplane order (R: its row
+// table, [l][k], ks entries per l).
+__device__ __forceinline__ long long hp_slot(const LuZone& Z, const int* __restrict__ R, int ks, int i, int j, int k) {
+  const int l = i + j + k;
+  return Z.off + R[(long long)l * ks + k] + (j - max(2, l - k - (Z.nx - 1)));
+}
+
+// The inverse table of the sweeps: slot -> the point's index within its zone.
+__global__ void __launch_bounds__(TPB) k_lu_points(LuDev D, const int* __restrict__ ri, int ls, int ks,
+                                                   int* __restrict__ pts, const LuWork* __restrict__ work) {
+  const LuWork w = work[blockIdx.x];
+  const LuZone Z = D.zones[w.zone];
+  int i, j, k;
+  const int q = w.first + threadIdx.x;
+  if (!decode(Z, q, i, j, k) || !interior(Z, i, j, k)) return;
+  pts[hp_slot(Z, ri + (long long)w.zone * ls * ks, ks, i, j, k)] = q;
 }
 
 // jacld's and jacu's blocks and d's factors (the Jacobian work of ssor,
@@ -680,10 +678,7 @@ __global__ void __launch_bounds__(TPB) k_lu_jac(LuDev D, const int* __restrict__
   const long long NP = D.NP, p = pidx(Z, i, j, k);
   const JC J{D.dt, Z.tx1, Z.tx2, Z.ty1, Z.ty2, Z.tz1, Z.tz2};
   const int* R = ri + (long long)zone * ls * ks;
-  auto slot = [&](int a, int b, int c) -> long long {
-    const int l = a + b + c;
-    return Z.off + R[(long long)l * ks + c] + (b - max(2, l - c - (Z.nx - 1)));
-  };
+  auto slot = [&](int a, int b, int c) -> long long { return hp_slot(Z, R, ks, a, b, c); };
   const double r1 = D.prim[PR_RHO * NP + p];
   double u[5];
   load5(D.u, NP, p, u);
@@ -706,7 +701,10 @@ __global__ void __launch_bounds__(TPB) k_lu_jac(LuDev D, const int* __restrict__
     jac_d(J, r1, u[1], u[2], u[3], u[4], b);
     const double rinv0 = 1.0e+00 / b[0][0];
 #pragma unroll
-    for (int r = 0; r < 5; ++r) jac[(FAC_T + r) * NP + h] = b[r][r];
+    for (int r = 0; r < 5; ++r) {
+      jac[(FAC_T + r) * NP + h] = b[r][r];
+      jac[(FAC_Y + r) * NP + h] = 1.0e+00 / b[r][r];
+    }
 #pragma unroll
     for (int r = 1; r < 5; ++r) jac[(FAC_R0 + r - 1) * NP + h] = rinv0 * b[r][0];
 #pragma unroll
@@ -714,40 +712,98 @@ __global__ void __launch_bounds__(TPB) k_lu_jac(LuDev D, const int* __restrict__
   }
 }
 
-// row M of the point's block (DIR, S) dotted with w, summed left to right as
-// the reference does (structural zeros skipped: a product with one is +-0
-// and adding it changes no sum's value)
-template <int DIR, int S, int M>
-__device__ __forceinline__ double row_dot(const double* __restrict__ jac, long long NP, long long h,
-                                          const double w[5]) {
+// ---- the wavefront sweeps (src/LU/blts.jl, src/LU/buts.jl) ------------------
+// The entries of a zone's off-diagonal blocks that do not depend on the state,
+// by the reference's expressions: [dir] k00 = -dt t1 d, kn = -+dt t2,
+// k4 = -+dt t2 c2 (S = 0 jacld's signs, S = 1 jacu's).
+struct RowConsts {
+  double k00[3], kn[3], k4[3];
+};
+template <int S>
+__device__ __forceinline__ RowConsts row_consts(double dt, const LuZone& Z) {
+  RowConsts K;
+  K.k00[0] = -dt * Z.tx1 * dx1;
+  K.k00[1] = -dt * Z.ty1 * dy1;
+  K.k00[2] = -dt * Z.tz1 * dz1;
+  const double t2[3] = {Z.tx2, Z.ty2, Z.tz2};
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    K.kn[d] = S == 0 ? -dt * t2[d] : dt * t2[d];
+    K.k4[d] = S == 0 ? -dt * t2[d] * c2 : dt * t2[d] * c2;
+  }
+  return K;
+}
+
+// What row M of one point needs besides rsd: its rows of the three
+// off-diagonal blocks and its part of d's factors.
+struct RowCoef {
+  double b[3][5];
+  double f[4];  // rows 1..3: f[0] = tmp_m0; row 4: tmp_40, tmp_41, tmp_42, tmp_43
+  double t, y;  // t_mm, 1 / t_mm
+};
+
+// Read-only load that stays where it is written: before the wait for the
+// previous hyperplane (the compiler would sink a plain one to its use).
+__device__ __forceinline__ double ld_early(const double* p) {
+  double v;
+  asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+
+template <int S, int M>
+__device__ __forceinline__ void load_row(const double* __restrict__ jac, long long NP, long long h,
+                                         const RowConsts& K, RowCoef& c) {
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+#pragma unroll
+    for (int e = 0; e < 5; ++e) {
+      if (off_zero(d, M, e)) continue;
+      if (off_const(d, M, e))
+        c.b[d][e] = M == 0 ? (e == 0 ? K.k00[d] : K.kn[d]) : K.k4[d];
+      else
+        c.b[d][e] = ld_early(jac + (FAC_BLK + (2 * d + S) * BLK_N + blk_idx(d, M, e)) * NP + h);
+    }
+  if (M > 0) c.f[0] = ld_early(jac + (FAC_R0 + M - 1) * NP + h);
+  if (M == 4) {
+#pragma unroll
+    for (int q = 1; q <= 3; ++q) c.f[q] = ld_early(jac + (FAC_4C + q - 1) * NP + h);
+  }
+  c.t = ld_early(jac + (FAC_T + M) * NP + h);
+  c.y = ld_early(jac + (FAC_Y + M) * NP + h);
+}
+
+// Row M of block z dotted with wz, summed left to right as the reference does
+// (structural zeros skipped: a product with one is +-0 and adding it changes
+// no sum's value).
+template <int M>
+__device__ __forceinline__ double row_dot_z(const RowCoef& c, const double wz[5]) {
   double s = 0.0;
   bool first = true;
 #pragma unroll
-  for (int c = 0; c < 5; ++c) {
-    if (off_zero(DIR, M, c)) continue;
-    const double t = jac[(FAC_BLK + (2 * DIR + S) * BLK_NZ + blk_idx(DIR, M, c)) * NP + h] * w[c];
+  for (int e = 0; e < 5; ++e) {
+    if (off_zero(2, M, e)) continue;
+    const double t = c.b[2][e] * wz[e];
     s = first ? t : s + t;
     first = false;
   }
   return s;
 }
 
-// sum over c of Y[M][c] wy[c] + X[M][c] wx[c] (y term first, as blts / buts
+// sum over e of Y[M][e] wy[e] + X[M][e] wx[e] (y term first, as blts / buts
 // write it)
-template <int S, int M>
-__device__ __forceinline__ double row_dot2(const double* __restrict__ jac, long long NP, long long h,
-                                           const double wy[5], const double wx[5]) {
+template <int M>
+__device__ __forceinline__ double row_dot_yx(const RowCoef& c, const double wy[5], const double wx[5]) {
   double s = 0.0;
   bool first = true;
 #pragma unroll
-  for (int c = 0; c < 5; ++c) {
-    if (!off_zero(1, M, c)) {
-      const double t = jac[(FAC_BLK + (2 + S) * BLK_NZ + blk_idx(1, M, c)) * NP + h] * wy[c];
+  for (int e = 0; e < 5; ++e) {
+    if (!off_zero(1, M, e)) {
+      const double t = c.b[1][e] * wy[e];
       s = first ? t : s + t;
       first = false;
     }
-    if (!off_zero(0, M, c)) {
-      const double t = jac[(FAC_BLK + S * BLK_NZ + blk_idx(0, M, c)) * NP + h] * wx[c];
+    if (!off_zero(0, M, e)) {
+      const double t = c.b[0][e] * wx[e];
       s = first ? t : s + t;
       first = false;
     }
@@ -755,131 +811,110 @@ __device__ __forceinline__ double row_dot2(const double* __restrict__ jac, long 
   return s;
 }
 
-// blts's two update loops for row M of one point (h: its jac index)
-template <int M, bool SCALE>
-__device__ __forceinline__ double lower_row(const LuDev& D, const double* __restrict__ jac, const LuZone& Z, int i,
-                                            int j, int k, long long h) {
-  const long long NP = D.NP, p = pidx(Z, i, j, k);
-  const double omega = D.omega;
-  double v = D.rsd[M * NP + p];
-  if (SCALE) v = D.dt * v;
-  double w[5], x[5];
-  load5(D.rsd, NP, pidx(Z, i, j, k - 1), w);
-  v = v - omega * row_dot<2, 0, M>(jac, NP, h, w);
-  load5(D.rsd, NP, pidx(Z, i, j - 1, k), w);
-  load5(D.rsd, NP, pidx(Z, i - 1, j, k), x);
-  v = v - omega * row_dot2<0, M>(jac, NP, h, w, x);
-  return v;
+// v / t from y = 1/t rounded to nearest: the quotient estimate v y, refined by
+// its FMA residuals (P. Markstein, IBM J. Res. Dev. 34(1), 1990: one step from
+// an estimate within one ulp, with the correctly rounded reciprocal, gives the
+// correctly rounded quotient; the first step here makes the estimate so).  A
+// dependent divide costs nine FP64 instructions where this takes five, and
+// the FP64 pipe binds the sweeps.  Operands whose residual could underflow or
+// overflow take the divide.
+__device__ __forceinline__ double div_y(double v, double t, double y) {
+  const unsigned ev = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu, et = ((unsigned)__double2hiint(t) >> 20) & 0x7ffu;
+  // exponents of v in [2^-600, 2^600) and of t in [2^-300, 2^300): v, t, y, q and every residual are normal
+  if (__builtin_expect(ev - 423u < 1200u && et - 723u < 600u, 1)) {
+    double q = v * y;
+    q = fma(fma(-t, q, v), y, q);
+    return fma(fma(-t, q, v), y, q);
+  }
+  return v / t;
 }
 
-// d's factors row m needs, loaded before the rows are exchanged (so that
-// their latency overlaps the row sums): f[0] = t_mm; rows 1..3 f[1] = tmp_m0;
-// row 4 f[1..4] = tmp_40, tmp_10, tmp_20, tmp_30, f[5..7] = tmp_41..tmp_43
-__device__ __forceinline__ void load_factors(const double* __restrict__ jac, long long NP, long long h, int m,
-                                             double f[8]) {
-  f[0] = jac[(FAC_T + m) * NP + h];
-  if (m >= 1 && m <= 3) f[1] = jac[(FAC_R0 + m - 1) * NP + h];
-  if (m == 4) {
-    f[1] = jac[(FAC_R0 + 3) * NP + h];
-#pragma unroll
-    for (int c = 1; c <= 3; ++c) {
-      f[1 + c] = jac[(FAC_R0 + c - 1) * NP + h];
-      f[4 + c] = jac[(FAC_4C + c - 1) * NP + h];
-    }
-  }
-}
-
-// the forward substitution with d's factors (rows exchanged through shared
-// memory); v: this thread's row, sv: every row of the point
-__device__ __forceinline__ double d_solve(const double f[8], int m, double v, const double sv[5]) {
-  const double v0 = sv[0];
-  if (m == 0) return v / f[0];
-  if (m < 4) {
-    v = v - v0 * f[1];
-    return v / f[0];
-  }
-  v = v - v0 * f[1];
-#pragma unroll
-  for (int c = 1; c <= 3; ++c) {
-    const double vc = sv[c] - v0 * f[1 + c];  // v_c after column 0, as row c has it
-    v = v - vc * f[4 + c];
-  }
-  return v / f[0];
-}
-
-// jacld + blts at every point of hyperplane l (blockIdx.y: zone - zone0),
-// five threads per point (threadIdx.y: row).  SCALE: rsd *= dt at the point
-// first (ssor's scaling, fused: blts reads only points it has already scaled
-// and solved, or boundary points, which the scaling does not touch).
-template <bool SCALE>
-__global__ void __launch_bounds__(HP * 5) k_lu_lower(LuDev D, const double* __restrict__ jac,
-                                                     const int* __restrict__ hps, int hstride, int l, int zone0) {
-  __shared__ double sv[HP][5];
-  const int m = threadIdx.y, a = threadIdx.x, z = zone0 + blockIdx.y;
-  const LuZone Z = D.zones[z];
-  const int t = blockIdx.x * HP + a;
-  int i = 0, j = 0, k = 0;
-  const bool ok = hyperplane_point(Z, l, t, i, j, k);
-  const long long h = ok ? Z.off + hps[(long long)z * hstride + l] + t : 0;
-  double v = 0.0, f[8];
-  if (ok) {
-    load_factors(jac, D.NP, h, m, f);
-    switch (m) {
-      case 0: v = lower_row<0, SCALE>(D, jac, Z, i, j, k, h); break;
-      case 1: v = lower_row<1, SCALE>(D, jac, Z, i, j, k, h); break;
-      case 2: v = lower_row<2, SCALE>(D, jac, Z, i, j, k, h); break;
-      case 3: v = lower_row<3, SCALE>(D, jac, Z, i, j, k, h); break;
-      default: v = lower_row<4, SCALE>(D, jac, Z, i, j, k, h); break;
-    }
-    sv[a][m] = v;
-  }
-  __syncthreads();
-  if (!ok) return;
-  D.rsd[m * D.NP + pidx(Z, i, j, k)] = d_solve(f, m, v, sv[a]);
-}
-
-// buts's two tv loops for row M of one point
-template <int M>
-__device__ __forceinline__ double upper_row(const LuDev& D, const double* __restrict__ jac, const LuZone& Z, int i,
-                                            int j, int k, long long h) {
+// Row M of one point of a sweep (UP false: blts, the neighbours at -1; UP
+// true: buts, the neighbours at +1); h: the point's slot, -1 for a lane
+// without one.  SCALE: rsd *= dt at the point first (ssor's scaling, fused:
+// blts reads only points it has already scaled and solved, or boundary
+// points, which it does not touch).
+template <bool UP, bool SCALE, int M>
+__device__ __forceinline__ void sweep_row(const LuDev& D, const LuSweep& S, const LuZone& Z, long long h, int lane,
+                                          double (*sv)[HP]) {
   const long long NP = D.NP;
-  const double omega = D.omega;
-  double w[5], x[5];
-  load5(D.rsd, NP, pidx(Z, i, j, k + 1), w);
-  double tv = omega * row_dot<2, 1, M>(jac, NP, h, w);
-  load5(D.rsd, NP, pidx(Z, i, j + 1, k), w);
-  load5(D.rsd, NP, pidx(Z, i + 1, j, k), x);
-  tv = tv + omega * row_dot2<1, M>(jac, NP, h, w, x);
-  return tv;
+  RowCoef c;
+  long long p = 0;
+  if (h >= 0) {
+    p = Z.off + __ldg(S.pts + h);
+    load_row<UP ? 1 : 0, M>(S.jac, NP, h, row_consts<UP ? 1 : 0>(D.dt, Z), c);
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the previous hyperplane's rsd from here on
+  double own = 0.0, v = 0.0;
+  if (h >= 0) {
+    const long long sgn = UP ? 1 : -1, sy = sgn * Z.nx, sz = sy * Z.ny;
+    double wz[5], wy[5], wx[5];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
+      const double* r = D.rsd + m * NP + p;
+      wz[m] = __ldcg(r + sz);
+      wy[m] = __ldcg(r + sy);
+      wx[m] = __ldcg(r + sgn);
+    }
+    own = __ldcg(D.rsd + M * NP + p);
+    const double omega = D.omega;
+    if (!UP) {
+      v = SCALE ? D.dt * own : own;
+      v = v - omega * row_dot_z<M>(c, wz);
+      v = v - omega * row_dot_yx<M>(c, wy, wx);
+    } else {
+      v = omega * row_dot_z<M>(c, wz);
+      v = v + omega * row_dot_yx<M>(c, wy, wx);
+    }
+  }
+  // the solve with d: rows 1..4 subtract v_0's part, then row 4 that of 1..3
+  if (M == 0) sv[0][lane] = v;
+  __syncthreads();
+  if (M > 0 && h >= 0) v = v - sv[0][lane] * c.f[0];
+  if (M > 0 && M < 4) sv[M][lane] = v;
+  __syncthreads();
+  if (h < 0) return;
+  if (M == 4) {
+#pragma unroll
+    for (int r = 1; r <= 3; ++r) v = v - sv[r][lane] * c.f[r];
+  }
+  v = div_y(v, c.t, c.y);
+  D.rsd[M * NP + p] = UP ? own - v : v;
 }
 
-// jacu + buts at every point of hyperplane l
-__global__ void __launch_bounds__(HP * 5) k_lu_upper(LuDev D, const double* __restrict__ jac,
-                                                     const int* __restrict__ hps, int hstride, int l, int zone0) {
-  __shared__ double sv[HP][5];
-  const int m = threadIdx.y, a = threadIdx.x, z = zone0 + blockIdx.y;
-  const LuZone Z = D.zones[z];
-  const int t = blockIdx.x * HP + a;
-  int i = 0, j = 0, k = 0;
-  const bool ok = hyperplane_point(Z, l, t, i, j, k);
-  const long long h = ok ? Z.off + hps[(long long)z * hstride + l] + t : 0;
-  double tv = 0.0, f[8], own = 0.0;
-  if (ok) {
-    load_factors(jac, D.NP, h, m, f);
-    own = D.rsd[m * D.NP + pidx(Z, i, j, k)];
-    switch (m) {
-      case 0: tv = upper_row<0>(D, jac, Z, i, j, k, h); break;
-      case 1: tv = upper_row<1>(D, jac, Z, i, j, k, h); break;
-      case 2: tv = upper_row<2>(D, jac, Z, i, j, k, h); break;
-      case 3: tv = upper_row<3>(D, jac, Z, i, j, k, h); break;
-      default: tv = upper_row<4>(D, jac, Z, i, j, k, h); break;
-    }
-    sv[a][m] = tv;
+// blts (UP false) / buts (UP true) at the points of hyperplane i+j+k = l of
+// zones z0 + blockIdx.y, five threads per point: one warp per row and HP
+// points.  Launched once per hyperplane, each launch a programmatic dependent
+// of the one before: its blocks take their place and fetch the coefficients,
+// which the sweep does not change, while the previous hyperplane still runs,
+// and wait for it before they read rsd.
+// Bound: an SM quarter takes an FP64 warp instruction every 64 cycles whatever
+// its active lanes, so the longest row's chain (45 FP64 instructions for row 4
+// without contraction) sets the time of a small hyperplane, and the sum of
+// the rows (about 160 per 32 points) that of a large one.  Rows 0 and 1, the
+// cheapest, run on warps 0 and 4, which share an SM quarter.
+// Both sweeps of one iteration (us, with block rows of 32 points, separate
+// loads and no overlap of the launches, and now): 64x64x8
+// 576 / 193, 304x208x17 contracted 3184 / 1456, 480x320x28 8180 / 4130.  One
+// launch for a whole sweep with one thread-block cluster per zone and cluster
+// barriers between the hyperplanes took 222, 1820 and 7150 there: a zone has
+// eight SMs then.
+template <bool UP, bool SCALE>
+__global__ void __launch_bounds__(HP * 5, 4) k_lu_sweep(LuDev D, LuSweep S, int l, int z0) {
+  __shared__ double sv[4][HP];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int zone = z0 + blockIdx.y, lane = threadIdx.x, t = blockIdx.x * HP + lane;
+  const LuZone Z = D.zones[zone];
+  const int* hps = S.hps + (long long)zone * S.hstride + l;
+  const int lo = __ldg(hps), n = __ldg(hps + 1) - lo;
+  const long long h = t < n ? Z.off + lo + t : -1;
+  switch (threadIdx.y) {
+    case 0: sweep_row<UP, SCALE, 0>(D, S, Z, h, lane, sv); break;
+    case 1: sweep_row<UP, SCALE, 4>(D, S, Z, h, lane, sv); break;
+    case 2: sweep_row<UP, SCALE, 2>(D, S, Z, h, lane, sv); break;
+    case 3: sweep_row<UP, SCALE, 3>(D, S, Z, h, lane, sv); break;
+    default: sweep_row<UP, SCALE, 1>(D, S, Z, h, lane, sv); break;
   }
-  __syncthreads();
-  if (!ok) return;
-  tv = d_solve(f, m, tv, sv[a]);
-  D.rsd[m * D.NP + pidx(Z, i, j, k)] = own - tv;
 }
 
 __device__ inline void face_sizes(const LuZone& Z, int nkp, long long& e, long long& s) {
@@ -1134,17 +1169,24 @@ void jac(bool hp_order, const LuDev& D, const int* fb, int fls, const int* ri, i
   else
     k_lu_jac<false><<<grid, TPB, 0, s>>>(D, fb, fls, ri, ls, ks, jac, z0);
 }
-void lower(bool scale, const LuDev& D, const double* jac, const int* hps, int hstride, int l, int z0, dim3 grid,
-           cudaStream_t s) {
-  const dim3 b(HP, 5);
-  if (scale)
-    k_lu_lower<true><<<grid, b, 0, s>>>(D, jac, hps, hstride, l, z0);
-  else
-    k_lu_lower<false><<<grid, b, 0, s>>>(D, jac, hps, hstride, l, z0);
+void points(const LuDev& D, const int* ri, int ls, int ks, int* pts, const LuWork* w, int n, cudaStream_t s) {
+  k_lu_points<<<n, TPB, 0, s>>>(D, ri, ls, ks, pts, w);
 }
-void upper(const LuDev& D, const double* jac, const int* hps, int hstride, int l, int z0, dim3 grid,
-           cudaStream_t s) {
-  k_lu_upper<<<grid, dim3(HP, 5), 0, s>>>(D, jac, hps, hstride, l, z0);
+// follows: the launch before it in the stream is the hyperplane before it
+cudaError_t sweep(bool up, bool scale, const LuDev& D, const LuSweep& S, int l, int z0, dim3 grid, bool follows,
+                  cudaStream_t s) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[1];
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(HP, 5);
+  cfg.stream = s;
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = follows ? 1 : 0;
+  if (up) return cudaLaunchKernelEx(&cfg, k_lu_sweep<true, false>, D, S, l, z0);
+  if (scale) return cudaLaunchKernelEx(&cfg, k_lu_sweep<false, true>, D, S, l, z0);
+  return cudaLaunchKernelEx(&cfg, k_lu_sweep<false, false>, D, S, l, z0);
 }
 void pack(const LuDev& D, const Faces& F, int nzones, dim3 grid, cudaStream_t s) {
   k_lu_pack<<<grid, TPB, 0, s>>>(D, F, nzones);

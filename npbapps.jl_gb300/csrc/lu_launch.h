@@ -14,10 +14,9 @@ namespace npbmz_lu {
   void pointwise(bool update, const LuDev& D, const LuWork* w, int n, double tmp, cudaStream_t s);                   \
   void jac(bool hp_order, const LuDev& D, const int* fb, int fls, const int* ri, int ls, int ks, double* jac,      \
            int z0, dim3 grid, cudaStream_t s);                                                                       \
-  void lower(bool scale, const LuDev& D, const double* jac, const int* hps, int hstride, int l, int z0, dim3 grid,  \
-             cudaStream_t s);                                                                                        \
-  void upper(const LuDev& D, const double* jac, const int* hps, int hstride, int l, int z0, dim3 grid,              \
-             cudaStream_t s);                                                                                        \
+  void points(const LuDev& D, const int* ri, int ls, int ks, int* pts, const LuWork* w, int n, cudaStream_t s);      \
+  cudaError_t sweep(bool up, bool scale, const LuDev& D, const LuSweep& S, int l, int z0, dim3 grid, bool follows,   \
+                    cudaStream_t s);                                                                                 \
   void pack(const LuDev& D, const Faces& F, int nzones, dim3 grid, cudaStream_t s);                                  \
   void unpack(const LuDev& D, const Faces& F, int nzones, dim3 grid, cudaStream_t s);                                \
   void norm_partial(int which, const LuDev& D, const LuWork* w, int n, const CeTable& ce, double* partial,          \

@@ -81,18 +81,28 @@ __host__ __device__ constexpr bool off_zero(int dir, int r, int c) {
                      (r == 3 && (c == 2 || c == 4)));
 }
 
-// Position of entry (r, c) among the 18 entries of block DIR that are not
-// structural zeros, row-major.
+// The entries that do not depend on the state (the reference assigns
+// -dt t1 d, -+dt t2 and -+dt t2 c2 there): the sweeps form them from the
+// zone's constants instead of reading them.
+__host__ __device__ constexpr bool off_const(int dir, int r, int c) {
+  return (r == 0 && (c == 0 || c == dir + 1)) || (r == dir + 1 && c == 4);
+}
+
+// Position of entry (r, c) among the 15 stored entries of block DIR,
+// row-major.
+__host__ __device__ constexpr bool off_stored(int dir, int r, int c) {
+  return !off_zero(dir, r, c) && !off_const(dir, r, c);
+}
 __host__ __device__ constexpr int blk_idx(int dir, int r, int c) {
   int n = 0;
   for (int rr = 0; rr < 5; ++rr)
     for (int cc = 0; cc < 5; ++cc) {
       if (rr == r && cc == c) return n;
-      if (!off_zero(dir, rr, cc)) ++n;
+      if (off_stored(dir, rr, cc)) ++n;
     }
   return n;
 }
-constexpr int BLK_NZ = 18;
+constexpr int BLK_N = 15;
 
 // The 5x5 solve of blts / buts (src/LU/blts.jl:106-193, src/LU/buts.jl:113-200)
 // with tmat = d.  d is lower triangular with d[2][1] = d[3][1] = d[3][2] = 0
@@ -107,16 +117,26 @@ constexpr int BLK_NZ = 18;
 // `jac` planes per interior point, stored at the point's hyperplane-ordered
 // index h = zone.off + hps[l] + t (t: its place in hyperplane l = i+j+k,
 // k then j ascending; hps[l]: the zone's interior points with i+j+k < l), so
-// that the sweeps, which run one hyperplane per launch, read them coalesced.
+// that the sweeps, which go hyperplane by hyperplane, read them coalesced.
 // Written by k_lu_jac before the sweeps (u does not change until the
 // update), each block by the point whose state it is built from:
 //   FAC_T + r, FAC_R0 + r-1, FAC_4C + c-1   t_rr, tmp_r0, tmp_4c of d
-//   FAC_BLK + (2 dir + s) * 18 + blk_idx    the non-zero entries of the
+//   FAC_Y + r                               1 / t_rr
+//   FAC_BLK + (2 dir + s) * BLK_N + blk_idx the stored entries of the
 //       off-diagonal block of direction dir: s = 0 jacld's (from the point
 //       at -1 in dir), s = 1 jacu's (from the point at +1)
-enum { FAC_T = 0, FAC_R0 = 5, FAC_4C = 9, FAC_BLK = 12, FAC_COUNT = 12 + 6 * 18 };
+enum { FAC_T = 0, FAC_R0 = 5, FAC_4C = 9, FAC_Y = 12, FAC_BLK = 17, FAC_COUNT = 17 + 6 * BLK_N };
 
 constexpr int HP = 32;  // points per block of the sweep kernels (x 5 rows)
+
+// The tables of the sweeps: hps as above (hstride ints per zone), and per slot
+// h the point's index within its zone.
+struct LuSweep {
+  const double* jac;
+  const int* hps;
+  const int* pts;
+  int hstride;
+};
 
 // ---- exch_qbc (src/LU/exchange_qbc.jl) --------------------------------------
 // Staging per zone: east face (j = ny-1) and west face (j = 2), nx*nkp points

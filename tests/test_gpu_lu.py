@@ -91,6 +91,24 @@ def test_iterations_are_bit_exact(name, niter, flags):
     np.testing.assert_allclose(a[2], b[2], rtol=1e-13)
 
 
+@pytest.mark.parametrize("zone", [(8, 8, 8), (9, 9, 9), (40, 5, 6), (5, 40, 7), (14, 13, 12)])
+@pytest.mark.parametrize("flags", [0, lu.GRAPH], ids=["direct", "graph"])
+def test_sweeps_at_block_edges_are_bit_exact(zone, flags):
+    """Zones whose hyperplanes end below, at and above the sweeps' blocks of 32
+    points, and long thin ones; the lower phase without the fused scaling too."""
+    from oracle import oracle
+
+    nx, ny, nz = zone
+    p, r = make(lu.lu_zone_setup(2 * nx, 2 * ny, nz, 2, 2), 0.5, flags)
+    for gp, op in [(lu.PHASE_LOWER, oracle.LU_LOWER), (lu.PHASE_UPPER, oracle.LU_UPPER)]:
+        p.phase(gp)
+        r.phase(op)
+        assert_state_equal(p, r, (lu.U, lu.RSD))
+    p.iterate(4)
+    r.iterate(4)
+    assert_state_equal(p, r, (lu.U, lu.RSD))
+
+
 def test_per_zone_ssor_equals_batched():
     g, dt = GEOMS["rect"]
     a, _ = make(g(), dt, lu.FACES_NPB)
