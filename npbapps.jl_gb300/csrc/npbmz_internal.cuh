@@ -14,6 +14,14 @@
 
 namespace npbmz {
 
+// Constants of one sweep direction of the FMA build's BT elimination
+// (bt_lines.cuh): dt t2, its products with c1 and c2, dt t1 times c3c4,
+// con43 c3c4 and c1345, and dt t1 times d.
+template <typename T>
+struct BtK {
+  T t2, c1, c2, two_m_c2, c2t2, c1t2, kc, k43, kg, t1d[5];
+};
+
 // set_constants (src/BT/set_constants.jl:1-130), evaluated on the host.
 struct Consts {
   double dt, dnxm1, dnym1, dnzm1;
@@ -39,7 +47,41 @@ struct Consts {
   float2 p_c1, p_c2, p_two_m_c2, p_k43, p_c3c4, p_c1345, p_k43m, p_c3c4m;
   float2 p_con43, p_c1c5, p_comz1, p_comz4, p_comz5, p_comz6, p_bt, p_c2iv;
   float2 p_dtt1[3], p_dtt2[3], p_c2dtt1[3], p_d[3][5], p_dmax[3];
+  BtK<double> bt64[3];
+  BtK<float> bt32[3];
 };
+
+// Fill bt64 and bt32 from the other constants (host).
+inline void make_bt_consts(Consts& k) {
+  const double t1[3] = {k.dttx1, k.dtty1, k.dttz1}, t2[3] = {k.dttx2, k.dtty2, k.dttz2};
+  const double d[3][5] = {{k.dx1, k.dx2, k.dx3, k.dx4, k.dx5}, {k.dy1, k.dy2, k.dy3, k.dy4, k.dy5},
+                          {k.dz1, k.dz2, k.dz3, k.dz4, k.dz5}};
+  for (int dir = 0; dir < 3; ++dir) {
+    BtK<double>& b = k.bt64[dir];
+    b.t2 = t2[dir];
+    b.c1 = k.c1;
+    b.c2 = k.c2;
+    b.two_m_c2 = 2.0 - k.c2;
+    b.c2t2 = k.c2 * t2[dir];
+    b.c1t2 = k.c1 * t2[dir];
+    b.kc = t1[dir] * k.c3c4;
+    b.k43 = t1[dir] * (k.con43 * k.c3c4);
+    b.kg = t1[dir] * k.c1345;
+    BtK<float>& f = k.bt32[dir];
+    f.t2 = (float)b.t2; f.c1 = (float)b.c1; f.c2 = (float)b.c2; f.two_m_c2 = (float)b.two_m_c2;
+    f.c2t2 = (float)b.c2t2; f.c1t2 = (float)b.c1t2; f.kc = (float)b.kc; f.k43 = (float)b.k43; f.kg = (float)b.kg;
+    for (int m = 0; m < 5; ++m) {
+      b.t1d[m] = t1[dir] * d[dir][m];
+      f.t1d[m] = (float)b.t1d[m];
+    }
+  }
+}
+template <typename T>
+__host__ __device__ inline const BtK<T>& bt_consts(const Consts& k, int dir);
+template <>
+__host__ __device__ inline const BtK<double>& bt_consts<double>(const Consts& k, int dir) { return k.bt64[dir]; }
+template <>
+__host__ __device__ inline const BtK<float>& bt_consts<float>(const Consts& k, int dir) { return k.bt32[dir]; }
 
 // The FP32 (T = float) or FP64 (T = double) copy of a constant.
 template <typename T>

@@ -722,8 +722,10 @@ __device__ __forceinline__ void bt_load_point(const Fields& F, int64_t pt, T& ri
   u5 = (T)F.u[4 * NP + pt];
 }
 
-// out: where the forward-eliminated rhs and the solution go (rhs itself for
-// the in-place solve; a separate buffer when a refinement pass follows).
+#if NPBMZ_HAS_FP32
+#include "bt_lines.cuh"
+#else
+// out: where the forward-eliminated rhs and the solution go (rhs itself).
 template <int DIR, typename T>
 __global__ void __launch_bounds__(128) k_bt_solve(Fields F, Consts K, const Work* __restrict__ work,
                                                   T* __restrict__ lhsc, int64_t nlt, int add_u,
@@ -860,6 +862,9 @@ __global__ void __launch_bounds__(128) k_bt_solve(Fields F, Consts K, const Work
   }
 }
 
+#endif  // NPBMZ_HAS_FP32
+
+#if NPBMZ_HAS_FP32
 // ============================================================================
 // Mixed-precision BT sweep (NPBMZ_MIXED): two kernels per sweep direction.
 //
@@ -914,87 +919,66 @@ template <int DIR>
 struct BtF32Carry {
   float Cp[5][5];     // C' at p-1
   float rp[5];        // forward-eliminated rhs at p-1
-  float Acur[5][5];   // lhsa at p   (structural nonzeros)
-  float Anext[5][5];  // lhsa at p+1
-  float Bcur[5][5];   // lhsb at p   (structural nonzeros)
+  float Pcur[5][5];   // -lhsa at p   (structural nonzeros)
+  float Pnext[5][5];  // -lhsa at p+1
+  float Bs[5][5];     // lhsb at p    (structural nonzeros)
 };
 
+constexpr int BT_SCR = 30;  // words per point of the FP32 line scratch: C' (25), r' (5)
+
+// G and H from the FP32 state s = ri, u2, u3, u4, u5, q.
 template <int DIR>
-__device__ __forceinline__ void bt_f32_consts(const Consts& K, float& tmp1, float& tmp2, float dd[5]) {
-  tmp1 = K.f_dtt1[DIR];
-  tmp2 = K.f_dtt2[DIR];
-#pragma unroll
-  for (int m = 0; m < 5; ++m) dd[m] = K.f_d[DIR][m];
+__device__ __forceinline__ void bt_gh_f32(const Consts& K, const float s[6], float G[5][5], float H[5][5]) {
+  const float v[3] = {s[1] * s[0], s[2] * s[0], s[3] * s[0]};
+  bt_gh<DIR, float>(bt_consts<float>(K, DIR), s[0], v, s[4] * s[0], s[5], G, H);
 }
 
-// Start of the elimination: Jacobians at points 0 and 1 (FP32 state s0, s1 =
-// ri, u2, u3, u4, u5, q).
+// Start of the elimination: Jacobians at points 0 and 1 (FP32 state s0, s1).
 template <int DIR>
-__device__ __forceinline__ void bt_f32_begin(const Consts& K, int n, const float s0[6], const float s1[6],
+__device__ __forceinline__ void bt_f32_begin(const Consts& K, const float s0[6], const float s1[6],
                                              BtF32Carry<DIR>& c) {
-  float tmp1, tmp2, dd[5], f[5][5], nj[5][5];
-  bt_f32_consts<DIR>(K, tmp1, tmp2, dd);
-  bt_jac<DIR, float>(K, s0[0], s0[1], s0[2], s0[3], s0[4], s0[5], f, nj);
-  bt_asm_a<DIR, float>(f, nj, tmp1, tmp2, dd, c.Acur);
-  bt_jac<DIR, float>(K, s1[0], s1[1], s1[2], s1[3], s1[4], s1[5], f, nj);
-  bt_asm_b<float>(nj, tmp1, dd, c.Bcur);
-  if (n - 2 >= 2) bt_asm_a<DIR, float>(f, nj, tmp1, tmp2, dd, c.Anext);
-}
-
-// One forward step at point p (1..n-2): r holds the rhs of row p on entry and
-// the eliminated rhs on exit; sn is the FP32 state at p+1.  C'_p and r'_p go
-// to scr[(p*30 + e) * nlt + gl].
-template <int DIR>
-__device__ __forceinline__ void bt_f32_step(const Consts& K, int p, int n, bool skip_first_matvec, float r[5],
-                                            const float sn[6], BtF32Carry<DIR>& c, float* __restrict__ scr,
-                                            int64_t nlt, int64_t gl) {
-  float tmp1, tmp2, dd[5];
-  bt_f32_consts<DIR>(K, tmp1, tmp2, dd);
-  if (p > 1 || !skip_first_matvec) {
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      float sacc = 0.f;
-#pragma unroll
-      for (int cc = 0; cc < 5; ++cc)
-        if (anz<DIR>(m, cc)) sacc += c.Acur[m][cc] * c.rp[cc];
-      r[m] -= sacc;
-    }
-  }
-  float B[5][5];
+  float G[5][5], H[5][5];
+  bt_gh_f32<DIR>(K, s0, G, H);
+  bt_form_p<DIR, float>(G, H, c.Pcur);
+  bt_gh_f32<DIR>(K, s1, G, H);
+  bt_form_p<DIR, float>(G, H, c.Pnext);
+  bt_form_b<DIR, float>(H, c.Bs);
 #pragma unroll
   for (int a = 0; a < 5; ++a)
 #pragma unroll
-    for (int b = 0; b < 5; ++b) {
-      float t = bnz(a, b) ? c.Bcur[a][b] : 0.f;
-      if (p > 1) {
-#pragma unroll
-        for (int cc = 0; cc < 5; ++cc)
-          if (anz<DIR>(a, cc)) t -= c.Acur[a][cc] * c.Cp[cc][b];
-      }
-      B[a][b] = t;
-    }
-  float f[5][5], nj[5][5], C[5][5];
-  bt_jac<DIR, float>(K, sn[0], sn[1], sn[2], sn[3], sn[4], sn[5], f, nj);
-  bt_asm_c<DIR, float>(f, nj, tmp1, tmp2, dd, C);
+    for (int b = 0; b < 5; ++b) c.Cp[a][b] = 0.f;
+}
+
+// One forward step at point p (1..n-2): r holds the rhs of row p on entry and
+// the eliminated rhs on exit; sn is the FP32 state at p+1.  C'_p (STORE_C)
+// and r'_p go to scr[(p*BT_SCR + e) * nlt + gl].
+template <int DIR, bool STORE_C>
+__device__ __forceinline__ void bt_f32_step(const Consts& K, int p, float r[5], const float sn[6], BtF32Carry<DIR>& c,
+                                            float* __restrict__ scr, int64_t nlt, int64_t gl) {
+  float B[5][5], C[5][5], G[5][5], H[5][5];
+  bt_add_px<DIR, float>(c.Pcur, c.rp, r);
+  bt_add_pc<DIR, float>(c.Pcur, c.Cp, c.Bs, B);
+  bt_gh_f32<DIR>(K, sn, G, H);
+  bt_form_c<DIR, float>(G, H, C);
 #pragma unroll
   for (int a = 0; a < 5; ++a)
 #pragma unroll
     for (int b = 0; b < 5; ++b)
-      if (anz<DIR>(a, b)) c.Acur[a][b] = c.Anext[a][b];
-  if (p + 1 <= n - 2) bt_asm_b<float>(nj, tmp1, dd, c.Bcur);
-  if (p + 2 <= n - 2) bt_asm_a<DIR, float>(f, nj, tmp1, tmp2, dd, c.Anext);
-  binvcrhs<float>(B, C, r);
+      if (anz<DIR>(a, b)) c.Pcur[a][b] = c.Pnext[a][b];
+  bt_form_p<DIR, float>(G, H, c.Pnext);
+  bt_form_b<DIR, float>(H, c.Bs);
+  bt_factor_solve<DIR, float>(B, C, r);
 #pragma unroll
   for (int a = 0; a < 5; ++a)
 #pragma unroll
     for (int b = 0; b < 5; ++b) {
       c.Cp[a][b] = C[a][b];
-      scr[((int64_t)p * 30 + a * 5 + b) * nlt + gl] = C[a][b];
+      if (STORE_C) scr[((int64_t)p * BT_SCR + a * 5 + b) * nlt + gl] = C[a][b];
     }
 #pragma unroll
   for (int m = 0; m < 5; ++m) {
     c.rp[m] = r[m];
-    scr[((int64_t)p * 30 + 25 + m) * nlt + gl] = r[m];
+    scr[((int64_t)p * BT_SCR + 25 + m) * nlt + gl] = r[m];
   }
 }
 
@@ -1043,7 +1027,7 @@ __global__ void __launch_bounds__(128) k_bt_mixed_solve(Fields F, Consts K, cons
   load_state_f32(F, base + st, s1);
 #pragma unroll
   for (int m = 0; m < 5; ++m) c.rp[m] = bload(m, base);
-  bt_f32_begin<DIR>(K, n, s0, s1, c);
+  bt_f32_begin<DIR>(K, s0, s1, c);
   float sn[6], bn[5];
   load_state_f32(F, base + 2 * st, sn);
 #pragma unroll
@@ -1059,7 +1043,7 @@ __global__ void __launch_bounds__(128) k_bt_mixed_solve(Fields F, Consts K, cons
 #pragma unroll
       for (int m = 0; m < 5; ++m) bn[m] = bload(m, base + (int64_t)(p + 1) * st);
     }
-    bt_f32_step<DIR>(K, p, n, false, r, s, c, scr, nlt, gl);
+    bt_f32_step<DIR, true>(K, p, r, s, c, scr, nlt, gl);
   }
   float rn[5];
 #pragma unroll
@@ -1067,11 +1051,11 @@ __global__ void __launch_bounds__(128) k_bt_mixed_solve(Fields F, Consts K, cons
   for (int p = n - 2; p >= 1; --p) {
     float r[5];
 #pragma unroll
-    for (int m = 0; m < 5; ++m) r[m] = (p == n - 2) ? c.rp[m] : scr[((int64_t)p * 30 + 25 + m) * nlt + gl];
+    for (int m = 0; m < 5; ++m) r[m] = (p == n - 2) ? c.rp[m] : scr[((int64_t)p * BT_SCR + 25 + m) * nlt + gl];
 #pragma unroll
     for (int m = 0; m < 5; ++m)
 #pragma unroll
-      for (int cc = 0; cc < 5; ++cc) r[m] -= scr[((int64_t)p * 30 + m * 5 + cc) * nlt + gl] * rn[cc];
+      for (int cc = 0; cc < 5; ++cc) r[m] -= scr[((int64_t)p * BT_SCR + m * 5 + cc) * nlt + gl] * rn[cc];
     const int64_t pt = base + p * st;
 #pragma unroll
     for (int m = 0; m < 5; ++m) {
@@ -1150,7 +1134,7 @@ __global__ void __launch_bounds__(128) k_bt_refine(Fields F, Consts K, const Wor
   BtF32Carry<DIR> c;
 #pragma unroll
   for (int m = 0; m < 5; ++m) c.rp[m] = 0.f;  // the boundary residual is exactly zero
-  bt_f32_begin<DIR>(K, n, s0, s1, c);
+  bt_f32_begin<DIR>(K, s0, s1, c);
   // prefetch point 2 and b_1
   double xn[5], sn[6], bn[5];
   load_x(2, xn);
@@ -1184,7 +1168,7 @@ __global__ void __launch_bounds__(128) k_bt_refine(Fields F, Consts K, const Wor
     }
 #pragma unroll
     for (int e = 0; e < 6; ++e) s[e] = (float)sq[e];
-    bt_f32_step<DIR>(K, p, n, true, r, s, c, scr, nlt, gl);
+    bt_f32_step<DIR, true>(K, p, r, s, c, scr, nlt, gl);
     (void)pt;
   }
   // back substitution of the correction d, then x = x0 + d
@@ -1193,11 +1177,11 @@ __global__ void __launch_bounds__(128) k_bt_refine(Fields F, Consts K, const Wor
     const int64_t pt = base + p * st;
     float d[5];
 #pragma unroll
-    for (int m = 0; m < 5; ++m) d[m] = (p == n - 2) ? c.rp[m] : scr[((int64_t)p * 30 + 25 + m) * nlt + gl];
+    for (int m = 0; m < 5; ++m) d[m] = (p == n - 2) ? c.rp[m] : scr[((int64_t)p * BT_SCR + 25 + m) * nlt + gl];
 #pragma unroll
     for (int m = 0; m < 5; ++m)
 #pragma unroll
-      for (int cc = 0; cc < 5; ++cc) d[m] -= scr[((int64_t)p * 30 + m * 5 + cc) * nlt + gl] * dn[cc];
+      for (int cc = 0; cc < 5; ++cc) d[m] -= scr[((int64_t)p * BT_SCR + m * 5 + cc) * nlt + gl] * dn[cc];
 #pragma unroll
     for (int m = 0; m < 5; ++m) {
       const double v = (double)x0f[m * NP + pt] + (double)d[m];
@@ -1395,7 +1379,7 @@ __global__ void __launch_bounds__(128) k_bt_refine_df(Fields F, Consts K, const 
 #pragma unroll
   for (int m = 0; m < 5; ++m) c.rp[m] = 0.f;
   // bt_f32_begin takes ri, u2, u3, u4, u5, q in that order (as sq)
-  bt_f32_begin<DIR>(K, n, s0, s1, c);
+  bt_f32_begin<DIR>(K, s0, s1, c);
   df64 xn[5], sn[6];
   // b of the next point: double-float planes (IN_DF) or FP64 rhs
   df64 bn[5];
@@ -1443,18 +1427,18 @@ __global__ void __launch_bounds__(128) k_bt_refine_df(Fields F, Consts K, const 
     }
 #pragma unroll
     for (int e = 0; e < 6; ++e) s[e] = sq[e].hi;
-    bt_f32_step<DIR>(K, p, n, true, r, s, c, scr, nlt, gl);
+    bt_f32_step<DIR, true>(K, p, r, s, c, scr, nlt, gl);
   }
   float dn[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
   for (int p = n - 2; p >= 1; --p) {
     const int64_t pt = base + p * st;
     float d[5];
 #pragma unroll
-    for (int m = 0; m < 5; ++m) d[m] = (p == n - 2) ? c.rp[m] : scr[((int64_t)p * 30 + 25 + m) * nlt + gl];
+    for (int m = 0; m < 5; ++m) d[m] = (p == n - 2) ? c.rp[m] : scr[((int64_t)p * BT_SCR + 25 + m) * nlt + gl];
 #pragma unroll
     for (int m = 0; m < 5; ++m)
 #pragma unroll
-      for (int cc = 0; cc < 5; ++cc) d[m] -= scr[((int64_t)p * 30 + m * 5 + cc) * nlt + gl] * dn[cc];
+      for (int cc = 0; cc < 5; ++cc) d[m] -= scr[((int64_t)p * BT_SCR + m * 5 + cc) * nlt + gl] * dn[cc];
 #pragma unroll
     for (int m = 0; m < 5; ++m) {
       if (OUT_DF) {
@@ -1471,7 +1455,6 @@ __global__ void __launch_bounds__(128) k_bt_refine_df(Fields F, Consts K, const 
   }
 }
 
-#if NPBMZ_HAS_FP32
 // ============================================================================
 // Software-pipelined refined FP32 BT sweep of a fused step (mode 4).  The
 // two passes above wait on memory once per point: a line advances one point
@@ -1516,15 +1499,16 @@ __device__ __forceinline__ void cpa_wait() {
 }
 
 constexpr int PL_MIXED_W = 30;   // words per slot, first pass
-constexpr int PL_REFINE_W = 35;  // words per slot, refinement pass
+constexpr int PL_REFINE_W = 45;  // words per slot, refinement pass
 
 // Dynamic shared memory of the pipelined kernels for tpb threads.
-// (the first pass keeps 5 more words per line: b at the line's last point)
+// (the first pass keeps 5 more words per line: b at the line's last point;
+// the refinement pass 10: the same in double-float)
 __host__ __device__ constexpr size_t pl_mixed_smem(int tpb) {
   return (size_t)(PIPE * PL_MIXED_W + 5) * tpb * sizeof(float);
 }
-__host__ __device__ constexpr size_t pl_refine_smem(int tpb, bool out_df) {
-  return (size_t)PIPE * 5 * tpb * sizeof(double) * (out_df ? 0 : 1) + (size_t)PIPE * PL_REFINE_W * tpb * sizeof(float);
+__host__ __device__ constexpr size_t pl_refine_smem(int tpb) {
+  return (size_t)(PIPE * PL_REFINE_W + 10) * tpb * sizeof(float);
 }
 
 template <int DIR>
@@ -1582,7 +1566,7 @@ __device__ __forceinline__ void bt_mixed_pl_item(const Fields& F, const Consts& 
     }
 #pragma unroll
     for (int m = 0; m < 5; ++m) c.rp[m] = *b_at(0, m);
-    bt_f32_begin<DIR>(K, n, s0, s1, c);
+    bt_f32_begin<DIR>(K, s0, s1, c);
   }
   for (int p = 1; p <= n - 2; ++p) {
     issue_fwd(p + PIPE - 1);
@@ -1593,7 +1577,7 @@ __device__ __forceinline__ void bt_mixed_pl_item(const Fields& F, const Consts& 
     for (int e = 0; e < 6; ++e) s[e] = *S(slot, e);
 #pragma unroll
     for (int m = 0; m < 5; ++m) r[m] = *S(slot, 6 + m);
-    bt_f32_step<DIR>(K, p, n, false, r, s, c, scr, nlt, gl);
+    bt_f32_step<DIR, true>(K, p, r, s, c, scr, nlt, gl);
     if (p + PIPE > n - 2) {
       // the ring does not refill this slot: C'_p and r'_p stay here for the
       // back substitution, which so starts without a trip to memory
@@ -1613,7 +1597,7 @@ __device__ __forceinline__ void bt_mixed_pl_item(const Fields& F, const Consts& 
     if (p >= 1) {
       const int slot = p % PIPE;
 #pragma unroll
-      for (int e = 0; e < 30; ++e) cpa4(S(slot, e), scr + ((int64_t)p * 30 + e) * nlt + gl);
+      for (int e = 0; e < 30; ++e) cpa4(S(slot, e), scr + ((int64_t)p * BT_SCR + e) * nlt + gl);
     }
     cpa_commit();
   };
@@ -1661,11 +1645,8 @@ __device__ __forceinline__ void bt_refine_pl_item(const Fields& F, const Consts&
   const int64_t gl = Z.lineoff[DIR] + line;
   const int64_t NP = F.NP;
   const int T = blockDim.x;
-  // the FP64 ring (u, z sweep only) first: 8-byte words
-  double* umy = reinterpret_cast<double*>(pl_smem) + threadIdx.x;
-  float* my = reinterpret_cast<float*>(pl_smem + (OUT_DF ? 0 : (size_t)PIPE * 5 * T * sizeof(double))) + threadIdx.x;
+  float* my = reinterpret_cast<float*>(pl_smem) + threadIdx.x;
   auto S = [&](int slot, int e) -> float* { return my + (slot * PL_REFINE_W + e) * T; };
-  auto SU = [&](int slot, int m) -> double* { return umy + (slot * 5 + m) * T; };
   double* __restrict__ rhs = F.rhs;
   float* __restrict__ bdf = F.rdf;
   const int order[6] = {PF_RHOI, PF_U2, PF_U3, PF_U4, PF_U5, PF_QS};
@@ -1708,32 +1689,49 @@ __device__ __forceinline__ void bt_refine_pl_item(const Fields& F, const Consts&
 #pragma unroll
     for (int e = 0; e < 6; ++e) s6[e] = df64{*st_at(q, order[e]), *st_at(q, PF_HI_COUNT + order[e])};
   };
-  // forward step p (1..n-2) consumes x and the state at p+1 and b_p:
-  // words 0..9 x (5 x0 values, or hi/lo of the line's end value), 10..21
-  // state hi/lo, 22..31 b hi/lo
+  // forward step p (1..n-2) consumes x0 and the state at p+1 and b_p: words
+  // 0..4 x0, 5..16 state hi/lo, 17..26 b hi/lo (the line's last point has b
+  // itself for x: words 0..9 of slot PIPE, fetched first)
   auto issue_fwd = [&](int p) {
     if (p <= n - 2) {
       const int slot = p % PIPE;
-      if (p + 1 == n - 1) {
-#pragma unroll
-        for (int e = 0; e < 10; ++e) cpa4(S(slot, e), b_at(p + 1, e));
-      } else {
+      if (p + 1 < n - 1) {
 #pragma unroll
         for (int m = 0; m < 5; ++m) cpa4(S(slot, m), x0_at(p + 1, m));
       }
 #pragma unroll
       for (int e = 0; e < 6; ++e) {
-        cpa4(S(slot, 10 + e), st_at(p + 1, order[e]));
-        cpa4(S(slot, 16 + e), st_at(p + 1, PF_HI_COUNT + order[e]));
+        cpa4(S(slot, 5 + e), st_at(p + 1, order[e]));
+        cpa4(S(slot, 11 + e), st_at(p + 1, PF_HI_COUNT + order[e]));
       }
 #pragma unroll
-      for (int e = 0; e < 10; ++e) cpa4(S(slot, 22 + e), b_at(p, e));
+      for (int e = 0; e < 10; ++e) cpa4(S(slot, 17 + e), b_at(p, e));
     }
     cpa_commit();
+  };
+  // back substitution step p (n-2 .. 1) consumes C'_p (the first pass's),
+  // r'_p, x0_p and u_p: words 0..24, 25..29, 30..34, 35..44 (u in two halves)
+  auto fetch_bwd = [&](int p, bool r_in_slot) {
+    const int slot = p % PIPE;
+#pragma unroll
+    for (int e = 0; e < 30; ++e)
+      if (e < 25 || !r_in_slot) cpa4(S(slot, e), scr + ((int64_t)p * BT_SCR + e) * nlt + gl);
+#pragma unroll
+    for (int m = 0; m < 5; ++m) cpa4(S(slot, 30 + m), x0_at(p, m));
+    if (!OUT_DF && add_u) {
+      const float* up = reinterpret_cast<const float*>(F.u + base + (int64_t)p * st);
+#pragma unroll
+      for (int m = 0; m < 5; ++m) {
+        cpa4(S(slot, 35 + 2 * m), up + 2 * m * NP);
+        cpa4(S(slot, 36 + 2 * m), up + 2 * m * NP + 1);
+      }
+    }
   };
 
   // the ring's first slots go out before the line's first points are read
   // directly, so that the two memory latencies overlap
+#pragma unroll
+  for (int e = 0; e < 10; ++e) cpa4(S(PIPE, e), b_at(n - 1, e));
 #pragma unroll
   for (int q = 1; q < PIPE; ++q) issue_fwd(q);
   df64 acc_c[5], acc_n[5], xq[5], sq[6], P[5], Q[5];
@@ -1759,7 +1757,7 @@ __device__ __forceinline__ void bt_refine_pl_item(const Fields& F, const Consts&
     for (int e = 0; e < 6; ++e) s1[e] = sq[e].hi;
 #pragma unroll
     for (int m = 0; m < 5; ++m) c.rp[m] = 0.f;
-    bt_f32_begin<DIR>(K, n, s0, s1, c);
+    bt_f32_begin<DIR>(K, s0, s1, c);
   }
   for (int p = 1; p <= n - 2; ++p) {
     issue_fwd(p + PIPE - 1);
@@ -1768,15 +1766,15 @@ __device__ __forceinline__ void bt_refine_pl_item(const Fields& F, const Consts&
     df64 bd[5];
     if (p + 1 == n - 1) {
 #pragma unroll
-      for (int m = 0; m < 5; ++m) xq[m] = df64{*S(slot, m), *S(slot, 5 + m)};
+      for (int m = 0; m < 5; ++m) xq[m] = df64{*S(PIPE, m), *S(PIPE, 5 + m)};
     } else {
 #pragma unroll
       for (int m = 0; m < 5; ++m) xq[m] = df64{*S(slot, m), 0.f};
     }
 #pragma unroll
-    for (int e = 0; e < 6; ++e) sq[e] = df64{*S(slot, 10 + e), *S(slot, 16 + e)};
+    for (int e = 0; e < 6; ++e) sq[e] = df64{*S(slot, 5 + e), *S(slot, 11 + e)};
 #pragma unroll
-    for (int m = 0; m < 5; ++m) bd[m] = df64{*S(slot, 22 + m), *S(slot, 27 + m)};
+    for (int m = 0; m < 5; ++m) bd[m] = df64{*S(slot, 17 + m), *S(slot, 22 + m)};
     pq(sq, xq, P, Q);
     float r[5], s[6];
 #pragma unroll
@@ -1789,45 +1787,25 @@ __device__ __forceinline__ void bt_refine_pl_item(const Fields& F, const Consts&
     }
 #pragma unroll
     for (int e = 0; e < 6; ++e) s[e] = sq[e].hi;
-    bt_f32_step<DIR>(K, p, n, true, r, s, c, scr, nlt, gl);
+    // the elimination runs again (its factors do not fit beside C'); C' is the
+    // first pass's, so only r' is stored
+    bt_f32_step<DIR, false>(K, p, r, s, c, scr, nlt, gl);
     if (p + PIPE > n - 2) {
-      // the ring does not refill this slot: C'_p and r'_p stay here for the
-      // back substitution, x0_p (and u_p) are fetched now, so that it starts
+      // the ring does not refill this slot: r'_p stays here for the back
+      // substitution, whose other operands are fetched now, so that it starts
       // without a trip to memory
 #pragma unroll
-      for (int a = 0; a < 5; ++a)
-#pragma unroll
-        for (int b = 0; b < 5; ++b) *S(slot, a * 5 + b) = c.Cp[a][b];
-#pragma unroll
-      for (int m = 0; m < 5; ++m) {
-        *S(slot, 25 + m) = c.rp[m];
-        cpa4(S(slot, 30 + m), x0_at(p, m));
-      }
-      if (!OUT_DF && add_u) {
-        const int64_t pt = base + (int64_t)p * st;
-#pragma unroll
-        for (int m = 0; m < 5; ++m) cpa8(SU(slot, m), F.u + m * NP + pt);
-      }
+      for (int m = 0; m < 5; ++m) *S(slot, 25 + m) = r[m];
+      fetch_bwd(p, true);
       cpa_commit();
     }
   }
   cpa_wait<0>();
-  // back substitution: step p (n-2 .. 1) consumes C'_p, r'_p, x0_p (and u_p)
-  // from slot p % PIPE: the last PIPE points as the forward pass left them,
-  // the others loaded PIPE steps ahead into the slot just consumed
+  // back substitution: step p (n-2 .. 1) from slot p % PIPE: the last PIPE
+  // points as the forward pass left them, the others fetched PIPE steps ahead
+  // into the slot just consumed
   auto issue_bwd = [&](int p) {
-    if (p >= 1) {
-      const int slot = p % PIPE;
-      const int64_t pt = base + (int64_t)p * st;
-#pragma unroll
-      for (int e = 0; e < 30; ++e) cpa4(S(slot, e), scr + ((int64_t)p * 30 + e) * nlt + gl);
-#pragma unroll
-      for (int m = 0; m < 5; ++m) cpa4(S(slot, 30 + m), x0_at(p, m));
-      if (!OUT_DF && add_u) {
-#pragma unroll
-        for (int m = 0; m < 5; ++m) cpa8(SU(slot, m), F.u + m * NP + pt);
-      }
-    }
+    if (p >= 1) fetch_bwd(p, false);
     cpa_commit();
   };
   float dn[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
@@ -1858,7 +1836,8 @@ __device__ __forceinline__ void bt_refine_pl_item(const Fields& F, const Consts&
         // exact FP32 -> FP64 by bits (a conversion instruction takes the FP64 pipe)
         const double v = f32_to_f64(xv) + f32_to_f64(d[m]);
         rhs[m * NP + pt] = v;
-        if (add_u) F.u[m * NP + pt] = *SU(slot, m) + v;
+        if (add_u)
+          F.u[m * NP + pt] = __hiloint2double(__float_as_int(*S(slot, 36 + 2 * m)), __float_as_int(*S(slot, 35 + 2 * m))) + v;
       }
       dn[m] = d[m];
     }
@@ -2523,9 +2502,16 @@ static void launch_solve_t(bool sp, int dir, const Fields& F, const Consts& K, c
     else if (dir == 1) k_sp_solve<1, T><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, out, transform);
     else k_sp_solve<2, T><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, out, transform);
   } else {
+#if NPBMZ_HAS_FP32
+    (void)out;
+    if (dir == 0) k_bt_line<0, T><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u);
+    else if (dir == 1) k_bt_line<1, T><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u);
+    else k_bt_line<2, T><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u);
+#else
     if (dir == 0) k_bt_solve<0, T><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, out);
     else if (dir == 1) k_bt_solve<1, T><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, out);
     else k_bt_solve<2, T><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, out);
+#endif
   }
 }
 
@@ -2566,7 +2552,7 @@ void launch_solve(bool sp, int mode, int dir, const Fields& F, const Consts& K, 
     // x-line-major copy), z writes FP64 rhs (and u)
     float* scr = reinterpret_cast<float*>(scratch);
     float* x0 = reinterpret_cast<float*>(xw);
-    const size_t sm_m = pl_mixed_smem(tpb), sm_r = pl_refine_smem(tpb, dir != 2);
+    const size_t sm_m = pl_mixed_smem(tpb), sm_r = pl_refine_smem(tpb);
 #define NPBMZ_PL(D, OD)                                                                                          \
   do {                                                                                                           \
     k_bt_mixed_pl<D><<<item_grid((const void*)k_bt_mixed_pl<D>, nwork, tpb, sm_m, persist, ctas_per_sm), tpb,     \
@@ -2629,7 +2615,7 @@ void launch_solve(bool sp, int mode, int dir, const Fields& F, const Consts& K, 
 // Opt the pipelined sweeps into their dynamic shared memory (above 48 KB for
 // 128 threads per CTA); called once per handle, outside any stream capture.
 int configure_kernels() {
-  size_t cap_b = pl_refine_smem(128, false);
+  size_t cap_b = pl_refine_smem(128);
   for (size_t b : {pl_mixed_smem(128), pls_mixed_smem(128), pls_refine_smem(128, false)})
     if (b > cap_b) cap_b = b;
   const int cap = (int)cap_b;

@@ -119,6 +119,40 @@ def test_each_phase_fast_path_within_1e12(oracle_mod, gname):
             p.upload(npbmz.RHS, z, o.get(npbmz.RHS, z))
 
 
+@pytest.mark.parametrize("flags", [0, npbmz.MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("nz", [3, 7, 13])
+def test_bt_line_solves_at_small_and_ragged_sizes(oracle_mod, nz, flags):
+    """Each BT sweep on zones from 3 points per axis up, with line counts and
+    lengths around the kernels' groups of lines and blocks of points, from
+    identical inputs: the FP64 solve to 1e-12, the refined FP32 solve to 1e-10."""
+    nx, ny, nzs, nbr = npbmz.zones_from_widths([3, 4, 8, 15], [3, 5, 9, 14], nz)
+    geom = npbmz.Geometry(npbmz.BT, nx, ny, nzs, nbr, 30, 31, nz, 4, 4)
+    p, o = make_pair(oracle_mod, geom, 0.0008, flags, npbmz.CE_REFERENCE)
+    rng = np.random.default_rng(5)
+    for z in range(geom.nzones):
+        p.phase(npbmz.PHASE_RHS, z)  # the primitive variables of u; rhs itself is drawn
+        o.phase(0, z)
+        for ph in (npbmz.PHASE_XSOLVE, npbmz.PHASE_YSOLVE, npbmz.PHASE_ZSOLVE):
+            r = rng.normal(size=p.zone_shape(z))
+            p.upload(npbmz.RHS, z, r)
+            o.set(npbmz.RHS, z, r)
+            p.phase(ph, z)
+            o.phase(ph, z)
+            compare(p, o, npbmz.RHS, 1e-10 if flags else FAST_REL, [z])
+
+
+@pytest.mark.parametrize("nz", [5, 7, 13])
+def test_bt_fused_mixed_steps_at_small_and_ragged_sizes(oracle_mod, nz):
+    """Whole refined FP32 steps (the pipelined sweeps) on zones of 5 points per
+    axis, the least that compute_rhs's stencils span, and up."""
+    nx, ny, nzs, nbr = npbmz.zones_from_widths([5, 6, 8, 15], [5, 7, 9, 14], nz)
+    geom = npbmz.Geometry(npbmz.BT, nx, ny, nzs, nbr, 34, 35, nz, 4, 4)
+    p, o = make_pair(oracle_mod, geom, 0.0008, npbmz.MIXED, npbmz.CE_REFERENCE)
+    p.step(4)
+    o.step(4)
+    compare(p, o, npbmz.U, 1e-10)
+
+
 DF_RHS_REL = 1e-12   # compute_rhs in double-float (FP32 pairs, about 48 bits)
 
 
