@@ -712,11 +712,29 @@ void* line_scratch(npbmz_t* h, int dir) {
   return (dir > 0 && h->scratch_yz[dir - 1]) ? h->scratch_yz[dir - 1] : h->scratch;
 }
 
+// FP64 BT sweeps with one thread per line take as long as their longest line
+// unless the lines give every SM quarter (608) a warp; six lanes per line take
+// 1.6 times the warp instructions but a quarter of the time per line.  The two
+// meet where the lines, as multiples of the longest, number about 11,000:
+// 128x128x16's z sweep (14,400) takes 235 us by threads and 303 by groups of
+// lanes, 304x208x17's x sweep (12,300) 1123 and 1177, 128x128x16's x sweep
+// (3,700) 746 and 381.
+bool few_lines(const npbmz_t* h, int dir, int zone) {
+  int64_t points = 0;
+  int longest = 1;
+  for (int z = zone < 0 ? 0 : zone; z < (zone < 0 ? h->nzones : zone + 1); ++z) {
+    const int n = zone_line_len(h->zh[z], dir);
+    points += (int64_t)zone_lines(h->zh[z], dir) * n;
+    longest = std::max(longest, n);
+  }
+  return points < 10000 * (int64_t)longest;
+}
+
 int phase_solve(npbmz_t* h, int dir, int zone, int add_u, bool fused = false) {
   const Fields F = fields(h);
   const bool sp = h->kind == NPBMZ_SP;
   const int mode = use_exact(h) ? 0
-                   : !use_fp32(h) ? 0
+                   : !use_fp32(h) ? (!sp && few_lines(h, dir, zone) ? 5 : 0)
                    : (h->flags & NPBMZ_FP32_NOREFINE) ? 1
                    : (h->flags & NPBMZ_REFINE_FP64) ? 3
                    : (fused && h->rdf ? 4 : 2);

@@ -928,21 +928,21 @@ constexpr int BT_SCR = 30;  // words per point of the FP32 line scratch: C' (25)
 
 // G and H from the FP32 state s = ri, u2, u3, u4, u5, q.
 template <int DIR>
-__device__ __forceinline__ void bt_gh_f32(const Consts& K, const float s[6], float G[5][5], float H[5][5]) {
+__device__ __forceinline__ void bt_gh_f32(const Consts& K, const float s[6], BtGH<DIR, float>& J) {
   const float v[3] = {s[1] * s[0], s[2] * s[0], s[3] * s[0]};
-  bt_gh<DIR, float>(bt_consts<float>(K, DIR), s[0], v, s[4] * s[0], s[5], G, H);
+  bt_gh<DIR, float>(bt_consts<float>(K, DIR), s[0], v, s[4] * s[0], s[5], J);
 }
 
 // Start of the elimination: Jacobians at points 0 and 1 (FP32 state s0, s1).
 template <int DIR>
 __device__ __forceinline__ void bt_f32_begin(const Consts& K, const float s0[6], const float s1[6],
                                              BtF32Carry<DIR>& c) {
-  float G[5][5], H[5][5];
-  bt_gh_f32<DIR>(K, s0, G, H);
-  bt_form_p<DIR, float>(G, H, c.Pcur);
-  bt_gh_f32<DIR>(K, s1, G, H);
-  bt_form_p<DIR, float>(G, H, c.Pnext);
-  bt_form_b<DIR, float>(H, c.Bs);
+  BtGH<DIR, float> J;
+  bt_gh_f32<DIR>(K, s0, J);
+  bt_form_p<DIR, float>(J, c.Pcur);
+  bt_gh_f32<DIR>(K, s1, J);
+  bt_form_p<DIR, float>(J, c.Pnext);
+  bt_form_b<DIR, float>(J, c.Bs);
 #pragma unroll
   for (int a = 0; a < 5; ++a)
 #pragma unroll
@@ -955,18 +955,19 @@ __device__ __forceinline__ void bt_f32_begin(const Consts& K, const float s0[6],
 template <int DIR, bool STORE_C>
 __device__ __forceinline__ void bt_f32_step(const Consts& K, int p, float r[5], const float sn[6], BtF32Carry<DIR>& c,
                                             float* __restrict__ scr, int64_t nlt, int64_t gl) {
-  float B[5][5], C[5][5], G[5][5], H[5][5];
+  float B[5][5], C[5][5];
+  BtGH<DIR, float> J;
   bt_add_px<DIR, float>(c.Pcur, c.rp, r);
   bt_add_pc<DIR, float>(c.Pcur, c.Cp, c.Bs, B);
-  bt_gh_f32<DIR>(K, sn, G, H);
-  bt_form_c<DIR, float>(G, H, C);
+  bt_gh_f32<DIR>(K, sn, J);
+  bt_form_c<DIR, float>(J, C);
 #pragma unroll
   for (int a = 0; a < 5; ++a)
 #pragma unroll
     for (int b = 0; b < 5; ++b)
       if (anz<DIR>(a, b)) c.Pcur[a][b] = c.Pnext[a][b];
-  bt_form_p<DIR, float>(G, H, c.Pnext);
-  bt_form_b<DIR, float>(H, c.Bs);
+  bt_form_p<DIR, float>(J, c.Pnext);
+  bt_form_b<DIR, float>(J, c.Bs);
   bt_factor_solve<DIR, float>(B, C, r);
 #pragma unroll
   for (int a = 0; a < 5; ++a)
@@ -2515,7 +2516,7 @@ static void launch_solve_t(bool sp, int dir, const Fields& F, const Consts& K, c
   }
 }
 
-// mode 0: FP64 in place; 1: FP32 in place; 2: FP32 + refinement with a
+// mode 0: FP64 in place (5: BT, six lanes per line); 1: FP32 in place; 2: FP32 + refinement with a
 // double-float residual (BT; SP: FP64 residual); 3: FP32 + refinement with
 // an FP64 residual (xw: a [5][NP] buffer for the first solution).
 void launch_solve(bool sp, int mode, int dir, const Fields& F, const Consts& K, const Work* work, int nwork, int tpb,
@@ -2606,6 +2607,16 @@ void launch_solve(bool sp, int mode, int dir, const Fields& F, const Consts& K, 
   }
 #else
   (void)xw;
+#endif
+#if NPBMZ_HAS_FP32
+  if (mode == 5) {
+    const dim3 grid(nwork, (tpb + BTS_LINES - 1) / BTS_LINES);
+    double* scr = reinterpret_cast<double*>(scratch);
+    if (dir == 0) k_bt_line6<0><<<grid, 32, BTS_SMEM, s>>>(F, K, work, tpb, scr, nlt, add_u);
+    else if (dir == 1) k_bt_line6<1><<<grid, 32, BTS_SMEM, s>>>(F, K, work, tpb, scr, nlt, add_u);
+    else k_bt_line6<2><<<grid, 32, BTS_SMEM, s>>>(F, K, work, tpb, scr, nlt, add_u);
+    return;
+  }
 #endif
   (void)mode;
   launch_solve_t<double>(sp, dir, F, K, work, nwork, tpb, scratch, nlt, add_u, F.rhs, 1, s);

@@ -141,6 +141,22 @@ def test_bt_line_solves_at_small_and_ragged_sizes(oracle_mod, nz, flags):
             compare(p, o, npbmz.RHS, 1e-10 if flags else FAST_REL, [z])
 
 
+def test_bt_few_line_solves_equal_full_launches():
+    """The FP64 sweeps of one zone (six lanes per line) give the bits of the
+    batched launch over class B's 64 zones (one thread per line)."""
+    geom, dt, _ = geom_class("BT", "B")
+    a, b = npbmz.Problem(geom, dt, 0), npbmz.Problem(geom, dt, 0)
+    for p in (a, b):
+        p.setup(npbmz.CE_REFERENCE)
+        p.exch_qbc()
+    a.adi(-1)
+    for z in range(geom.nzones):
+        b.adi(z)
+    for z in range(geom.nzones):
+        np.testing.assert_array_equal(a.download(npbmz.U, z), b.download(npbmz.U, z), err_msg=f"zone {z}")
+        np.testing.assert_array_equal(a.download(npbmz.RHS, z), b.download(npbmz.RHS, z), err_msg=f"zone {z}")
+
+
 @pytest.mark.parametrize("nz", [5, 7, 13])
 def test_bt_fused_mixed_steps_at_small_and_ragged_sizes(oracle_mod, nz):
     """Whole refined FP32 steps (the pipelined sweeps) on zones of 5 points per
