@@ -289,6 +289,7 @@ struct npbmz_handle {
   int tpb_bkt[3][HandleLimits::MAXB] = {{64, 64, 64}, {64, 64, 64}, {64, 64, 64}};
   std::vector<Range> gb_line[3];   // per (group, bucket): slice of the line list
   int cur_bucket = -1;             // >= 0: line launches of that bucket only
+  int64_t problem_lines[3] = {0, 0, 0};  // of the whole problem, from its grid
   int64_t nlines[3] = {0, 0, 0};
   // execution
   cudaStream_t stream = nullptr;
@@ -730,6 +731,16 @@ bool few_lines(const npbmz_t* h, int dir, int zone) {
   return points < 10000 * (int64_t)longest;
 }
 
+// The refined FP32 BT sweeps with two threads per line, by the lines of the
+// whole problem (all ranks' zones, so that every split of it solves alike).
+// One thread per line fills the chip at 152 SMs x 256 lines; half of that, 128
+// lines per SM, is what two threads per line keep at once.  x, y, z sweeps in
+// us, one / two threads: 64x64x8 (1344, 1344, 3136 lines) 85, 72, 33 / 61, 55,
+// 27; 338x118x8 (10,200 to 33,000) 106, 114, 48 / 91, 92, 62; 37x389x12 x
+// (14,300) 59 / 58; 192x104x27 (35,200, 32,000, 14,100) 107, 73, 96 / 117, 97,
+// 96; 480x320x28 (from 119,000) 586, 568, 635 / 668, 694, 708.
+bool two_ended(const npbmz_t* h, int dir) { return h->problem_lines[dir] < 14000; }
+
 int phase_solve(npbmz_t* h, int dir, int zone, int add_u, bool fused = false) {
   const Fields F = fields(h);
   const bool sp = h->kind == NPBMZ_SP;
@@ -737,7 +748,8 @@ int phase_solve(npbmz_t* h, int dir, int zone, int add_u, bool fused = false) {
                    : !use_fp32(h) ? (!sp && few_lines(h, dir, zone) ? 5 : 0)
                    : (h->flags & NPBMZ_FP32_NOREFINE) ? 1
                    : (h->flags & NPBMZ_REFINE_FP64) ? 3
-                   : (fused && h->rdf ? 4 : 2);
+                   : !(fused && h->rdf) ? 2
+                   : !sp && two_ended(h, dir) ? 6 : 4;
   return line_launches(h, dir, zone, [&](int lo, int hi, int tpb) {
     if (use_exact(h))
       exact::launch_solve(sp, 0, dir, F, h->K, h->wline_d[dir] + lo, hi - lo, tpb, line_scratch(h, dir),
@@ -1484,6 +1496,13 @@ int npbmz_create(int kind, int nzones, const int* nx, const int* ny, const int* 
     h->max_face = std::max(h->max_face, 5 * std::max(d.nx, d.ny) * d.nz);
   }
   h->NP = std::max<int64_t>(off, 32);
+  {
+    const int64_t xz = (int64_t)params[4], yz = (int64_t)params[5];
+    const int64_t ix = (int64_t)params[1] - 2 * xz, iy = (int64_t)params[2] - 2 * yz, iz = (int64_t)params[3] - 2;
+    h->problem_lines[0] = xz * iy * iz;
+    h->problem_lines[1] = yz * ix * iz;
+    h->problem_lines[2] = ix * iy;
+  }
   for (int dir = 0; dir < 3; ++dir) {
     h->nlines[dir] = lines[dir];
     int maxlen = 0;

@@ -47,6 +47,7 @@ struct Consts {
   float2 p_c1, p_c2, p_two_m_c2, p_k43, p_c3c4, p_c1345, p_k43m, p_c3c4m;
   float2 p_con43, p_c1c5, p_comz1, p_comz4, p_comz5, p_comz6, p_bt, p_c2iv;
   float2 p_dtt1[3], p_dtt2[3], p_c2dtt1[3], p_d[3][5], p_dmax[3];
+  float2 p_t1d[3][5];  // dt t1 d
   BtK<double> bt64[3];
   BtK<float> bt32[3];
 };
@@ -72,6 +73,8 @@ inline void make_bt_consts(Consts& k) {
     f.c2t2 = (float)b.c2t2; f.c1t2 = (float)b.c1t2; f.kc = (float)b.kc; f.k43 = (float)b.k43; f.kg = (float)b.kg;
     for (int m = 0; m < 5; ++m) {
       b.t1d[m] = t1[dir] * d[dir][m];
+      k.p_t1d[dir][m].x = (float)b.t1d[m];
+      k.p_t1d[dir][m].y = (float)(b.t1d[m] - (double)k.p_t1d[dir][m].x);
       f.t1d[m] = (float)b.t1d[m];
     }
   }

@@ -928,19 +928,19 @@ constexpr int BT_SCR = 30;  // words per point of the FP32 line scratch: C' (25)
 
 // G and H from the FP32 state s = ri, u2, u3, u4, u5, q.
 template <int DIR>
-__device__ __forceinline__ void bt_gh_f32(const Consts& K, const float s[6], BtGH<DIR, float>& J) {
+__device__ __forceinline__ void bt_gh_f32(const BtK<float>& k, const float s[6], BtGH<DIR, float>& J) {
   const float v[3] = {s[1] * s[0], s[2] * s[0], s[3] * s[0]};
-  bt_gh<DIR, float>(bt_consts<float>(K, DIR), s[0], v, s[4] * s[0], s[5], J);
+  bt_gh<DIR, float>(k, s[0], v, s[4] * s[0], s[5], J);
 }
 
 // Start of the elimination: Jacobians at points 0 and 1 (FP32 state s0, s1).
 template <int DIR>
-__device__ __forceinline__ void bt_f32_begin(const Consts& K, const float s0[6], const float s1[6],
+__device__ __forceinline__ void bt_f32_begin(const BtK<float>& k, const float s0[6], const float s1[6],
                                              BtF32Carry<DIR>& c) {
   BtGH<DIR, float> J;
-  bt_gh_f32<DIR>(K, s0, J);
+  bt_gh_f32<DIR>(k, s0, J);
   bt_form_p<DIR, float>(J, c.Pcur);
-  bt_gh_f32<DIR>(K, s1, J);
+  bt_gh_f32<DIR>(k, s1, J);
   bt_form_p<DIR, float>(J, c.Pnext);
   bt_form_b<DIR, float>(J, c.Bs);
 #pragma unroll
@@ -951,15 +951,15 @@ __device__ __forceinline__ void bt_f32_begin(const Consts& K, const float s0[6],
 
 // One forward step at point p (1..n-2): r holds the rhs of row p on entry and
 // the eliminated rhs on exit; sn is the FP32 state at p+1.  C'_p (STORE_C)
-// and r'_p go to scr[(p*BT_SCR + e) * nlt + gl].
+// and r'_p go to out[e * nlt] (the point's words of the line scratch).
 template <int DIR, bool STORE_C>
-__device__ __forceinline__ void bt_f32_step(const Consts& K, int p, float r[5], const float sn[6], BtF32Carry<DIR>& c,
-                                            float* __restrict__ scr, int64_t nlt, int64_t gl) {
+__device__ __forceinline__ void bt_f32_step(const BtK<float>& k, float r[5], const float sn[6], BtF32Carry<DIR>& c,
+                                            float* __restrict__ out, int64_t nlt) {
   float B[5][5], C[5][5];
   BtGH<DIR, float> J;
   bt_add_px<DIR, float>(c.Pcur, c.rp, r);
   bt_add_pc<DIR, float>(c.Pcur, c.Cp, c.Bs, B);
-  bt_gh_f32<DIR>(K, sn, J);
+  bt_gh_f32<DIR>(k, sn, J);
   bt_form_c<DIR, float>(J, C);
 #pragma unroll
   for (int a = 0; a < 5; ++a)
@@ -974,12 +974,12 @@ __device__ __forceinline__ void bt_f32_step(const Consts& K, int p, float r[5], 
 #pragma unroll
     for (int b = 0; b < 5; ++b) {
       c.Cp[a][b] = C[a][b];
-      if (STORE_C) scr[((int64_t)p * BT_SCR + a * 5 + b) * nlt + gl] = C[a][b];
+      if (STORE_C) out[(a * 5 + b) * nlt] = C[a][b];
     }
 #pragma unroll
   for (int m = 0; m < 5; ++m) {
     c.rp[m] = r[m];
-    scr[((int64_t)p * BT_SCR + 25 + m) * nlt + gl] = r[m];
+    out[(25 + m) * nlt] = r[m];
   }
 }
 
@@ -1028,7 +1028,7 @@ __global__ void __launch_bounds__(128) k_bt_mixed_solve(Fields F, Consts K, cons
   load_state_f32(F, base + st, s1);
 #pragma unroll
   for (int m = 0; m < 5; ++m) c.rp[m] = bload(m, base);
-  bt_f32_begin<DIR>(K, s0, s1, c);
+  bt_f32_begin<DIR>(bt_consts<float>(K, DIR), s0, s1, c);
   float sn[6], bn[5];
   load_state_f32(F, base + 2 * st, sn);
 #pragma unroll
@@ -1044,7 +1044,7 @@ __global__ void __launch_bounds__(128) k_bt_mixed_solve(Fields F, Consts K, cons
 #pragma unroll
       for (int m = 0; m < 5; ++m) bn[m] = bload(m, base + (int64_t)(p + 1) * st);
     }
-    bt_f32_step<DIR, true>(K, p, r, s, c, scr, nlt, gl);
+    bt_f32_step<DIR, true>(bt_consts<float>(K, DIR), r, s, c, scr + (int64_t)p * BT_SCR * nlt + gl, nlt);
   }
   float rn[5];
 #pragma unroll
@@ -1135,7 +1135,7 @@ __global__ void __launch_bounds__(128) k_bt_refine(Fields F, Consts K, const Wor
   BtF32Carry<DIR> c;
 #pragma unroll
   for (int m = 0; m < 5; ++m) c.rp[m] = 0.f;  // the boundary residual is exactly zero
-  bt_f32_begin<DIR>(K, s0, s1, c);
+  bt_f32_begin<DIR>(bt_consts<float>(K, DIR), s0, s1, c);
   // prefetch point 2 and b_1
   double xn[5], sn[6], bn[5];
   load_x(2, xn);
@@ -1169,7 +1169,7 @@ __global__ void __launch_bounds__(128) k_bt_refine(Fields F, Consts K, const Wor
     }
 #pragma unroll
     for (int e = 0; e < 6; ++e) s[e] = (float)sq[e];
-    bt_f32_step<DIR, true>(K, p, r, s, c, scr, nlt, gl);
+    bt_f32_step<DIR, true>(bt_consts<float>(K, DIR), r, s, c, scr + (int64_t)p * BT_SCR * nlt + gl, nlt);
     (void)pt;
   }
   // back substitution of the correction d, then x = x0 + d
@@ -1258,42 +1258,99 @@ __device__ __forceinline__ df64 df_from(double d) {
   return {h, __double2float_rn(d - (double)h)};
 }
 
-// F = fjac x and N = njac x in double-float (the formulas of bt_jx).
+// The same without renormalisation (the low word may exceed half an ulp of the
+// high one by a few times): the residual's sums and products.  A product keeps
+// the operands' low words' product where both operands are themselves sums, so
+// that nothing above 2^-46 of the operands' magnitude is dropped, as in the
+// normalised forms: 4 or 5 operations instead of 7, 8 instead of 11 for a sum.
+// With the plain FP32 operands the residual takes 640 instructions a point
+// instead of 1040 (480x320x28 sweeps 586, 568, 635 -> 550, 527, 582 us); u's
+// error against 64 bits after 20 steps of 64x64x8 is 2.8e-15 (before 3.5e-15),
+// after 10 of 480x320x28 1.3e-15 (1.5e-15).
+__device__ __forceinline__ df64 du_mul(df64 a, df64 b) {
+  const float p = __fmul_rn(a.hi, b.hi);
+  float e = __fmaf_rn(a.hi, b.hi, -p);
+  e = __fmaf_rn(a.hi, b.lo, e);
+  return {p, __fmaf_rn(a.lo, b.hi, e)};
+}
+__device__ __forceinline__ df64 du_mul_ss(df64 a, df64 b) {  // both operands sums
+  const df64 r = du_mul(a, b);
+  return {r.hi, __fmaf_rn(a.lo, b.lo, r.lo)};
+}
+__device__ __forceinline__ df64 du_add(df64 a, df64 b) {
+  const df64 s = df_two_sum(a.hi, b.hi);
+  return {s.hi, __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo))};
+}
+__device__ __forceinline__ df64 du_sub(df64 a, df64 b) { return du_add(a, df_neg(b)); }
+// with a plain FP32 operand: the first pass's solution inside the line
+__device__ __forceinline__ df64 du_mul(df64 a, float b) {
+  const float p = __fmul_rn(a.hi, b);
+  return {p, __fmaf_rn(a.lo, b, __fmaf_rn(a.hi, b, -p))};
+}
+__device__ __forceinline__ df64 du_add(df64 a, float b) {
+  const df64 s = df_two_sum(a.hi, b);
+  return {s.hi, __fadd_rn(s.lo, a.lo)};
+}
+
+// Constants of the residual in one direction (pairs); t2 carries the sign of
+// the direction the line is walked in.
+struct BtResid {
+  df64 t1, t2, t1d[5], c1, c2, two_m_c2, k43, c3c4, c1345, k43m, c3c4m;
+};
 template <int DIR>
-__device__ __forceinline__ void bt_jx_df(const df64 c1, const df64 c2, const df64 two_m_c2, const df64 k43,
-                                         const df64 c3c4, const df64 c1345, const df64 k43m, const df64 c3c4m,
-                                         const df64 st[6], const df64 x[5], df64 Fx[5], df64 Nx[5]) {
+__device__ __forceinline__ BtResid bt_resid_consts(const Consts& K, bool turned) {
+  BtResid c;
+  c.t1 = f2df(K.p_dtt1[DIR]);
+  c.t2 = f2df(K.p_dtt2[DIR]);
+  if (turned) c.t2 = df_neg(c.t2);
+#pragma unroll
+  for (int m = 0; m < 5; ++m) c.t1d[m] = f2df(K.p_t1d[DIR][m]);
+  c.c1 = f2df(K.p_c1);
+  c.c2 = f2df(K.p_c2);
+  c.two_m_c2 = f2df(K.p_two_m_c2);
+  c.k43 = f2df(K.p_k43);
+  c.c3c4 = f2df(K.p_c3c4);
+  c.c1345 = f2df(K.p_c1345);
+  c.k43m = f2df(K.p_k43m);
+  c.c3c4m = f2df(K.p_c3c4m);
+  return c;
+}
+
+// P = tmp2 fjac x and Q = tmp1 (njac + D) x of one point (the formulas of
+// bt_jx); X = float inside the line, df64 at its ends.
+template <int DIR, typename X>
+__device__ __forceinline__ void bt_pq(const BtResid& k, const df64 st[6], const X x[5], df64 P[5], df64 Q[5]) {
   // st = ri, u2, u3, u4, u5, q
   const df64 ri = st[0], q = st[5];
-  const df64 vel[3] = {df_mul(st[1], ri), df_mul(st[2], ri), df_mul(st[3], ri)};
-  const df64 E = df_mul(st[4], ri);
-  constexpr int a = DIR + 1;
+  const df64 vel[3] = {du_mul(st[1], ri), du_mul(st[2], ri), du_mul(st[3], ri)};
+  const df64 E = du_mul(st[4], ri);
+  constexpr int a = DIR + 1, m1 = DIR == 0 ? 1 : 0, m2 = DIR == 2 ? 1 : 2;
   const df64 vn = vel[DIR];
   df64 d[3];
 #pragma unroll
-  for (int m = 0; m < 3; ++m) d[m] = df_sub(x[m + 1], df_mul(vel[m], x[0]));
-  df64 tang = {0.f, 0.f};
-  Fx[0] = x[a];
+  for (int m = 0; m < 3; ++m) d[m] = du_add(df_neg(du_mul(vel[m], x[0])), x[m + 1]);
+  df64 Fx[5];
+#pragma unroll
+  for (int m = 0; m < 3; ++m)
+    if (m != DIR) Fx[m + 1] = du_add(du_mul_ss(vn, d[m]), du_mul(vel[m], x[a]));
+  const df64 tang = du_add(du_mul(vel[m1], x[m1 + 1]), du_mul(vel[m2], x[m2 + 1]));
+  const df64 c2q = du_mul(k.c2, q), vn2 = du_mul(vn, vn), c1E = du_mul(k.c1, E);
+  Fx[a] = du_add(du_sub(du_mul(du_sub(c2q, vn2), x[0]), du_mul(k.c2, tang)),
+                 du_add(du_mul(du_mul(k.two_m_c2, vn), x[a]), du_mul(k.c2, x[4])));
+  Fx[4] = du_add(du_sub(du_mul(du_mul_ss(du_sub(df_scale2(c2q), c1E), vn), x[0]), du_mul_ss(du_mul(k.c2, vn), tang)),
+                 du_add(du_mul(du_sub(c1E, du_mul(k.c2, du_add(q, vn2))), x[a]), du_mul(du_mul(k.c1, vn), x[4])));
+  df64 s4 = du_mul(k.c1345, du_add(df_neg(du_mul(E, x[0])), x[4]));
+  const df64 k43ri = du_mul(k.k43, ri), c3c4ri = du_mul(k.c3c4, ri);
+  P[0] = du_mul(k.t2, x[a]);
+  Q[0] = du_mul(k.t1d[0], x[0]);
 #pragma unroll
   for (int m = 0; m < 3; ++m) {
-    if (m == DIR) continue;
-    Fx[m + 1] = df_add(df_mul(vn, d[m]), df_mul(vel[m], x[a]));
-    tang = df_add(tang, df_mul(vel[m], x[m + 1]));
+    Q[m + 1] = du_add(du_mul(k.t1, du_mul_ss(m == DIR ? k43ri : c3c4ri, d[m])), du_mul(k.t1d[m + 1], x[m + 1]));
+    s4 = du_add(s4, du_mul_ss(du_mul(m == DIR ? k.k43m : k.c3c4m, vel[m]), d[m]));
   }
-  const df64 c2q = df_mul(c2, q), vn2 = df_mul(vn, vn), c1E = df_mul(c1, E);
-  Fx[a] = df_add(df_add(df_mul(df_sub(c2q, vn2), x[0]), df_neg(df_mul(c2, tang))),
-                 df_add(df_mul(df_mul(two_m_c2, vn), x[a]), df_mul(c2, x[4])));
-  Fx[4] = df_add(df_add(df_mul(df_mul(df_sub(df_scale2(c2q), c1E), vn), x[0]), df_neg(df_mul(df_mul(c2, vn), tang))),
-                 df_add(df_mul(df_sub(c1E, df_mul(c2, df_add(q, vn2))), x[a]), df_mul(df_mul(c1, vn), x[4])));
-  df64 s4 = df_mul(c1345, df_sub(x[4], df_mul(E, x[0])));
-  const df64 k43ri = df_mul(k43, ri), c3c4ri = df_mul(c3c4, ri);
-  Nx[0] = {0.f, 0.f};
+  Q[4] = du_add(du_mul(k.t1, du_mul_ss(ri, s4)), du_mul(k.t1d[4], x[4]));
 #pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    Nx[m + 1] = df_mul(m == DIR ? k43ri : c3c4ri, d[m]);
-    s4 = df_add(s4, df_mul(df_mul(m == DIR ? k43m : c3c4m, vel[m]), d[m]));
-  }
-  Nx[4] = df_mul(ri, s4);
+  for (int m = 1; m < 5; ++m) P[m] = du_mul(k.t2, Fx[m]);
 }
 
 __device__ __forceinline__ void load_state_df(const Fields& F, int64_t pt, df64 s[6]) {
@@ -1328,15 +1385,7 @@ __global__ void __launch_bounds__(128) k_bt_refine_df(Fields F, Consts K, const 
   double* __restrict__ rhs = F.rhs;
   float* __restrict__ bdf = F.rdf;
 
-  const df64 t1 = f2df(K.p_dtt1[DIR]);
-  const df64 t2 = f2df(K.p_dtt2[DIR]);
-  df64 D[5];
-#pragma unroll
-  for (int m = 0; m < 5; ++m) D[m] = f2df(K.p_d[DIR][m]);
-  const df64 c1 = f2df(K.p_c1), c2 = f2df(K.p_c2), two_m_c2 = f2df(K.p_two_m_c2);
-  const df64 k43 = f2df(K.p_k43), c3c4 = f2df(K.p_c3c4), c1345 = f2df(K.p_c1345);
-  const df64 k43m = f2df(K.p_k43m), c3c4m = f2df(K.p_c3c4m);
-
+  const BtResid kr = bt_resid_consts<DIR>(K, false);
   auto load_x = [&](int q, df64 x[5]) {
     const int64_t pt = base + (int64_t)q * st;
     if (q == 0 || q == n - 1) {
@@ -1347,28 +1396,18 @@ __global__ void __launch_bounds__(128) k_bt_refine_df(Fields F, Consts K, const 
       for (int m = 0; m < 5; ++m) x[m] = {x0f[m * NP + pt], 0.f};
     }
   };
-  // P and Q of one point
-  auto pq = [&](const df64 s[6], const df64 x[5], df64 P[5], df64 Q[5]) {
-    df64 Fq[5], Nq[5];
-    bt_jx_df<DIR>(c1, c2, two_m_c2, k43, c3c4, c1345, k43m, c3c4m, s, x, Fq, Nq);
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      P[m] = df_mul(t2, Fq[m]);
-      Q[m] = df_mul(t1, df_add(Nq[m], df_mul(D[m], x[m])));
-    }
-  };
   df64 acc_c[5], acc_n[5], xq[5], sq[6], P[5], Q[5];
   float s0[6], s1[6];
   load_x(0, xq);
   load_state_df(F, base, sq);
-  pq(sq, xq, P, Q);
+  bt_pq<DIR>(kr, sq, xq, P, Q);
 #pragma unroll
   for (int m = 0; m < 5; ++m) acc_c[m] = df_neg(df_add(P[m], Q[m]));
 #pragma unroll
   for (int e = 0; e < 6; ++e) s0[e] = sq[e].hi;
   load_x(1, xq);
   load_state_df(F, base + st, sq);
-  pq(sq, xq, P, Q);
+  bt_pq<DIR>(kr, sq, xq, P, Q);
 #pragma unroll
   for (int m = 0; m < 5; ++m) {
     acc_c[m] = df_add(acc_c[m], df_add(xq[m], df_scale2(Q[m])));
@@ -1380,7 +1419,7 @@ __global__ void __launch_bounds__(128) k_bt_refine_df(Fields F, Consts K, const 
 #pragma unroll
   for (int m = 0; m < 5; ++m) c.rp[m] = 0.f;
   // bt_f32_begin takes ri, u2, u3, u4, u5, q in that order (as sq)
-  bt_f32_begin<DIR>(K, s0, s1, c);
+  bt_f32_begin<DIR>(bt_consts<float>(K, DIR), s0, s1, c);
   df64 xn[5], sn[6];
   // b of the next point: double-float planes (IN_DF) or FP64 rhs
   df64 bn[5];
@@ -1412,7 +1451,7 @@ __global__ void __launch_bounds__(128) k_bt_refine_df(Fields F, Consts K, const 
       load_state_df(F, base + (int64_t)(p + 2) * st, sn);
       load_b(base + (int64_t)(p + 1) * st);
     }
-    pq(sq, xq, P, Q);
+    bt_pq<DIR>(kr, sq, xq, P, Q);
     float r[5], s[6];
 #pragma unroll
     for (int m = 0; m < 5; ++m) {
@@ -1428,7 +1467,7 @@ __global__ void __launch_bounds__(128) k_bt_refine_df(Fields F, Consts K, const 
     }
 #pragma unroll
     for (int e = 0; e < 6; ++e) s[e] = sq[e].hi;
-    bt_f32_step<DIR, true>(K, p, r, s, c, scr, nlt, gl);
+    bt_f32_step<DIR, true>(bt_consts<float>(K, DIR), r, s, c, scr + (int64_t)p * BT_SCR * nlt + gl, nlt);
   }
   float dn[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
   for (int p = n - 2; p >= 1; --p) {
@@ -1457,15 +1496,24 @@ __global__ void __launch_bounds__(128) k_bt_refine_df(Fields F, Consts K, const 
 }
 
 // ============================================================================
-// Software-pipelined refined FP32 BT sweep of a fused step (mode 4).  The
-// two passes above wait on memory once per point: a line advances one point
-// per DRAM round trip, and with 8-12 resident warps per SM nothing hides it.
-// Here each thread streams its own line's data PIPE points ahead with
-// cp.async into a ring of PIPE slots in shared memory (word e of slot s of
-// thread t at ring[(s * W + e) * T + t]: a warp's copies land in consecutive
-// banks), in the forward elimination and in the back substitution alike.
-// The arithmetic is that of k_bt_mixed_solve<DIR, true> and
-// k_bt_refine_df<DIR, true, OUT_DF>.
+// Software-pipelined refined FP32 BT sweep of a fused step (mode 4).
+// Each thread streams its data PIPE points ahead with cp.async into a ring of
+// PIPE slots in shared memory (word e of slot s of thread t at
+// ring[(s * W + e) * T + t]: a warp's copies land in consecutive banks), in
+// the forward elimination and in the back substitution alike.
+//
+// TWO: two threads per line, eliminating from both ends: thread t of the first
+// half of the block takes rows 1..L0 of its line from point 0 up, thread
+// t + lines the rows n-2..L0+1 from point n-1 down (L0 = (n-1)/2 rows, L1 the
+// rest).  Seen from the far end the line is the same one with the sign of the
+// convective terms turned (G -> -G: lhsa and lhsc trade places), so both
+// halves run the same code on a local index j, q = j or n-1-j.  At the seam
+//   x_A = r'_A - C'_A x_B,  x_B = r'_B - C'_B x_A
+// (A, B the two middle rows), so each half solves (I - C'_A C'_B) x_A =
+// r'_A - C'_A r'_B with its partner's C' and r' and substitutes back toward
+// its own end.  A line then takes half as many dependent steps for 8 % more
+// instructions and a barrier: faster while the lines are too few to fill the
+// chip one per thread (two_ended in npbmz_api.cu draws the line).
 // ============================================================================
 #ifndef NPBMZ_PIPE
 #define NPBMZ_PIPE 4
@@ -1501,151 +1549,241 @@ __device__ __forceinline__ void cpa_wait() {
 
 constexpr int PL_MIXED_W = 30;   // words per slot, first pass
 constexpr int PL_REFINE_W = 45;  // words per slot, refinement pass
+// Words per thread beside the ring: at the seam C' and r' (TWO), else b at the
+// line's last point in double-float.
+constexpr int pl_end_words(bool two) { return two ? 30 : 10; }
 
-// Dynamic shared memory of the pipelined kernels for tpb threads.
-// (the first pass keeps 5 more words per line: b at the line's last point;
-// the refinement pass 10: the same in double-float)
-__host__ __device__ constexpr size_t pl_mixed_smem(int tpb) {
-  return (size_t)(PIPE * PL_MIXED_W + 5) * tpb * sizeof(float);
+// Dynamic shared memory of the pipelined kernels for tpb lines per block.
+__host__ __device__ constexpr size_t pl_mixed_smem(int tpb, bool two) {
+  return (size_t)(PIPE * PL_MIXED_W + pl_end_words(two)) * (two ? 2 : 1) * tpb * sizeof(float);
 }
-__host__ __device__ constexpr size_t pl_refine_smem(int tpb) {
-  return (size_t)(PIPE * PL_REFINE_W + 10) * tpb * sizeof(float);
+__host__ __device__ constexpr size_t pl_refine_smem(int tpb, bool two) {
+  return (size_t)(PIPE * PL_REFINE_W + pl_end_words(two)) * (two ? 2 : 1) * tpb * sizeof(float);
 }
 
+// A thread's part of a line (TWO: one half): local point j is point q(j).
+template <int DIR, bool TWO>
+struct BtHalf {
+  int n, L;           // points of the line, rows of this half
+  bool far;           // the half that starts at point n-1
+  bool active;        // the block's last lines may be missing
+  int64_t base, st, gl;
+  __device__ __forceinline__ int q(int j) const { return TWO && far ? n - 1 - j : j; }
+  __device__ __forceinline__ int64_t pt(int j) const { return base + (int64_t)q(j) * st; }
+};
+template <int DIR, bool TWO>
+__device__ __forceinline__ BtHalf<DIR, TWO> bt_half(const ZoneDev& Z, int first) {
+  BtHalf<DIR, TWO> h;
+  const int lines = TWO ? blockDim.x >> 1 : blockDim.x;
+  h.far = TWO && (int)threadIdx.x >= lines;
+  const int line = first + (int)threadIdx.x - (h.far ? lines : 0);
+  h.active = line < zone_lines(Z, DIR);
+  h.n = zone_line_len(Z, DIR);
+  const int L0 = TWO ? (h.n - 1) >> 1 : h.n - 2;
+  h.L = h.far ? h.n - 2 - L0 : L0;
+  if (h.active) line_geometry(Z, DIR, line, h.base, h.st);
+  h.gl = Z.lineoff[DIR] + line;
+  return h;
+}
+
+// The direction's constants with the sign of the convective terms turned for
+// the far half.
 template <int DIR>
+__device__ __forceinline__ BtK<float> bt_half_consts(const Consts& K, bool far) {
+  BtK<float> k = bt_consts<float>(K, DIR);
+  if (far) {
+    k.t2 = -k.t2;
+    k.c2t2 = -k.c2t2;
+    k.c1t2 = -k.c1t2;
+  }
+  return k;
+}
+
+// The seam: x of this half's last row from its own and its partner's C', r'
+// (join: 30 words per thread).  All threads of the block call it.
+__device__ __forceinline__ void bt_join(float* join, bool far, const float C[5][5], const float r[5], float x[5]) {
+  const int T = blockDim.x, lines = T >> 1, t = threadIdx.x, u = far ? t - lines : t + lines;
+#pragma unroll
+  for (int e = 0; e < 25; ++e) join[e * T + t] = C[e / 5][e % 5];
+#pragma unroll
+  for (int m = 0; m < 5; ++m) join[(25 + m) * T + t] = r[m];
+  __syncthreads();
+  float M[5][5];
+#pragma unroll
+  for (int m = 0; m < 5; ++m) {
+    x[m] = r[m];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+      x[m] = fmaf(-C[m][c], join[(25 + c) * T + u], x[m]);
+      M[m][c] = m == c ? 1.f : 0.f;
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 5; ++e)
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+      const float b = join[(e * 5 + c) * T + u];
+#pragma unroll
+      for (int m = 0; m < 5; ++m) M[m][c] = fmaf(-C[m][e], b, M[m][c]);
+    }
+#pragma unroll
+  for (int p = 0; p < 5; ++p) {
+    const float piv = bt_recip(M[p][p]);
+#pragma unroll
+    for (int c = p + 1; c < 5; ++c) M[p][c] *= piv;
+    x[p] *= piv;
+#pragma unroll
+    for (int q = p + 1; q < 5; ++q) {
+#pragma unroll
+      for (int c = p + 1; c < 5; ++c) M[q][c] = fmaf(-M[q][p], M[p][c], M[q][c]);
+      x[q] = fmaf(-M[q][p], x[p], x[q]);
+    }
+  }
+#pragma unroll
+  for (int p = 4; p > 0; --p)
+#pragma unroll
+    for (int q = 0; q < p; ++q) x[q] = fmaf(-M[q][p], x[p], x[q]);
+  __syncthreads();  // join may be written again (the block's next item)
+}
+
+template <int DIR, bool TWO>
 __device__ __forceinline__ void bt_mixed_pl_item(const Fields& F, const Consts& K, const Work w,
                                                  float* __restrict__ scr, int64_t nlt, float* __restrict__ x0,
                                                  unsigned char* pl_smem) {
   const ZoneDev Z = F.zones[w.zone];
-  const int line = w.first + threadIdx.x;
-  if (line >= zone_lines(Z, DIR)) return;
-  int64_t base, st;
-  line_geometry(Z, DIR, line, base, st);
-  const int n = zone_line_len(Z, DIR);
-  const int64_t gl = Z.lineoff[DIR] + line;
+  const BtHalf<DIR, TWO> h = bt_half<DIR, TWO>(Z, w.first);
+  if (!TWO && !h.active) return;
   const int64_t NP = F.NP;
-  const int T = blockDim.x;
+  const int T = blockDim.x, L = h.L;
   float* my = reinterpret_cast<float*>(pl_smem) + threadIdx.x;
   auto S = [&](int slot, int e) -> float* { return my + (slot * PL_MIXED_W + e) * T; };
   const int order[6] = {PF_RHOI, PF_U2, PF_U3, PF_U4, PF_U5, PF_QS};
   // the x sweep reads its x-line-major copies, y and z the zone layout
-  auto st_at = [&](int q, int plane) -> const float* {
-    return DIR == 0 ? F.pfx + ((int64_t)q * PF_COUNT + plane) * F.nlx + gl : F.primf + plane * NP + base + (int64_t)q * st;
+  auto st_at = [&](int j, int plane) -> const float* {
+    return DIR == 0 ? F.pfx + ((int64_t)h.q(j) * PF_COUNT + plane) * F.nlx + h.gl : F.primf + plane * NP + h.pt(j);
   };
-  auto b_at = [&](int q, int e) -> const float* {
-    return DIR == 0 ? F.rdx + ((int64_t)q * 10 + e) * F.nlx + gl : F.rdf + e * NP + base + (int64_t)q * st;
+  auto b_at = [&](int j, int e) -> const float* {
+    return DIR == 0 ? F.rdx + ((int64_t)h.q(j) * 10 + e) * F.nlx + h.gl : F.rdf + e * NP + h.pt(j);
   };
-  auto x0_at = [&](int q, int m) -> float* {
-    return DIR == 0 ? F.x0x + ((int64_t)q * 5 + m) * F.nlx + gl : x0 + m * NP + base + (int64_t)q * st;
+  auto x0_at = [&](int j, int m) -> float* {
+    return DIR == 0 ? F.x0x + ((int64_t)h.q(j) * 5 + m) * F.nlx + h.gl : x0 + m * NP + h.pt(j);
   };
-
-  // forward step p (1..n-2) consumes b_p and the state at p+1
-  auto issue_fwd = [&](int p) {
-    if (p <= n - 2) {
-      const int slot = p % PIPE;
+  auto scr_at = [&](int j, int e) -> float* { return scr + ((int64_t)h.q(j) * BT_SCR + e) * nlt + h.gl; };
+  // forward step j (1..L) consumes b_j and the state at j+1
+  auto issue_fwd = [&](int j) {
+    if (j <= L) {
+      const int slot = j % PIPE;
 #pragma unroll
-      for (int e = 0; e < 6; ++e) cpa4(S(slot, e), st_at(p + 1, order[e]));
+      for (int e = 0; e < 6; ++e) cpa4(S(slot, e), st_at(j + 1, order[e]));
 #pragma unroll
-      for (int m = 0; m < 5; ++m) cpa4(S(slot, 6 + m), b_at(p, m));
+      for (int m = 0; m < 5; ++m) cpa4(S(slot, 6 + m), b_at(j, m));
     }
     cpa_commit();
   };
-  // the ring's first slots (and b at the last point, which the back
-  // substitution starts from) go out before the line's first points are read
-  // directly, so that the memory latencies overlap
-#pragma unroll
-  for (int m = 0; m < 5; ++m) cpa4(S(PIPE, m), b_at(n - 1, m));
-#pragma unroll
-  for (int q = 1; q < PIPE; ++q) issue_fwd(q);
+  const BtK<float> k = bt_half_consts<DIR>(K, h.far);
   BtF32Carry<DIR> c;
-  {
-    float s0[6], s1[6];
+  float* ends = reinterpret_cast<float*>(pl_smem) + (size_t)PIPE * PL_MIXED_W * T;
+  if (h.active) {
+    // the ring's first slots (and b at the last point, which a whole line's
+    // back substitution starts from) go out before the line's first points
+    // are read directly, so that the memory latencies overlap
+    if (!TWO) {
 #pragma unroll
-    for (int e = 0; e < 6; ++e) {
-      s0[e] = *st_at(0, order[e]);
-      s1[e] = *st_at(1, order[e]);
+      for (int m = 0; m < 5; ++m) cpa4(ends + m * T + threadIdx.x, b_at(h.n - 1, m));
     }
 #pragma unroll
-    for (int m = 0; m < 5; ++m) c.rp[m] = *b_at(0, m);
-    bt_f32_begin<DIR>(K, s0, s1, c);
-  }
-  for (int p = 1; p <= n - 2; ++p) {
-    issue_fwd(p + PIPE - 1);
-    cpa_wait<PIPE - 1>();
-    const int slot = p % PIPE;
-    float r[5], s[6];
+    for (int j = 1; j < PIPE; ++j) issue_fwd(j);
+    {
+      float s0[6], s1[6];
 #pragma unroll
-    for (int e = 0; e < 6; ++e) s[e] = *S(slot, e);
+      for (int e = 0; e < 6; ++e) {
+        s0[e] = *st_at(0, order[e]);
+        s1[e] = *st_at(1, order[e]);
+      }
 #pragma unroll
-    for (int m = 0; m < 5; ++m) r[m] = *S(slot, 6 + m);
-    bt_f32_step<DIR, true>(K, p, r, s, c, scr, nlt, gl);
-    if (p + PIPE > n - 2) {
-      // the ring does not refill this slot: C'_p and r'_p stay here for the
-      // back substitution, which so starts without a trip to memory
-#pragma unroll
-      for (int a = 0; a < 5; ++a)
-#pragma unroll
-        for (int b = 0; b < 5; ++b) *S(slot, a * 5 + b) = c.Cp[a][b];
-#pragma unroll
-      for (int m = 0; m < 5; ++m) *S(slot, 25 + m) = c.rp[m];
+      for (int m = 0; m < 5; ++m) c.rp[m] = *b_at(0, m);
+      bt_f32_begin<DIR>(k, s0, s1, c);
     }
-  }
-  cpa_wait<0>();
-  // back substitution: step p (n-2 .. 1) consumes C'_p and r'_p from slot
-  // p % PIPE: the last PIPE points as the forward pass left them, the others
-  // loaded PIPE steps ahead into the slot just consumed
-  auto issue_bwd = [&](int p) {
-    if (p >= 1) {
-      const int slot = p % PIPE;
+    for (int j = 1; j <= L; ++j) {
+      issue_fwd(j + PIPE - 1);
+      cpa_wait<PIPE - 1>();
+      const int slot = j % PIPE;
+      float r[5], s[6];
 #pragma unroll
-      for (int e = 0; e < 30; ++e) cpa4(S(slot, e), scr + ((int64_t)p * BT_SCR + e) * nlt + gl);
+      for (int e = 0; e < 6; ++e) s[e] = *S(slot, e);
+#pragma unroll
+      for (int m = 0; m < 5; ++m) r[m] = *S(slot, 6 + m);
+      bt_f32_step<DIR, true>(k, r, s, c, scr_at(j, 0), nlt);
+      if (j + PIPE > L) {
+        // the ring does not refill this slot: C'_j and r'_j stay here for the
+        // back substitution, which so starts without a trip to memory
+#pragma unroll
+        for (int a = 0; a < 5; ++a)
+#pragma unroll
+          for (int b = 0; b < 5; ++b) *S(slot, a * 5 + b) = c.Cp[a][b];
+#pragma unroll
+        for (int m = 0; m < 5; ++m) *S(slot, 25 + m) = c.rp[m];
+      }
+    }
+    cpa_wait<0>();
+  }
+  float rn[5];
+  if (TWO) {
+    bt_join(ends, h.far, c.Cp, c.rp, rn);
+    if (!h.active) return;
+  } else {
+#pragma unroll
+    for (int m = 0; m < 5; ++m) rn[m] = ends[m * T + threadIdx.x];
+  }
+  // back substitution (TWO: row L is the seam's): step j consumes C'_j and
+  // r'_j from slot j % PIPE: the last PIPE rows as the forward pass left
+  // them, the others loaded PIPE steps ahead into the slot just consumed
+  auto issue_bwd = [&](int j) {
+    if (j >= 1) {
+      const int slot = j % PIPE;
+#pragma unroll
+      for (int e = 0; e < 30; ++e) cpa4(S(slot, e), scr_at(j, e));
     }
     cpa_commit();
   };
-  float rn[5];
+  for (int j = L; j >= 1; --j) {
+    if (j + PIPE <= L) cpa_wait<PIPE - 1>();
+    const int slot = j % PIPE;
+    if (!TWO || j < L) {
+      float r[5];
 #pragma unroll
-  for (int m = 0; m < 5; ++m) rn[m] = *S(PIPE, m);
-  for (int p = n - 2; p >= 1; --p) {
-    if (p + PIPE <= n - 2) cpa_wait<PIPE - 1>();
-    const int slot = p % PIPE;
-    float r[5];
+      for (int m = 0; m < 5; ++m) {
+        float t = *S(slot, 25 + m);
 #pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      float t = *S(slot, 25 + m);
+        for (int cc = 0; cc < 5; ++cc) t -= *S(slot, m * 5 + cc) * rn[cc];
+        r[m] = t;
+      }
 #pragma unroll
-      for (int cc = 0; cc < 5; ++cc) t -= *S(slot, m * 5 + cc) * rn[cc];
-      r[m] = t;
+      for (int m = 0; m < 5; ++m) rn[m] = r[m];
     }
 #pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      *x0_at(p, m) = r[m];
-      rn[m] = r[m];
-    }
-    issue_bwd(p - PIPE);
+    for (int m = 0; m < 5; ++m) *x0_at(j, m) = rn[m];
+    issue_bwd(j - PIPE);
   }
   cpa_wait<0>();
 }
 
-template <int DIR>
-__global__ void __launch_bounds__(128, NPBMZ_BT_MIXED_MINB) k_bt_mixed_pl(Fields F, Consts K, const Work* __restrict__ work, int nwork,
+template <int DIR, bool TWO>
+__global__ void __launch_bounds__(TWO ? 256 : 128, NPBMZ_BT_MIXED_MINB) k_bt_mixed_pl(Fields F, Consts K, const Work* __restrict__ work, int nwork,
                                                      float* __restrict__ scr, int64_t nlt, float* __restrict__ x0) {
   extern __shared__ __align__(16) unsigned char pl_smem[];
-  for (int it = blockIdx.x; it < nwork; it += gridDim.x) bt_mixed_pl_item<DIR>(F, K, work[it], scr, nlt, x0, pl_smem);
+  for (int it = blockIdx.x; it < nwork; it += gridDim.x) bt_mixed_pl_item<DIR, TWO>(F, K, work[it], scr, nlt, x0, pl_smem);
 }
 
-template <int DIR, bool OUT_DF>
+template <int DIR, bool OUT_DF, bool TWO>
 __device__ __forceinline__ void bt_refine_pl_item(const Fields& F, const Consts& K, const Work w,
                                                   float* __restrict__ scr, int64_t nlt, int add_u,
                                                   const float* __restrict__ x0f, unsigned char* pl_smem) {
   const ZoneDev Z = F.zones[w.zone];
-  const int line = w.first + threadIdx.x;
-  if (line >= zone_lines(Z, DIR)) return;
-  int64_t base, st;
-  line_geometry(Z, DIR, line, base, st);
-  const int n = zone_line_len(Z, DIR);
-  const int64_t gl = Z.lineoff[DIR] + line;
+  const BtHalf<DIR, TWO> h = bt_half<DIR, TWO>(Z, w.first);
+  if (!TWO && !h.active) return;
   const int64_t NP = F.NP;
-  const int T = blockDim.x;
+  const int T = blockDim.x, L = h.L;
   float* my = reinterpret_cast<float*>(pl_smem) + threadIdx.x;
   auto S = [&](int slot, int e) -> float* { return my + (slot * PL_REFINE_W + e) * T; };
   double* __restrict__ rhs = F.rhs;
@@ -1653,74 +1791,58 @@ __device__ __forceinline__ void bt_refine_pl_item(const Fields& F, const Consts&
   const int order[6] = {PF_RHOI, PF_U2, PF_U3, PF_U4, PF_U5, PF_QS};
   // the x sweep reads its x-line-major copies, y and z the zone layout; the
   // result always goes to the zone layout (the next sweep reads it there)
-  auto st_at = [&](int q, int plane) -> const float* {
-    return DIR == 0 ? F.pfx + ((int64_t)q * PF_COUNT + plane) * F.nlx + gl : F.primf + plane * NP + base + (int64_t)q * st;
+  auto st_at = [&](int j, int plane) -> const float* {
+    return DIR == 0 ? F.pfx + ((int64_t)h.q(j) * PF_COUNT + plane) * F.nlx + h.gl : F.primf + plane * NP + h.pt(j);
   };
-  auto b_at = [&](int q, int e) -> const float* {
-    return DIR == 0 ? F.rdx + ((int64_t)q * 10 + e) * F.nlx + gl : bdf + e * NP + base + (int64_t)q * st;
+  auto b_at = [&](int j, int e) -> float* {
+    return DIR == 0 ? F.rdx + ((int64_t)h.q(j) * 10 + e) * F.nlx + h.gl : bdf + e * NP + h.pt(j);
   };
-  auto x0_at = [&](int q, int m) -> const float* {
-    return DIR == 0 ? F.x0x + ((int64_t)q * 5 + m) * F.nlx + gl : x0f + m * NP + base + (int64_t)q * st;
+  auto x0_at = [&](int j, int m) -> const float* {
+    return DIR == 0 ? F.x0x + ((int64_t)h.q(j) * 5 + m) * F.nlx + h.gl : x0f + m * NP + h.pt(j);
   };
+  auto scr_at = [&](int j, int e) -> float* { return scr + ((int64_t)h.q(j) * BT_SCR + e) * nlt + h.gl; };
 
-  const df64 t1 = f2df(K.p_dtt1[DIR]);
-  const df64 t2 = f2df(K.p_dtt2[DIR]);
-  df64 D[5];
-#pragma unroll
-  for (int m = 0; m < 5; ++m) D[m] = f2df(K.p_d[DIR][m]);
-  const df64 c1 = f2df(K.p_c1), c2 = f2df(K.p_c2), two_m_c2 = f2df(K.p_two_m_c2);
-  const df64 k43 = f2df(K.p_k43), c3c4 = f2df(K.p_c3c4), c1345 = f2df(K.p_c1345);
-  const df64 k43m = f2df(K.p_k43m), c3c4m = f2df(K.p_c3c4m);
-
-  auto pq = [&](const df64 s[6], const df64 x[5], df64 P[5], df64 Q[5]) {
-    df64 Fq[5], Nq[5];
-    bt_jx_df<DIR>(c1, c2, two_m_c2, k43, c3c4, c1345, k43m, c3c4m, s, x, Fq, Nq);
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      P[m] = df_mul(t2, Fq[m]);
-      Q[m] = df_mul(t1, df_add(Nq[m], df_mul(D[m], x[m])));
-    }
-  };
-  auto load_x = [&](int q, df64 x[5]) {  // direct loads (prologue)
+  const BtResid kr = bt_resid_consts<DIR>(K, h.far);
+  // x at local point j: b itself at the line's ends, else the first pass's
+  auto load_x = [&](int j, df64 x[5]) {
 #pragma unroll
     for (int m = 0; m < 5; ++m)
-      x[m] = (q == 0 || q == n - 1) ? df64{*b_at(q, m), *b_at(q, 5 + m)} : df64{*x0_at(q, m), 0.f};
+      x[m] = (j == 0 || j == h.n - 1) ? df64{*b_at(j, m), *b_at(j, 5 + m)} : df64{*x0_at(j, m), 0.f};
   };
-  auto load_sdf = [&](int q, df64 s6[6]) {
+  auto load_sdf = [&](int j, df64 s6[6]) {
 #pragma unroll
-    for (int e = 0; e < 6; ++e) s6[e] = df64{*st_at(q, order[e]), *st_at(q, PF_HI_COUNT + order[e])};
+    for (int e = 0; e < 6; ++e) s6[e] = df64{*st_at(j, order[e]), *st_at(j, PF_HI_COUNT + order[e])};
   };
-  // forward step p (1..n-2) consumes x0 and the state at p+1 and b_p: words
-  // 0..4 x0, 5..16 state hi/lo, 17..26 b hi/lo (the line's last point has b
-  // itself for x: words 0..9 of slot PIPE, fetched first)
-  auto issue_fwd = [&](int p) {
-    if (p <= n - 2) {
-      const int slot = p % PIPE;
-      if (p + 1 < n - 1) {
+  // forward step j (1..L) consumes x0 and the state at j+1 and b_j: words
+  // 0..4 x0, 5..16 state hi/lo, 17..26 b hi/lo
+  auto issue_fwd = [&](int j) {
+    if (j <= L) {
+      const int slot = j % PIPE;
+      if (j + 1 < h.n - 1) {
 #pragma unroll
-        for (int m = 0; m < 5; ++m) cpa4(S(slot, m), x0_at(p + 1, m));
+        for (int m = 0; m < 5; ++m) cpa4(S(slot, m), x0_at(j + 1, m));
       }
 #pragma unroll
       for (int e = 0; e < 6; ++e) {
-        cpa4(S(slot, 5 + e), st_at(p + 1, order[e]));
-        cpa4(S(slot, 11 + e), st_at(p + 1, PF_HI_COUNT + order[e]));
+        cpa4(S(slot, 5 + e), st_at(j + 1, order[e]));
+        cpa4(S(slot, 11 + e), st_at(j + 1, PF_HI_COUNT + order[e]));
       }
 #pragma unroll
-      for (int e = 0; e < 10; ++e) cpa4(S(slot, 17 + e), b_at(p, e));
+      for (int e = 0; e < 10; ++e) cpa4(S(slot, 17 + e), b_at(j, e));
     }
     cpa_commit();
   };
-  // back substitution step p (n-2 .. 1) consumes C'_p (the first pass's),
-  // r'_p, x0_p and u_p: words 0..24, 25..29, 30..34, 35..44 (u in two halves)
-  auto fetch_bwd = [&](int p, bool r_in_slot) {
-    const int slot = p % PIPE;
+  // back substitution step j consumes C'_j (the first pass's), r'_j, x0_j and
+  // u_j: words 0..24, 25..29, 30..34, 35..44 (u in two halves)
+  auto fetch_bwd = [&](int j, bool r_in_slot) {
+    const int slot = j % PIPE;
 #pragma unroll
     for (int e = 0; e < 30; ++e)
-      if (e < 25 || !r_in_slot) cpa4(S(slot, e), scr + ((int64_t)p * BT_SCR + e) * nlt + gl);
+      if (e < 25 || !r_in_slot) cpa4(S(slot, e), scr_at(j, e));
 #pragma unroll
-    for (int m = 0; m < 5; ++m) cpa4(S(slot, 30 + m), x0_at(p, m));
+    for (int m = 0; m < 5; ++m) cpa4(S(slot, 30 + m), x0_at(j, m));
     if (!OUT_DF && add_u) {
-      const float* up = reinterpret_cast<const float*>(F.u + base + (int64_t)p * st);
+      const float* up = reinterpret_cast<const float*>(F.u + h.pt(j));
 #pragma unroll
       for (int m = 0; m < 5; ++m) {
         cpa4(S(slot, 35 + 2 * m), up + 2 * m * NP);
@@ -1728,99 +1850,123 @@ __device__ __forceinline__ void bt_refine_pl_item(const Fields& F, const Consts&
       }
     }
   };
-
-  // the ring's first slots go out before the line's first points are read
-  // directly, so that the two memory latencies overlap
-#pragma unroll
-  for (int e = 0; e < 10; ++e) cpa4(S(PIPE, e), b_at(n - 1, e));
-#pragma unroll
-  for (int q = 1; q < PIPE; ++q) issue_fwd(q);
-  df64 acc_c[5], acc_n[5], xq[5], sq[6], P[5], Q[5];
+  const BtK<float> k = bt_half_consts<DIR>(K, h.far);
   BtF32Carry<DIR> c;
-  {
-    float s0[6], s1[6];
-    load_x(0, xq);
-    load_sdf(0, sq);
-    pq(sq, xq, P, Q);
+  float* ends = reinterpret_cast<float*>(pl_smem) + (size_t)PIPE * PL_REFINE_W * T;
+  if (h.active) {
+    // the ring's first slots (and x at a whole line's last point, b itself) go
+    // out before the line's first points are read directly, so that the
+    // memory latencies overlap
+    if (!TWO) {
 #pragma unroll
-    for (int m = 0; m < 5; ++m) acc_c[m] = df_neg(df_add(P[m], Q[m]));
-#pragma unroll
-    for (int e = 0; e < 6; ++e) s0[e] = sq[e].hi;
-    load_x(1, xq);
-    load_sdf(1, sq);
-    pq(sq, xq, P, Q);
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      acc_c[m] = df_add(acc_c[m], df_add(xq[m], df_scale2(Q[m])));
-      acc_n[m] = df_neg(df_add(P[m], Q[m]));
+      for (int e = 0; e < 10; ++e) cpa4(ends + e * T + threadIdx.x, b_at(h.n - 1, e));
     }
 #pragma unroll
-    for (int e = 0; e < 6; ++e) s1[e] = sq[e].hi;
+    for (int j = 1; j < PIPE; ++j) issue_fwd(j);
+    // partial sums of T x0: rows j and j + 1
+    df64 acc_c[5], acc_n[5], sq[6], P[5], Q[5];
+    {
+      float s0[6], s1[6];
+      df64 xe[5];
+      load_x(0, xe);
+      load_sdf(0, sq);
+      bt_pq<DIR>(kr, sq, xe, P, Q);
 #pragma unroll
-    for (int m = 0; m < 5; ++m) c.rp[m] = 0.f;
-    bt_f32_begin<DIR>(K, s0, s1, c);
+      for (int m = 0; m < 5; ++m) acc_c[m] = df_neg(du_add(P[m], Q[m]));
+#pragma unroll
+      for (int e = 0; e < 6; ++e) s0[e] = sq[e].hi;
+      load_x(1, xe);
+      load_sdf(1, sq);
+      bt_pq<DIR>(kr, sq, xe, P, Q);
+#pragma unroll
+      for (int m = 0; m < 5; ++m) {
+        acc_c[m] = du_add(acc_c[m], du_add(df_scale2(Q[m]), xe[m]));
+        acc_n[m] = df_neg(du_add(P[m], Q[m]));
+      }
+#pragma unroll
+      for (int e = 0; e < 6; ++e) s1[e] = sq[e].hi;
+#pragma unroll
+      for (int m = 0; m < 5; ++m) c.rp[m] = 0.f;
+      bt_f32_begin<DIR>(k, s0, s1, c);
+    }
+    for (int j = 1; j <= L; ++j) {
+      issue_fwd(j + PIPE - 1);
+      cpa_wait<PIPE - 1>();
+      const int slot = j % PIPE;
+      df64 bd[5];
+      float r[5], s[6];
+#pragma unroll
+      for (int e = 0; e < 6; ++e) sq[e] = df64{*S(slot, 5 + e), *S(slot, 11 + e)};
+#pragma unroll
+      for (int m = 0; m < 5; ++m) bd[m] = df64{*S(slot, 17 + m), *S(slot, 22 + m)};
+#pragma unroll
+      for (int e = 0; e < 6; ++e) s[e] = sq[e].hi;
+      if (j + 1 < h.n - 1) {
+        float xq[5];
+#pragma unroll
+        for (int m = 0; m < 5; ++m) xq[m] = *S(slot, m);
+        bt_pq<DIR>(kr, sq, xq, P, Q);
+#pragma unroll
+        for (int m = 0; m < 5; ++m) {
+          const df64 rr = du_sub(bd[m], du_add(acc_c[m], du_sub(P[m], Q[m])));
+          r[m] = rr.hi + rr.lo;
+          acc_c[m] = du_add(acc_n[m], du_add(df_scale2(Q[m]), xq[m]));
+          acc_n[m] = df_neg(du_add(P[m], Q[m]));
+        }
+      } else {  // the line's last point: completes the last row
+        df64 xe[5];
+        if (TWO) {  // a line of one row
+          load_x(j + 1, xe);
+        } else {
+#pragma unroll
+          for (int m = 0; m < 5; ++m) xe[m] = df64{ends[m * T + threadIdx.x], ends[(5 + m) * T + threadIdx.x]};
+        }
+        bt_pq<DIR>(kr, sq, xe, P, Q);
+#pragma unroll
+        for (int m = 0; m < 5; ++m) {
+          const df64 rr = du_sub(bd[m], du_add(acc_c[m], du_sub(P[m], Q[m])));
+          r[m] = rr.hi + rr.lo;
+        }
+      }
+      // the elimination runs again (its factors would be 25 more words to
+      // write and read, and the sweep is bound by memory); C' is the first
+      // pass's, so only r' is stored
+      bt_f32_step<DIR, false>(k, r, s, c, scr_at(j, 0), nlt);
+      if (j + PIPE > L) {
+        // the ring does not refill this slot: r'_j stays here for the back
+        // substitution, whose other operands are fetched now, so that it
+        // starts without a trip to memory
+#pragma unroll
+        for (int m = 0; m < 5; ++m) *S(slot, 25 + m) = r[m];
+        fetch_bwd(j, true);
+        cpa_commit();
+      }
+    }
   }
-  for (int p = 1; p <= n - 2; ++p) {
-    issue_fwd(p + PIPE - 1);
-    cpa_wait<PIPE - 1>();
-    const int slot = p % PIPE;
-    df64 bd[5];
-    if (p + 1 == n - 1) {
-#pragma unroll
-      for (int m = 0; m < 5; ++m) xq[m] = df64{*S(PIPE, m), *S(PIPE, 5 + m)};
-    } else {
-#pragma unroll
-      for (int m = 0; m < 5; ++m) xq[m] = df64{*S(slot, m), 0.f};
-    }
-#pragma unroll
-    for (int e = 0; e < 6; ++e) sq[e] = df64{*S(slot, 5 + e), *S(slot, 11 + e)};
-#pragma unroll
-    for (int m = 0; m < 5; ++m) bd[m] = df64{*S(slot, 17 + m), *S(slot, 22 + m)};
-    pq(sq, xq, P, Q);
-    float r[5], s[6];
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      const df64 tx = df_add(acc_c[m], df_sub(P[m], Q[m]));
-      const df64 rr = df_sub(bd[m], tx);
-      r[m] = rr.hi + rr.lo;
-      acc_c[m] = df_add(acc_n[m], df_add(xq[m], df_scale2(Q[m])));
-      acc_n[m] = df_neg(df_add(P[m], Q[m]));
-    }
-#pragma unroll
-    for (int e = 0; e < 6; ++e) s[e] = sq[e].hi;
-    // the elimination runs again (its factors do not fit beside C'); C' is the
-    // first pass's, so only r' is stored
-    bt_f32_step<DIR, false>(K, p, r, s, c, scr, nlt, gl);
-    if (p + PIPE > n - 2) {
-      // the ring does not refill this slot: r'_p stays here for the back
-      // substitution, whose other operands are fetched now, so that it starts
-      // without a trip to memory
-#pragma unroll
-      for (int m = 0; m < 5; ++m) *S(slot, 25 + m) = r[m];
-      fetch_bwd(p, true);
-      cpa_commit();
-    }
+  float dn[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+  if (TWO) {
+    bt_join(ends, h.far, c.Cp, c.rp, dn);
+    if (!h.active) return;
   }
   cpa_wait<0>();
-  // back substitution: step p (n-2 .. 1) from slot p % PIPE: the last PIPE
-  // points as the forward pass left them, the others fetched PIPE steps ahead
-  // into the slot just consumed
-  auto issue_bwd = [&](int p) {
-    if (p >= 1) fetch_bwd(p, false);
-    cpa_commit();
-  };
-  float dn[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int p = n - 2; p >= 1; --p) {
-    if (p + PIPE <= n - 2) cpa_wait<PIPE - 1>();
-    const int slot = p % PIPE;
-    const int64_t pt = base + (int64_t)p * st;
-    float d[5];
+  // back substitution (TWO: row L is the seam's): step j from slot
+  // j % PIPE: the last PIPE rows as the forward pass left them, the others
+  // fetched PIPE steps ahead into the slot just consumed
+  for (int j = L; j >= 1; --j) {
+    if (j + PIPE <= L) cpa_wait<PIPE - 1>();
+    const int slot = j % PIPE;
+    const int64_t pt = h.pt(j);
+    if (!TWO || j < L) {
+      float d[5];
 #pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      float t = *S(slot, 25 + m);
+      for (int m = 0; m < 5; ++m) {
+        float t = *S(slot, 25 + m);
 #pragma unroll
-      for (int cc = 0; cc < 5; ++cc) t -= *S(slot, m * 5 + cc) * dn[cc];
-      d[m] = t;
+        for (int cc = 0; cc < 5; ++cc) t -= *S(slot, m * 5 + cc) * dn[cc];
+        d[m] = t;
+      }
+#pragma unroll
+      for (int m = 0; m < 5; ++m) dn[m] = d[m];
     }
 #pragma unroll
     for (int m = 0; m < 5; ++m) {
@@ -1828,32 +1974,30 @@ __device__ __forceinline__ void bt_refine_pl_item(const Fields& F, const Consts&
       if (OUT_DF) {
         // x: in place of b in the x-line-major copy (k_xline_back moves it
         // to rdf); y: rdf
-        const df64 v = df_two_sum(xv, d[m]);
-        float* o = DIR == 0 ? F.rdx + ((int64_t)p * 10 + m) * F.nlx + gl : bdf + m * NP + pt;
-        const int64_t lo_off = DIR == 0 ? 5 * F.nlx : 5 * NP;
-        o[0] = v.hi;
-        o[lo_off] = v.lo;
+        const df64 v = df_two_sum(xv, dn[m]);
+        *b_at(j, m) = v.hi;
+        *b_at(j, 5 + m) = v.lo;
       } else {
         // exact FP32 -> FP64 by bits (a conversion instruction takes the FP64 pipe)
-        const double v = f32_to_f64(xv) + f32_to_f64(d[m]);
+        const double v = f32_to_f64(xv) + f32_to_f64(dn[m]);
         rhs[m * NP + pt] = v;
         if (add_u)
           F.u[m * NP + pt] = __hiloint2double(__float_as_int(*S(slot, 36 + 2 * m)), __float_as_int(*S(slot, 35 + 2 * m))) + v;
       }
-      dn[m] = d[m];
     }
-    issue_bwd(p - PIPE);
+    if (j - PIPE >= 1) fetch_bwd(j - PIPE, false);
+    cpa_commit();
   }
   cpa_wait<0>();
 }
 
-template <int DIR, bool OUT_DF>
-__global__ void __launch_bounds__(128, NPBMZ_BT_REFINE_MINB) k_bt_refine_pl(Fields F, Consts K, const Work* __restrict__ work, int nwork,
+template <int DIR, bool OUT_DF, bool TWO>
+__global__ void __launch_bounds__(TWO ? 256 : 128, NPBMZ_BT_REFINE_MINB) k_bt_refine_pl(Fields F, Consts K, const Work* __restrict__ work, int nwork,
                                                       float* __restrict__ scr, int64_t nlt, int add_u,
                                                       const float* __restrict__ x0f) {
   extern __shared__ __align__(16) unsigned char pl_smem[];
   for (int it = blockIdx.x; it < nwork; it += gridDim.x)
-    bt_refine_pl_item<DIR, OUT_DF>(F, K, work[it], scr, nlt, add_u, x0f, pl_smem);
+    bt_refine_pl_item<DIR, OUT_DF, TWO>(F, K, work[it], scr, nlt, add_u, x0f, pl_smem);
 }
 #endif  // NPBMZ_HAS_FP32
 
@@ -2516,7 +2660,8 @@ static void launch_solve_t(bool sp, int dir, const Fields& F, const Consts& K, c
   }
 }
 
-// mode 0: FP64 in place (5: BT, six lanes per line); 1: FP32 in place; 2: FP32 + refinement with a
+// mode 4: one fused refined FP32 step (6: BT, two threads per line); mode 0:
+// FP64 in place (5: BT, six lanes per line); 1: FP32 in place; 2: FP32 + refinement with a
 // double-float residual (BT; SP: FP64 residual); 3: FP32 + refinement with
 // an FP64 residual (xw: a [5][NP] buffer for the first solution).
 void launch_solve(bool sp, int mode, int dir, const Fields& F, const Consts& K, const Work* work, int nwork, int tpb,
@@ -2547,27 +2692,34 @@ void launch_solve(bool sp, int mode, int dir, const Fields& F, const Consts& K, 
 #undef NPBMZ_SPL
     return;
   }
-  if (mode == 4 && !sp) {
+  if ((mode == 4 || mode == 6) && !sp) {
     // one fused step: b of the x sweep comes from compute_rhs's double-float
     // copy, x and y hand their results on as double-float (x through its
     // x-line-major copy), z writes FP64 rhs (and u)
     float* scr = reinterpret_cast<float*>(scratch);
     float* x0 = reinterpret_cast<float*>(xw);
-    const size_t sm_m = pl_mixed_smem(tpb), sm_r = pl_refine_smem(tpb);
-#define NPBMZ_PL(D, OD)                                                                                          \
-  do {                                                                                                           \
-    k_bt_mixed_pl<D><<<item_grid((const void*)k_bt_mixed_pl<D>, nwork, tpb, sm_m, persist, ctas_per_sm), tpb,     \
-                       sm_m, s>>>(                                                                                \
-        F, K, work, nwork, scr, nlt, x0);                                                                        \
-    k_bt_refine_pl<D, OD><<<item_grid((const void*)k_bt_refine_pl<D, OD>, nwork, tpb, sm_r, persist, ctas_per_sm), \
-                            tpb, sm_r,                                                                            \
-                            s>>>(F, K, work, nwork, scr, nlt, add_u, x0);                                        \
+    const bool two = mode == 6;
+    const int thr = two ? 2 * tpb : tpb;
+    const size_t sm_m = pl_mixed_smem(tpb, two), sm_r = pl_refine_smem(tpb, two);
+#define NPBMZ_PL(D, OD, TW)                                                                                          \
+  do {                                                                                                               \
+    k_bt_mixed_pl<D, TW><<<item_grid((const void*)k_bt_mixed_pl<D, TW>, nwork, thr, sm_m, persist, ctas_per_sm), thr, \
+                           sm_m, s>>>(F, K, work, nwork, scr, nlt, x0);                                              \
+    k_bt_refine_pl<D, OD, TW><<<item_grid((const void*)k_bt_refine_pl<D, OD, TW>, nwork, thr, sm_r, persist,         \
+                                          ctas_per_sm),                                                              \
+                                thr, sm_r, s>>>(F, K, work, nwork, scr, nlt, add_u, x0);                             \
   } while (0)
     if (dir == 0) {
-      NPBMZ_PL(0, true);
+      if (two) NPBMZ_PL(0, true, true);
+      else NPBMZ_PL(0, true, false);
       k_xline_back<<<nwork, 256, 0, s>>>(F, work, nwork, tpb);
-    } else if (dir == 1) NPBMZ_PL(1, true);
-    else NPBMZ_PL(2, false);
+    } else if (dir == 1) {
+      if (two) NPBMZ_PL(1, true, true);
+      else NPBMZ_PL(1, true, false);
+    } else {
+      if (two) NPBMZ_PL(2, false, true);
+      else NPBMZ_PL(2, false, false);
+    }
 #undef NPBMZ_PL
     return;
   }
@@ -2626,8 +2778,8 @@ void launch_solve(bool sp, int mode, int dir, const Fields& F, const Consts& K, 
 // Opt the pipelined sweeps into their dynamic shared memory (above 48 KB for
 // 128 threads per CTA); called once per handle, outside any stream capture.
 int configure_kernels() {
-  size_t cap_b = pl_refine_smem(128);
-  for (size_t b : {pl_mixed_smem(128), pls_mixed_smem(128), pls_refine_smem(128, false)})
+  size_t cap_b = pl_refine_smem(128, true);
+  for (size_t b : {pl_mixed_smem(128, true), pls_mixed_smem(128), pls_refine_smem(128, false)})
     if (b > cap_b) cap_b = b;
   const int cap = (int)cap_b;
   cudaError_t e = cudaSuccess;
@@ -2635,12 +2787,18 @@ int configure_kernels() {
     const cudaError_t r = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
     if (r != cudaSuccess) e = r;
   };
-  set((const void*)k_bt_mixed_pl<0>);
-  set((const void*)k_bt_mixed_pl<1>);
-  set((const void*)k_bt_mixed_pl<2>);
-  set((const void*)k_bt_refine_pl<0, true>);
-  set((const void*)k_bt_refine_pl<1, true>);
-  set((const void*)k_bt_refine_pl<2, false>);
+  set((const void*)k_bt_mixed_pl<0, false>);
+  set((const void*)k_bt_mixed_pl<0, true>);
+  set((const void*)k_bt_mixed_pl<1, false>);
+  set((const void*)k_bt_mixed_pl<1, true>);
+  set((const void*)k_bt_mixed_pl<2, false>);
+  set((const void*)k_bt_mixed_pl<2, true>);
+  set((const void*)k_bt_refine_pl<0, true, false>);
+  set((const void*)k_bt_refine_pl<0, true, true>);
+  set((const void*)k_bt_refine_pl<1, true, false>);
+  set((const void*)k_bt_refine_pl<1, true, true>);
+  set((const void*)k_bt_refine_pl<2, false, false>);
+  set((const void*)k_bt_refine_pl<2, false, true>);
   set((const void*)k_sp_mixed_pl<0>);
   set((const void*)k_sp_mixed_pl<1>);
   set((const void*)k_sp_mixed_pl<2>);

@@ -169,6 +169,18 @@ def test_bt_fused_mixed_steps_at_small_and_ragged_sizes(oracle_mod, nz):
     compare(p, o, npbmz.U, 1e-10)
 
 
+def test_bt_fused_mixed_steps_many_ragged_zones(oracle_mod):
+    """The same with enough lines that every sweep takes one thread per line
+    (the smaller problems take two)."""
+    w = [5, 6, 7, 8, 9, 11, 13, 17, 5, 6, 7, 10, 19, 23, 34, 35]
+    nx, ny, nzs, nbr = npbmz.zones_from_widths(w, w[::-1], 9)
+    geom = npbmz.Geometry(npbmz.BT, nx, ny, nzs, nbr, sum(w), sum(w), 9, 16, 16)
+    p, o = make_pair(oracle_mod, geom, 0.0003, npbmz.MIXED | npbmz.GRAPH, npbmz.CE_REFERENCE)
+    p.step(3)
+    o.step(3)
+    compare(p, o, npbmz.U, 1e-10)
+
+
 DF_RHS_REL = 1e-12   # compute_rhs in double-float (FP32 pairs, about 48 bits)
 
 
