@@ -55,9 +55,9 @@ WORKLOADS = {
 # point of the zones): jac reads u and 1/u1 (48 B) and writes 107 planes of
 # blocks and factors per interior point (856 B); the sweeps read rsd and the
 # 62 planes of their direction (rsd in, rsd out: 80 B + 496 B); rhs reads u,
-# frct and ten planes of flux quantities and writes rsd (200 B); update reads
-# u and rsd and writes u and the flux quantities (200 B).
-LU_BYTES_PER_POINT = {"jac": 904.0, "lower": 576.0, "upper": 576.0, "rhs": 200.0, "update": 200.0, "exch": 0.0}
+# frct and 18 planes of flux quantities and writes rsd (264 B); update reads
+# u and rsd and writes u and the flux quantities (264 B).
+LU_BYTES_PER_POINT = {"jac": 904.0, "lower": 576.0, "upper": 576.0, "rhs": 264.0, "update": 264.0, "exch": 0.0}
 LU_KERNELS = {"jac": "k_lu_jac", "lower": "k_lu_sweep<0, 1>", "upper": "k_lu_sweep<1, 0>", "rhs": "k_lu_rhs<0>",
               "update": "k_lu_pointwise<1>", "exch": "k_lu_pack+k_lu_unpack"}
 SEED = 20261203

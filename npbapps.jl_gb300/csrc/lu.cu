@@ -16,7 +16,7 @@
 //   Jacobians      k_lu_jac: jacld's and jacu's off-diagonal blocks and the
 //                  factors of d at every point, fully parallel
 //   flux prims     per-point quantities of the flux functions (1/u1, the
-//                  viscous u21.., the convective u21 and q), refreshed where
+//                  viscous u21.., the convective fluxes), refreshed where
 //                  u changes: k_lu_unpack (ghost faces), k_lu_pointwise<1>
 //                  (update), uploads; read by the sweeps and rhs
 //   blts           k_lu_sweep<false>, one launch per hyperplane i+j+k = l,
@@ -197,10 +197,8 @@ int launch_jac(npbmz_lu_t* h, int z0, int nzs) {
     maxnp = std::max(maxnp, h->zh[z].np);
   }
   const dim3 g((maxnp + TPB - 1) / TPB, nzs);
-  // thread order: hyperplane order (coalesced block writes) for the FMA
-  // build, natural order (coalesced state reads) for the FP64-bound exact one
-  (h->fast ? lu_fast::jac : lu_exact::jac)(h->fast, dev(h), h->fb_d, h->fb_ls, h->ri_d, h->hstride, h->ri_ks, h->fac,
-                                          z0, g, h->stream);
+  (h->fast ? lu_fast::jac : lu_exact::jac)(dev(h), h->fb_d, h->fb_ls, h->ri_d, h->hstride, h->ri_ks, h->fac, z0, g,
+                                          h->stream);
   LU_CK(h, cudaGetLastError());
   return 0;
 }

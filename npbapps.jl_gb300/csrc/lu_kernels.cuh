@@ -34,7 +34,26 @@ __device__ inline double visc_up(double o, double a, double b) {
   return ERHS ? (o + a) + b : o + (a + b);
 }
 
-__device__ __forceinline__ void prim_point(const double g[5], double pr[PR_COUNT]) {
+// v / t from y = 1/t rounded to nearest: the quotient estimate v y, refined by
+// its FMA residuals (P. Markstein, IBM J. Res. Dev. 34(1), 1990: one step from
+// an estimate within one ulp, with the correctly rounded reciprocal, gives the
+// correctly rounded quotient; the first step here makes the estimate so).  A
+// dependent divide costs nine FP64 instructions where this takes five, and
+// the FP64 pipe binds the sweeps.  Operands whose residual could underflow or
+// overflow take the divide.
+__device__ __forceinline__ double div_y(double v, double t, double y) {
+  const unsigned ev = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu, et = ((unsigned)__double2hiint(t) >> 20) & 0x7ffu;
+  // exponents of v in [2^-600, 2^600) and of t in [2^-300, 2^300): v, t, y, q and every residual are normal
+  if (__builtin_expect(ev - 423u < 1200u && et - 723u < 600u, 1)) {
+    double q = v * y;
+    q = fma(fma(-t, q, v), y, q);
+    return fma(fma(-t, q, v), y, q);
+  }
+  return v / t;
+}
+
+// The flux quantities of one point; returns q.
+__device__ __forceinline__ double prim_point(const double g[5], double pr[PR_COUNT]) {
   const double tmp = 1.0e+00 / g[0];
   pr[PR_RHO] = tmp;
   pr[PR_U21] = tmp * g[1];
@@ -42,10 +61,20 @@ __device__ __forceinline__ void prim_point(const double g[5], double pr[PR_COUNT
   pr[PR_U41] = tmp * g[3];
   pr[PR_U51] = tmp * g[4];
   pr[PR_S] = pr[PR_U21] * pr[PR_U21] + pr[PR_U31] * pr[PR_U31] + pr[PR_U41] * pr[PR_U41];
-  pr[PR_C21] = g[1] / g[0];
-  pr[PR_C31] = g[2] / g[0];
-  pr[PR_C41] = g[3] / g[0];
-  pr[PR_Q] = 0.50e+00 * (g[1] * g[1] + g[2] * g[2] + g[3] * g[3]) / g[0];
+  const double u21 = div_y(g[1], g[0], tmp), u31 = div_y(g[2], g[0], tmp), u41 = div_y(g[3], g[0], tmp);
+  const double q = div_y(0.50e+00 * (g[1] * g[1] + g[2] * g[2] + g[3] * g[3]), g[0], tmp);
+  const double pres = c2 * (g[4] - q), h = c1 * g[4] - c2 * q;
+  const double vel[3] = {u21, u31, u41};
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      const double f = g[m + 1] * vel[d];
+      pr[PR_F + 4 * d + m] = m == d ? f + pres : f;
+    }
+    pr[PR_F + 4 * d + 3] = h * vel[d];
+  }
+  return q;
 }
 
 __device__ __forceinline__ void store_prim(double* prim, long long NP, long long p, const double g[5]) {
@@ -55,149 +84,82 @@ __device__ __forceinline__ void store_prim(double* prim, long long NP, long long
   for (int q = 0; q < PR_COUNT; ++q) prim[q * NP + p] = pr[q];
 }
 
+// Products with 2, 4 and dssp = 1/4 are exact, so fma rounds them and the sum
+// once, as the separate operations do: the second differences and the
+// fourth-difference dissipation take an FP64 instruction less for each.
+static_assert(dssp == 0.25, "the dissipation's fma needs a power of two");
+
+// o - dssp times the fourth difference of u at position q (1-based, 2..n-1) of
+// an axis of n >= 6 points: the reference's start, middle and end stencils are
+// the middle one, whose missing terms enter as zeros (x - 0 and 0 + x are x),
+// with 5 instead of 6 at the centre of the outermost two; no lane diverges.
+__device__ __forceinline__ double dissip(double o, int q, int n, double um2, double um1, double u0, double up1,
+                                         double up2) {
+  const double a = q >= 4 ? um2 : 0.0, b = q >= 3 ? um1 : 0.0, d = q <= n - 2 ? up1 : 0.0, e = q <= n - 3 ? up2 : 0.0;
+  const double w = q == 2 || q == n - 1 ? 5.0e+00 : 6.0e+00;
+  return fma(-dssp, fma(-4.0e+00, d, fma(-4.0e+00, b, a) + w * u0) + e, o);
+}
+// The same on an axis of 5 points, where two stencils apply at the middle one.
+__device__ __noinline__ double dissip5(double o, int q, double um2, double um1, double u0, double up1, double up2) {
+  if (q == 2) o = o - dssp * (+5.0e+00 * u0 - 4.0e+00 * up1 + up2);
+  if (q == 3) o = o - dssp * (-4.0e+00 * um1 + 6.0e+00 * u0 - 4.0e+00 * up1 + up2);
+  if (q == 3) o = o - dssp * (um2 - 4.0e+00 * um1 + 6.0e+00 * u0 - 4.0e+00 * up1);
+  if (q == 4) o = o - dssp * (um2 - 4.0e+00 * um1 + 5.0e+00 * u0);
+  return o;
+}
+
+// One direction of the operator at point p (position q of an axis of n points,
+// stride st): the reference's statements, in their order.
+template <bool ERHS, int D>
+__device__ __forceinline__ void flux_dir(const double* __restrict__ g, const double* __restrict__ prim, long long NP,
+                                         long long p, long long st, int q, int n, double t1, double t2, double t3,
+                                         double d1, double o[5]) {
+  const long long a = p + st, b = p - st;
+  // convective flux
+  o[0] = o[0] - t2 * (g[(D + 1) * NP + a] - g[(D + 1) * NP + b]);
+#pragma unroll
+  for (int m = 1; m < 5; ++m) {
+    const double* f = prim + (PR_F + 4 * D + m - 1) * NP;
+    o[m] = o[m] - t2 * (f[a] - f[b]);
+  }
+  // viscous fluxes between the point and its neighbours
+  auto visc = [&](long long hi, long long lo, double f[5]) {
+#pragma unroll
+    for (int m = 0; m < 3; ++m)
+      f[m + 1] = (D == m ? (4.0e+00 / 3.0e+00) * t3 : t3) * (prim[(PR_U21 + m) * NP + hi] - prim[(PR_U21 + m) * NP + lo]);
+    const double ui = prim[(PR_U21 + D) * NP + hi], um = prim[(PR_U21 + D) * NP + lo];
+    f[4] = 0.50e+00 * (1.0e+00 - c1 * c5) * t3 * (prim[PR_S * NP + hi] - prim[PR_S * NP + lo]) +
+           (1.0e+00 / 6.0e+00) * t3 * (ui * ui - um * um) +
+           c1 * c5 * t3 * (prim[PR_U51 * NP + hi] - prim[PR_U51 * NP + lo]);
+  };
+  double fp[5], fm[5];
+  visc(a, p, fp);
+  visc(p, b, fm);
+  // second difference: x and y take g(-1) first; z too in rhs, g(+1) in erhs
+  auto second = [&](int m) {
+    const double* u = g + m * NP;
+    const double x = D == 2 && ERHS ? u[a] : u[b], y = D == 2 && ERHS ? u[b] : u[a];
+    return fma(-2.0e+00, u[p], x) + y;
+  };
+  o[0] = o[0] + d1 * t1 * second(0);
+#pragma unroll
+  for (int m = 1; m < 5; ++m) o[m] = visc_up<ERHS>(o[m], t3 * c3 * c4 * (fp[m] - fm[m]), d1 * t1 * second(m));
+  const long long p2 = q <= n - 2 ? a + st : p, m2 = q >= 3 ? b - st : p;
+#pragma unroll
+  for (int m = 0; m < 5; ++m) {
+    const double* u = g + m * NP;
+    o[m] = n == 5 ? dissip5(o[m], q, u[m2], u[b], u[p], u[a], u[p2]) : dissip(o[m], q, n, u[m2], u[b], u[p], u[a], u[p2]);
+  }
+}
+
 template <bool ERHS>
-__device__ void flux_point(const double* __restrict__ g, const double* __restrict__ prim, long long NP,
-                           const LuZone& Z, int i, int j, int k, double o[5]) {
-  const int nx = Z.nx, ny = Z.ny, nz = Z.nz;
-  auto G = [&](int m, int ii, int jj, int kk) -> double { return g[m * NP + pidx(Z, ii, jj, kk)]; };
-  auto P = [&](int q, int ii, int jj, int kk) -> double { return prim[q * NP + pidx(Z, ii, jj, kk)]; };
-  const double tx1 = Z.tx1, tx2 = Z.tx2, tx3 = Z.tx3, ty1 = Z.ty1, ty2 = Z.ty2, ty3 = Z.ty3, tz1 = Z.tz1,
-               tz2 = Z.tz2, tz3 = Z.tz3;
-  // convective flux of direction D (0 x, 1 y, 2 z) at a point
-  auto conv = [&](int D, int ii, int jj, int kk, double f[5]) {
-    const double g2 = G(1, ii, jj, kk), g3 = G(2, ii, jj, kk), g4 = G(3, ii, jj, kk), g5 = G(4, ii, jj, kk);
-    const double q = P(PR_Q, ii, jj, kk);
-    if (D == 0) {
-      const double u21 = P(PR_C21, ii, jj, kk);
-      f[0] = g2;
-      f[1] = g2 * u21 + c2 * (g5 - q);
-      f[2] = g3 * u21;
-      f[3] = g4 * u21;
-      f[4] = (c1 * g5 - c2 * q) * u21;
-    } else if (D == 1) {
-      const double u31 = P(PR_C31, ii, jj, kk);
-      f[0] = g3;
-      f[1] = g2 * u31;
-      f[2] = g3 * u31 + c2 * (g5 - q);
-      f[3] = g4 * u31;
-      f[4] = (c1 * g5 - c2 * q) * u31;
-    } else {
-      const double u41 = P(PR_C41, ii, jj, kk);
-      f[0] = g4;
-      f[1] = g2 * u41;
-      f[2] = g3 * u41;
-      f[3] = g4 * u41 + c2 * (g5 - q);
-      f[4] = (c1 * g5 - c2 * q) * u41;
-    }
-  };
-  // viscous flux of direction D between point b (the - side) and point a
-  auto visc = [&](int D, double t3, int ai, int aj, int ak, int bi, int bj, int bk, double f[5]) {
-    const double u21i = P(PR_U21, ai, aj, ak), u31i = P(PR_U31, ai, aj, ak), u41i = P(PR_U41, ai, aj, ak),
-                 u51i = P(PR_U51, ai, aj, ak), si = P(PR_S, ai, aj, ak);
-    const double u21m = P(PR_U21, bi, bj, bk), u31m = P(PR_U31, bi, bj, bk), u41m = P(PR_U41, bi, bj, bk),
-                 u51m = P(PR_U51, bi, bj, bk), sm = P(PR_S, bi, bj, bk);
-    f[1] = (D == 0 ? (4.0e+00 / 3.0e+00) * t3 : t3) * (u21i - u21m);
-    f[2] = (D == 1 ? (4.0e+00 / 3.0e+00) * t3 : t3) * (u31i - u31m);
-    f[3] = (D == 2 ? (4.0e+00 / 3.0e+00) * t3 : t3) * (u41i - u41m);
-    const double ui = D == 0 ? u21i : (D == 1 ? u31i : u41i), um = D == 0 ? u21m : (D == 1 ? u31m : u41m);
-    f[4] = 0.50e+00 * (1.0e+00 - c1 * c5) * t3 * (si - sm) + (1.0e+00 / 6.0e+00) * t3 * (ui * ui - um * um) +
-           c1 * c5 * t3 * (u51i - u51m);
-  };
-  // ---------------- xi ----------------
-  {
-    double fp[5], fm[5];
-    conv(0, i + 1, j, k, fp);
-    conv(0, i - 1, j, k, fm);
-#pragma unroll
-    for (int m = 0; m < 5; ++m) o[m] = o[m] - tx2 * (fp[m] - fm[m]);
-    visc(0, tx3, i + 1, j, k, i, j, k, fp);
-    visc(0, tx3, i, j, k, i - 1, j, k, fm);
-    o[0] = o[0] + dx1 * tx1 * (G(0, i - 1, j, k) - 2.0e+00 * G(0, i, j, k) + G(0, i + 1, j, k));
-    const double dxm[5] = {dx1, dx2, dx3, dx4, dx5};
-#pragma unroll
-    for (int m = 1; m < 5; ++m)
-      o[m] = visc_up<ERHS>(o[m], tx3 * c3 * c4 * (fp[m] - fm[m]),
-                           dxm[m] * tx1 * (G(m, i - 1, j, k) - 2.0e+00 * G(m, i, j, k) + G(m, i + 1, j, k)));
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      if (i == 2) o[m] = o[m] - dssp * (+5.0e+00 * G(m, 2, j, k) - 4.0e+00 * G(m, 3, j, k) + G(m, 4, j, k));
-      if (i == 3)
-        o[m] = o[m] - dssp * (-4.0e+00 * G(m, 2, j, k) + 6.0e+00 * G(m, 3, j, k) - 4.0e+00 * G(m, 4, j, k) +
-                              G(m, 5, j, k));
-      if (i >= 4 && i <= nx - 3)
-        o[m] = o[m] - dssp * (G(m, i - 2, j, k) - 4.0e+00 * G(m, i - 1, j, k) + 6.0e+00 * G(m, i, j, k) -
-                              4.0e+00 * G(m, i + 1, j, k) + G(m, i + 2, j, k));
-      if (i == nx - 2)
-        o[m] = o[m] - dssp * (G(m, nx - 4, j, k) - 4.0e+00 * G(m, nx - 3, j, k) + 6.0e+00 * G(m, nx - 2, j, k) -
-                              4.0e+00 * G(m, nx - 1, j, k));
-      if (i == nx - 1)
-        o[m] = o[m] - dssp * (G(m, nx - 3, j, k) - 4.0e+00 * G(m, nx - 2, j, k) + 5.0e+00 * G(m, nx - 1, j, k));
-    }
-  }
-  // ---------------- eta ----------------
-  {
-    double fp[5], fm[5];
-    conv(1, i, j + 1, k, fp);
-    conv(1, i, j - 1, k, fm);
-#pragma unroll
-    for (int m = 0; m < 5; ++m) o[m] = o[m] - ty2 * (fp[m] - fm[m]);
-    visc(1, ty3, i, j + 1, k, i, j, k, fp);
-    visc(1, ty3, i, j, k, i, j - 1, k, fm);
-    o[0] = o[0] + dy1 * ty1 * (G(0, i, j - 1, k) - 2.0e+00 * G(0, i, j, k) + G(0, i, j + 1, k));
-    const double dym[5] = {dy1, dy2, dy3, dy4, dy5};
-#pragma unroll
-    for (int m = 1; m < 5; ++m)
-      o[m] = visc_up<ERHS>(o[m], ty3 * c3 * c4 * (fp[m] - fm[m]),
-                           dym[m] * ty1 * (G(m, i, j - 1, k) - 2.0e+00 * G(m, i, j, k) + G(m, i, j + 1, k)));
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      if (j == 2) o[m] = o[m] - dssp * (+5.0e+00 * G(m, i, 2, k) - 4.0e+00 * G(m, i, 3, k) + G(m, i, 4, k));
-      if (j == 3)
-        o[m] = o[m] - dssp * (-4.0e+00 * G(m, i, 2, k) + 6.0e+00 * G(m, i, 3, k) - 4.0e+00 * G(m, i, 4, k) +
-                              G(m, i, 5, k));
-      if (j >= 4 && j <= ny - 3)
-        o[m] = o[m] - dssp * (G(m, i, j - 2, k) - 4.0e+00 * G(m, i, j - 1, k) + 6.0e+00 * G(m, i, j, k) -
-                              4.0e+00 * G(m, i, j + 1, k) + G(m, i, j + 2, k));
-      if (j == ny - 2)
-        o[m] = o[m] - dssp * (G(m, i, ny - 4, k) - 4.0e+00 * G(m, i, ny - 3, k) + 6.0e+00 * G(m, i, ny - 2, k) -
-                              4.0e+00 * G(m, i, ny - 1, k));
-      if (j == ny - 1)
-        o[m] = o[m] - dssp * (G(m, i, ny - 3, k) - 4.0e+00 * G(m, i, ny - 2, k) + 5.0e+00 * G(m, i, ny - 1, k));
-    }
-  }
-  // ---------------- zeta ----------------
-  {
-    double fp[5], fm[5];
-    conv(2, i, j, k + 1, fp);
-    conv(2, i, j, k - 1, fm);
-#pragma unroll
-    for (int m = 0; m < 5; ++m) o[m] = o[m] - tz2 * (fp[m] - fm[m]);
-    visc(2, tz3, i, j, k + 1, i, j, k, fp);
-    visc(2, tz3, i, j, k, i, j, k - 1, fm);
-    auto sd = [&](int m) {
-      return ERHS ? (G(m, i, j, k + 1) - 2.0e+00 * G(m, i, j, k) + G(m, i, j, k - 1))
-                  : (G(m, i, j, k - 1) - 2.0e+00 * G(m, i, j, k) + G(m, i, j, k + 1));
-    };
-    o[0] = o[0] + dz1 * tz1 * sd(0);
-    const double dzm[5] = {dz1, dz2, dz3, dz4, dz5};
-#pragma unroll
-    for (int m = 1; m < 5; ++m) o[m] = visc_up<ERHS>(o[m], tz3 * c3 * c4 * (fp[m] - fm[m]), dzm[m] * tz1 * sd(m));
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      if (k == 2) o[m] = o[m] - dssp * (+5.0e+00 * G(m, i, j, 2) - 4.0e+00 * G(m, i, j, 3) + G(m, i, j, 4));
-      if (k == 3)
-        o[m] = o[m] - dssp * (-4.0e+00 * G(m, i, j, 2) + 6.0e+00 * G(m, i, j, 3) - 4.0e+00 * G(m, i, j, 4) +
-                              G(m, i, j, 5));
-      if (k >= 4 && k <= nz - 3)
-        o[m] = o[m] - dssp * (G(m, i, j, k - 2) - 4.0e+00 * G(m, i, j, k - 1) + 6.0e+00 * G(m, i, j, k) -
-                              4.0e+00 * G(m, i, j, k + 1) + G(m, i, j, k + 2));
-      if (k == nz - 2)
-        o[m] = o[m] - dssp * (G(m, i, j, nz - 4) - 4.0e+00 * G(m, i, j, nz - 3) + 6.0e+00 * G(m, i, j, nz - 2) -
-                              4.0e+00 * G(m, i, j, nz - 1));
-      if (k == nz - 1)
-        o[m] = o[m] - dssp * (G(m, i, j, nz - 3) - 4.0e+00 * G(m, i, j, nz - 2) + 5.0e+00 * G(m, i, j, nz - 1));
-    }
-  }
+__device__ __forceinline__ void flux_point(const double* __restrict__ g, const double* __restrict__ prim, long long NP,
+                                           const LuZone& Z, int i, int j, int k, double o[5]) {
+  static_assert(dx1 == dx5 && dy1 == dy5 && dz1 == dz5, "one factor per direction");
+  const long long p = pidx(Z, i, j, k);
+  flux_dir<ERHS, 0>(g, prim, NP, p, 1, i, Z.nx, Z.tx1, Z.tx2, Z.tx3, dx1, o);
+  flux_dir<ERHS, 1>(g, prim, NP, p, Z.nx, j, Z.ny, Z.ty1, Z.ty2, Z.ty3, dy1, o);
+  flux_dir<ERHS, 2>(g, prim, NP, p, (long long)Z.nx * Z.ny, k, Z.nz, Z.tz1, Z.tz2, Z.tz3, dz1, o);
 }
 
 __device__ inline bool decode(const LuZone& Z, int q, int& i, int& j, int& k) {
@@ -212,6 +174,10 @@ __device__ inline bool interior(const LuZone& Z, int i, int j, int k) {
   return i >= 2 && i <= Z.nx - 1 && j >= 2 && j <= Z.ny - 1 && k >= 2 && k <= Z.nz - 1;
 }
 
+// Bound by the FP64 pipe: about 330 FP64 instructions a point without
+// contraction (444 with the convective fluxes formed at every neighbour, the
+// products with 2, 4 and 1/4 apart, and a divergent branch per stencil).
+// 480x320x28: 5.00 -> 2.58 ms; contracted 3.2 -> 1.98 ms.
 // rhs (ERHS = false: g = u, out = rsd starting at -frct) or erhs's flux part
 // (ERHS = true: g = the exact polynomial in rsd, out = frct starting at 0)
 template <bool ERHS>
@@ -302,12 +268,12 @@ __global__ void __launch_bounds__(TPB) k_lu_pointwise(LuDev D, const LuWork* __r
       D.u[m * D.NP + p] = g[m];
     }
     double pr[PR_COUNT];
-    prim_point(g, pr);
+    const double qk = prim_point(g, pr);
 #pragma unroll
     for (int q = 0; q < PR_COUNT; ++q) D.prim[q * D.NP + p] = pr[q];
     if (D.health) {
       // on the bit patterns (integer pipe): positive and finite
-      const double pres = g[4] - pr[PR_Q];
+      const double pres = g[4] - qk;
       const unsigned long long br = (unsigned long long)__double_as_longlong(g[0]);
       const unsigned long long bp = (unsigned long long)__double_as_longlong(pres);
       const bool rho_ok = br - 1ull < 0x7FEFFFFFFFFFFFFFull, p_ok = bp - 1ull < 0x7FEFFFFFFFFFFFFFull;
@@ -377,211 +343,95 @@ __device__ __forceinline__ void jac_d(const JC& J, double r1, double u2, double 
             dt * 2.0e+00 * (tx1 * dx5 + ty1 * dy5 + tz1 * dz5);
 }
 
-// Off-diagonal block of direction DIR (0 x, 1 y, 2 z) from the neighbour's
-// state; SG = -1: jacld's (the neighbour at -1), SG = +1: jacu's (at +1).
-// The entries are the reference's statements.  r1 = 1/u1 of the neighbour
-// (the reference's tmp1: the PR_RHO plane).
-template <int DIR, int SG>
+// The state-dependent entries of jacld's (lo: the block the point at +1 in DIR
+// reads) and jacu's (up: the point at -1) off-diagonal blocks of direction
+// DIR (0 x, 1 y, 2 z) from one point's state; r1 = 1/u1 (the reference's tmp1:
+// the PR_RHO plane).  The entries are the reference's statements; jacld's
+// differ from jacu's in the sign of the convective term, their first, alone,
+// so each term is formed once and the two entries are its sums: about 95 FP64
+// operations a direction.
+template <int DIR>
 __device__ __forceinline__ void jac_off(const JC& J, double r1, double u2, double u3, double u4, double u5,
-                                        double a[5][5]) {
+                                        double lo[5][5], double up[5][5]) {
   const double dt = J.dt;
   const double tmp1 = r1, tmp2 = tmp1 * tmp1, tmp3 = tmp1 * tmp2;
+#define NPBMZ_LU_OFF(r, c, P, rest) \
+  {                                 \
+    const double conv = P;          \
+    lo[r][c] = -conv rest;          \
+    up[r][c] = conv rest;           \
+  }
   if (DIR == 2) {
     const double tz1 = J.tz1, tz2 = J.tz2;
-    if (SG < 0) {
-      a[0][0] = -dt * tz1 * dz1;
-      a[0][1] = 0.0;
-      a[0][2] = 0.0;
-      a[0][3] = -dt * tz2;
-      a[0][4] = 0.0;
-      a[1][0] = -dt * tz2 * (-(u2 * u4) * tmp2) - dt * tz1 * (-c34 * tmp2 * u2);
-      a[1][1] = -dt * tz2 * (u4 * tmp1) - dt * tz1 * c34 * tmp1 - dt * tz1 * dz2;
-      a[1][2] = 0.0;
-      a[1][3] = -dt * tz2 * (u2 * tmp1);
-      a[1][4] = 0.0;
-      a[2][0] = -dt * tz2 * (-(u3 * u4) * tmp2) - dt * tz1 * (-c34 * tmp2 * u3);
-      a[2][1] = 0.0;
-      a[2][2] = -dt * tz2 * (u4 * tmp1) - dt * tz1 * (c34 * tmp1) - dt * tz1 * dz3;
-      a[2][3] = -dt * tz2 * (u3 * tmp1);
-      a[2][4] = 0.0;
-      a[3][0] = -dt * tz2 * (-((u4 * tmp1) * (u4 * tmp1)) + 0.50e+00 * c2 * ((u2 * u2 + u3 * u3 + u4 * u4) * tmp2)) -
-                dt * tz1 * (-r43 * c34 * tmp2 * u4);
-      a[3][1] = -dt * tz2 * (-c2 * (u2 * tmp1));
-      a[3][2] = -dt * tz2 * (-c2 * (u3 * tmp1));
-      a[3][3] = -dt * tz2 * (2.0e+00 - c2) * (u4 * tmp1) - dt * tz1 * (r43 * c34 * tmp1) - dt * tz1 * dz4;
-      a[3][4] = -dt * tz2 * c2;
-      a[4][0] = -dt * tz2 * ((c2 * (u2 * u2 + u3 * u3 + u4 * u4) * tmp2 - c1 * (u5 * tmp1)) * (u4 * tmp1)) -
-                dt * tz1 *
-                    (-(c34 - c1345) * tmp3 * (u2 * u2) - (c34 - c1345) * tmp3 * (u3 * u3) -
-                     (r43 * c34 - c1345) * tmp3 * (u4 * u4) - c1345 * tmp2 * u5);
-      a[4][1] = -dt * tz2 * (-c2 * (u2 * u4) * tmp2) - dt * tz1 * (c34 - c1345) * tmp2 * u2;
-      a[4][2] = -dt * tz2 * (-c2 * (u3 * u4) * tmp2) - dt * tz1 * (c34 - c1345) * tmp2 * u3;
-      a[4][3] = -dt * tz2 * (c1 * (u5 * tmp1) - 0.50e+00 * c2 * ((u2 * u2 + u3 * u3 + 3.0e+00 * u4 * u4) * tmp2)) -
-                dt * tz1 * (r43 * c34 - c1345) * tmp2 * u4;
-      a[4][4] = -dt * tz2 * (c1 * (u4 * tmp1)) - dt * tz1 * c1345 * tmp1 - dt * tz1 * dz5;
-    } else {
-      a[0][0] = -dt * tz1 * dz1;
-      a[0][1] = 0.0;
-      a[0][2] = 0.0;
-      a[0][3] = dt * tz2;
-      a[0][4] = 0.0;
-      a[1][0] = dt * tz2 * (-(u2 * u4) * tmp2) - dt * tz1 * (-c34 * tmp2 * u2);
-      a[1][1] = dt * tz2 * (u4 * tmp1) - dt * tz1 * c34 * tmp1 - dt * tz1 * dz2;
-      a[1][2] = 0.0;
-      a[1][3] = dt * tz2 * (u2 * tmp1);
-      a[1][4] = 0.0;
-      a[2][0] = dt * tz2 * (-(u3 * u4) * tmp2) - dt * tz1 * (-c34 * tmp2 * u3);
-      a[2][1] = 0.0;
-      a[2][2] = dt * tz2 * (u4 * tmp1) - dt * tz1 * (c34 * tmp1) - dt * tz1 * dz3;
-      a[2][3] = dt * tz2 * (u3 * tmp1);
-      a[2][4] = 0.0;
-      a[3][0] = dt * tz2 * (-((u4 * tmp1) * (u4 * tmp1)) + 0.50e+00 * c2 * ((u2 * u2 + u3 * u3 + u4 * u4) * tmp2)) -
-                dt * tz1 * (-r43 * c34 * tmp2 * u4);
-      a[3][1] = dt * tz2 * (-c2 * (u2 * tmp1));
-      a[3][2] = dt * tz2 * (-c2 * (u3 * tmp1));
-      a[3][3] = dt * tz2 * (2.0e+00 - c2) * (u4 * tmp1) - dt * tz1 * (r43 * c34 * tmp1) - dt * tz1 * dz4;
-      a[3][4] = dt * tz2 * c2;
-      a[4][0] = dt * tz2 * ((c2 * (u2 * u2 + u3 * u3 + u4 * u4) * tmp2 - c1 * (u5 * tmp1)) * (u4 * tmp1)) -
-                dt * tz1 *
-                    (-(c34 - c1345) * tmp3 * (u2 * u2) - (c34 - c1345) * tmp3 * (u3 * u3) -
-                     (r43 * c34 - c1345) * tmp3 * (u4 * u4) - c1345 * tmp2 * u5);
-      a[4][1] = dt * tz2 * (-c2 * (u2 * u4) * tmp2) - dt * tz1 * (c34 - c1345) * tmp2 * u2;
-      a[4][2] = dt * tz2 * (-c2 * (u3 * u4) * tmp2) - dt * tz1 * (c34 - c1345) * tmp2 * u3;
-      a[4][3] = dt * tz2 * (c1 * (u5 * tmp1) - 0.50e+00 * c2 * ((u2 * u2 + u3 * u3 + 3.0e+00 * u4 * u4) * tmp2)) -
-                dt * tz1 * (r43 * c34 - c1345) * tmp2 * u4;
-      a[4][4] = dt * tz2 * (c1 * (u4 * tmp1)) - dt * tz1 * c1345 * tmp1 - dt * tz1 * dz5;
-    }
+    NPBMZ_LU_OFF(1, 0, (dt * tz2 * (-(u2 * u4) * tmp2)), - dt * tz1 * (-c34 * tmp2 * u2))
+    NPBMZ_LU_OFF(1, 1, (dt * tz2 * (u4 * tmp1)), - dt * tz1 * c34 * tmp1 - dt * tz1 * dz2)
+    NPBMZ_LU_OFF(1, 3, (dt * tz2 * (u2 * tmp1)), )
+    NPBMZ_LU_OFF(2, 0, (dt * tz2 * (-(u3 * u4) * tmp2)), - dt * tz1 * (-c34 * tmp2 * u3))
+    NPBMZ_LU_OFF(2, 2, (dt * tz2 * (u4 * tmp1)), - dt * tz1 * (c34 * tmp1) - dt * tz1 * dz3)
+    NPBMZ_LU_OFF(2, 3, (dt * tz2 * (u3 * tmp1)), )
+    NPBMZ_LU_OFF(3, 0, (dt * tz2 * (-((u4 * tmp1) * (u4 * tmp1)) + 0.50e+00 * c2 * ((u2 * u2 + u3 * u3 + u4 * u4) *
+                 tmp2))),
+                 - dt * tz1 * (-r43 * c34 * tmp2 * u4))
+    NPBMZ_LU_OFF(3, 1, (dt * tz2 * (-c2 * (u2 * tmp1))), )
+    NPBMZ_LU_OFF(3, 2, (dt * tz2 * (-c2 * (u3 * tmp1))), )
+    NPBMZ_LU_OFF(3, 3, (dt * tz2 * (2.0e+00 - c2) * (u4 * tmp1)), - dt * tz1 * (r43 * c34 * tmp1) - dt * tz1 * dz4)
+    NPBMZ_LU_OFF(4, 0, (dt * tz2 * ((c2 * (u2 * u2 + u3 * u3 + u4 * u4) * tmp2 - c1 * (u5 * tmp1)) * (u4 * tmp1))),
+                 - dt * tz1 * (-(c34 - c1345) * tmp3 * (u2 * u2) - (c34 - c1345) * tmp3 * (u3 * u3) - (r43 * c34 -
+                 c1345) * tmp3 * (u4 * u4) - c1345 * tmp2 * u5))
+    NPBMZ_LU_OFF(4, 1, (dt * tz2 * (-c2 * (u2 * u4) * tmp2)), - dt * tz1 * (c34 - c1345) * tmp2 * u2)
+    NPBMZ_LU_OFF(4, 2, (dt * tz2 * (-c2 * (u3 * u4) * tmp2)), - dt * tz1 * (c34 - c1345) * tmp2 * u3)
+    NPBMZ_LU_OFF(4, 3, (dt * tz2 * (c1 * (u5 * tmp1) - 0.50e+00 * c2 * ((u2 * u2 + u3 * u3 + 3.0e+00 * u4 * u4) *
+                 tmp2))),
+                 - dt * tz1 * (r43 * c34 - c1345) * tmp2 * u4)
+    NPBMZ_LU_OFF(4, 4, (dt * tz2 * (c1 * (u4 * tmp1))), - dt * tz1 * c1345 * tmp1 - dt * tz1 * dz5)
   } else if (DIR == 1) {
     const double ty1 = J.ty1, ty2 = J.ty2;
-    if (SG < 0) {
-      a[0][0] = -dt * ty1 * dy1;
-      a[0][1] = 0.0;
-      a[0][2] = -dt * ty2;
-      a[0][3] = 0.0;
-      a[0][4] = 0.0;
-      a[1][0] = -dt * ty2 * (-(u2 * u3) * tmp2) - dt * ty1 * (-c34 * tmp2 * u2);
-      a[1][1] = -dt * ty2 * (u3 * tmp1) - dt * ty1 * (c34 * tmp1) - dt * ty1 * dy2;
-      a[1][2] = -dt * ty2 * (u2 * tmp1);
-      a[1][3] = 0.0;
-      a[1][4] = 0.0;
-      a[2][0] = -dt * ty2 * (-((u3 * tmp1) * (u3 * tmp1)) + 0.50e+00 * c2 * ((u2 * u2 + u3 * u3 + u4 * u4) * tmp2)) -
-                dt * ty1 * (-r43 * c34 * tmp2 * u3);
-      a[2][1] = -dt * ty2 * (-c2 * (u2 * tmp1));
-      a[2][2] = -dt * ty2 * ((2.0e+00 - c2) * (u3 * tmp1)) - dt * ty1 * (r43 * c34 * tmp1) - dt * ty1 * dy3;
-      a[2][3] = -dt * ty2 * (-c2 * (u4 * tmp1));
-      a[2][4] = -dt * ty2 * c2;
-      a[3][0] = -dt * ty2 * (-(u3 * u4) * tmp2) - dt * ty1 * (-c34 * tmp2 * u4);
-      a[3][1] = 0.0;
-      a[3][2] = -dt * ty2 * (u4 * tmp1);
-      a[3][3] = -dt * ty2 * (u3 * tmp1) - dt * ty1 * (c34 * tmp1) - dt * ty1 * dy4;
-      a[3][4] = 0.0;
-      a[4][0] = -dt * ty2 * ((c2 * (u2 * u2 + u3 * u3 + u4 * u4) * tmp2 - c1 * (u5 * tmp1)) * (u3 * tmp1)) -
-                dt * ty1 *
-                    (-(c34 - c1345) * tmp3 * (u2 * u2) - (r43 * c34 - c1345) * tmp3 * (u3 * u3) -
-                     (c34 - c1345) * tmp3 * (u4 * u4) - c1345 * tmp2 * u5);
-      a[4][1] = -dt * ty2 * (-c2 * (u2 * u3) * tmp2) - dt * ty1 * (c34 - c1345) * tmp2 * u2;
-      a[4][2] = -dt * ty2 * (c1 * (u5 * tmp1) - 0.50e+00 * c2 * ((u2 * u2 + 3.0e+00 * u3 * u3 + u4 * u4) * tmp2)) -
-                dt * ty1 * (r43 * c34 - c1345) * tmp2 * u3;
-      a[4][3] = -dt * ty2 * (-c2 * (u3 * u4) * tmp2) - dt * ty1 * (c34 - c1345) * tmp2 * u4;
-      a[4][4] = -dt * ty2 * (c1 * (u3 * tmp1)) - dt * ty1 * c1345 * tmp1 - dt * ty1 * dy5;
-    } else {
-      a[0][0] = -dt * ty1 * dy1;
-      a[0][1] = 0.0;
-      a[0][2] = dt * ty2;
-      a[0][3] = 0.0;
-      a[0][4] = 0.0;
-      a[1][0] = dt * ty2 * (-(u2 * u3) * tmp2) - dt * ty1 * (-c34 * tmp2 * u2);
-      a[1][1] = dt * ty2 * (u3 * tmp1) - dt * ty1 * (c34 * tmp1) - dt * ty1 * dy2;
-      a[1][2] = dt * ty2 * (u2 * tmp1);
-      a[1][3] = 0.0;
-      a[1][4] = 0.0;
-      a[2][0] = dt * ty2 * (-((u3 * tmp1) * (u3 * tmp1)) + 0.50e+00 * c2 * ((u2 * u2 + u3 * u3 + u4 * u4) * tmp2)) -
-                dt * ty1 * (-r43 * c34 * tmp2 * u3);
-      a[2][1] = dt * ty2 * (-c2 * (u2 * tmp1));
-      a[2][2] = dt * ty2 * ((2.0e+00 - c2) * (u3 * tmp1)) - dt * ty1 * (r43 * c34 * tmp1) - dt * ty1 * dy3;
-      a[2][3] = dt * ty2 * (-c2 * (u4 * tmp1));
-      a[2][4] = dt * ty2 * c2;
-      a[3][0] = dt * ty2 * (-(u3 * u4) * tmp2) - dt * ty1 * (-c34 * tmp2 * u4);
-      a[3][1] = 0.0;
-      a[3][2] = dt * ty2 * (u4 * tmp1);
-      a[3][3] = dt * ty2 * (u3 * tmp1) - dt * ty1 * (c34 * tmp1) - dt * ty1 * dy4;
-      a[3][4] = 0.0;
-      a[4][0] = dt * ty2 * ((c2 * (u2 * u2 + u3 * u3 + u4 * u4) * tmp2 - c1 * (u5 * tmp1)) * (u3 * tmp1)) -
-                dt * ty1 *
-                    (-(c34 - c1345) * tmp3 * (u2 * u2) - (r43 * c34 - c1345) * tmp3 * (u3 * u3) -
-                     (c34 - c1345) * tmp3 * (u4 * u4) - c1345 * tmp2 * u5);
-      a[4][1] = dt * ty2 * (-c2 * (u2 * u3) * tmp2) - dt * ty1 * (c34 - c1345) * tmp2 * u2;
-      a[4][2] = dt * ty2 * (c1 * (u5 * tmp1) - 0.50e+00 * c2 * ((u2 * u2 + 3.0e+00 * u3 * u3 + u4 * u4) * tmp2)) -
-                dt * ty1 * (r43 * c34 - c1345) * tmp2 * u3;
-      a[4][3] = dt * ty2 * (-c2 * (u3 * u4) * tmp2) - dt * ty1 * (c34 - c1345) * tmp2 * u4;
-      a[4][4] = dt * ty2 * (c1 * (u3 * tmp1)) - dt * ty1 * c1345 * tmp1 - dt * ty1 * dy5;
-    }
+    NPBMZ_LU_OFF(1, 0, (dt * ty2 * (-(u2 * u3) * tmp2)), - dt * ty1 * (-c34 * tmp2 * u2))
+    NPBMZ_LU_OFF(1, 1, (dt * ty2 * (u3 * tmp1)), - dt * ty1 * (c34 * tmp1) - dt * ty1 * dy2)
+    NPBMZ_LU_OFF(1, 2, (dt * ty2 * (u2 * tmp1)), )
+    NPBMZ_LU_OFF(2, 0, (dt * ty2 * (-((u3 * tmp1) * (u3 * tmp1)) + 0.50e+00 * c2 * ((u2 * u2 + u3 * u3 + u4 * u4) *
+                 tmp2))),
+                 - dt * ty1 * (-r43 * c34 * tmp2 * u3))
+    NPBMZ_LU_OFF(2, 1, (dt * ty2 * (-c2 * (u2 * tmp1))), )
+    NPBMZ_LU_OFF(2, 2, (dt * ty2 * ((2.0e+00 - c2) * (u3 * tmp1))), - dt * ty1 * (r43 * c34 * tmp1) - dt * ty1 * dy3)
+    NPBMZ_LU_OFF(2, 3, (dt * ty2 * (-c2 * (u4 * tmp1))), )
+    NPBMZ_LU_OFF(3, 0, (dt * ty2 * (-(u3 * u4) * tmp2)), - dt * ty1 * (-c34 * tmp2 * u4))
+    NPBMZ_LU_OFF(3, 2, (dt * ty2 * (u4 * tmp1)), )
+    NPBMZ_LU_OFF(3, 3, (dt * ty2 * (u3 * tmp1)), - dt * ty1 * (c34 * tmp1) - dt * ty1 * dy4)
+    NPBMZ_LU_OFF(4, 0, (dt * ty2 * ((c2 * (u2 * u2 + u3 * u3 + u4 * u4) * tmp2 - c1 * (u5 * tmp1)) * (u3 * tmp1))),
+                 - dt * ty1 * (-(c34 - c1345) * tmp3 * (u2 * u2) - (r43 * c34 - c1345) * tmp3 * (u3 * u3) - (c34 -
+                 c1345) * tmp3 * (u4 * u4) - c1345 * tmp2 * u5))
+    NPBMZ_LU_OFF(4, 1, (dt * ty2 * (-c2 * (u2 * u3) * tmp2)), - dt * ty1 * (c34 - c1345) * tmp2 * u2)
+    NPBMZ_LU_OFF(4, 2, (dt * ty2 * (c1 * (u5 * tmp1) - 0.50e+00 * c2 * ((u2 * u2 + 3.0e+00 * u3 * u3 + u4 * u4) *
+                 tmp2))),
+                 - dt * ty1 * (r43 * c34 - c1345) * tmp2 * u3)
+    NPBMZ_LU_OFF(4, 3, (dt * ty2 * (-c2 * (u3 * u4) * tmp2)), - dt * ty1 * (c34 - c1345) * tmp2 * u4)
+    NPBMZ_LU_OFF(4, 4, (dt * ty2 * (c1 * (u3 * tmp1))), - dt * ty1 * c1345 * tmp1 - dt * ty1 * dy5)
   } else {
     const double tx1 = J.tx1, tx2 = J.tx2;
-    if (SG < 0) {
-      a[0][0] = -dt * tx1 * dx1;
-      a[0][1] = -dt * tx2;
-      a[0][2] = 0.0;
-      a[0][3] = 0.0;
-      a[0][4] = 0.0;
-      a[1][0] = -dt * tx2 * (-((u2 * tmp1) * (u2 * tmp1)) + c2 * 0.50e+00 * (u2 * u2 + u3 * u3 + u4 * u4) * tmp2) -
-                dt * tx1 * (-r43 * c34 * tmp2 * u2);
-      a[1][1] = -dt * tx2 * ((2.0e+00 - c2) * (u2 * tmp1)) - dt * tx1 * (r43 * c34 * tmp1) - dt * tx1 * dx2;
-      a[1][2] = -dt * tx2 * (-c2 * (u3 * tmp1));
-      a[1][3] = -dt * tx2 * (-c2 * (u4 * tmp1));
-      a[1][4] = -dt * tx2 * c2;
-      a[2][0] = -dt * tx2 * (-(u2 * u3) * tmp2) - dt * tx1 * (-c34 * tmp2 * u3);
-      a[2][1] = -dt * tx2 * (u3 * tmp1);
-      a[2][2] = -dt * tx2 * (u2 * tmp1) - dt * tx1 * (c34 * tmp1) - dt * tx1 * dx3;
-      a[2][3] = 0.0;
-      a[2][4] = 0.0;
-      a[3][0] = -dt * tx2 * (-(u2 * u4) * tmp2) - dt * tx1 * (-c34 * tmp2 * u4);
-      a[3][1] = -dt * tx2 * (u4 * tmp1);
-      a[3][2] = 0.0;
-      a[3][3] = -dt * tx2 * (u2 * tmp1) - dt * tx1 * (c34 * tmp1) - dt * tx1 * dx4;
-      a[3][4] = 0.0;
-      a[4][0] = -dt * tx2 * ((c2 * (u2 * u2 + u3 * u3 + u4 * u4) * tmp2 - c1 * (u5 * tmp1)) * (u2 * tmp1)) -
-                dt * tx1 *
-                    (-(r43 * c34 - c1345) * tmp3 * (u2 * u2) - (c34 - c1345) * tmp3 * (u3 * u3) -
-                     (c34 - c1345) * tmp3 * (u4 * u4) - c1345 * tmp2 * u5);
-      a[4][1] = -dt * tx2 * (c1 * (u5 * tmp1) - 0.50e+00 * c2 * ((3.0e+00 * u2 * u2 + u3 * u3 + u4 * u4) * tmp2)) -
-                dt * tx1 * (r43 * c34 - c1345) * tmp2 * u2;
-      a[4][2] = -dt * tx2 * (-c2 * (u3 * u2) * tmp2) - dt * tx1 * (c34 - c1345) * tmp2 * u3;
-      a[4][3] = -dt * tx2 * (-c2 * (u4 * u2) * tmp2) - dt * tx1 * (c34 - c1345) * tmp2 * u4;
-      a[4][4] = -dt * tx2 * (c1 * (u2 * tmp1)) - dt * tx1 * c1345 * tmp1 - dt * tx1 * dx5;
-    } else {
-      a[0][0] = -dt * tx1 * dx1;
-      a[0][1] = dt * tx2;
-      a[0][2] = 0.0;
-      a[0][3] = 0.0;
-      a[0][4] = 0.0;
-      a[1][0] = dt * tx2 * (-((u2 * tmp1) * (u2 * tmp1)) + c2 * 0.50e+00 * (u2 * u2 + u3 * u3 + u4 * u4) * tmp2) -
-                dt * tx1 * (-r43 * c34 * tmp2 * u2);
-      a[1][1] = dt * tx2 * ((2.0e+00 - c2) * (u2 * tmp1)) - dt * tx1 * (r43 * c34 * tmp1) - dt * tx1 * dx2;
-      a[1][2] = dt * tx2 * (-c2 * (u3 * tmp1));
-      a[1][3] = dt * tx2 * (-c2 * (u4 * tmp1));
-      a[1][4] = dt * tx2 * c2;
-      a[2][0] = dt * tx2 * (-(u2 * u3) * tmp2) - dt * tx1 * (-c34 * tmp2 * u3);
-      a[2][1] = dt * tx2 * (u3 * tmp1);
-      a[2][2] = dt * tx2 * (u2 * tmp1) - dt * tx1 * (c34 * tmp1) - dt * tx1 * dx3;
-      a[2][3] = 0.0;
-      a[2][4] = 0.0;
-      a[3][0] = dt * tx2 * (-(u2 * u4) * tmp2) - dt * tx1 * (-c34 * tmp2 * u4);
-      a[3][1] = dt * tx2 * (u4 * tmp1);
-      a[3][2] = 0.0;
-      a[3][3] = dt * tx2 * (u2 * tmp1) - dt * tx1 * (c34 * tmp1) - dt * tx1 * dx4;
-      a[3][4] = 0.0;
-      a[4][0] = dt * tx2 * ((c2 * (u2 * u2 + u3 * u3 + u4 * u4) * tmp2 - c1 * (u5 * tmp1)) * (u2 * tmp1)) -
-                dt * tx1 *
-                    (-(r43 * c34 - c1345) * tmp3 * (u2 * u2) - (c34 - c1345) * tmp3 * (u3 * u3) -
-                     (c34 - c1345) * tmp3 * (u4 * u4) - c1345 * tmp2 * u5);
-      a[4][1] = dt * tx2 * (c1 * (u5 * tmp1) - 0.50e+00 * c2 * ((3.0e+00 * u2 * u2 + u3 * u3 + u4 * u4) * tmp2)) -
-                dt * tx1 * (r43 * c34 - c1345) * tmp2 * u2;
-      a[4][2] = dt * tx2 * (-c2 * (u3 * u2) * tmp2) - dt * tx1 * (c34 - c1345) * tmp2 * u3;
-      a[4][3] = dt * tx2 * (-c2 * (u4 * u2) * tmp2) - dt * tx1 * (c34 - c1345) * tmp2 * u4;
-      a[4][4] = dt * tx2 * (c1 * (u2 * tmp1)) - dt * tx1 * c1345 * tmp1 - dt * tx1 * dx5;
-    }
+    NPBMZ_LU_OFF(1, 0, (dt * tx2 * (-((u2 * tmp1) * (u2 * tmp1)) + c2 * 0.50e+00 * (u2 * u2 + u3 * u3 + u4 * u4) *
+                 tmp2)),
+                 - dt * tx1 * (-r43 * c34 * tmp2 * u2))
+    NPBMZ_LU_OFF(1, 1, (dt * tx2 * ((2.0e+00 - c2) * (u2 * tmp1))), - dt * tx1 * (r43 * c34 * tmp1) - dt * tx1 * dx2)
+    NPBMZ_LU_OFF(1, 2, (dt * tx2 * (-c2 * (u3 * tmp1))), )
+    NPBMZ_LU_OFF(1, 3, (dt * tx2 * (-c2 * (u4 * tmp1))), )
+    NPBMZ_LU_OFF(2, 0, (dt * tx2 * (-(u2 * u3) * tmp2)), - dt * tx1 * (-c34 * tmp2 * u3))
+    NPBMZ_LU_OFF(2, 1, (dt * tx2 * (u3 * tmp1)), )
+    NPBMZ_LU_OFF(2, 2, (dt * tx2 * (u2 * tmp1)), - dt * tx1 * (c34 * tmp1) - dt * tx1 * dx3)
+    NPBMZ_LU_OFF(3, 0, (dt * tx2 * (-(u2 * u4) * tmp2)), - dt * tx1 * (-c34 * tmp2 * u4))
+    NPBMZ_LU_OFF(3, 1, (dt * tx2 * (u4 * tmp1)), )
+    NPBMZ_LU_OFF(3, 3, (dt * tx2 * (u2 * tmp1)), - dt * tx1 * (c34 * tmp1) - dt * tx1 * dx4)
+    NPBMZ_LU_OFF(4, 0, (dt * tx2 * ((c2 * (u2 * u2 + u3 * u3 + u4 * u4) * tmp2 - c1 * (u5 * tmp1)) * (u2 * tmp1))),
+                 - dt * tx1 * (-(r43 * c34 - c1345) * tmp3 * (u2 * u2) - (c34 - c1345) * tmp3 * (u3 * u3) - (c34 -
+                 c1345) * tmp3 * (u4 * u4) - c1345 * tmp2 * u5))
+    NPBMZ_LU_OFF(4, 1, (dt * tx2 * (c1 * (u5 * tmp1) - 0.50e+00 * c2 * ((3.0e+00 * u2 * u2 + u3 * u3 + u4 * u4) *
+                 tmp2))),
+                 - dt * tx1 * (r43 * c34 - c1345) * tmp2 * u2)
+    NPBMZ_LU_OFF(4, 2, (dt * tx2 * (-c2 * (u3 * u2) * tmp2)), - dt * tx1 * (c34 - c1345) * tmp2 * u3)
+    NPBMZ_LU_OFF(4, 3, (dt * tx2 * (-c2 * (u4 * u2) * tmp2)), - dt * tx1 * (c34 - c1345) * tmp2 * u4)
+    NPBMZ_LU_OFF(4, 4, (dt * tx2 * (c1 * (u2 * tmp1))), - dt * tx1 * c1345 * tmp1 - dt * tx1 * dx5)
   }
+#undef NPBMZ_LU_OFF
 }
 
 __device__ __forceinline__ void load5(const double* f, long long NP, long long p, double v[5]) {
@@ -598,26 +448,16 @@ __device__ __forceinline__ void store_blk(double* jac, long long NP, long long h
       if (off_stored(DIR, r, c)) jac[(FAC_BLK + (2 * DIR + S) * BLK_N + blk_idx(DIR, r, c)) * NP + h] = b[r][c];
 }
 
-// jacld's (SG = -1) and jacu's (SG = +1) blocks of direction DIR built from
-// this point's state (r1 = 1/u1, u), stored at the interior consumers: the
-// point at +1 in DIR reads the jacld block, the point at -1 the jacu block.
-// Both signs from one state share most of their subexpressions.
+// Both blocks of direction DIR built from this point's state, stored at the
+// interior consumers: the point at +1 in DIR reads jacld's, the point at -1
+// jacu's.
 template <int DIR>
 __device__ __forceinline__ void jac_dir(const JC& J, double r1, const double u[5], double* __restrict__ jac,
                                         long long NP, bool lo, long long slot_lo, bool up, long long slot_up) {
   double b[5][5], c[5][5];
-  if (lo && up) {
-    jac_off<DIR, -1>(J, r1, u[1], u[2], u[3], u[4], b);
-    jac_off<DIR, 1>(J, r1, u[1], u[2], u[3], u[4], c);
-    store_blk<DIR, 0>(jac, NP, slot_lo, b);
-    store_blk<DIR, 1>(jac, NP, slot_up, c);
-  } else if (lo) {
-    jac_off<DIR, -1>(J, r1, u[1], u[2], u[3], u[4], b);
-    store_blk<DIR, 0>(jac, NP, slot_lo, b);
-  } else if (up) {
-    jac_off<DIR, 1>(J, r1, u[1], u[2], u[3], u[4], c);
-    store_blk<DIR, 1>(jac, NP, slot_up, c);
-  }
+  jac_off<DIR>(J, r1, u[1], u[2], u[3], u[4], b, c);
+  if (lo) store_blk<DIR, 0>(jac, NP, slot_lo, b);
+  if (up) store_blk<DIR, 1>(jac, NP, slot_up, c);
 }
 
 // Slot of interior point (i, j, k) in the zone's hyperplane order (R: its row
@@ -644,37 +484,31 @@ __global__ void __launch_bounds__(TPB) k_lu_points(LuDev D, const int* __restric
 // j), so that consecutive threads write consecutive consumer slots.
 // fb: per zone, l and k, the first full-box point of row k of hyperplane l;
 // ri: the same for the interior points (the consumers' slots).
-// HP_ORDER false: threads in the zone's natural order instead (coalesced
-// reads of the point's state, scattered block writes).  The FP64-bound
-// uncontracted build is faster so, the FMA build with HP_ORDER; the values
-// written are the same either way.
-template <bool HP_ORDER>
+// Bound by the FP64 pipe.  480x320x28, us without / with contraction: 4913 /
+// 4400 with jacld's and jacu's entries formed apart and a branch per missing
+// consumer, 4343 / 3535 with each term formed once, 3705 / 3190 with the three
+// directions of every point together (their squares and products shared).
+// The zone's natural order instead of the hyperplane order (coalesced reads,
+// scattered writes) costs 4670 / 4614 where this order takes 4343 / 3535.
 __global__ void __launch_bounds__(TPB) k_lu_jac(LuDev D, const int* __restrict__ fb, int fls, const int* __restrict__ ri,
                                                 int ls, int ks, double* __restrict__ jac, int z0) {
   const int zone = z0 + blockIdx.y;
   const LuZone Z = D.zones[zone];
   const int T = blockIdx.x * TPB + threadIdx.x;
   if (T >= Z.np) return;
-  int i, j, k;
-  if (HP_ORDER) {
-    const int* FB = fb + (long long)zone * fls * ks;
-    int lo = 3, hi = Z.nx + Z.ny + Z.nz;  // the hyperplane: largest l starting at or before T
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) / 2;
-      if (FB[mid * ks] <= T) lo = mid; else hi = mid - 1;
-    }
-    const int l = lo;
-    int klo = 1, khi = Z.nz;  // the row: largest k starting at or before T
-    while (klo < khi) {
-      const int mid = (klo + khi + 1) / 2;
-      if (FB[l * ks + mid] <= T) klo = mid; else khi = mid - 1;
-    }
-    k = klo;
-    j = max(1, l - k - Z.nx) + (T - FB[l * ks + k]);
-    i = l - j - k;
-  } else {
-    decode(Z, T, i, j, k);
+  const int* FB = fb + (long long)zone * fls * ks;
+  int lo = 3, hi = Z.nx + Z.ny + Z.nz;  // the hyperplane: largest l starting at or before T
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) / 2;
+    if (FB[mid * ks] <= T) lo = mid; else hi = mid - 1;
   }
+  const int l = lo;
+  int klo = 1, khi = Z.nz;  // the row: largest k starting at or before T
+  while (klo < khi) {
+    const int mid = (klo + khi + 1) / 2;
+    if (FB[l * ks + mid] <= T) klo = mid; else khi = mid - 1;
+  }
+  const int k = klo, j = max(1, l - k - Z.nx) + (T - FB[l * ks + k]), i = l - j - k;
   const long long NP = D.NP, p = pidx(Z, i, j, k);
   const JC J{D.dt, Z.tx1, Z.tx2, Z.ty1, Z.ty2, Z.tz1, Z.tz2};
   const int* R = ri + (long long)zone * ls * ks;
@@ -683,16 +517,18 @@ __global__ void __launch_bounds__(TPB) k_lu_jac(LuDev D, const int* __restrict__
   double u[5];
   load5(D.u, NP, p, u);
   const bool ii = i >= 2 && i <= Z.nx - 1, jj = j >= 2 && j <= Z.ny - 1, kk = k >= 2 && k <= Z.nz - 1;
-  if (jj && kk) {
-    const bool lo = i <= Z.nx - 2, up = i >= 3;
+  // every point forms the blocks of the three directions (the shared products
+  // once), and stores those that have a consumer
+  {
+    const bool lo = jj && kk && i <= Z.nx - 2, up = jj && kk && i >= 3;
     jac_dir<0>(J, r1, u, jac, NP, lo, lo ? slot(i + 1, j, k) : 0, up, up ? slot(i - 1, j, k) : 0);
   }
-  if (ii && kk) {
-    const bool lo = j <= Z.ny - 2, up = j >= 3;
+  {
+    const bool lo = ii && kk && j <= Z.ny - 2, up = ii && kk && j >= 3;
     jac_dir<1>(J, r1, u, jac, NP, lo, lo ? slot(i, j + 1, k) : 0, up, up ? slot(i, j - 1, k) : 0);
   }
-  if (ii && jj) {
-    const bool lo = k <= Z.nz - 2, up = k >= 3;
+  {
+    const bool lo = ii && jj && k <= Z.nz - 2, up = ii && jj && k >= 3;
     jac_dir<2>(J, r1, u, jac, NP, lo, lo ? slot(i, j, k + 1) : 0, up, up ? slot(i, j, k - 1) : 0);
   }
   if (ii && jj && kk) {
@@ -809,24 +645,6 @@ __device__ __forceinline__ double row_dot_yx(const RowCoef& c, const double wy[5
     }
   }
   return s;
-}
-
-// v / t from y = 1/t rounded to nearest: the quotient estimate v y, refined by
-// its FMA residuals (P. Markstein, IBM J. Res. Dev. 34(1), 1990: one step from
-// an estimate within one ulp, with the correctly rounded reciprocal, gives the
-// correctly rounded quotient; the first step here makes the estimate so).  A
-// dependent divide costs nine FP64 instructions where this takes five, and
-// the FP64 pipe binds the sweeps.  Operands whose residual could underflow or
-// overflow take the divide.
-__device__ __forceinline__ double div_y(double v, double t, double y) {
-  const unsigned ev = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu, et = ((unsigned)__double2hiint(t) >> 20) & 0x7ffu;
-  // exponents of v in [2^-600, 2^600) and of t in [2^-300, 2^300): v, t, y, q and every residual are normal
-  if (__builtin_expect(ev - 423u < 1200u && et - 723u < 600u, 1)) {
-    double q = v * y;
-    q = fma(fma(-t, q, v), y, q);
-    return fma(fma(-t, q, v), y, q);
-  }
-  return v / t;
 }
 
 // Row M of one point of a sweep (UP false: blts, the neighbours at -1; UP
@@ -1162,12 +980,9 @@ void pointwise(bool update, const LuDev& D, const LuWork* w, int n, double tmp, 
   else
     k_lu_pointwise<false><<<n, TPB, 0, s>>>(D, w, tmp);
 }
-void jac(bool hp_order, const LuDev& D, const int* fb, int fls, const int* ri, int ls, int ks, double* jac, int z0,
-         dim3 grid, cudaStream_t s) {
-  if (hp_order)
-    k_lu_jac<true><<<grid, TPB, 0, s>>>(D, fb, fls, ri, ls, ks, jac, z0);
-  else
-    k_lu_jac<false><<<grid, TPB, 0, s>>>(D, fb, fls, ri, ls, ks, jac, z0);
+void jac(const LuDev& D, const int* fb, int fls, const int* ri, int ls, int ks, double* jac, int z0, dim3 grid,
+         cudaStream_t s) {
+  k_lu_jac<<<grid, TPB, 0, s>>>(D, fb, fls, ri, ls, ks, jac, z0);
 }
 void points(const LuDev& D, const int* ri, int ls, int ks, int* pts, const LuWork* w, int n, cudaStream_t s) {
   k_lu_points<<<n, TPB, 0, s>>>(D, ri, ls, ks, pts, w);

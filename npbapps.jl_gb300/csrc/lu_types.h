@@ -58,9 +58,10 @@ __host__ __device__ inline long long pidx(const LuZone& Z, int i, int j, int k) 
 //   PR_RHO  1/g1                          (the viscous tmp, jacld's tmp1)
 //   PR_U21..PR_U51  tmp*g2 .. tmp*g5      (the viscous u21i .. u51i)
 //   PR_S    u21^2 + u31^2 + u41^2         (their sum of squares)
-//   PR_C21, PR_C31, PR_C41  g2/g1, g3/g1, g4/g1  (the convective u21, u31, u41)
-//   PR_Q    0.5 (g2^2 + g3^2 + g4^2) / g1 (the convective q)
-enum { PR_RHO = 0, PR_U21, PR_U31, PR_U41, PR_U51, PR_S, PR_C21, PR_C31, PR_C41, PR_Q, PR_COUNT };
+//   PR_F + 4 dir + m-1                    component m = 1..4 of the convective
+//       flux of direction dir (component 0 is g itself), from g2/g1, g3/g1,
+//       g4/g1 and q = 0.5 (g2^2 + g3^2 + g4^2) / g1
+enum { PR_RHO = 0, PR_U21, PR_U31, PR_U41, PR_U51, PR_S, PR_F, PR_COUNT = PR_F + 12 };
 
 struct JC {
   double dt, tx1, tx2, ty1, ty2, tz1, tz2;

@@ -109,6 +109,18 @@ def test_sweeps_at_block_edges_are_bit_exact(zone, flags):
     assert_state_equal(p, r, (lu.U, lu.RSD))
 
 
+@pytest.mark.parametrize("zone", [(5, 6, 7), (6, 7, 5), (7, 5, 6), (8, 9, 6), (33, 6, 5)])
+def test_rhs_stencils_at_short_axes_are_bit_exact(zone):
+    """rhs and erhs (setup) on axes of 5 points, where two dissipation stencils
+    meet, 6, where every stencil is an end one, and longer."""
+    nx, ny, nz = zone
+    p, r = make(lu.lu_zone_setup(2 * nx, 2 * ny, nz, 2, 2), 0.5, lu.FACES_NPB)
+    assert_state_equal(p, r)
+    p.iterate(3)
+    r.iterate(3)
+    assert_state_equal(p, r, (lu.U, lu.RSD))
+
+
 def test_per_zone_ssor_equals_batched():
     g, dt = GEOMS["rect"]
     a, _ = make(g(), dt, lu.FACES_NPB)
