@@ -9,9 +9,10 @@
 //       transposed blocks),  vb -= (d(Td(v) xd)/dv)^T y  (xd = the forward
 //       solution of that sweep);  the next rdb is y;
 //   vb += (dR/dv)^T rb,  fb += (dR/df)^T rb;   ub_prev = E^T vb.
-// The pointwise derivatives (of the flux-Jacobian products and of the
-// compute_rhs flux and viscous terms) are taken with forward-mode dual
-// numbers over the five conserved variables of one point.
+// The pointwise derivatives of the BT flux-Jacobian products are written out
+// (k_adj_lin); those of the compute_rhs flux and viscous terms and of SP are
+// taken with forward-mode dual numbers over the five conserved variables of
+// one point.
 //
 // SP (src/SP/adi.jl:6-258): r0 = R(u', f), r = Tx(u') r0 (txinvr), and per
 // sweep d = x, y, z: y_d = L_d(u')^-1 x_{d-1} (three scalar pentadiagonal
@@ -112,41 +113,35 @@ __device__ __forceinline__ void seed_state(const Fields& F, int64_t pt, D5 u[5])
   }
 }
 
-// F = fjac(u) x and N = njac(u) x with dual u (the formulas of bt_jx, with
-// ri = 1/u1 and qs = square / u1 derived from u as compute_rhs does).
-template <int DIR>
-__device__ __forceinline__ void jx_dual(const Consts& K, const D5 u[5], const double x[5], D5 Fx[5], D5 Nx[5]) {
-  const D5 ri = dinv(u[0]);
-  const D5 vel[3] = {u[1] * ri, u[2] * ri, u[3] * ri};
-  const D5 E = u[4] * ri;
-  const D5 q = 0.5 * ((u[1] * u[1] + u[2] * u[2] + u[3] * u[3]) * ri) * ri;
-  constexpr int a = DIR + 1;
-  const D5 vn = vel[DIR];
-  const double c1 = K.c1, c2 = K.c2;
-  D5 d[3];
+// Dense L U of M (no pivoting; unit-diagonal U) applied to U and r.
+__device__ __forceinline__ void lu_solve(double M[5][5], double U[5][5], double r[5]) {
 #pragma unroll
-  for (int m = 0; m < 3; ++m) d[m] = dconst(x[m + 1]) - vel[m] * x[0];
-  D5 tang = dconst(0.0);
-  Fx[0] = dconst(x[a]);
+  for (int p = 0; p < 5; ++p) {
+    const double piv = nr_rcp(M[p][p]);
 #pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    if (m == DIR) continue;
-    Fx[m + 1] = vn * d[m] + vel[m] * x[a];
-    tang = tang + vel[m] * x[m + 1];
+    for (int c = 0; c < 5; ++c) {
+      if (c > p) M[p][c] *= piv;
+      U[p][c] *= piv;
+    }
+    r[p] *= piv;
+#pragma unroll
+    for (int q = p + 1; q < 5; ++q) {
+#pragma unroll
+      for (int c = 0; c < 5; ++c) {
+        if (c > p) M[q][c] = fma(-M[q][p], M[p][c], M[q][c]);
+        U[q][c] = fma(-M[q][p], U[p][c], U[q][c]);
+      }
+      r[q] = fma(-M[q][p], r[p], r[q]);
+    }
   }
-  Fx[a] = (c2 * q - vn * vn) * x[0] - c2 * tang + ((2.0 - c2) * vn) * x[a] + dconst(c2 * x[4]);
-  Fx[4] = ((2.0 * c2) * q - c1 * E) * vn * x[0] - (c2 * vn) * tang + (c1 * E - c2 * (q + vn * vn)) * x[a] +
-          (c1 * vn) * x[4];
-  const double k43 = K.con43 * K.c3c4, c3c4 = K.c3c4, c1345 = K.c1345;
-  D5 s4 = c1345 * (dconst(x[4]) - E * x[0]);
-  Nx[0] = dconst(0.0);
 #pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    const double cm = (m == DIR) ? k43 : c3c4;
-    Nx[m + 1] = (cm * ri) * d[m];
-    s4 = s4 + ((cm - c1345) * vel[m]) * d[m];
-  }
-  Nx[4] = ri * s4;
+  for (int p = 4; p > 0; --p)
+#pragma unroll
+    for (int q = 0; q < p; ++q) {
+#pragma unroll
+      for (int c = 0; c < 5; ++c) U[q][c] = fma(-M[q][p], U[p][c], U[q][c]);
+      r[q] = fma(-M[q][p], r[p], r[q]);
+    }
 }
 
 // ---- transposed sweep --------------------------------------------------------
@@ -155,14 +150,12 @@ __device__ __forceinline__ void jx_dual(const Consts& K, const D5 u[5], const do
 //   L_p = C_{p-1}^T (zero for p = 1, where C_0 is the boundary's zero block),
 //   D_p = B_p^T (identity on the boundary rows 0 and n-1),
 //   U_p = A_{p+1}^T (zero for p = n-2, where A_{n-1} is zero).
-// Block LU (forward: G_p, g_p to the scratch), back substitution, then the
-// linearisation vb_q -= J_F(q)^T w_q + J_N(q)^T z_q with
-//   w_q = tmp2 (y_{q-1} - y_{q+1}),  z_q = -tmp1 (y_{q-1} - 2 y_q + y_{q+1})
-// over the interior rows only.
+// Block LU (forward: G_p, g_p to the scratch), back substitution; the
+// linearisation in x of the solution y is a kernel of its own over the points
+// (k_adj_lin).
 template <int DIR>
 __global__ void __launch_bounds__(128) k_adj_solve(Fields F, Consts K, const Work* __restrict__ work,
-                                                  double* __restrict__ yb, const double* __restrict__ xs,
-                                                  double* __restrict__ vb, double* __restrict__ scr, int64_t nlt) {
+                                                  double* __restrict__ yb, double* __restrict__ scr, int64_t nlt) {
   const Work w = work[blockIdx.x];
   const ZoneDev Z = F.zones[w.zone];
   const int line = w.first + threadIdx.x;
@@ -172,28 +165,19 @@ __global__ void __launch_bounds__(128) k_adj_solve(Fields F, Consts K, const Wor
   const int n = zone_line_len(Z, DIR);
   const int64_t gl = Z.lineoff[DIR] + line;
   const int64_t NP = F.NP;
-  const double tmp1 = DIR == 0 ? K.dttx1 : DIR == 1 ? K.dtty1 : K.dttz1;
-  const double tmp2 = DIR == 0 ? K.dttx2 : DIR == 1 ? K.dtty2 : K.dttz2;
-  double dd[5];
-  if (DIR == 0) { dd[0] = K.dx1; dd[1] = K.dx2; dd[2] = K.dx3; dd[3] = K.dx4; dd[4] = K.dx5; }
-  else if (DIR == 1) { dd[0] = K.dy1; dd[1] = K.dy2; dd[2] = K.dy3; dd[3] = K.dy4; dd[4] = K.dy5; }
-  else { dd[0] = K.dz1; dd[1] = K.dz2; dd[2] = K.dz3; dd[3] = K.dz4; dd[4] = K.dz5; }
+  const BtK<double>& k = bt_consts<double>(K, DIR);
   auto G = [&](int p, int e) -> double& { return scr[((int64_t)p * 30 + e) * nlt + gl]; };
 
   double Gp[5][5], gp[5];
   for (int p = 0; p < n; ++p) {
     const int64_t pt = base + (int64_t)p * st;
-    double f[5][5], nj[5][5];
-    bt_jac<DIR, double>(K, F.prim[PR_RHOI * NP + pt], F.u[NP + pt], F.u[2 * NP + pt], F.u[3 * NP + pt],
-                        F.u[4 * NP + pt], F.prim[PR_QS * NP + pt], f, nj);
-    double A[5][5], B[5][5], C[5][5];
-#pragma unroll
-    for (int a = 0; a < 5; ++a)
-#pragma unroll
-      for (int b = 0; b < 5; ++b) { A[a][b] = 0.0; B[a][b] = 0.0; C[a][b] = 0.0; }
-    bt_asm_a<DIR, double>(f, nj, tmp1, tmp2, dd, A);   // A_{p+1}
-    bt_asm_b<double>(nj, tmp1, dd, B);                  // B_p
-    bt_asm_c<DIR, double>(f, nj, tmp1, tmp2, dd, C);   // C_{p-1}
+    const BtState<double> u = bt_load_state<double>(F, pt);
+    BtGH<DIR, double> J;
+    bt_gh<DIR, double>(k, u.ri, u.v, u.u5 * u.ri, u.q, J);
+    double P[5][5], B[5][5], C[5][5];
+    bt_form_p<DIR, double>(J, P);  // -A_{p+1}
+    bt_form_b<DIR, double>(J, B);  // B_p
+    bt_form_c<DIR, double>(J, C);  // C_{p-1}
     const bool bnd = (p == 0 || p == n - 1);
     double M[5][5], U[5][5], r[5];
 #pragma unroll
@@ -201,8 +185,8 @@ __global__ void __launch_bounds__(128) k_adj_solve(Fields F, Consts K, const Wor
       r[a] = yb[a * NP + pt];
 #pragma unroll
       for (int b = 0; b < 5; ++b) {
-        M[a][b] = bnd ? (a == b ? 1.0 : 0.0) : B[b][a];
-        U[a][b] = (p <= n - 3) ? A[b][a] : 0.0;
+        M[a][b] = bnd ? (a == b ? 1.0 : 0.0) : hnz<DIR>(b, a) ? B[b][a] : 0.0;
+        U[a][b] = p <= n - 3 && anz<DIR>(b, a) ? -P[b][a] : 0.0;
       }
     }
     if (p >= 2) {  // L_p = C_{p-1}^T; M -= L G_{p-1}; r -= L g_{p-1}
@@ -212,16 +196,18 @@ __global__ void __launch_bounds__(128) k_adj_solve(Fields F, Consts K, const Wor
         for (int b = 0; b < 5; ++b) {
           double t = M[a][b];
 #pragma unroll
-          for (int c = 0; c < 5; ++c) t -= C[c][a] * Gp[c][b];
+          for (int c = 0; c < 5; ++c)
+            if (anz<DIR>(c, a)) t -= C[c][a] * Gp[c][b];
           M[a][b] = t;
         }
         double t = r[a];
 #pragma unroll
-        for (int c = 0; c < 5; ++c) t -= C[c][a] * gp[c];
+        for (int c = 0; c < 5; ++c)
+          if (anz<DIR>(c, a)) t -= C[c][a] * gp[c];
         r[a] = t;
       }
     }
-    binvcrhs<double>(M, U, r);
+    lu_solve(M, U, r);
 #pragma unroll
     for (int a = 0; a < 5; ++a) {
       gp[a] = r[a];
@@ -233,56 +219,109 @@ __global__ void __launch_bounds__(128) k_adj_solve(Fields F, Consts K, const Wor
       }
     }
   }
-  // back substitution y_p = g_p - G_p y_{p+1}; linearisation of point q = p+1
-  double y_next[5], y_cur[5], y_nn[5];  // y_{p+1}, y_p, y_{p+2}
+  // back substitution y_p = g_p - G_p y_{p+1}
+  double y[5];
 #pragma unroll
-  for (int m = 0; m < 5; ++m) { y_next[m] = gp[m]; y_nn[m] = 0.0; }
-#pragma unroll
-  for (int m = 0; m < 5; ++m) yb[m * NP + base + (int64_t)(n - 1) * st] = y_next[m];
-  auto lin = [&](int q, const double ym[5], const double yc[5], const double yp[5]) {
-    // rows outside 1..n-2 do not depend on the state
-    const double km = (q - 1 >= 1 && q - 1 <= n - 2) ? 1.0 : 0.0;
-    const double kc = (q >= 1 && q <= n - 2) ? 1.0 : 0.0;
-    const double kp = (q + 1 >= 1 && q + 1 <= n - 2) ? 1.0 : 0.0;
-    double wv[5], zv[5];
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      wv[m] = tmp2 * (km * ym[m] - kp * yp[m]);
-      zv[m] = -tmp1 * (km * ym[m] - 2.0 * kc * yc[m] + kp * yp[m]);
-    }
-    const int64_t pt = base + (int64_t)q * st;
-    D5 u[5], Fx[5], Nx[5];
-    seed_state(F, pt, u);
-    double x[5];
-#pragma unroll
-    for (int m = 0; m < 5; ++m) x[m] = xs[m * NP + pt];
-    jx_dual<DIR>(K, u, x, Fx, Nx);
-#pragma unroll
-    for (int c = 0; c < 5; ++c) {
-      double g = 0.0;
-#pragma unroll
-      for (int a = 0; a < 5; ++a) g += wv[a] * Fx[a].d[c] + zv[a] * Nx[a].d[c];
-      vb[c * NP + pt] -= g;
-    }
-  };
+  for (int m = 0; m < 5; ++m) {
+    y[m] = gp[m];
+    yb[m * NP + base + (int64_t)(n - 1) * st] = gp[m];
+  }
   for (int p = n - 2; p >= 0; --p) {
+    double t[5];
 #pragma unroll
     for (int m = 0; m < 5; ++m) {
-      double t = G(p, 25 + m);
+      t[m] = G(p, 25 + m);
 #pragma unroll
-      for (int c = 0; c < 5; ++c) t -= G(p, m * 5 + c) * y_next[c];
-      y_cur[m] = t;
+      for (int c = 0; c < 5; ++c) t[m] -= G(p, m * 5 + c) * y[c];
     }
 #pragma unroll
-    for (int m = 0; m < 5; ++m) yb[m * NP + base + (int64_t)p * st] = y_cur[m];
-    lin(p + 1, y_cur, y_next, y_nn);
+    for (int m = 0; m < 5; ++m) {
+      y[m] = t[m];
+      yb[m * NP + base + (int64_t)p * st] = t[m];
+    }
+  }
+}
+
+// The same with six lanes per line (few lines: see k_bt_line6).
+template <int DIR>
+__global__ void __launch_bounds__(32, 1) k_adj_line6(Fields F, Consts K, const Work* __restrict__ work, int lpi,
+                                                     double* __restrict__ yb, double* __restrict__ scr, int64_t nlt) {
+  extern __shared__ double bts[];
+  bt_line6<DIR, true>(F, K, work, lpi, yb, scr, nlt, 0, bts);
+}
+
+// The state dependence of T along one direction: at point q of every line,
+// vb_q -= (dF/du)^T w + (dN/du)^T z with F = fjac(u) x, N = njac(u) x (the
+// formulas of bt_jx), x the forward solution and
+//   w = tmp2 (y_{q-1} - y_{q+1}),  z = -tmp1 (y_{q-1} - 2 y_q + y_{q+1})
+// over the interior rows only.  F and N depend on u through the velocities, q,
+// E = u5/rho and 1/rho: the derivative of w.F + z.N in those six, then the
+// chain rule to u (about 110 FP64 instructions; five dual numbers through F
+// and N took about 700, inside the serial back substitution of the line).
+template <int DIR>
+__global__ void __launch_bounds__(128) k_adj_lin(Fields F, Consts K, const Work* __restrict__ work,
+                                                 const double* __restrict__ yb, const double* __restrict__ xs,
+                                                 double* __restrict__ vb) {
+  const Work wk = work[blockIdx.x];
+  const ZoneDev Z = F.zones[wk.zone];
+  const int t = wk.first + threadIdx.x;
+  if (t >= Z.nx * Z.ny * Z.nz) return;
+  const int ijk[3] = {t % Z.nx, (t / Z.nx) % Z.ny, t / (Z.nx * Z.ny)};
+  const int nn[3] = {Z.nx, Z.ny, Z.nz};
 #pragma unroll
-    for (int m = 0; m < 5; ++m) { y_nn[m] = y_next[m]; y_next[m] = y_cur[m]; }
+  for (int d = 0; d < 3; ++d)
+    if (d != DIR && (ijk[d] < 1 || ijk[d] > nn[d] - 2)) return;
+  const int q = ijk[DIR], n = nn[DIR];
+  const int64_t st = DIR == 0 ? 1 : DIR == 1 ? Z.nx : (int64_t)Z.nx * Z.ny;
+  const int64_t NP = F.NP, pt = Z.off + t;
+  const double tmp1 = DIR == 0 ? K.dttx1 : DIR == 1 ? K.dtty1 : K.dttz1;
+  const double tmp2 = DIR == 0 ? K.dttx2 : DIR == 1 ? K.dtty2 : K.dttz2;
+  const bool has_m = q - 1 >= 1 && q - 1 <= n - 2, has_c = q >= 1 && q <= n - 2, has_p = q + 1 >= 1 && q + 1 <= n - 2;
+  double w[5], z[5], x[5];
+#pragma unroll
+  for (int m = 0; m < 5; ++m) {
+    const double ym = has_m ? yb[m * NP + pt - st] : 0.0, yc = has_c ? yb[m * NP + pt] : 0.0,
+                 yp = has_p ? yb[m * NP + pt + st] : 0.0;
+    w[m] = tmp2 * (ym - yp);
+    z[m] = -tmp1 * (ym - 2.0 * yc + yp);
+    x[m] = xs[m * NP + pt];
   }
-  {
-    double zero[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    lin(0, zero, y_next, y_nn);
+  const BtState<double> s = bt_load_state<double>(F, pt);
+  const double ri = s.ri, qs = s.q, E = s.u5 * ri, *v = s.v;
+  constexpr int a = DIR + 1;
+  const double c1 = K.c1, c2 = K.c2, vn = v[DIR];
+  const double cn = K.con43 * K.c3c4, ct = K.c3c4, c1345 = K.c1345;
+  double d[3], tang = 0.0;
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    d[m] = x[m + 1] - v[m] * x[0];
+    if (m != DIR) tang += v[m] * x[m + 1];
   }
+  const double w4vn = w[4] * vn, z4r = z[4] * ri;
+  double gv[3], g_ri = z[4] * (c1345 * (x[4] - E * x[0]));
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    const double cm = m == DIR ? cn : ct;
+    gv[m] = z4r * (cm - c1345) * (d[m] - v[m] * x[0]) - z[m + 1] * (cm * ri) * x[0];
+    if (m != DIR) gv[m] += w[m + 1] * (x[a] - vn * x[0]) - c2 * x[m + 1] * (w[a] + w4vn);
+    g_ri += z[m + 1] * (cm * d[m]) + z[4] * ((cm - c1345) * v[m] * d[m]);
+  }
+#pragma unroll
+  for (int m = 0; m < 3; ++m)
+    if (m != DIR) gv[DIR] += w[m + 1] * d[m];
+  gv[DIR] += w[a] * ((2.0 - c2) * x[a] - 2.0 * vn * x[0]) +
+             w[4] * ((2.0 * c2 * qs - c1 * E) * x[0] - c2 * tang - 2.0 * c2 * vn * x[a] + c1 * x[4]);
+  const double g_q = c2 * (w[a] * x[0] + 2.0 * w4vn * x[0] - w[4] * x[a]);
+  const double g_E = c1 * (w[4] * x[a] - w4vn * x[0]) - z4r * c1345 * x[0];
+  double g0 = ri * g_ri + E * g_E;
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    const double g = gv[m] + v[m] * g_q;
+    g0 += v[m] * g;
+    vb[(m + 1) * NP + pt] -= ri * g;
+  }
+  vb[pt] += ri * g0;
+  vb[4 * NP + pt] -= ri * g_E;
 }
 
 // ---- compute_rhs adjoint --------------------------------------------------------
@@ -757,13 +796,28 @@ __global__ void __launch_bounds__(128) k_adj_sp_solve(Fields F, Consts K, const 
 }  // namespace adjk
 
 // ================================ launchers ================================
-void adj_launch_solve(int dir, const Fields& F, const Consts& K, const Work* work, int nwork, int tpb, double* yb,
-                      const double* xs, double* vb, double* scr, int64_t nlt, cudaStream_t s) {
+void adj_launch_solve(int dir, bool few, const Fields& F, const Consts& K, const Work* work, int nwork, int tpb,
+                      double* yb, double* scr, int64_t nlt, cudaStream_t s) {
   if (nwork <= 0) return;
+  if (few) {
+    const dim3 grid(nwork, (tpb + adjk::BTS_LINES - 1) / adjk::BTS_LINES);
+    if (dir == 0) adjk::k_adj_line6<0><<<grid, 32, adjk::BTS_SMEM, s>>>(F, K, work, tpb, yb, scr, nlt);
+    else if (dir == 1) adjk::k_adj_line6<1><<<grid, 32, adjk::BTS_SMEM, s>>>(F, K, work, tpb, yb, scr, nlt);
+    else adjk::k_adj_line6<2><<<grid, 32, adjk::BTS_SMEM, s>>>(F, K, work, tpb, yb, scr, nlt);
+    return;
+  }
   // one CTA of tpb (<= 128) threads per work item of tpb lines
-  if (dir == 0) adjk::k_adj_solve<0><<<nwork, tpb, 0, s>>>(F, K, work, yb, xs, vb, scr, nlt);
-  else if (dir == 1) adjk::k_adj_solve<1><<<nwork, tpb, 0, s>>>(F, K, work, yb, xs, vb, scr, nlt);
-  else adjk::k_adj_solve<2><<<nwork, tpb, 0, s>>>(F, K, work, yb, xs, vb, scr, nlt);
+  if (dir == 0) adjk::k_adj_solve<0><<<nwork, tpb, 0, s>>>(F, K, work, yb, scr, nlt);
+  else if (dir == 1) adjk::k_adj_solve<1><<<nwork, tpb, 0, s>>>(F, K, work, yb, scr, nlt);
+  else adjk::k_adj_solve<2><<<nwork, tpb, 0, s>>>(F, K, work, yb, scr, nlt);
+}
+
+void adj_launch_lin(int dir, const Fields& F, const Consts& K, const Work* work, int nwork, const double* yb,
+                    const double* xs, double* vb, cudaStream_t s) {
+  if (nwork <= 0) return;
+  if (dir == 0) adjk::k_adj_lin<0><<<nwork, 128, 0, s>>>(F, K, work, yb, xs, vb);
+  else if (dir == 1) adjk::k_adj_lin<1><<<nwork, 128, 0, s>>>(F, K, work, yb, xs, vb);
+  else adjk::k_adj_lin<2><<<nwork, 128, 0, s>>>(F, K, work, yb, xs, vb);
 }
 
 void adj_launch_rhs(const Fields& F, const Consts& K, const Work* work, int nwork, const double* rb, double* vb,

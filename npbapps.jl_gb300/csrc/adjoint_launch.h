@@ -8,11 +8,15 @@
 
 namespace npbmz {
 // Transposed block-tridiagonal sweep `dir` over the line work list (tpb lines
-// per item): yb (in: adjoint of the sweep's output, out: of its input),
-// vb -= the state linearisation; xs is the forward sweep's solution; scr
-// holds 30 doubles per line point ([(p*30+e)*nlt + line]).
-void adj_launch_solve(int dir, const Fields& F, const Consts& K, const Work* work, int nwork, int tpb, double* yb,
-                      const double* xs, double* vb, double* scr, int64_t nlt, cudaStream_t s);
+// per item; few: six lanes per line): yb (in: adjoint of the sweep's output,
+// out: of its input); scr holds 30 doubles per line point
+// ([(p*30+e)*nlt + line]).
+void adj_launch_solve(int dir, bool few, const Fields& F, const Consts& K, const Work* work, int nwork, int tpb,
+                      double* yb, double* scr, int64_t nlt, cudaStream_t s);
+// vb -= the sweep's state linearisation over the all-points work list; xs is
+// the forward sweep's solution.
+void adj_launch_lin(int dir, const Fields& F, const Consts& K, const Work* work, int nwork, const double* yb,
+                    const double* xs, double* vb, cudaStream_t s);
 // compute_rhs adjoint over the all-points work list (128 points per item).
 void adj_launch_rhs(const Fields& F, const Consts& K, const Work* work, int nwork, const double* rb, double* vb,
                     double* fb, cudaStream_t s);

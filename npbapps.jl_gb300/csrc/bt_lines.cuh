@@ -360,10 +360,13 @@ __host__ __device__ constexpr int bt_pidx(int r, int c) {  // place of P's entry
   return n;
 }
 
-template <int DIR>
-__global__ void __launch_bounds__(32, 1) k_bt_line6(Fields F, Consts K, const Work* __restrict__ work, int lpi,
-                                                 double* __restrict__ lhsc, int64_t nlt, int add_u) {
-  extern __shared__ double bts[];
+// ADJ: the transposed system of the adjoint instead (rows 0..n-1 of T^T, all
+// blocks of row p from the Jacobian at p): -C^T, B^T and -P^T in the places of
+// P, B and C, identity rows at the ends, r the adjoint in place.
+template <int DIR, bool ADJ>
+__device__ __forceinline__ void bt_line6(const Fields& F, const Consts& K, const Work* __restrict__ work, int lpi,
+                                         double* __restrict__ rhs, double* __restrict__ lhsc, int64_t nlt, int add_u,
+                                         double* bts) {
   const Work w = work[blockIdx.x];
   const ZoneDev Z = F.zones[w.zone];
   const int lane = threadIdx.x, g = lane < 30 ? lane / BTS_LANES : 0, c = lane < 30 ? lane - g * BTS_LANES : 5;
@@ -376,7 +379,6 @@ __global__ void __launch_bounds__(32, 1) k_bt_line6(Fields F, Consts K, const Wo
   line_geometry(Z, DIR, line, base, st);
   const int n = zone_line_len(Z, DIR);
   const int64_t gl = Z.lineoff[DIR] + line, NP = F.NP;
-  double* __restrict__ rhs = F.rhs;
   const BtK<double>& k = bt_consts<double>(K, DIR);
   auto at = [&](int q, int e) -> double& { return bts[((q % (2 * BTS_PTS)) * BTS_E + e) * BTS_LINES + g]; };
   const unsigned all = 0xffffffffu;
@@ -396,22 +398,29 @@ __global__ void __launch_bounds__(32, 1) k_bt_line6(Fields F, Consts K, const Wo
     double M[5][5];
     const int q = q0 + c;
     bt_gh<DIR, double>(k, s.ri, s.v, s.u5 * s.ri, s.q, J);
+    const bool end = ADJ && (q == 0 || q >= n - 1);
     bt_form_p<DIR, double>(J, M);
 #pragma unroll
     for (int i = 0; i < 5; ++i)
 #pragma unroll
-      for (int j = 0; j < 5; ++j)
-        if (anz<DIR>(i, j)) at(q, bt_pidx<DIR>(i, j)) = M[i][j];
+      for (int j = 0; j < 5; ++j) {
+        if (ADJ) at(q, 43 + j * 5 + i) = anz<DIR>(i, j) && q <= n - 3 ? -M[i][j] : 0.0;
+        else if (anz<DIR>(i, j)) at(q, bt_pidx<DIR>(i, j)) = M[i][j];
+      }
     bt_form_b<DIR, double>(J, M);
 #pragma unroll
     for (int i = 0; i < 5; ++i)
 #pragma unroll
-      for (int j = 0; j < 5; ++j) at(q, 18 + i * 5 + j) = hnz<DIR>(i, j) ? M[i][j] : 0.0;
+      for (int j = 0; j < 5; ++j)
+        at(q, 18 + (ADJ ? j * 5 + i : i * 5 + j)) = end ? (i == j ? 1.0 : 0.0) : hnz<DIR>(i, j) ? M[i][j] : 0.0;
     bt_form_c<DIR, double>(J, M);
 #pragma unroll
     for (int i = 0; i < 5; ++i)
 #pragma unroll
-      for (int j = 0; j < 5; ++j) at(q, 43 + i * 5 + j) = anz<DIR>(i, j) ? M[i][j] : 0.0;
+      for (int j = 0; j < 5; ++j) {
+        if (!ADJ) at(q, 43 + i * 5 + j) = anz<DIR>(i, j) ? M[i][j] : 0.0;
+        else if (anz<DIR>(i, j)) at(q, bt_pidx<DIR>(i, j)) = q >= 2 ? -M[i][j] : 0.0;
+      }
 #pragma unroll
     for (int m = 0; m < 5; ++m) at(q, 68 + m) = fr[m];
   };
@@ -423,12 +432,14 @@ __global__ void __launch_bounds__(32, 1) k_bt_line6(Fields F, Consts K, const Wo
   __syncwarp();
   double x[5];  // column c of C'_{p-1}, or r'_{p-1}
 #pragma unroll
-  for (int m = 0; m < 5; ++m) x[m] = is_r ? at(0, 68 + m) : 0.0;
-  for (int p = 1; p <= n - 2; ++p) {
-    if (p + 1 < n && (p + 1) % BTS_PTS == 0) {
+  for (int m = 0; m < 5; ++m) x[m] = is_r && !ADJ ? at(0, 68 + m) : 0.0;
+  const int first = ADJ ? 0 : 1, fin = ADJ ? n - 1 : n - 2;
+  for (int p = first; p <= fin; ++p) {
+    const int last_q = ADJ ? p : p + 1;  // the last point row p needs
+    if (last_q > 0 && last_q % BTS_PTS == 0) {
       __syncwarp();  // the slots of the block before the last are free
-      assemble(p + 1);
-      load(p + 1 + BTS_PTS);
+      assemble(last_q);
+      load(last_q + BTS_PTS);
       __syncwarp();
     }
     double b[5];
@@ -437,11 +448,12 @@ __global__ void __launch_bounds__(32, 1) k_bt_line6(Fields F, Consts K, const Wo
       b[i] = is_r ? at(p, 68 + i) : at(p, 18 + i * 5 + col);
 #pragma unroll
       for (int e = 0; e < 5; ++e)
-        if (anz<DIR>(i, e)) b[i] = fma(at(p - 1, bt_pidx<DIR>(i, e)), x[e], b[i]);
+        if (anz<DIR>(ADJ ? e : i, ADJ ? i : e))
+          b[i] = fma(at(ADJ ? p : p - 1, bt_pidx<DIR>(ADJ ? e : i, ADJ ? i : e)), x[e], b[i]);
     }
-    // right-hand side column: C_p's, from the state at p + 1, or r'
+    // right-hand side column: C_p's, or r'
 #pragma unroll
-    for (int i = 0; i < 5; ++i) x[i] = is_r ? b[i] : at(p + 1, 43 + i * 5 + col);
+    for (int i = 0; i < 5; ++i) x[i] = is_r ? b[i] : at(last_q, 43 + i * 5 + col);
     double up[5][5];  // the pivot columns' entries above the diagonal, for the back step
 #pragma unroll
     for (int t = 0; t < 5; ++t) {
@@ -484,21 +496,21 @@ __global__ void __launch_bounds__(32, 1) k_bt_line6(Fields F, Consts K, const Wo
   const int row = col;
   double cq[BACK][5], rq[BACK], uq[BACK];
   auto fetch = [&](int p, int slot) {
-    if (p < 1) return;
+    if (p < first) return;
     const int64_t pt = base + (int64_t)p * st;
 #pragma unroll
     for (int e = 0; e < 5; ++e) cq[slot][e] = lhsc[((int64_t)p * 25 + row * 5 + e) * nlt + gl];
     rq[slot] = rhs[row * NP + pt];
     uq[slot] = add_u ? F.u[row * NP + pt] : 0.0;
   };
-  double y = rhs[row * NP + base + (int64_t)(n - 1) * st];
+  double y = ADJ ? 0.0 : rhs[row * NP + base + (int64_t)(n - 1) * st];
 #pragma unroll
-  for (int q = 0; q < BACK; ++q) fetch(n - 2 - q, q);
-  for (int p0 = n - 2; p0 >= 1; p0 -= BACK) {
+  for (int q = 0; q < BACK; ++q) fetch(fin - q, q);
+  for (int p0 = fin; p0 >= first; p0 -= BACK) {
 #pragma unroll
     for (int q = 0; q < BACK; ++q) {
       const int p = p0 - q;
-      if (p < 1) break;
+      if (p < first) break;
       double t = rq[q];
 #pragma unroll
       for (int e = 0; e < 5; ++e) t = fma(-cq[q][e], __shfl_sync(all, y, src0 + e), t);
@@ -511,4 +523,11 @@ __global__ void __launch_bounds__(32, 1) k_bt_line6(Fields F, Consts K, const Wo
       fetch(p - BACK, q);
     }
   }
+}
+
+template <int DIR>
+__global__ void __launch_bounds__(32, 1) k_bt_line6(Fields F, Consts K, const Work* __restrict__ work, int lpi,
+                                                    double* __restrict__ lhsc, int64_t nlt, int add_u) {
+  extern __shared__ double bts[];
+  bt_line6<DIR, false>(F, K, work, lpi, F.rhs, lhsc, nlt, add_u, bts);
 }

@@ -1267,12 +1267,14 @@ int adjoint_back_step(npbmz_t* h, double* const x[3], double* ub, double* vb, do
   // the sweeps in reverse order
   for (int dir = 2; dir >= 0; --dir) {
     if (line_launches(h, dir, -1, [&](int lo, int hi, int tpb) {
-          adj_launch_solve(dir, F, h->K, h->wline_d[dir] + lo, hi - lo, tpb, yb, x[dir], vb, scr, h->nlines[dir],
-                           h->stream);
+          adj_launch_solve(dir, few_lines(h, dir, -1), F, h->K, h->wline_d[dir] + lo, hi - lo, tpb, yb, scr,
+                           h->nlines[dir], h->stream);
           CKL(h);
           return 0;
         }))
       return -1;
+    adj_launch_lin(dir, F, h->K, h->wpts_d, h->nwpts, yb, x[dir], vb, h->stream);
+    CKL(h);
   }
   // compute_rhs (yb is now the adjoint of rhs)
   adj_launch_rhs(F, h->K, h->wpts_d, h->nwpts, yb, vb, fb, h->stream);

@@ -216,6 +216,33 @@ def test_single_zone_adjoint_without_exchange():
         assert max(errs) <= ADJ_REL, errs
 
 
+@pytest.mark.parametrize("xw,yw,nz", [([5, 6, 8, 15], [5, 7, 9, 14], 5), ([8, 13], [6, 20], 14),
+                                      ([5, 6, 7, 8, 9, 11, 13, 17, 5, 6, 7, 10, 12, 19, 23, 24],
+                                       [5, 6, 7, 8, 9, 11, 13, 17, 5, 6, 7, 10, 12, 19, 23, 24], 12)],
+                         ids=["ragged-nz5", "ragged-nz14", "many-lines"])
+def test_bt_adjoint_matches_dual_numbers_on_ragged_zones(xw, yw, nz):
+    """Two steps on zones whose lines end around the kernels' groups of lines
+    and blocks of points, and on enough lines for one thread per line, along
+    one direction in u_0 and one in the forcing."""
+    from oracle import oracle
+
+    nx, ny, nzs, nbr = npbmz.zones_from_widths(xw, yw, nz)
+    g = npbmz.Geometry(npbmz.BT, nx, ny, nzs, nbr, sum(xw), sum(yw), nz, len(xw), len(yw))
+    p, _, target = build_case(g, 0.0008, seed=9)
+    J, gf, gu = p.adjoint(2, target, checkpoint_every=2)
+    u0, f0 = p.flatten(p.download_all(npbmz.U)), p.flatten(p.download_all(npbmz.FORCING))
+    rng = np.random.default_rng(2)
+    du = np.zeros((16, u0.size))
+    df = np.zeros((16, u0.size))
+    du[0] = rng.standard_normal(u0.size) * variable_scale(p, u0)
+    df[1] = rng.standard_normal(u0.size) * variable_scale(p, f0)
+    Jd, dJ, _ = oracle.tangent_objective(oracle.KIND_BT, g.nx, g.ny, g.nz, g.nbr, p.dt, g.gx, g.gy, g.gz, g.x_zones,
+                                         g.y_zones, u0, f0, p.flatten(target), 2, du0=du, dforcing=df)
+    assert J == pytest.approx(Jd, rel=1e-10)
+    ad = (du @ p.flatten(gu) + df @ p.flatten(gf))[:2]
+    assert np.all(np.abs(ad - dJ[:2]) <= DUAL_REL * np.abs(dJ[:2])), (ad, dJ[:2])
+
+
 def test_adjoint_rejects_bad_arguments(bt64):
     p, target, _ = bt64
     with pytest.raises(npbmz.NpbmzError, match="checkpoint_every"):
