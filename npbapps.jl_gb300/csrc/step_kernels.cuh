@@ -143,15 +143,27 @@ __global__ void __launch_bounds__(128) k_prim_w(Fields F, Consts K, const Work* 
 // ============================================================================
 
 // Fourth-order dissipation term at position q of an axis of n points
-// (1 <= q <= n-2): the start / middle / end stencils of the reference,
-// applied in the reference's order when n is so small that they overlap.
-__device__ __forceinline__ void dissip(double& r, int q, int n, double dssp, double um2, double um1, double u0,
-                                       double up1, double up2) {
-  if (q == 1) r -= dssp * (5.0e0 * u0 - 4.0e0 * up1 + up2);
-  if (q == 2) r -= dssp * (-4.0e0 * um1 + 6.0e0 * u0 - 4.0e0 * up1 + up2);
-  if (q >= 3 && q <= n - 4) r -= dssp * (um2 - 4.0e0 * um1 + 6.0 * u0 - 4.0e0 * up1 + up2);
-  if (q == n - 3) r -= dssp * (um2 - 4.0e0 * um1 + 6.0e0 * u0 - 4.0e0 * up1);
-  if (q == n - 2) r -= dssp * (um2 - 4.0e0 * um1 + 5.0e0 * u0);
+// (1 <= q <= n-2).  On six points and more one of the reference's start,
+// middle and end stencils applies: the middle one, whose missing terms enter
+// as zeros (0 + x and x - 0 are x), with 5 instead of 6 at the centre of the
+// outermost two -- no lane diverges, and the products with 4 and with dssp
+// (0.25 for every problem: set_constants) are exact, so fma rounds them and
+// their sum once, as the separate operations do.
+constexpr double DSSP = 0.25;
+__device__ __forceinline__ double dissip(double r, int q, int n, double um2, double um1, double u0, double up1,
+                                         double up2) {
+  if (n >= 6) {
+    const double a = q >= 3 ? um2 : 0.0, b = q >= 2 ? um1 : 0.0, d = q <= n - 3 ? up1 : 0.0, e = q <= n - 4 ? up2 : 0.0;
+    const double w = q == 1 || q == n - 2 ? 5.0e0 : 6.0e0;
+    return fma(-DSSP, fma(-4.0e0, d, fma(-4.0e0, b, a) + w * u0) + e, r);
+  }
+  // shorter axes: several stencils at one point, in the reference's order
+  if (q == 1) r -= DSSP * (5.0e0 * u0 - 4.0e0 * up1 + up2);
+  if (q == 2) r -= DSSP * (-4.0e0 * um1 + 6.0e0 * u0 - 4.0e0 * up1 + up2);
+  if (q >= 3 && q <= n - 4) r -= DSSP * (um2 - 4.0e0 * um1 + 6.0 * u0 - 4.0e0 * up1 + up2);
+  if (q == n - 3) r -= DSSP * (um2 - 4.0e0 * um1 + 6.0e0 * u0 - 4.0e0 * up1);
+  if (q == n - 2) r -= DSSP * (um2 - 4.0e0 * um1 + 5.0e0 * u0);
+  return r;
 }
 
 // Safe neighbour load along an axis: positions outside 0..n-1 are never used
@@ -161,30 +173,12 @@ __device__ __forceinline__ double ld_axis(const double* __restrict__ a, int64_t 
   return (qq >= 0 && qq < n) ? a[p + d * st] : a[p];
 }
 
-// Weighted form of the dissipation stencils at position q of an axis of n
-// points: the sum of the start / middle / end stencils that apply at q.  Used
-// by the FMA build (no lane divergence at zone edges); the exact build keeps
-// dissip() and the reference's operation order.
-__device__ __forceinline__ void dissip_weights(int q, int n, double w[5]) {
-  w[0] = w[1] = w[2] = w[3] = w[4] = 0.0;
-  if (q == 1) { w[2] += 5.0; w[3] -= 4.0; w[4] += 1.0; }
-  if (q == 2) { w[1] -= 4.0; w[2] += 6.0; w[3] -= 4.0; w[4] += 1.0; }
-  if (q >= 3 && q <= n - 4) { w[0] += 1.0; w[1] -= 4.0; w[2] += 6.0; w[3] -= 4.0; w[4] += 1.0; }
-  if (q == n - 3) { w[0] += 1.0; w[1] -= 4.0; w[2] += 6.0; w[3] -= 4.0; }
-  if (q == n - 2) { w[0] += 1.0; w[1] -= 4.0; w[2] += 5.0; }
-}
+// up - 2 u0 + um, left to right: 2 u0 is exact, so fma rounds the difference once
+__device__ __forceinline__ double d2(double up, double u0, double um) { return fma(-2.0e0, u0, up) + um; }
 
-#if NPBMZ_HAS_FP32
-#define NPBMZ_DISSIP(r, q, n, dssp, um2, um1, u0, up1, up2)                                        \
-  do {                                                                                              \
-    double w_[5];                                                                                   \
-    dissip_weights((q), (n), w_);                                                                   \
-    (r) -= (dssp) * (w_[0] * (um2) + w_[1] * (um1) + w_[2] * (u0) + w_[3] * (up1) + w_[4] * (up2)); \
-  } while (0)
-#else
-#define NPBMZ_DISSIP(r, q, n, dssp, um2, um1, u0, up1, up2) dissip((r), (q), (n), (dssp), (um2), (um1), (u0), (up1), (up2))
-#endif
-
+// Bound by the FP64 pipe in both builds; this kernel is the exact build's:
+// 304x208x17 938 -> 560 us with the products with 2, 4 and dssp fused (exactly)
+// into the sums and no branch per stencil.
 // One thread per INTERIOR point of a zone (the work list counts interior
 // points only): the boundary rhs equals the forcing and no solve rewrites
 // it, so it is set when the forcing or rhs is set, not every step.
@@ -214,25 +208,25 @@ __global__ void __launch_bounds__(128) k_rhs(Fields F, Consts K, const Work* __r
       double r[5];
       for (int m = 0; m < 5; ++m) r[m] = F.forcing[m * NP + p];
       const int64_t sx = 1, sy = Z.nx, sz = (int64_t)Z.nx * Z.ny;
-      const double c1 = K.c1, c2 = K.c2, con43 = K.con43, dssp = K.dssp;
+      const double c1 = K.c1, c2 = K.c2, con43 = K.con43;
       // ---------------- xi direction ----------------
       {
         const int64_t a = p + sx, b = p - sx;
         const double uijk = us[p], up1 = us[a], um1 = us[b];
-        r[0] += K.dx1tx1 * (u[a] - 2.0e0 * u[p] + u[b]) - K.tx2 * (u[NP + a] - u[NP + b]);
-        r[1] += K.dx2tx1 * (u[NP + a] - 2.0e0 * u[NP + p] + u[NP + b]) + K.xxcon2 * con43 * (up1 - 2.0e0 * uijk + um1) -
+        r[0] += K.dx1tx1 * d2(u[a], u[p], u[b]) - K.tx2 * (u[NP + a] - u[NP + b]);
+        r[1] += K.dx2tx1 * d2(u[NP + a], u[NP + p], u[NP + b]) + K.xxcon2 * con43 * d2(up1, uijk, um1) -
                 K.tx2 * (u[NP + a] * up1 - u[NP + b] * um1 + (u[4 * NP + a] - sqr[a] - u[4 * NP + b] + sqr[b]) * c2);
-        r[2] += K.dx3tx1 * (u[2 * NP + a] - 2.0e0 * u[2 * NP + p] + u[2 * NP + b]) +
-                K.xxcon2 * (vs[a] - 2.0e0 * vs[p] + vs[b]) - K.tx2 * (u[2 * NP + a] * up1 - u[2 * NP + b] * um1);
-        r[3] += K.dx4tx1 * (u[3 * NP + a] - 2.0e0 * u[3 * NP + p] + u[3 * NP + b]) +
-                K.xxcon2 * (ws[a] - 2.0e0 * ws[p] + ws[b]) - K.tx2 * (u[3 * NP + a] * up1 - u[3 * NP + b] * um1);
-        r[4] += K.dx5tx1 * (u[4 * NP + a] - 2.0e0 * u[4 * NP + p] + u[4 * NP + b]) +
-                K.xxcon3 * (qs[a] - 2.0e0 * qs[p] + qs[b]) + K.xxcon4 * (up1 * up1 - 2.0e0 * uijk * uijk + um1 * um1) +
-                K.xxcon5 * (u[4 * NP + a] * ri[a] - 2.0e0 * u[4 * NP + p] * ri[p] + u[4 * NP + b] * ri[b]) -
+        r[2] += K.dx3tx1 * d2(u[2 * NP + a], u[2 * NP + p], u[2 * NP + b]) +
+                K.xxcon2 * d2(vs[a], vs[p], vs[b]) - K.tx2 * (u[2 * NP + a] * up1 - u[2 * NP + b] * um1);
+        r[3] += K.dx4tx1 * d2(u[3 * NP + a], u[3 * NP + p], u[3 * NP + b]) +
+                K.xxcon2 * d2(ws[a], ws[p], ws[b]) - K.tx2 * (u[3 * NP + a] * up1 - u[3 * NP + b] * um1);
+        r[4] += K.dx5tx1 * d2(u[4 * NP + a], u[4 * NP + p], u[4 * NP + b]) +
+                K.xxcon3 * d2(qs[a], qs[p], qs[b]) + K.xxcon4 * d2(up1 * up1, uijk * uijk, um1 * um1) +
+                K.xxcon5 * d2(u[4 * NP + a] * ri[a], u[4 * NP + p] * ri[p], u[4 * NP + b] * ri[b]) -
                 K.tx2 * ((c1 * u[4 * NP + a] - c2 * sqr[a]) * up1 - (c1 * u[4 * NP + b] - c2 * sqr[b]) * um1);
         for (int m = 0; m < 5; ++m) {
           const double* um = u + m * NP;
-          NPBMZ_DISSIP(r[m], i, Z.nx, dssp, ld_axis(um, p, sx, i, -2, Z.nx), um[p - sx], um[p], um[p + sx],
+          r[m] = dissip(r[m], i, Z.nx, ld_axis(um, p, sx, i, -2, Z.nx), um[p - sx], um[p], um[p + sx],
                        ld_axis(um, p, sx, i, 2, Z.nx));
         }
       }
@@ -240,21 +234,21 @@ __global__ void __launch_bounds__(128) k_rhs(Fields F, Consts K, const Work* __r
       {
         const int64_t a = p + sy, b = p - sy;
         const double vijk = vs[p], vp1 = vs[a], vm1 = vs[b];
-        r[0] += K.dy1ty1 * (u[a] - 2.0e0 * u[p] + u[b]) - K.ty2 * (u[2 * NP + a] - u[2 * NP + b]);
-        r[1] += K.dy2ty1 * (u[NP + a] - 2.0e0 * u[NP + p] + u[NP + b]) + K.yycon2 * (us[a] - 2.0e0 * us[p] + us[b]) -
+        r[0] += K.dy1ty1 * d2(u[a], u[p], u[b]) - K.ty2 * (u[2 * NP + a] - u[2 * NP + b]);
+        r[1] += K.dy2ty1 * d2(u[NP + a], u[NP + p], u[NP + b]) + K.yycon2 * d2(us[a], us[p], us[b]) -
                 K.ty2 * (u[NP + a] * vp1 - u[NP + b] * vm1);
-        r[2] += K.dy3ty1 * (u[2 * NP + a] - 2.0e0 * u[2 * NP + p] + u[2 * NP + b]) +
-                K.yycon2 * con43 * (vp1 - 2.0e0 * vijk + vm1) -
+        r[2] += K.dy3ty1 * d2(u[2 * NP + a], u[2 * NP + p], u[2 * NP + b]) +
+                K.yycon2 * con43 * d2(vp1, vijk, vm1) -
                 K.ty2 * (u[2 * NP + a] * vp1 - u[2 * NP + b] * vm1 + (u[4 * NP + a] - sqr[a] - u[4 * NP + b] + sqr[b]) * c2);
-        r[3] += K.dy4ty1 * (u[3 * NP + a] - 2.0e0 * u[3 * NP + p] + u[3 * NP + b]) +
-                K.yycon2 * (ws[a] - 2.0e0 * ws[p] + ws[b]) - K.ty2 * (u[3 * NP + a] * vp1 - u[3 * NP + b] * vm1);
-        r[4] += K.dy5ty1 * (u[4 * NP + a] - 2.0e0 * u[4 * NP + p] + u[4 * NP + b]) +
-                K.yycon3 * (qs[a] - 2.0e0 * qs[p] + qs[b]) + K.yycon4 * (vp1 * vp1 - 2.0e0 * vijk * vijk + vm1 * vm1) +
-                K.yycon5 * (u[4 * NP + a] * ri[a] - 2.0e0 * u[4 * NP + p] * ri[p] + u[4 * NP + b] * ri[b]) -
+        r[3] += K.dy4ty1 * d2(u[3 * NP + a], u[3 * NP + p], u[3 * NP + b]) +
+                K.yycon2 * d2(ws[a], ws[p], ws[b]) - K.ty2 * (u[3 * NP + a] * vp1 - u[3 * NP + b] * vm1);
+        r[4] += K.dy5ty1 * d2(u[4 * NP + a], u[4 * NP + p], u[4 * NP + b]) +
+                K.yycon3 * d2(qs[a], qs[p], qs[b]) + K.yycon4 * d2(vp1 * vp1, vijk * vijk, vm1 * vm1) +
+                K.yycon5 * d2(u[4 * NP + a] * ri[a], u[4 * NP + p] * ri[p], u[4 * NP + b] * ri[b]) -
                 K.ty2 * ((c1 * u[4 * NP + a] - c2 * sqr[a]) * vp1 - (c1 * u[4 * NP + b] - c2 * sqr[b]) * vm1);
         for (int m = 0; m < 5; ++m) {
           const double* um = u + m * NP;
-          NPBMZ_DISSIP(r[m], j, Z.ny, dssp, ld_axis(um, p, sy, j, -2, Z.ny), um[p - sy], um[p], um[p + sy],
+          r[m] = dissip(r[m], j, Z.ny, ld_axis(um, p, sy, j, -2, Z.ny), um[p - sy], um[p], um[p + sy],
                        ld_axis(um, p, sy, j, 2, Z.ny));
         }
       }
@@ -262,21 +256,21 @@ __global__ void __launch_bounds__(128) k_rhs(Fields F, Consts K, const Work* __r
       {
         const int64_t a = p + sz, b = p - sz;
         const double wijk = ws[p], wp1 = ws[a], wm1 = ws[b];
-        r[0] += K.dz1tz1 * (u[a] - 2.0e0 * u[p] + u[b]) - K.tz2 * (u[3 * NP + a] - u[3 * NP + b]);
-        r[1] += K.dz2tz1 * (u[NP + a] - 2.0e0 * u[NP + p] + u[NP + b]) + K.zzcon2 * (us[a] - 2.0e0 * us[p] + us[b]) -
+        r[0] += K.dz1tz1 * d2(u[a], u[p], u[b]) - K.tz2 * (u[3 * NP + a] - u[3 * NP + b]);
+        r[1] += K.dz2tz1 * d2(u[NP + a], u[NP + p], u[NP + b]) + K.zzcon2 * d2(us[a], us[p], us[b]) -
                 K.tz2 * (u[NP + a] * wp1 - u[NP + b] * wm1);
-        r[2] += K.dz3tz1 * (u[2 * NP + a] - 2.0e0 * u[2 * NP + p] + u[2 * NP + b]) +
-                K.zzcon2 * (vs[a] - 2.0e0 * vs[p] + vs[b]) - K.tz2 * (u[2 * NP + a] * wp1 - u[2 * NP + b] * wm1);
-        r[3] += K.dz4tz1 * (u[3 * NP + a] - 2.0e0 * u[3 * NP + p] + u[3 * NP + b]) +
-                K.zzcon2 * con43 * (wp1 - 2.0e0 * wijk + wm1) -
+        r[2] += K.dz3tz1 * d2(u[2 * NP + a], u[2 * NP + p], u[2 * NP + b]) +
+                K.zzcon2 * d2(vs[a], vs[p], vs[b]) - K.tz2 * (u[2 * NP + a] * wp1 - u[2 * NP + b] * wm1);
+        r[3] += K.dz4tz1 * d2(u[3 * NP + a], u[3 * NP + p], u[3 * NP + b]) +
+                K.zzcon2 * con43 * d2(wp1, wijk, wm1) -
                 K.tz2 * (u[3 * NP + a] * wp1 - u[3 * NP + b] * wm1 + (u[4 * NP + a] - sqr[a] - u[4 * NP + b] + sqr[b]) * c2);
-        r[4] += K.dz5tz1 * (u[4 * NP + a] - 2.0e0 * u[4 * NP + p] + u[4 * NP + b]) +
-                K.zzcon3 * (qs[a] - 2.0e0 * qs[p] + qs[b]) + K.zzcon4 * (wp1 * wp1 - 2.0e0 * wijk * wijk + wm1 * wm1) +
-                K.zzcon5 * (u[4 * NP + a] * ri[a] - 2.0e0 * u[4 * NP + p] * ri[p] + u[4 * NP + b] * ri[b]) -
+        r[4] += K.dz5tz1 * d2(u[4 * NP + a], u[4 * NP + p], u[4 * NP + b]) +
+                K.zzcon3 * d2(qs[a], qs[p], qs[b]) + K.zzcon4 * d2(wp1 * wp1, wijk * wijk, wm1 * wm1) +
+                K.zzcon5 * d2(u[4 * NP + a] * ri[a], u[4 * NP + p] * ri[p], u[4 * NP + b] * ri[b]) -
                 K.tz2 * ((c1 * u[4 * NP + a] - c2 * sqr[a]) * wp1 - (c1 * u[4 * NP + b] - c2 * sqr[b]) * wm1);
         for (int m = 0; m < 5; ++m) {
           const double* um = u + m * NP;
-          NPBMZ_DISSIP(r[m], k, Z.nz, dssp, ld_axis(um, p, sz, k, -2, Z.nz), um[p - sz], um[p], um[p + sz],
+          r[m] = dissip(r[m], k, Z.nz, ld_axis(um, p, sz, k, -2, Z.nz), um[p - sz], um[p], um[p + sz],
                        ld_axis(um, p, sz, k, 2, Z.nz));
         }
       }
@@ -627,9 +621,22 @@ __device__ __forceinline__ void bt_jac(const Consts& K, T tmp1, T u2, T u3, T u4
   }
 }
 
+// f <- tmp2 * f, n <- tmp1 * n: the products lhsa, lhsb and lhsc are sums of
+// (-tmp2 * f is their negative, tmp1 * 2.0 * n their double, both exactly).
+template <int DIR, typename T>
+__device__ __forceinline__ void bt_scale(T f[5][5], T n[5][5], T tmp1, T tmp2) {
+#pragma unroll
+  for (int a = 0; a < 5; ++a)
+#pragma unroll
+    for (int b = 0; b < 5; ++b) {
+      if (fnz<DIR>(a, b)) f[a][b] = tmp2 * f[a][b];
+      if (nnz(a, b)) n[a][b] = tmp1 * n[a][b];
+    }
+}
+
 // lhsa at the point after the Jacobian point: -tmp2*f - tmp1*n - tmp1*d (diag).
 template <int DIR, typename T>
-__device__ __forceinline__ void bt_asm_a(const T f[5][5], const T n[5][5], T tmp1, T tmp2, const T dd[5], T A[5][5]) {
+__device__ __forceinline__ void bt_asm_a(const T f[5][5], const T n[5][5], T tmp1, const T dd[5], T A[5][5]) {
 #pragma unroll
   for (int a = 0; a < 5; ++a)
 #pragma unroll
@@ -637,8 +644,8 @@ __device__ __forceinline__ void bt_asm_a(const T f[5][5], const T n[5][5], T tmp
       if (!anz<DIR>(a, b)) continue;
       T t;
       bool have = false;
-      if (fnz<DIR>(a, b)) { t = -tmp2 * f[a][b]; have = true; }
-      if (nnz(a, b)) { t = have ? t - tmp1 * n[a][b] : -(tmp1 * n[a][b]); have = true; }
+      if (fnz<DIR>(a, b)) { t = -f[a][b]; have = true; }
+      if (nnz(a, b)) { t = have ? t - n[a][b] : -n[a][b]; have = true; }
       if (a == b) { t = have ? t - tmp1 * dd[a] : -(tmp1 * dd[a]); }
       A[a][b] = t;
     }
@@ -646,15 +653,15 @@ __device__ __forceinline__ void bt_asm_a(const T f[5][5], const T n[5][5], T tmp
 
 // lhsc at the point before the Jacobian point: tmp2*f - tmp1*n - tmp1*d (diag).
 template <int DIR, typename T>
-__device__ __forceinline__ void bt_asm_c(const T f[5][5], const T n[5][5], T tmp1, T tmp2, const T dd[5], T C[5][5]) {
+__device__ __forceinline__ void bt_asm_c(const T f[5][5], const T n[5][5], T tmp1, const T dd[5], T C[5][5]) {
 #pragma unroll
   for (int a = 0; a < 5; ++a)
 #pragma unroll
     for (int b = 0; b < 5; ++b) {
       T t = (T)0.0;
       bool have = false;
-      if (fnz<DIR>(a, b)) { t = tmp2 * f[a][b]; have = true; }
-      if (nnz(a, b)) { t = have ? t - tmp1 * n[a][b] : -(tmp1 * n[a][b]); have = true; }
+      if (fnz<DIR>(a, b)) { t = f[a][b]; have = true; }
+      if (nnz(a, b)) { t = have ? t - n[a][b] : -n[a][b]; have = true; }
       if (a == b) { t = have ? t - tmp1 * dd[a] : -(tmp1 * dd[a]); }
       C[a][b] = t;
     }
@@ -670,25 +677,36 @@ __device__ __forceinline__ void bt_asm_b(const T n[5][5], T tmp1, const T dd[5],
       if (!bnz(a, b)) continue;
       if (a == b) {
         T t = (T)1.0;
-        if (nnz(a, b)) t = t + tmp1 * (T)2.0 * n[a][b];
+        if (nnz(a, b)) t = fma((T)2.0, n[a][b], t);
         B[a][b] = t + tmp1 * (T)2.0 * dd[a];
       } else {
-        B[a][b] = tmp1 * (T)2.0 * n[a][b];
+        B[a][b] = (T)2.0 * n[a][b];
       }
     }
 }
 
-// Pivot reciprocal: IEEE division in FP64 (the reference's arithmetic); in
-// the FP32 solves, which a double-float refinement corrects, the fast
-// reciprocal (within 2 ulp).
+// Pivot reciprocal: correctly rounded in FP64 (the reference's division), in
+// the FMA build within one ulp; in the FP32 solves, which a double-float
+// refinement corrects, the fast reciprocal (within 2 ulp).
 template <typename T>
-__device__ __forceinline__ T pivot_recip(T b) { return (T)1.0 / b; }
+__device__ __forceinline__ T pivot_recip(T b) { return NPBMZ_HAS_FP32 ? nr_rcp(b) : rcp_rn(b); }
 template <>
 __device__ __forceinline__ float pivot_recip<float>(float b) { return __fdividef(1.0f, b); }
 
+// Columns of C that are nonzero in pivot row p when it is reached: the block's
+// own, and all once the row of the normal momentum (all nonzero) has been the
+// pivot; the other columns hold exact zeros, whose operations are skipped.
+template <int DIR>
+__host__ __device__ constexpr bool cfull(int p, int c) {
+  if (p > DIR + 1) return true;
+  for (int q = 0; q <= p; ++q)
+    if (anz<DIR>(q, c)) return true;
+  return false;
+}
+
 // binvcrhs (src/BT/solve_subs.jl:468-723): Gauss-Jordan on B, no pivoting,
 // applied to C and r.
-template <typename T>
+template <int DIR, typename T>
 __device__ __forceinline__ void binvcrhs(T B[5][5], T C[5][5], T r[5]) {
 #pragma unroll
   for (int p = 0; p < 5; ++p) {
@@ -696,7 +714,8 @@ __device__ __forceinline__ void binvcrhs(T B[5][5], T C[5][5], T r[5]) {
 #pragma unroll
     for (int c = p + 1; c < 5; ++c) B[p][c] *= pivot;
 #pragma unroll
-    for (int c = 0; c < 5; ++c) C[p][c] *= pivot;
+    for (int c = 0; c < 5; ++c)
+      if (cfull<DIR>(p, c)) C[p][c] *= pivot;
     r[p] *= pivot;
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
@@ -705,7 +724,8 @@ __device__ __forceinline__ void binvcrhs(T B[5][5], T C[5][5], T r[5]) {
 #pragma unroll
       for (int c = p + 1; c < 5; ++c) B[q][c] -= coeff * B[p][c];
 #pragma unroll
-      for (int c = 0; c < 5; ++c) C[q][c] -= coeff * C[p][c];
+      for (int c = 0; c < 5; ++c)
+        if (cfull<DIR>(p, c)) C[q][c] -= coeff * C[p][c];
       r[q] -= coeff * r[p];
     }
   }
@@ -763,11 +783,13 @@ __global__ void __launch_bounds__(128) k_bt_solve(Fields F, Consts K, const Work
   // Jacobian at point 0 -> lhsa at 1; at point 1 -> lhsb at 1 and lhsa at 2.
   bt_load_point<DIR, T>(F, base, ri, u2, u3, u4, u5, q);
   bt_jac<DIR, T>(K, ri, u2, u3, u4, u5, q, f, nj);
-  bt_asm_a<DIR, T>(f, nj, tmp1, tmp2, dd, Acur);
+  bt_scale<DIR, T>(f, nj, tmp1, tmp2);
+  bt_asm_a<DIR, T>(f, nj, tmp1, dd, Acur);
   bt_load_point<DIR, T>(F, base + st, ri, u2, u3, u4, u5, q);
   bt_jac<DIR, T>(K, ri, u2, u3, u4, u5, q, f, nj);
+  bt_scale<DIR, T>(f, nj, tmp1, tmp2);
   bt_asm_b<T>(nj, tmp1, dd, Bcur);
-  if (n - 2 >= 2) bt_asm_a<DIR, T>(f, nj, tmp1, tmp2, dd, Anext);
+  if (n - 2 >= 2) bt_asm_a<DIR, T>(f, nj, tmp1, dd, Anext);
 
   for (int p = 1; p <= n - 2; ++p) {
     const int64_t pt = base + p * st;
@@ -808,16 +830,17 @@ __global__ void __launch_bounds__(128) k_bt_solve(Fields F, Consts K, const Work
     // Jacobian at p+1 -> lhsc_p, lhsb_{p+1}, lhsa_{p+2}
     bt_load_point<DIR, T>(F, pt + st, ri, u2, u3, u4, u5, q);
     bt_jac<DIR, T>(K, ri, u2, u3, u4, u5, q, f, nj);
+    bt_scale<DIR, T>(f, nj, tmp1, tmp2);
     T C[5][5];
-    bt_asm_c<DIR, T>(f, nj, tmp1, tmp2, dd, C);
+    bt_asm_c<DIR, T>(f, nj, tmp1, dd, C);
 #pragma unroll
     for (int a = 0; a < 5; ++a)
 #pragma unroll
       for (int b = 0; b < 5; ++b)
         if (anz<DIR>(a, b)) Acur[a][b] = Anext[a][b];
     if (p + 1 <= n - 2) bt_asm_b<T>(nj, tmp1, dd, Bcur);
-    if (p + 2 <= n - 2) bt_asm_a<DIR, T>(f, nj, tmp1, tmp2, dd, Anext);
-    binvcrhs<T>(B, C, r);
+    if (p + 2 <= n - 2) bt_asm_a<DIR, T>(f, nj, tmp1, dd, Anext);
+    binvcrhs<DIR, T>(B, C, r);
 #pragma unroll
     for (int a = 0; a < 5; ++a)
 #pragma unroll
