@@ -242,12 +242,12 @@ __global__ void __launch_bounds__(128) k_adj_solve(Fields F, Consts K, const Wor
   }
 }
 
-// The same with six lanes per line (few lines: see k_bt_line6).
+// The same with twelve lanes per line (few lines: see bt_line12).
 template <int DIR>
-__global__ void __launch_bounds__(32, 1) k_adj_line6(Fields F, Consts K, const Work* __restrict__ work, int lpi,
+__global__ void __launch_bounds__(64, 1) k_adj_line12(Fields F, Consts K, const Work* __restrict__ work, int lpi,
                                                      double* __restrict__ yb, double* __restrict__ scr, int64_t nlt) {
   extern __shared__ double bts[];
-  bt_line6<DIR, true>(F, K, work, lpi, yb, scr, nlt, 0, bts);
+  bt_line12<DIR, true>(F, K, work, lpi, yb, scr, nlt, 0, bts);
 }
 
 // The state dependence of T along one direction: at point q of every line,
@@ -801,9 +801,9 @@ void adj_launch_solve(int dir, bool few, const Fields& F, const Consts& K, const
   if (nwork <= 0) return;
   if (few) {
     const dim3 grid(nwork, (tpb + adjk::BTS_LINES - 1) / adjk::BTS_LINES);
-    if (dir == 0) adjk::k_adj_line6<0><<<grid, 32, adjk::BTS_SMEM, s>>>(F, K, work, tpb, yb, scr, nlt);
-    else if (dir == 1) adjk::k_adj_line6<1><<<grid, 32, adjk::BTS_SMEM, s>>>(F, K, work, tpb, yb, scr, nlt);
-    else adjk::k_adj_line6<2><<<grid, 32, adjk::BTS_SMEM, s>>>(F, K, work, tpb, yb, scr, nlt);
+    if (dir == 0) adjk::k_adj_line12<0><<<grid, 64, adjk::BTS_SMEM, s>>>(F, K, work, tpb, yb, scr, nlt);
+    else if (dir == 1) adjk::k_adj_line12<1><<<grid, 64, adjk::BTS_SMEM, s>>>(F, K, work, tpb, yb, scr, nlt);
+    else adjk::k_adj_line12<2><<<grid, 64, adjk::BTS_SMEM, s>>>(F, K, work, tpb, yb, scr, nlt);
     return;
   }
   // one CTA of tpb (<= 128) threads per work item of tpb lines

@@ -8,7 +8,7 @@
 
 namespace npbmz {
 // Transposed block-tridiagonal sweep `dir` over the line work list (tpb lines
-// per item; few: six lanes per line): yb (in: adjoint of the sweep's output,
+// per item; few: twelve lanes per line): yb (in: adjoint of the sweep's output,
 // out: of its input); scr holds 30 doubles per line point
 // ([(p*30+e)*nlt + line]).
 void adj_launch_solve(int dir, bool few, const Fields& F, const Consts& K, const Work* work, int nwork, int tpb,

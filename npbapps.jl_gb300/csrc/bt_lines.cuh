@@ -14,9 +14,7 @@
 // on the right-hand sides.  The elimination visits the row of rho first, then
 // the two tangential momenta, the normal momentum and the energy: the rows
 // visited first have few nonzeros in C, whose zero columns are skipped until
-// they fill.  Every multiply-add is written as fma, so that the two mappings
-// of the FP64 solve (one thread per line, six lanes per line) give the same
-// bits.  One point takes 389 FP64 instructions (531 with the blocks
+// they fill.  One point takes 389 FP64 instructions (531 with the blocks
 // formed entry by entry and Gauss-Jordan): five steps of 128x128x16 went from
 // 11.16 to 9.17 ms.  The FP32 sweeps of 480x320x28 (whose second pass also no
 // longer stores C' again) went from 640, 610 and 681 to 586, 568 and 635 us.
@@ -323,31 +321,38 @@ __global__ void __launch_bounds__(128) k_bt_line(Fields F, Consts K, const Work*
 }
 
 // ---------------------------------------------------------------------------
-// The same solve with six lanes per line (FP64), five lines per warp, one
-// warp per block: for launches with too few lines to give every SM quarter a
-// warp.  An SM quarter takes an FP64 warp instruction every 64 cycles
-// whatever its active lanes, and a line advances one point per 389
-// instructions of k_bt_line; here the work of a point is spread over the
-// group's lanes, about 95 instructions per lane (and 1.6 times k_bt_line's
-// warp instructions in all, so full launches keep that one).  Sweeps (us,
-// k_bt_line / here): 24x24x6 x and y 217 / 74, z 65 / 25; 64x64x8 362 / 120,
-// 95 / 39; 128x128x16 746 / 381, z 235 / 303; 304x208x17 x 1123 / 1177, z
-// 653 / 1105 (few_lines in npbmz_api.cu draws the line).
+// The same solve for launches with too few lines to give every SM quarter a
+// warp (FP64): twelve lanes per line, five lines per block of two warps.  An
+// SM quarter takes an FP64 warp instruction every 64 cycles whatever its
+// active lanes, and a line advances one point per 389 instructions of
+// k_bt_line; here its work is spread over lanes and over both its ends.
+//   - Warp 0 eliminates each line from point 0 up to the middle, warp 1 from
+//     point n-1 down (the same line with G turned to -G).  At the seam
+//     x_A = r'_A - C'_A x_B and x_B = r'_B - C'_B x_A, so each half solves
+//     (I - C'_A C'_B) x_A = r'_A - C'_A r'_B and substitutes back to its end.
 //   - G, H, P, B, C of six consecutive points at a time, one point per lane,
-//     into shared memory (they do not depend on the elimination);
-//   - lane c < 5 keeps column c of C', lane 5 keeps r': B' and r' are one
+//     into shared memory (they do not depend on the elimination).
+//   - Lane c < 5 keeps column c of C', lane 5 keeps r': B' and r' are one
 //     column per lane (18 multiply-adds), and each step of the elimination
 //     takes the pivot column from its lane by shuffles and updates the lane's
-//     column of B' and its column of C (lane 5: r');
-//   - back substitution: lane i < 5 holds row i.
-// Each element sees the operations of k_bt_line in the same order (those
-// k_bt_line skips multiply structural zeros), so the results are the same.
+//     column of B' and its column of C (lane 5: r'), about 95 instructions per
+//     lane and point.
+//   - Back substitution: lane i < 5 holds row i.
+// ADJ: the transposed system of the adjoint (rows 0..n-1 of T^T, all blocks of
+// row p from the Jacobian at p): -C^T, B^T and -P^T in the places of P, B and
+// C, identity rows at the ends, r the adjoint in place.
+// Sweeps in us, k_bt_line / six lanes from one end / here: 24x24x6 x and y
+// 217 / 74 / 45, z 65 / 25 / 20; 64x64x8 362 / 120 / 81, z (8 points) 95 / 39 /
+// 52; 128x128x16 x 746 / 383 / 340 (few_lines in npbmz_api.cu draws the line).
 // ---------------------------------------------------------------------------
-constexpr int BTS_LINES = 5;   // lines per warp
-constexpr int BTS_LANES = 6;   // lanes per line
+constexpr int BTS_LINES = 5;   // lines per block
+constexpr int BTS_LANES = 6;   // lanes per half of a line
 constexpr int BTS_PTS = 6;     // points assembled at a time
+constexpr int BTS_SLOTS = 8;   // points kept: a block of points and the two before it
 constexpr int BTS_E = 18 + 25 + 25 + 5;  // doubles per point: P (nonzeros), B, C, rhs
-constexpr size_t BTS_SMEM = (size_t)2 * BTS_PTS * BTS_E * BTS_LINES * sizeof(double);
+constexpr int BTS_RING = BTS_SLOTS * BTS_E * BTS_LINES;  // doubles per warp
+constexpr size_t BTS_SMEM = (size_t)(2 * BTS_RING + 2 * BTS_LINES * 30) * sizeof(double);
+static_assert(BTS_SMEM <= 48 * 1024, "no opt-in to larger shared memory");
 
 template <int DIR>
 __host__ __device__ constexpr int bt_pidx(int r, int c) {  // place of P's entry (r, c) among its 18 nonzeros
@@ -360,100 +365,108 @@ __host__ __device__ constexpr int bt_pidx(int r, int c) {  // place of P's entry
   return n;
 }
 
-// ADJ: the transposed system of the adjoint instead (rows 0..n-1 of T^T, all
-// blocks of row p from the Jacobian at p): -C^T, B^T and -P^T in the places of
-// P, B and C, identity rows at the ends, r the adjoint in place.
 template <int DIR, bool ADJ>
-__device__ __forceinline__ void bt_line6(const Fields& F, const Consts& K, const Work* __restrict__ work, int lpi,
-                                         double* __restrict__ rhs, double* __restrict__ lhsc, int64_t nlt, int add_u,
-                                         double* bts) {
+__device__ __forceinline__ void bt_line12(const Fields& F, const Consts& K, const Work* __restrict__ work, int lpi,
+                                          double* __restrict__ rhs, double* __restrict__ lhsc, int64_t nlt, int add_u,
+                                          double* smem) {
   const Work w = work[blockIdx.x];
   const ZoneDev Z = F.zones[w.zone];
-  const int lane = threadIdx.x, g = lane < 30 ? lane / BTS_LANES : 0, c = lane < 30 ? lane - g * BTS_LANES : 5;
+  const int half = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane < 30 ? lane / BTS_LANES : 0, c = lane < 30 ? lane - g * BTS_LANES : 5;
   const int off = blockIdx.y * BTS_LINES;
   const int last = min(w.first + lpi, zone_lines(Z, DIR)) - 1, want = w.first + off + g;
-  if (w.first + off > last) return;  // the whole warp
+  if (w.first + off > last) return;  // the whole block
   const bool own = lane < 30 && want <= last;  // lanes without a line of their own compute line `last`, store nothing
   const int line = min(want, last);
   int64_t base, st;
   line_geometry(Z, DIR, line, base, st);
   const int n = zone_line_len(Z, DIR);
   const int64_t gl = Z.lineoff[DIR] + line, NP = F.NP;
-  const BtK<double>& k = bt_consts<double>(K, DIR);
-  auto at = [&](int q, int e) -> double& { return bts[((q % (2 * BTS_PTS)) * BTS_E + e) * BTS_LINES + g]; };
+  // rows first .. fin of this half, in its own index j: point j from its end
+  const int rows = ADJ ? n : n - 2, near = (rows + 1) >> 1;
+  const int first = ADJ ? 0 : 1, fin = first - 1 + (half ? rows - near : near);
+  auto gq = [&](int j) -> int { return half ? n - 1 - j : j; };
+  auto pnt = [&](int j) -> int64_t { return base + (int64_t)gq(j) * st; };
+  BtK<double> k = bt_consts<double>(K, DIR);
+  if (half) {
+    k.t2 = -k.t2;
+    k.c2t2 = -k.c2t2;
+    k.c1t2 = -k.c1t2;
+  }
+  double* ring = smem + half * BTS_RING;
+  auto at = [&](int j, int e) -> double& { return ring[((j % BTS_SLOTS) * BTS_E + e) * BTS_LINES + g]; };
   const unsigned all = 0xffffffffu;
   const int src0 = g * BTS_LANES;  // the group's lane 0
-  // this lane's point of the block of points q0 .. q0+5
+  const bool is_r = c == 5;
+  const int col = is_r ? 0 : c;
+  // this lane's point of the block of points j0 .. j0+5
   BtState<double> s;
   double fr[5];
-  auto load = [&](int q0) {
-    const int q = min(q0 + c, n - 1);
-    s = bt_load_state<double>(F, base + (int64_t)q * st);
+  auto load = [&](int j0) {
+    const int j = min(j0 + c, n - 1);
+    s = bt_load_state<double>(F, pnt(j));
 #pragma unroll
-    for (int m = 0; m < 5; ++m) fr[m] = rhs[m * NP + base + (int64_t)q * st];
+    for (int m = 0; m < 5; ++m) fr[m] = j <= fin || j == 0 ? rhs[m * NP + pnt(j)] : 0.0;
   };
-  auto assemble = [&](int q0) {
+  auto assemble = [&](int j0) {
     if (lane >= 30) return;
     BtGH<DIR, double> J;
     double M[5][5];
-    const int q = q0 + c;
+    const int j = j0 + c;
+    const bool end = ADJ && (j == 0 || j >= n - 1);
     bt_gh<DIR, double>(k, s.ri, s.v, s.u5 * s.ri, s.q, J);
-    const bool end = ADJ && (q == 0 || q >= n - 1);
     bt_form_p<DIR, double>(J, M);
 #pragma unroll
-    for (int i = 0; i < 5; ++i)
+    for (int a = 0; a < 5; ++a)
 #pragma unroll
-      for (int j = 0; j < 5; ++j) {
-        if (ADJ) at(q, 43 + j * 5 + i) = anz<DIR>(i, j) && q <= n - 3 ? -M[i][j] : 0.0;
-        else if (anz<DIR>(i, j)) at(q, bt_pidx<DIR>(i, j)) = M[i][j];
+      for (int b = 0; b < 5; ++b) {
+        if (ADJ) at(j, 43 + b * 5 + a) = anz<DIR>(a, b) && j <= n - 3 ? -M[a][b] : 0.0;
+        else if (anz<DIR>(a, b)) at(j, bt_pidx<DIR>(a, b)) = M[a][b];
       }
     bt_form_b<DIR, double>(J, M);
 #pragma unroll
-    for (int i = 0; i < 5; ++i)
+    for (int a = 0; a < 5; ++a)
 #pragma unroll
-      for (int j = 0; j < 5; ++j)
-        at(q, 18 + (ADJ ? j * 5 + i : i * 5 + j)) = end ? (i == j ? 1.0 : 0.0) : hnz<DIR>(i, j) ? M[i][j] : 0.0;
+      for (int b = 0; b < 5; ++b)
+        at(j, 18 + (ADJ ? b * 5 + a : a * 5 + b)) = end ? (a == b ? 1.0 : 0.0) : hnz<DIR>(a, b) ? M[a][b] : 0.0;
     bt_form_c<DIR, double>(J, M);
 #pragma unroll
-    for (int i = 0; i < 5; ++i)
+    for (int a = 0; a < 5; ++a)
 #pragma unroll
-      for (int j = 0; j < 5; ++j) {
-        if (!ADJ) at(q, 43 + i * 5 + j) = anz<DIR>(i, j) ? M[i][j] : 0.0;
-        else if (anz<DIR>(i, j)) at(q, bt_pidx<DIR>(i, j)) = q >= 2 ? -M[i][j] : 0.0;
+      for (int b = 0; b < 5; ++b) {
+        if (!ADJ) at(j, 43 + a * 5 + b) = anz<DIR>(a, b) ? M[a][b] : 0.0;
+        else if (anz<DIR>(a, b)) at(j, bt_pidx<DIR>(a, b)) = j >= 2 ? -M[a][b] : 0.0;
       }
 #pragma unroll
-    for (int m = 0; m < 5; ++m) at(q, 68 + m) = fr[m];
+    for (int m = 0; m < 5; ++m) at(j, 68 + m) = fr[m];
   };
-  const bool is_r = c == 5;
-  const int col = is_r ? 0 : c;
   load(0);
   assemble(0);
   load(BTS_PTS);
   __syncwarp();
-  double x[5];  // column c of C'_{p-1}, or r'_{p-1}
+  double x[5];  // column c of C'_{j-1}, or r'_{j-1}
 #pragma unroll
   for (int m = 0; m < 5; ++m) x[m] = is_r && !ADJ ? at(0, 68 + m) : 0.0;
-  const int first = ADJ ? 0 : 1, fin = ADJ ? n - 1 : n - 2;
-  for (int p = first; p <= fin; ++p) {
-    const int last_q = ADJ ? p : p + 1;  // the last point row p needs
-    if (last_q > 0 && last_q % BTS_PTS == 0) {
-      __syncwarp();  // the slots of the block before the last are free
-      assemble(last_q);
-      load(last_q + BTS_PTS);
+  for (int j = first; j <= fin; ++j) {
+    const int next = ADJ ? j : j + 1;  // the last point row j needs
+    if (next > 0 && next % BTS_PTS == 0) {
+      __syncwarp();  // the slots of the block before are free but its last two
+      assemble(next);
+      load(next + BTS_PTS);
       __syncwarp();
     }
     double b[5];
 #pragma unroll
     for (int i = 0; i < 5; ++i) {
-      b[i] = is_r ? at(p, 68 + i) : at(p, 18 + i * 5 + col);
+      b[i] = is_r ? at(j, 68 + i) : at(j, 18 + i * 5 + col);
 #pragma unroll
       for (int e = 0; e < 5; ++e)
         if (anz<DIR>(ADJ ? e : i, ADJ ? i : e))
-          b[i] = fma(at(ADJ ? p : p - 1, bt_pidx<DIR>(ADJ ? e : i, ADJ ? i : e)), x[e], b[i]);
+          b[i] = fma(at(ADJ ? j : j - 1, bt_pidx<DIR>(ADJ ? e : i, ADJ ? i : e)), x[e], b[i]);
     }
-    // right-hand side column: C_p's, or r'
+    // right-hand side column: C_j's, or r'
 #pragma unroll
-    for (int i = 0; i < 5; ++i) x[i] = is_r ? b[i] : at(last_q, 43 + i * 5 + col);
+    for (int i = 0; i < 5; ++i) x[i] = is_r ? b[i] : at(next, 43 + i * 5 + col);
     double up[5][5];  // the pivot columns' entries above the diagonal, for the back step
 #pragma unroll
     for (int t = 0; t < 5; ++t) {
@@ -482,52 +495,92 @@ __device__ __forceinline__ void bt_line6(const Fields& F, const Consts& K, const
         if (bt_rank<DIR>(i) < t) x[i] = fma(-up[i][pr], x[pr], x[i]);
     }
     if (own) {
-      const int64_t pt = base + (int64_t)p * st;
 #pragma unroll
       for (int i = 0; i < 5; ++i) {
-        if (is_r) rhs[i * NP + pt] = x[i];
-        else lhsc[((int64_t)p * 25 + i * 5 + c) * nlt + gl] = x[i];
+        if (is_r) rhs[i * NP + pnt(j)] = x[i];
+        else lhsc[((int64_t)gq(j) * 25 + i * 5 + c) * nlt + gl] = x[i];
       }
     }
   }
-  // back substitution by rows; row c of C'_p and r'_p are loaded BACK steps ahead
-  __syncwarp();
-  constexpr int BACK = 4;
+  // the seam
+  double* mine = smem + 2 * BTS_RING + (half * BTS_LINES + g) * 30;
+  const double* other = smem + 2 * BTS_RING + ((1 - half) * BTS_LINES + g) * 30;
+  if (lane < 30) {
+#pragma unroll
+    for (int i = 0; i < 5; ++i) mine[is_r ? 25 + i : i * 5 + c] = x[i];
+  }
+  __syncthreads();
+  double y;  // row `row` of the solution at row fin
   const int row = col;
+  {
+    double b[5], up[5][5];
+#pragma unroll
+    for (int i = 0; i < 5; ++i) b[i] = is_r ? x[i] : i == c ? 1.0 : 0.0;
+#pragma unroll
+    for (int e = 0; e < 5; ++e) {
+      const double v = is_r ? other[25 + e] : other[e * 5 + col];
+#pragma unroll
+      for (int i = 0; i < 5; ++i) b[i] = fma(-mine[i * 5 + e], v, b[i]);
+    }
+#pragma unroll
+    for (int t = 0; t < 5; ++t) {
+      double m[5];
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        m[i] = __shfl_sync(all, b[i], src0 + t);
+        if (i < t) up[i][t] = m[i];
+      }
+      b[t] *= bt_recip(m[t]);
+#pragma unroll
+      for (int i = t + 1; i < 5; ++i) b[i] = fma(-m[i], b[t], b[i]);
+    }
+#pragma unroll
+    for (int t = 4; t > 0; --t)
+#pragma unroll
+      for (int i = 0; i < t; ++i) b[i] = fma(-up[i][t], b[t], b[i]);
+    y = 0.0;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const double v = __shfl_sync(all, b[i], src0 + 5);
+      if (row == i) y = v;
+    }
+  }
+  // back substitution by rows; row c of C'_j and r'_j are loaded BACK steps ahead
+  constexpr int BACK = 4;
   double cq[BACK][5], rq[BACK], uq[BACK];
-  auto fetch = [&](int p, int slot) {
-    if (p < first) return;
-    const int64_t pt = base + (int64_t)p * st;
+  auto fetch = [&](int j, int slot) {
+    if (j < first) return;
 #pragma unroll
-    for (int e = 0; e < 5; ++e) cq[slot][e] = lhsc[((int64_t)p * 25 + row * 5 + e) * nlt + gl];
-    rq[slot] = rhs[row * NP + pt];
-    uq[slot] = add_u ? F.u[row * NP + pt] : 0.0;
+    for (int e = 0; e < 5; ++e) cq[slot][e] = lhsc[((int64_t)gq(j) * 25 + row * 5 + e) * nlt + gl];
+    rq[slot] = rhs[row * NP + pnt(j)];
+    uq[slot] = add_u ? F.u[row * NP + pnt(j)] : 0.0;
   };
-  double y = ADJ ? 0.0 : rhs[row * NP + base + (int64_t)(n - 1) * st];
+  auto store = [&](int j, double uv) {
+    if (!own || is_r) return;
+    rhs[row * NP + pnt(j)] = y;
+    if (add_u) F.u[row * NP + pnt(j)] = uv + y;
+  };
 #pragma unroll
-  for (int q = 0; q < BACK; ++q) fetch(fin - q, q);
-  for (int p0 = fin; p0 >= first; p0 -= BACK) {
+  for (int q = 0; q < BACK; ++q) fetch(fin - 1 - q, q);
+  if (fin >= first) store(fin, add_u ? F.u[row * NP + pnt(fin)] : 0.0);
+  for (int j0 = fin - 1; j0 >= first; j0 -= BACK) {
 #pragma unroll
     for (int q = 0; q < BACK; ++q) {
-      const int p = p0 - q;
-      if (p < first) break;
+      const int j = j0 - q;
+      if (j < first) break;
       double t = rq[q];
 #pragma unroll
       for (int e = 0; e < 5; ++e) t = fma(-cq[q][e], __shfl_sync(all, y, src0 + e), t);
       y = t;
-      if (own && !is_r) {
-        const int64_t pt = base + (int64_t)p * st;
-        rhs[row * NP + pt] = y;
-        if (add_u) F.u[row * NP + pt] = uq[q] + y;
-      }
-      fetch(p - BACK, q);
+      store(j, uq[q]);
+      fetch(j - BACK, q);
     }
   }
 }
 
 template <int DIR>
-__global__ void __launch_bounds__(32, 1) k_bt_line6(Fields F, Consts K, const Work* __restrict__ work, int lpi,
-                                                    double* __restrict__ lhsc, int64_t nlt, int add_u) {
+__global__ void __launch_bounds__(64, 1) k_bt_line12(Fields F, Consts K, const Work* __restrict__ work, int lpi,
+                                                     double* __restrict__ lhsc, int64_t nlt, int add_u) {
   extern __shared__ double bts[];
-  bt_line6<DIR, false>(F, K, work, lpi, F.rhs, lhsc, nlt, add_u, bts);
+  bt_line12<DIR, false>(F, K, work, lpi, F.rhs, lhsc, nlt, add_u, bts);
 }

@@ -713,43 +713,36 @@ void* line_scratch(npbmz_t* h, int dir) {
   return (dir > 0 && h->scratch_yz[dir - 1]) ? h->scratch_yz[dir - 1] : h->scratch;
 }
 
-// FP64 BT sweeps with one thread per line take as long as their longest line
-// unless the lines give every SM quarter (608) a warp; six lanes per line take
-// 1.6 times the warp instructions but a quarter of the time per line.  The two
-// meet where the lines, as multiples of the longest, number about 11,000:
-// 128x128x16's z sweep (14,400) takes 235 us by threads and 303 by groups of
-// lanes, 304x208x17's x sweep (12,300) 1123 and 1177, 128x128x16's x sweep
-// (3,700) 746 and 381.
-bool few_lines(const npbmz_t* h, int dir, int zone) {
-  int64_t points = 0;
-  int longest = 1;
-  for (int z = zone < 0 ? 0 : zone; z < (zone < 0 ? h->nzones : zone + 1); ++z) {
-    const int n = zone_line_len(h->zh[z], dir);
-    points += (int64_t)zone_lines(h->zh[z], dir) * n;
-    longest = std::max(longest, n);
-  }
-  return points < 10000 * (int64_t)longest;
-}
-
-// The refined FP32 BT sweeps with two threads per line, by the lines of the
-// whole problem (all ranks' zones, so that every split of it solves alike).
-// One thread per line fills the chip at 152 SMs x 256 lines; half of that, 128
-// lines per SM, is what two threads per line keep at once.  x, y, z sweeps in
-// us, one / two threads: 64x64x8 (1344, 1344, 3136 lines) 85, 72, 33 / 61, 55,
-// 27; 338x118x8 (10,200 to 33,000) 106, 114, 48 / 91, 92, 62; 37x389x12 x
+// The BT sweeps' mappings for few lines (FP64: twelve lanes per line, refined
+// FP32: two threads per line), by the lines of the whole problem (all ranks'
+// zones, so that every split of it solves alike).
+// FP64: one thread per line takes its longest line's time, about 13 us a row,
+// until the lines give every SM quarter (608) a warp; twelve lanes per line
+// take about 1.65 ns per row and line.  They meet at 9000 lines of equal
+// length (z, where all have the zones' nz points) and later where the longest
+// is well above the mean.  Thread / twelve lanes, us: 128x128x16 x (6720 lines,
+// 13 to 58 points) 748 / 340, z (14,400) 235 / 288; 120x120x14 z (12,544) 196 /
+// 247; 160x128x16 x (13,440, up to 38) 484 / 368; 176x160x20 x (20,736) 402 /
+// 542; 304x208x17 x (23,040, up to 72) 1052 / 1071.
+// FP32: one thread per line fills the chip at 152 SMs x 256 lines; half of
+// that, 128 lines per SM, is what two threads per line keep at once.  x, y, z
+// in us, one / two threads: 64x64x8 (1344, 1344, 3136 lines) 85, 72, 33 / 61,
+// 55, 27; 338x118x8 (10,200 to 33,000) 106, 114, 48 / 91, 92, 62; 37x389x12 x
 // (14,300) 59 / 58; 192x104x27 (35,200, 32,000, 14,100) 107, 73, 96 / 117, 97,
 // 96; 480x320x28 (from 119,000) 586, 568, 635 / 668, 694, 708.
-bool two_ended(const npbmz_t* h, int dir) { return h->problem_lines[dir] < 14000; }
+bool few_lines(const npbmz_t* h, int dir) {
+  return h->problem_lines[dir] < (use_fp32(h) ? 14000 : dir == 2 ? 9000 : 12000);
+}
 
 int phase_solve(npbmz_t* h, int dir, int zone, int add_u, bool fused = false) {
   const Fields F = fields(h);
   const bool sp = h->kind == NPBMZ_SP;
   const int mode = use_exact(h) ? 0
-                   : !use_fp32(h) ? (!sp && few_lines(h, dir, zone) ? 5 : 0)
+                   : !use_fp32(h) ? (!sp && few_lines(h, dir) ? 5 : 0)
                    : (h->flags & NPBMZ_FP32_NOREFINE) ? 1
                    : (h->flags & NPBMZ_REFINE_FP64) ? 3
                    : !(fused && h->rdf) ? 2
-                   : !sp && two_ended(h, dir) ? 6 : 4;
+                   : !sp && few_lines(h, dir) ? 6 : 4;
   return line_launches(h, dir, zone, [&](int lo, int hi, int tpb) {
     if (use_exact(h))
       exact::launch_solve(sp, 0, dir, F, h->K, h->wline_d[dir] + lo, hi - lo, tpb, line_scratch(h, dir),
@@ -1267,7 +1260,7 @@ int adjoint_back_step(npbmz_t* h, double* const x[3], double* ub, double* vb, do
   // the sweeps in reverse order
   for (int dir = 2; dir >= 0; --dir) {
     if (line_launches(h, dir, -1, [&](int lo, int hi, int tpb) {
-          adj_launch_solve(dir, few_lines(h, dir, -1), F, h->K, h->wline_d[dir] + lo, hi - lo, tpb, yb, scr,
+          adj_launch_solve(dir, few_lines(h, dir), F, h->K, h->wline_d[dir] + lo, hi - lo, tpb, yb, scr,
                            h->nlines[dir], h->stream);
           CKL(h);
           return 0;
@@ -1565,7 +1558,7 @@ int npbmz_create(int kind, int nzones, const int* nx, const int* ny, const int* 
   // the SMs more evenly (bit-exact step of 304x208x17 6.47 ms with 64 lines per
   // block, 5.93 with 32; 480x320x28 FP64 z sweep 2.64 / 2.49)
   for (int dir = 0; dir < 3; ++dir)
-    if (!use_fp32(h) && (use_exact(h) || kind == NPBMZ_SP || !few_lines(h, dir, -1)))
+    if (!use_fp32(h) && (use_exact(h) || kind == NPBMZ_SP || !few_lines(h, dir)))
       for (int& t : h->tpb_bkt[dir]) t = 32;
   if (!rc) rc = build_work_lists(h);
   if (!rc) rc = build_line_lists(h);

@@ -1536,7 +1536,7 @@ __global__ void __launch_bounds__(128) k_bt_refine_df(Fields F, Consts K, const 
 // r'_A - C'_A r'_B with its partner's C' and r' and substitutes back toward
 // its own end.  A line then takes half as many dependent steps for 8 % more
 // instructions and a barrier: faster while the lines are too few to fill the
-// chip one per thread (two_ended in npbmz_api.cu draws the line).
+// chip one per thread (few_lines in npbmz_api.cu draws the line).
 // ============================================================================
 #ifndef NPBMZ_PIPE
 #define NPBMZ_PIPE 4
@@ -2684,7 +2684,7 @@ static void launch_solve_t(bool sp, int dir, const Fields& F, const Consts& K, c
 }
 
 // mode 4: one fused refined FP32 step (6: BT, two threads per line); mode 0:
-// FP64 in place (5: BT, six lanes per line); 1: FP32 in place; 2: FP32 + refinement with a
+// FP64 in place (5: BT, twelve lanes per line); 1: FP32 in place; 2: FP32 + refinement with a
 // double-float residual (BT; SP: FP64 residual); 3: FP32 + refinement with
 // an FP64 residual (xw: a [5][NP] buffer for the first solution).
 void launch_solve(bool sp, int mode, int dir, const Fields& F, const Consts& K, const Work* work, int nwork, int tpb,
@@ -2787,9 +2787,9 @@ void launch_solve(bool sp, int mode, int dir, const Fields& F, const Consts& K, 
   if (mode == 5) {
     const dim3 grid(nwork, (tpb + BTS_LINES - 1) / BTS_LINES);
     double* scr = reinterpret_cast<double*>(scratch);
-    if (dir == 0) k_bt_line6<0><<<grid, 32, BTS_SMEM, s>>>(F, K, work, tpb, scr, nlt, add_u);
-    else if (dir == 1) k_bt_line6<1><<<grid, 32, BTS_SMEM, s>>>(F, K, work, tpb, scr, nlt, add_u);
-    else k_bt_line6<2><<<grid, 32, BTS_SMEM, s>>>(F, K, work, tpb, scr, nlt, add_u);
+    if (dir == 0) k_bt_line12<0><<<grid, 64, BTS_SMEM, s>>>(F, K, work, tpb, scr, nlt, add_u);
+    else if (dir == 1) k_bt_line12<1><<<grid, 64, BTS_SMEM, s>>>(F, K, work, tpb, scr, nlt, add_u);
+    else k_bt_line12<2><<<grid, 64, BTS_SMEM, s>>>(F, K, work, tpb, scr, nlt, add_u);
     return;
   }
 #endif

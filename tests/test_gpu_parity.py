@@ -141,10 +141,11 @@ def test_bt_line_solves_at_small_and_ragged_sizes(oracle_mod, nz, flags):
             compare(p, o, npbmz.RHS, 1e-10 if flags else FAST_REL, [z])
 
 
-def test_bt_few_line_solves_equal_full_launches():
-    """The FP64 sweeps of one zone (six lanes per line) give the bits of the
-    batched launch over class B's 64 zones (one thread per line)."""
-    geom, dt, _ = geom_class("BT", "B")
+def test_bt_per_zone_solves_equal_batched_ones():
+    """Launches over one zone give the bits of the batched launch on class A,
+    whose x and y sweeps take twelve lanes per line and whose z sweep one
+    thread: the mapping follows the problem, not the launch."""
+    geom, dt, _ = geom_class("BT", "A")
     a, b = npbmz.Problem(geom, dt, 0), npbmz.Problem(geom, dt, 0)
     for p in (a, b):
         p.setup(npbmz.CE_REFERENCE)
