@@ -77,23 +77,40 @@ __device__ __forceinline__ df64 sp_rhon_df(const SpDfK& c, df64 ri) {
 }
 
 // Bands of interior row q (1..n-2) of the three systems in double-float from
-// cv, rhon and speed at q-1, q, q+1 (the statements of sp_assemble).
+// cv, rhon and speed at q-1, q, q+1 (the statements of sp_assemble).  From six
+// points up one position class applies to a row, so its constants are selected
+// and each added once.  (Normalised: unnormalised bands took 14 us less of the
+// three sweeps of 480x320x28 but doubled u's error on 64x64x8 to 7e-15.)
 __device__ __forceinline__ void sp_assemble_df(const SpDfK& c, int q, int n, const df64 cv[3], const df64 rh[3],
                                                const df64 sp[3], df64 L[3][5]) {
   const df64 z = {0.f, 0.f};
-  df64 L1 = z;
-  df64 L2 = df_sub(df_neg(df_mul(c.dtt2, cv[0])), df_mul(c.dtt1, rh[0]));
-  df64 L3 = df_add(df64{1.f, 0.f}, df_mul(c.c2dtt1, rh[1]));
-  df64 L4 = df_sub(df_mul(c.dtt2, cv[2]), df_mul(c.dtt1, rh[2]));
-  df64 L5 = z;
-  if (q == 1) { L3 = df_add(L3, c.comz5); L4 = df_sub(L4, c.comz4); L5 = df_add(L5, c.comz1); }
-  if (q == 2) { L2 = df_sub(L2, c.comz4); L3 = df_add(L3, c.comz6); L4 = df_sub(L4, c.comz4); L5 = df_add(L5, c.comz1); }
-  if (q >= 3 && q <= n - 4) {
-    L1 = df_add(L1, c.comz1); L2 = df_sub(L2, c.comz4); L3 = df_add(L3, c.comz6); L4 = df_sub(L4, c.comz4);
-    L5 = df_add(L5, c.comz1);
+  if (n < 6) {  // short lines: several stencils at one row
+    df64 L1 = z;
+    df64 L2 = df_sub(df_neg(df_mul(c.dtt2, cv[0])), df_mul(c.dtt1, rh[0]));
+    df64 L3 = df_add(df64{1.f, 0.f}, df_mul(c.c2dtt1, rh[1]));
+    df64 L4 = df_sub(df_mul(c.dtt2, cv[2]), df_mul(c.dtt1, rh[2]));
+    df64 L5 = z;
+    if (q == 1) { L3 = df_add(L3, c.comz5); L4 = df_sub(L4, c.comz4); L5 = df_add(L5, c.comz1); }
+    if (q == 2) { L2 = df_sub(L2, c.comz4); L3 = df_add(L3, c.comz6); L4 = df_sub(L4, c.comz4); L5 = df_add(L5, c.comz1); }
+    if (q >= 3 && q <= n - 4) {
+      L1 = df_add(L1, c.comz1); L2 = df_sub(L2, c.comz4); L3 = df_add(L3, c.comz6); L4 = df_sub(L4, c.comz4);
+      L5 = df_add(L5, c.comz1);
+    }
+    if (q == n - 3) { L1 = df_add(L1, c.comz1); L2 = df_sub(L2, c.comz4); L3 = df_add(L3, c.comz6); L4 = df_sub(L4, c.comz4); }
+    if (q == n - 2) { L1 = df_add(L1, c.comz1); L2 = df_sub(L2, c.comz4); L3 = df_add(L3, c.comz5); }
+    const df64 s0 = df_mul(c.dtt2, sp[0]), s2 = df_mul(c.dtt2, sp[2]);
+    L[0][0] = L1; L[0][1] = L2; L[0][2] = L3; L[0][3] = L4; L[0][4] = L5;
+    L[1][0] = L1; L[1][1] = df_sub(L2, s0); L[1][2] = L3; L[1][3] = df_add(L4, s2); L[1][4] = L5;
+    L[2][0] = L1; L[2][1] = df_add(L2, s0); L[2][2] = L3; L[2][3] = df_sub(L4, s2); L[2][4] = L5;
+    return;
   }
-  if (q == n - 3) { L1 = df_add(L1, c.comz1); L2 = df_sub(L2, c.comz4); L3 = df_add(L3, c.comz6); L4 = df_sub(L4, c.comz4); }
-  if (q == n - 2) { L1 = df_add(L1, c.comz1); L2 = df_sub(L2, c.comz4); L3 = df_add(L3, c.comz5); }
+  const bool lo1 = q == 1, hi1 = q == n - 2;
+  const df64 L1 = q >= 3 ? c.comz1 : z, L5 = q <= n - 4 ? c.comz1 : z;
+  df64 L2 = df_add(df_neg(df_mul(c.dtt2, cv[0])), df_neg(df_mul(c.dtt1, rh[0])));
+  df64 L4 = df_sub(df_mul(c.dtt2, cv[2]), df_mul(c.dtt1, rh[2]));
+  const df64 L3 = df_add(df_add(df_mul(c.c2dtt1, rh[1]), df64{1.f, 0.f}), lo1 || hi1 ? c.comz5 : c.comz6);
+  L2 = df_sub(L2, lo1 ? z : c.comz4);
+  L4 = df_sub(L4, hi1 ? z : c.comz4);
   const df64 s0 = df_mul(c.dtt2, sp[0]), s2 = df_mul(c.dtt2, sp[2]);
   L[0][0] = L1; L[0][1] = L2; L[0][2] = L3; L[0][3] = L4; L[0][4] = L5;
   L[1][0] = L1; L[1][1] = df_sub(L2, s0); L[1][2] = L3; L[1][3] = df_add(L4, s2); L[1][4] = L5;
@@ -392,8 +409,9 @@ __device__ __forceinline__ void sp_refine_pl_item(const Fields& F, const Consts&
   for (int q = 0; q < PIPE - 1; ++q) issue_fwd(q);
   // geometry window (cv, rhon, speed at q-1, q, q+1) and x window (q-2 .. q+2)
   df64 gcv[3], grh[3], gsp[3];
-  df64 xw[5][5];
-  const df64 z0 = {0.f, 0.f};
+  // x0 inside the line is plain FP32; at the line's ends x is b, whose low
+  // words (xe0, xen) enter the rows that reach them as a correction
+  float xw[5][5], xe0[5], xen[5];
   {
     const df64 cv = {*Ln.state(0, pcv), *Ln.state(0, PS_HI_COUNT + pcv)};
     const df64 ri = {*Ln.state(0, PS_RHOI), *Ln.state(0, PS_HI_COUNT + PS_RHOI)};
@@ -402,10 +420,12 @@ __device__ __forceinline__ void sp_refine_pl_item(const Fields& F, const Consts&
     gcv[0] = gcv[1] = cv; grh[0] = grh[1] = rh; gsp[0] = gsp[1] = sp;
 #pragma unroll
     for (int m = 0; m < 5; ++m) {
-      xw[0][m] = z0;
-      xw[1][m] = z0;
-      xw[2][m] = df64{*Ln.b(0, m), *Ln.b(0, 5 + m)};     // row 0 is an identity row: x = b
-      xw[3][m] = df64{*Ln.x0_at(1, m), 0.f};              // n >= 3: point 1 is interior
+      xw[0][m] = 0.f;
+      xw[1][m] = 0.f;
+      xw[2][m] = *Ln.b(0, m);      // row 0 is an identity row: x = b
+      xe0[m] = *Ln.b(0, 5 + m);
+      xw[3][m] = *Ln.x0_at(1, m);  // n >= 3: point 1 is interior
+      xen[m] = 0.f;
     }
   }
   auto row = [&](int q, float L[3][5], float r[5]) {
@@ -419,8 +439,10 @@ __device__ __forceinline__ void sp_refine_pl_item(const Fields& F, const Consts&
     }
     const int qx = q + 2;
 #pragma unroll
-    for (int m = 0; m < 5; ++m)
-      xw[4][m] = qx > n - 1 ? z0 : (qx == n - 1 ? df64{*S(slot, 6 + m), *S(slot, 11 + m)} : df64{*S(slot, 6 + m), 0.f});
+    for (int m = 0; m < 5; ++m) {
+      xw[4][m] = qx > n - 1 ? 0.f : *S(slot, 6 + m);
+      if (qx == n - 1) xen[m] = *S(slot, 11 + m);
+    }
     if (q == 0 || q == n - 1) {
       sp_identity_rows(L);
 #pragma unroll
@@ -435,13 +457,18 @@ __device__ __forceinline__ void sp_refine_pl_item(const Fields& F, const Consts&
 #pragma unroll
       for (int m = 0; m < 5; ++m) {
         const int s = m < 3 ? 0 : m - 2;
-        df64 t = df_mul(Ld[s][2], xw[2][m]);
-        t = df_add(t, df_mul(Ld[s][1], xw[1][m]));
-        t = df_add(t, df_mul(Ld[s][3], xw[3][m]));
-        t = df_add(t, df_mul(Ld[s][0], xw[0][m]));
-        t = df_add(t, df_mul(Ld[s][4], xw[4][m]));
+        // unnormalised sums with the plain FP32 x: 275 instead of 450
+        // instructions a row (sweeps of 480x320x28 366, 308, 586 -> 347, 287,
+        // 541 us; u's error unchanged, 2.8e-15 after 20 steps of 64x64x8)
+        df64 t = du_mul(Ld[s][2], xw[2][m]);
+        t = du_add(t, du_mul(Ld[s][1], xw[1][m]));
+        t = du_add(t, du_mul(Ld[s][3], xw[3][m]));
+        t = du_add(t, du_mul(Ld[s][0], xw[0][m]));
+        t = du_add(t, du_mul(Ld[s][4], xw[4][m]));
+        if (q <= 2) t.lo = fmaf(q == 1 ? Ld[s][1].hi : Ld[s][0].hi, xe0[m], t.lo);
+        if (q >= n - 3) t.lo = fmaf(q == n - 2 ? Ld[s][3].hi : Ld[s][4].hi, xen[m], t.lo);
         const df64 b = {*S(slot, 16 + m), *S(slot, 21 + m)};
-        const df64 rr = df_sub(b, t);
+        const df64 rr = du_sub(b, t);
         r[m] = rr.hi + rr.lo;
       }
     }

@@ -170,6 +170,18 @@ def test_bt_fused_mixed_steps_at_small_and_ragged_sizes(oracle_mod, nz):
     compare(p, o, npbmz.U, 1e-10)
 
 
+@pytest.mark.parametrize("nz", [5, 6, 7, 13])
+def test_sp_fused_mixed_steps_at_small_and_ragged_sizes(oracle_mod, nz):
+    """Whole refined FP32 SP steps on zones of 5 points per axis (two stencils
+    at a row), 6 (every row an end one) and up."""
+    nx, ny, nzs, nbr = npbmz.zones_from_widths([5, 6, 8, 15], [5, 7, 6, 14], nz)
+    geom = npbmz.Geometry(npbmz.SP, nx, ny, nzs, nbr, 34, 32, nz, 4, 4)
+    p, o = make_pair(oracle_mod, geom, 0.0015, npbmz.MIXED, npbmz.CE_REFERENCE)
+    p.step(4)
+    o.step(4)
+    compare(p, o, npbmz.U, 1e-10)
+
+
 def test_bt_fused_mixed_steps_many_ragged_zones(oracle_mod):
     """The same with enough lines that every sweep takes one thread per line
     (the smaller problems take two)."""
