@@ -258,9 +258,11 @@ int npbmz_adjoint(npbmz_t* h, int nsteps, int checkpoint_every, const double* u_
  * branch.  Each branch starts when the previous group's compute_rhs is done,
  * so FP64-bound phases of one group run beside the FP32 sweeps of the
  * previous one.  Results are unchanged (zones are independent within a step
- * after exch_qbc).  npbmz_create sets 2 groups for NPBMZ_GRAPH handles with
- * at least 8 zones (not NPBMZ_EXACT or NPBMZ_PERZONE).  No counterpart in the
- * reference. */
+ * after exch_qbc).  npbmz_create gives NPBMZ_GRAPH handles with at least 8
+ * zones (not NPBMZ_EXACT or NPBMZ_PERZONE) 2 branches; with NPBMZ_MIXED and
+ * from 2 M points 6 groups, by which npbmz_step_inout and npbmz_step_download
+ * copy (BT: three to a branch of the resident step); this call makes every
+ * group a branch.  No counterpart in the reference. */
 int npbmz_set_step_groups(npbmz_t* h, int groups);
 
 /* How the zone-group branches of the step graph share the SMs.

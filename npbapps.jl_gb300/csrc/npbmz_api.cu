@@ -254,7 +254,9 @@ struct npbmz_handle {
   int ngroups = 1;
   std::vector<int> zone_group;     // per zone
   std::vector<Range> grp_pts, grp_int, grp_line[3];
-  int cur_group = -1;              // >= 0 while the phases of one group are issued
+  int step_merge = 1;              // groups per branch of the resident step graph (npbmz_step_inout: one each)
+  int cur_group = -1;              // >= 0 while the phases of groups cur_group .. + cur_span - 1 are issued
+  int cur_span = 1;
   cudaStream_t grp_stream[8] = {};
   // the x sweep's x-line-major state copies made by the compute_rhs launch
   // (k_rhs_flux_xc) instead of a kernel of their own (npbmz_set_copy_fusion)
@@ -610,7 +612,11 @@ int line_launches(npbmz_t* h, int dir, int zone, Fn fn) {
   }
   if (h->cur_group < 0 && h->cur_bucket < 0 && h->nbkt == 1)  // one shape: the whole list in one launch
     return h->nwline[dir] > 0 ? fn(0, h->nwline[dir], h->tpb_bkt[dir][0]) : 0;
-  const int g0 = h->cur_group >= 0 ? h->cur_group : 0, g1 = h->cur_group >= 0 ? h->cur_group + 1 : h->ngroups;
+  const int g0 = h->cur_group >= 0 ? h->cur_group : 0, g1 = h->cur_group >= 0 ? h->cur_group + h->cur_span : h->ngroups;
+  if (h->cur_group >= 0 && h->cur_span > 1 && h->cur_bucket < 0 && h->nbkt == 1) {  // adjacent ranges of one shape
+    const int lo = h->gb_line[dir][g0].lo, hi = h->gb_line[dir][g1 - 1].hi;
+    return hi > lo ? fn(lo, hi, h->tpb_bkt[dir][0]) : 0;
+  }
   for (int g = g0; g < g1; ++g)
     for (int b = 0; b < h->nbkt; ++b) {
       if (h->cur_bucket >= 0 && b != h->cur_bucket) continue;
@@ -662,7 +668,7 @@ int phase_prim(npbmz_t* h, int zone, bool fused = false) {
     // over the point work list
     int wlo = 0, whi = h->nwpts;
     if (zone >= 0) { wlo = h->pts_range[zone].lo; whi = h->pts_range[zone].hi; }
-    else if (h->cur_group >= 0) { wlo = h->grp_pts[h->cur_group].lo; whi = h->grp_pts[h->cur_group].hi; }
+    else if (h->cur_group >= 0) { wlo = h->grp_pts[h->cur_group].lo; whi = h->grp_pts[h->cur_group + h->cur_span - 1].hi; }
     Fields Fp = F;
     Fp.pfx = nullptr;  // the x-line-major state copies come from k_xline_copy
     if (h->dfrhs)
@@ -691,7 +697,7 @@ int phase_rhs(npbmz_t* h, int zone, bool tx, bool norm, bool fused = false) {
   F.rhs64 = !fused;
   int lo = 0, hi = h->nwint;
   if (zone >= 0) { lo = h->int_range[zone].lo; hi = h->int_range[zone].hi; }
-  else if (h->cur_group >= 0) { lo = h->grp_int[h->cur_group].lo; hi = h->grp_int[h->cur_group].hi; }
+  else if (h->cur_group >= 0) { lo = h->grp_int[h->cur_group].lo; hi = h->grp_int[h->cur_group + h->cur_span - 1].hi; }
   if (use_exact(h)) exact::launch_rhs(tx, norm, F, h->K, h->wint_d + lo, hi - lo, h->part_rhs + 5 * lo, h->stream);
   else if (h->dfrhs)
     fast::launch_rhs_df(tx, norm, F, h->rdc, h->wint_d + lo, hi - lo, h->part_rhs + 5 * lo, h->stream,
@@ -829,13 +835,13 @@ void drop_graph(npbmz_t* h) {
 // caller runs it between the two parts of the upload) and group g's branch
 // first waits for up_ev[g], the upload of its zones.
 int grouped_step(npbmz_t* h, cudaStream_t cs, bool inout) {
-  const int G = h->ngroups;
+  const int G = h->ngroups, M = inout ? 1 : h->step_merge;  // a branch: M adjacent groups
   const bool sp = h->kind == NPBMZ_SP;
   if (!inout && phase_exch(h)) return -1;
   cudaEvent_t start = h->grp_ev[2 * G];
   CK(h, cudaEventRecord(start, cs));
   int rc = 0;
-  for (int g = 0; g < G && !rc; ++g) {
+  for (int g = 0; g < G && !rc; g += M) {
     cudaStream_t S = inout ? h->io_grp_stream[g] : h->grp_stream[g];
     // prim + compute_rhs of group g: on the priority stream (in group order),
     // or on the group's own stream after group g-1's compute_rhs (always so
@@ -843,22 +849,25 @@ int grouped_step(npbmz_t* h, cudaStream_t cs, bool inout) {
     cudaStream_t P = h->fp64_prio && !inout ? h->prio_stream : S;
     rc |= cudaStreamWaitEvent(P, start, 0) != cudaSuccess;
     if (inout) rc |= cudaStreamWaitEvent(P, h->up_ev[g], cudaEventWaitExternal) != cudaSuccess;
-    if (g > 0 && P == S) rc |= cudaStreamWaitEvent(S, h->grp_ev[2 * (g - 1)], 0) != cudaSuccess;
+    if (g > 0 && P == S) rc |= cudaStreamWaitEvent(S, h->grp_ev[2 * (g - M)], 0) != cudaSuccess;
     h->stream = P;
     h->cur_group = g;
+    h->cur_span = std::min(M, G - g);
     if (!rc) rc = phase_prim(h, -1, true);
     if (!rc) rc = phase_rhs(h, -1, sp, false, true);
     if (!rc) rc = cudaEventRecord(h->grp_ev[2 * g], P) != cudaSuccess;
     if (!rc && P != S) rc = cudaStreamWaitEvent(S, h->grp_ev[2 * g], 0) != cudaSuccess;
     h->stream = S;
     for (int dir = 0; dir < 3 && !rc; ++dir) rc = phase_solve(h, dir, -1, dir == 2 ? 1 : 0, true);
-    // group g's u is final: an event that work outside the graph can wait on
-    if (!rc) rc = cudaEventRecordWithFlags(h->grp_out_ev[g], S, cudaEventRecordExternal) != cudaSuccess;
+    // the groups' u is final: events that work outside the graph can wait on
+    for (int q = g; q < g + h->cur_span && !rc; ++q)
+      rc = cudaEventRecordWithFlags(h->grp_out_ev[q], S, cudaEventRecordExternal) != cudaSuccess;
     if (!rc) rc = cudaEventRecord(h->grp_ev[2 * g + 1], S) != cudaSuccess;
   }
   h->stream = cs;
   h->cur_group = -1;
-  for (int g = 0; g < G && !rc; ++g) rc = cudaStreamWaitEvent(cs, h->grp_ev[2 * g + 1], 0) != cudaSuccess;
+  h->cur_span = 1;
+  for (int g = 0; g < G && !rc; g += M) rc = cudaStreamWaitEvent(cs, h->grp_ev[2 * g + 1], 0) != cudaSuccess;
   if (rc && h->err.empty()) h->err = "grouped step capture failed";
   return rc ? -1 : 0;
 }
@@ -998,7 +1007,7 @@ int count_launches(npbmz_t* h) {
   const int adi = 2 + (h->pfx && !h->copy_fusion ? 1 : 0) + 3 * (refined ? 2 : 1) + (h->rdx ? 1 : 0);
   int batches = 1;
   if (h->flags & NPBMZ_PERZONE) batches = h->nzones;
-  else if ((h->flags & NPBMZ_GRAPH) && h->ngroups > 1 && !(h->flags & NPBMZ_EXACT)) batches = h->ngroups;
+  else if ((h->flags & NPBMZ_GRAPH) && h->ngroups > 1 && !(h->flags & NPBMZ_EXACT)) batches = (h->ngroups + h->step_merge - 1) / h->step_merge;
   return (h->nzones > 1 ? 1 : 0) + adi * batches;
 }
 
@@ -1356,6 +1365,35 @@ int adjoint_run(npbmz_t* h, int nsteps, int every, const double* u_target, doubl
   return 0;
 }
 
+// Zone groups of the step graph; merge adjacent ones share a branch of the
+// resident graph.
+int set_groups(npbmz_t* h, int groups, int merge) {
+  CK(h, cudaStreamSynchronize(h->stream));
+  drop_graph(h);
+  h->ngroups = groups;
+  h->step_merge = merge;
+  assign_zone_groups(h);
+  if (build_work_lists(h) || build_line_lists(h)) return -1;
+  {  // zones of each group (npbmz_step_download)
+    std::vector<int> zl;
+    h->grp_zone_off.assign(h->ngroups + 1, 0);
+    for (int g = 0; g < h->ngroups; ++g) {
+      for (int z = 0; z < h->nzones; ++z)
+        if (h->zone_group[z] == g) zl.push_back(z);
+      h->grp_zone_off[g + 1] = (int)zl.size();
+    }
+    if (!h->grp_zones_d) CK(h, cudaMalloc((void**)&h->grp_zones_d, std::max(1, h->nzones) * sizeof(int)));
+    CK(h, cudaMemcpy(h->grp_zones_d, zl.data(), zl.size() * sizeof(int), cudaMemcpyHostToDevice));
+  }
+  if (h->ngroups > 1 && !h->scratch_yz[0])
+    for (int d = 0; d < 2; ++d) {
+      CK(h, cudaMalloc(&h->scratch_yz[d], std::max<size_t>(h->scratch_bytes, 16)));
+      h->device_bytes += (int64_t)h->scratch_bytes;
+    }
+  h->launches_per_step = count_launches(h);
+  return 0;
+}
+
 }  // namespace
 
 // =============================== C ABI ======================================
@@ -1605,9 +1643,20 @@ int npbmz_create(int kind, int nzones, const int* nx, const int* ny, const int* 
   if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess) { h->stream = s; h->own_stream = true; }
   h->launches_per_step = count_launches(h);
   *out = h;
-  // the step graph of a batched FMA-build step runs in zone-group branches
+  // The step graph of a batched FMA-build step runs in zone-group branches:
+  // two, on large mixed problems of several groups each, since
+  // npbmz_step_inout, whose copies overlap the groups' work, gains by more (us
+  // by groups, 480x320x28 in and out every step: BT 2: 4809, 4: 4232, 6: 3899,
+  // 8: 3872, SP 4723, 4112, 3787, 3624; BT 240x208x17 1218, 1151, 1168, 1251).
+  // The resident graph keeps two branches on BT (ten steps of 480x320x28 with
+  // 2: 29.73 ms, 6: 29.96; 240x208x17 7.36, 9.47); SP's six are faster there
+  // too (27.5, 26.2).
+  int64_t npts = 0;
+  for (const ZoneDev& z : h->zh) npts += (int64_t)z.nx * z.ny * z.nz;
+  const bool large = use_fp32(h) && npts >= 2000000 && nzones >= 24;
+  const int groups = large ? 6 : 2, merge = large && kind == NPBMZ_BT ? 3 : 1;
   if ((variant_flags & NPBMZ_GRAPH) && !(variant_flags & (NPBMZ_EXACT | NPBMZ_PERZONE)) && nzones >= 8 &&
-      npbmz_set_step_groups(h, 2)) {
+      set_groups(h, groups, merge)) {
     const std::string msg = h->err;
     npbmz_destroy(h);
     *out = nullptr;
@@ -1932,29 +1981,7 @@ int npbmz_phase(npbmz_t* h, int phase, int zone) {
 int npbmz_set_step_groups(npbmz_t* h, int groups) {
   if (!h) return fail(nullptr, "null handle");
   if (groups < 1 || groups > 8) return fail(h, "groups must be 1..8");
-  CK(h, cudaStreamSynchronize(h->stream));
-  drop_graph(h);
-  h->ngroups = groups;
-  assign_zone_groups(h);
-  if (build_work_lists(h) || build_line_lists(h)) return -1;
-  {  // zones of each group (npbmz_step_download)
-    std::vector<int> zl;
-    h->grp_zone_off.assign(h->ngroups + 1, 0);
-    for (int g = 0; g < h->ngroups; ++g) {
-      for (int z = 0; z < h->nzones; ++z)
-        if (h->zone_group[z] == g) zl.push_back(z);
-      h->grp_zone_off[g + 1] = (int)zl.size();
-    }
-    if (!h->grp_zones_d) CK(h, cudaMalloc((void**)&h->grp_zones_d, std::max(1, h->nzones) * sizeof(int)));
-    CK(h, cudaMemcpy(h->grp_zones_d, zl.data(), zl.size() * sizeof(int), cudaMemcpyHostToDevice));
-  }
-  if (h->ngroups > 1 && !h->scratch_yz[0])
-    for (int d = 0; d < 2; ++d) {
-      CK(h, cudaMalloc(&h->scratch_yz[d], std::max<size_t>(h->scratch_bytes, 16)));
-      h->device_bytes += (int64_t)h->scratch_bytes;
-    }
-  h->launches_per_step = count_launches(h);
-  return 0;
+  return set_groups(h, groups, 1);
 }
 
 int npbmz_state_check(npbmz_t* h, int* bits, int* zone, int* i, int* j, int* k) {

@@ -141,6 +141,31 @@ def test_bt_line_solves_at_small_and_ragged_sizes(oracle_mod, nz, flags):
             compare(p, o, npbmz.RHS, 1e-10 if flags else FAST_REL, [z])
 
 
+@pytest.mark.parametrize("kind", ["BT", "SP"])
+def test_default_zone_groups_equal_one_branch(kind):
+    """The default groups of a graph handle (class C: six, on BT three to a
+    branch, the copies of npbmz_step_inout and npbmz_step_download by group)
+    against one branch without groups."""
+    import torch
+
+    geom, dt, _ = geom_class(kind, "C")
+    a, b = (npbmz.Problem(geom, dt, npbmz.MIXED | npbmz.GRAPH) for _ in range(2))
+    b.set_step_groups(1)
+    out = []
+    for p in (a, b):
+        p.setup(npbmz.CE_REFERENCE)
+        u = torch.zeros(p.dense_total(), dtype=torch.float64).pin_memory()
+        v = torch.zeros(p.dense_total(), dtype=torch.float64).pin_memory()
+        p.transfer_raw(npbmz.U, -1, npbmz.LAYOUT_DENSE, u.data_ptr(), False)
+        p.step_inout(3, npbmz.LAYOUT_DENSE, u.data_ptr(), v.data_ptr())
+        first = v.numpy().copy()
+        p.step_download(2, npbmz.LAYOUT_DENSE, v.data_ptr())
+        out.append((first, v.numpy().copy(), p.flatten(p.download_all(npbmz.U))))
+    for x, y in zip(*out):
+        np.testing.assert_array_equal(x, y)
+    np.testing.assert_array_equal(out[0][1], out[0][2])
+
+
 def test_bt_per_zone_solves_equal_batched_ones():
     """Launches over one zone give the bits of the batched launch on class A,
     whose x and y sweeps take twelve lanes per line and whose z sweep one
