@@ -120,7 +120,7 @@ bool make_lin_weights(const Consts& k, LinWeights& lw) {
 }
 
 // The FMA build's compute_rhs constants: every factor times dt.
-void make_rhs_f64_consts(const Consts& k, const LinWeights& lw, RhsF64Consts& c) {
+void make_rhs_f64_consts(const Consts& k, const LinWeights& lw, bool sp, RhsF64Consts& c) {
   for (int d = 0; d < 3; ++d)
     for (int cl = 0; cl < 32; ++cl)
       for (int o = 0; o < 5; ++o) c.w[d][cl][o] = k.dt * lw.w[d][cl][o];
@@ -133,7 +133,8 @@ void make_rhs_f64_consts(const Consts& k, const LinWeights& lw, RhsF64Consts& c)
   c.t2[0] = k.dttx2;
   c.t2[1] = k.dtty2;
   c.t2[2] = k.dttz2;
-  c.dt = k.dt;
+  const double kw[3] = {k.xxcon2, k.yycon2, k.zzcon2};
+  for (int d = 0; d < 3; ++d) c.kw[d] = sp ? k.dt : k.dt * kw[d];
 }
 
 float2 split_const(double v) {
@@ -1571,7 +1572,7 @@ int npbmz_create(int kind, int nzones, const int* nx, const int* ny, const int* 
       rc |= dalloc(h, &h->xd, (size_t)XD_COUNT * h->NP);
       rc |= dalloc(h, &h->fd, 5 * (size_t)h->NP);
     } else {
-      make_rhs_f64_consts(h->K, h->lw, h->rc64);
+      make_rhs_f64_consts(h->K, h->lw, h->kind == NPBMZ_SP, h->rc64);
       rc |= dalloc(h, &h->flux, (size_t)PX_COUNT * h->NP);
       rc |= dalloc(h, &h->fdt, 5 * (size_t)h->NP);
     }

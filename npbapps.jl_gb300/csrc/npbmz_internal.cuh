@@ -129,12 +129,12 @@ enum { PS_RHOI = 0, PS_US, PS_VS, PS_WS, PS_SPEED, PS_HI_COUNT, PS_COUNT = 2 * P
 // build (one value per point, shared by both neighbours that difference it):
 // the off-diagonal momentum fluxes (u2 u3 / u1 = u3 us = u2 vs, ...), the
 // normal momentum fluxes with the pressure term, the energy fluxes and the
-// viscous energy terms of each direction.
+// viscous energy terms of each direction (BT: without their factor c3c4 t3^2).
 enum {
   PX_UV = 0, PX_UW, PX_VW,   // u2*u3/u1, u2*u4/u1, u3*u4/u1
   PX_XX, PX_YY, PX_ZZ,       // u2*us + c2*(u5 - square), u3*vs + ..., u4*ws + ...
   PX_EX, PX_EY, PX_EZ,       // (c1*u5 - c2*square) * us / vs / ws
-  PX_WX, PX_WY, PX_WZ,       // con3*qs + con4*vel^2 + con5*u5/u1 with the x / y / z constants
+  PX_WX, PX_WY, PX_WZ,       // con3*qs + con4*vel^2 + con5*u5/u1 (BT: conz1, con16, c1c5)
   PX_COUNT
 };
 
@@ -274,7 +274,7 @@ struct RhsF64Consts {
   double t2[3];
   double vc[3][3];
   double vcc[3];
-  double dt;
+  double kw[3];  // factor of the viscous energy plane: dt (SP), dt c3c4 t3^2 (BT)
 };
 
 // FP64 value -> FP32 pair (hi = rn(v), lo = rn(v - hi)), the same bits as the

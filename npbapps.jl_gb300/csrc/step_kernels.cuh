@@ -90,8 +90,13 @@ __device__ __forceinline__ void prim_point(const Fields& F, const Consts& K, int
       const double u5 = F.u[4 * NP + p];
       const double us = u2 * rho_inv, vs = u3 * rho_inv, ws = u4 * rho_inv;
       const double press = K.c2 * (u5 - square);
-      const double h = K.c1 * u5 - K.c2 * square;
       const double qs = square * rho_inv, e = u5 * rho_inv;
+      // BT: the enthalpy from the pressure (c1 = 1 + c2) and the viscous term
+      // without its direction's factor, which compute_rhs applies; class C
+      // primitives 380 -> 336 us. SP keeps the expanded forms: with the short
+      // ones (529 -> 492 us) its adjoint's central differences, which stand on
+      // their rounding noise, went from 6.7e-7 to 3e-6 .. 5e-6 at worst.
+      const double h = SP ? K.c1 * u5 - K.c2 * square : u5 + press;
       X[PX_UV * NP + p] = u3 * us;
       X[PX_UW * NP + p] = u4 * us;
       X[PX_VW * NP + p] = u4 * vs;
@@ -101,9 +106,16 @@ __device__ __forceinline__ void prim_point(const Fields& F, const Consts& K, int
       X[PX_EX * NP + p] = h * us;
       X[PX_EY * NP + p] = h * vs;
       X[PX_EZ * NP + p] = h * ws;
-      X[PX_WX * NP + p] = K.xxcon3 * qs + K.xxcon4 * (us * us) + K.xxcon5 * e;
-      X[PX_WY * NP + p] = K.yycon3 * qs + K.yycon4 * (vs * vs) + K.yycon5 * e;
-      X[PX_WZ * NP + p] = K.zzcon3 * qs + K.zzcon4 * (ws * ws) + K.zzcon5 * e;
+      if (SP) {
+        X[PX_WX * NP + p] = K.xxcon3 * qs + K.xxcon4 * (us * us) + K.xxcon5 * e;
+        X[PX_WY * NP + p] = K.yycon3 * qs + K.yycon4 * (vs * vs) + K.yycon5 * e;
+        X[PX_WZ * NP + p] = K.zzcon3 * qs + K.zzcon4 * (ws * ws) + K.zzcon5 * e;
+      } else {
+        const double base = K.conz1 * qs + K.c1c5 * e;
+        X[PX_WX * NP + p] = fma(K.con16 * us, us, base);
+        X[PX_WY * NP + p] = fma(K.con16 * vs, vs, base);
+        X[PX_WZ * NP + p] = fma(K.con16 * ws, ws, base);
+      }
     }
 #endif
   }
@@ -322,11 +334,11 @@ __device__ __forceinline__ int dissip_class(int q, int n) {
 // W[2], is summed over the directions by the caller), flux planes of
 // variables 1..4 (fx[0..3]), normal momentum plane (variable a = 1 + dir),
 // velocity-term factors vc[3] (their centre term likewise), viscous energy
-// plane wv, t2; every factor carries dt.
+// plane wv and its factor kw, t2; every factor carries dt.
 __device__ __forceinline__ void rhs_dir(double r[5], const double* __restrict__ u, int64_t NP, int64_t p, int64_t st,
                                         int q, int n, const double* __restrict__ W, const double* const fx[4],
                                         const double* __restrict__ un, const double* const vel[3], const double vc[3],
-                                        const double* __restrict__ wv, double t2, double dt) {
+                                        const double* __restrict__ wv, double t2, double kw) {
   const int64_t pm2 = q >= 2 ? p - 2 * st : p;
   const int64_t pp2 = q + 2 <= n - 1 ? p + 2 * st : p;
   const double w0 = W[0], w1 = W[1], w3 = W[3], w4 = W[4];
@@ -343,7 +355,7 @@ __device__ __forceinline__ void rhs_dir(double r[5], const double* __restrict__ 
   for (int m = 0; m < 4; ++m) r[m + 1] = fma(-t2, fx[m][p + st] - fx[m][p - st], r[m + 1]);
 #pragma unroll
   for (int m = 0; m < 3; ++m) r[m + 1] = fma(vc[m], vel[m][p + st] + vel[m][p - st], r[m + 1]);
-  r[4] = fma(dt, (wv[p + st] + wv[p - st]) - 2.0 * wv[p], r[4]);
+  r[4] = fma(kw, (wv[p + st] + wv[p - st]) - 2.0 * wv[p], r[4]);
 }
 
 // One work item (128 interior points of one zone) of compute_rhs; wt: the
@@ -372,16 +384,16 @@ __device__ __forceinline__ void rhs_flux_item(const Fields& F, const Consts& K, 
     const double* Wz = wt + (2 * 32 + dissip_class(k, Z.nz)) * 5;
     {
       const double* fx[4] = {X + PX_XX * NP, X + PX_UV * NP, X + PX_UW * NP, X + PX_EX * NP};
-      rhs_dir(r, u, NP, p, 1, i, Z.nx, Wx, fx, u + NP, vel, RC.vc[0], X + PX_WX * NP, RC.t2[0], RC.dt);
+      rhs_dir(r, u, NP, p, 1, i, Z.nx, Wx, fx, u + NP, vel, RC.vc[0], X + PX_WX * NP, RC.t2[0], RC.kw[0]);
     }
     {
       const double* fx[4] = {X + PX_UV * NP, X + PX_YY * NP, X + PX_VW * NP, X + PX_EY * NP};
-      rhs_dir(r, u, NP, p, Z.nx, j, Z.ny, Wy, fx, u + 2 * NP, vel, RC.vc[1], X + PX_WY * NP, RC.t2[1], RC.dt);
+      rhs_dir(r, u, NP, p, Z.nx, j, Z.ny, Wy, fx, u + 2 * NP, vel, RC.vc[1], X + PX_WY * NP, RC.t2[1], RC.kw[1]);
     }
     {
       const double* fx[4] = {X + PX_UW * NP, X + PX_VW * NP, X + PX_ZZ * NP, X + PX_EZ * NP};
       rhs_dir(r, u, NP, p, (int64_t)Z.nx * Z.ny, k, Z.nz, Wz, fx, u + 3 * NP, vel, RC.vc[2], X + PX_WZ * NP,
-              RC.t2[2], RC.dt);
+              RC.t2[2], RC.kw[2]);
     }
     // centre point: the three directions' stencil weights and velocity
     // factors summed first
@@ -1574,7 +1586,7 @@ constexpr int PL_MIXED_W = 30;   // words per slot, first pass
 constexpr int PL_REFINE_W = 45;  // words per slot, refinement pass
 // Words per thread beside the ring: at the seam C' and r' (TWO), else b at the
 // line's last point in double-float.
-constexpr int pl_end_words(bool two) { return two ? 30 : 10; }
+__host__ __device__ constexpr int pl_end_words(bool two) { return two ? 30 : 10; }
 
 // Dynamic shared memory of the pipelined kernels for tpb lines per block.
 __host__ __device__ constexpr size_t pl_mixed_smem(int tpb, bool two) {
