@@ -465,8 +465,7 @@ def run_gpu_lu(args, cls, desc):
         te = time.perf_counter() - t0
         moved = 5 * 8 * pts  # the interior points of the reference arrays, each way
         extra["e2e"] = {"value": pts * world * args.steps / te / 1e6, "unit": "Mgridpt-steps/s",
-                        "h2d_bytes_per_step": moved, "d2h_bytes_per_step": moved, "step_groups": best_g,
-                        "ms_per_call_by_step_groups": {str(k): round(v, 3) for k, v in e2e_groups.items()},
+                        "h2d_bytes_per_step": moved, "d2h_bytes_per_step": moved,
                         "path": "npbmz_lu_upload + npbmz_lu_iterate(1) + npbmz_lu_download (zone=-1, "
                                 "NPBMZ_LAYOUT_REF) on page-locked reference-layout u, read and written in place "
                                 "(interior points only) by one kernel per zone each way"}
