@@ -259,10 +259,11 @@ int npbmz_adjoint(npbmz_t* h, int nsteps, int checkpoint_every, const double* u_
  * so FP64-bound phases of one group run beside the FP32 sweeps of the
  * previous one.  Results are unchanged (zones are independent within a step
  * after exch_qbc).  npbmz_create gives NPBMZ_GRAPH handles with at least 8
- * zones (not NPBMZ_EXACT or NPBMZ_PERZONE) 2 branches; with NPBMZ_MIXED and
- * from 2 M points 6 groups, by which npbmz_step_inout and npbmz_step_download
- * copy (BT: three to a branch of the resident step); this call makes every
- * group a branch.  No counterpart in the reference. */
+ * zones (not NPBMZ_EXACT or NPBMZ_PERZONE) 2 groups, with NPBMZ_MIXED and from
+ * 2 M points 6, by which npbmz_step_inout and npbmz_step_download copy; the
+ * resident step runs them as one branch where a branch would not fill the chip
+ * (mixed below 1 M points, SP below 2 M), on BT from 2 M three to a branch.
+ * This call makes every group a branch.  No counterpart in the reference. */
 int npbmz_set_step_groups(npbmz_t* h, int groups);
 
 /* How the zone-group branches of the step graph share the SMs.

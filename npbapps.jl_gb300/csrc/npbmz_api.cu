@@ -1644,18 +1644,24 @@ int npbmz_create(int kind, int nzones, const int* nx, const int* ny, const int* 
   if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess) { h->stream = s; h->own_stream = true; }
   h->launches_per_step = count_launches(h);
   *out = h;
-  // The step graph of a batched FMA-build step runs in zone-group branches:
-  // two, on large mixed problems of several groups each, since
-  // npbmz_step_inout, whose copies overlap the groups' work, gains by more (us
-  // by groups, 480x320x28 in and out every step: BT 2: 4809, 4: 4232, 6: 3899,
-  // 8: 3872, SP 4723, 4112, 3787, 3624; BT 240x208x17 1218, 1151, 1168, 1251).
-  // The resident graph keeps two branches on BT (ten steps of 480x320x28 with
-  // 2: 29.73 ms, 6: 29.96; 240x208x17 7.36, 9.47); SP's six are faster there
-  // too (27.5, 26.2).
+  // Zone groups and branches of the step graph of a batched FMA-build step.
+  // Large mixed problems: six groups, since npbmz_step_inout, whose copies
+  // overlap the groups' work, gains by them (us by groups, 480x320x28 in and
+  // out every step: BT 2: 4809, 4: 4232, 6: 3899, 8: 3872, SP 4723, 4112,
+  // 3787, 3624); the resident graph runs BT's as two branches (ten steps 29.73
+  // ms, six 29.96), SP's as six (2: 27.5, 6: 26.2).  Others: two groups.  Two
+  // branches overlap FP64 phases with FP32 sweeps, which pays only where each
+  // branch still fills the chip; below that they double a chain of launches
+  // that does not.  Step us with one branch / two: mixed BT 64x64x8 147 / 183,
+  // 128x128x16 315 / 403, 304x208x17 818 / 807; SP 126 / 148, 280 / 303, 750 /
+  // 760; 480x320x14 1343 / 1298; SP FP64, bound by one pipe throughout,
+  // 64x64x8 175 / 187, 304x208x17 930 / 1069, 480x320x28 3561 / 3513; BT FP64
+  // 64x64x8 209 / 198, 304x208x17 2691 / 2951, 368x400x13 3900 / 3722.
   int64_t npts = 0;
   for (const ZoneDev& z : h->zh) npts += (int64_t)z.nx * z.ny * z.nz;
   const bool large = use_fp32(h) && npts >= 2000000 && nzones >= 24;
-  const int groups = large ? 6 : 2, merge = large && kind == NPBMZ_BT ? 3 : 1;
+  const bool branches = kind == NPBMZ_BT ? !use_fp32(h) || npts >= 1000000 : npts >= 2000000;
+  const int groups = large ? 6 : 2, merge = large && kind == NPBMZ_BT ? 3 : branches ? 1 : groups;
   if ((variant_flags & NPBMZ_GRAPH) && !(variant_flags & (NPBMZ_EXACT | NPBMZ_PERZONE)) && nzones >= 8 &&
       set_groups(h, groups, merge)) {
     const std::string msg = h->err;

@@ -166,6 +166,32 @@ def test_default_zone_groups_equal_one_branch(kind):
     np.testing.assert_array_equal(out[0][1], out[0][2])
 
 
+@pytest.mark.parametrize("kind,cls,flags", [("BT", "W", npbmz.MIXED), ("SP", "W", npbmz.MIXED), ("BT", "A", npbmz.MIXED),
+                                            ("SP", "A", 0), ("BT", "W", 0), ("SP", "W", npbmz.MIXED | npbmz.RHS_DF)])
+def test_default_groups_of_small_problems_equal_one_group(kind, cls, flags):
+    """Below the sizes whose branches fill the chip a graph handle's two groups
+    share one branch; the copies still follow the groups."""
+    import torch
+
+    geom, dt, _ = geom_class(kind, cls)
+    a, b = (npbmz.Problem(geom, dt, flags | npbmz.GRAPH) for _ in range(2))
+    b.set_step_groups(1)
+    out = []
+    for p in (a, b):
+        p.setup(npbmz.CE_REFERENCE)
+        p.step(3)
+        first = p.flatten(p.download_all(npbmz.U))
+        u = torch.from_numpy(first.copy()).pin_memory()
+        v = torch.zeros(p.dense_total(), dtype=torch.float64).pin_memory()
+        p.step_inout(2, npbmz.LAYOUT_DENSE, u.data_ptr(), v.data_ptr())
+        second = v.numpy().copy()
+        p.step_download(2, npbmz.LAYOUT_DENSE, v.data_ptr())
+        out.append((first, second, v.numpy().copy(), p.flatten(p.download_all(npbmz.U))))
+    for x, y in zip(*out):
+        np.testing.assert_array_equal(x, y)
+    np.testing.assert_array_equal(out[0][2], out[0][3])
+
+
 def test_bt_per_zone_solves_equal_batched_ones():
     """Launches over one zone give the bits of the batched launch on class A,
     whose x and y sweeps take twelve lanes per line and whose z sweep one
