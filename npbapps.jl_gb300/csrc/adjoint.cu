@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(128) k_adj_solve(Fields F, Consts K, const Wor
     const int64_t pt = base + (int64_t)p * st;
     const BtState<double> u = bt_load_state<double>(F, pt);
     BtGH<DIR, double> J;
-    bt_gh<DIR, double>(k, u.ri, u.v, u.u5 * u.ri, u.q, J);
+    bt_gh<DIR, double>(k, u, J);
     double P[5][5], B[5][5], C[5][5];
     bt_form_p<DIR, double>(J, P);  // -A_{p+1}
     bt_form_b<DIR, double>(J, B);  // B_p
@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(128) k_adj_lin(Fields F, Consts K, const Work*
     x[m] = xs[m * NP + pt];
   }
   const BtState<double> s = bt_load_state<double>(F, pt);
-  const double ri = s.ri, qs = s.q, E = s.u5 * ri, *v = s.v;
+  const double ri = s.ri, qs = s.q, E = s.u[3] * ri, v[3] = {s.u[0] * ri, s.u[1] * ri, s.u[2] * ri};
   constexpr int a = DIR + 1;
   const double c1 = K.c1, c2 = K.c2, vn = v[DIR];
   const double cn = K.con43 * K.c3c4, ct = K.c3c4, c1345 = K.c1345;

@@ -207,22 +207,29 @@ __device__ __forceinline__ void bt_add_pc(const T P[5][5], const T Cp[5][5], con
     }
 }
 
-// State of one point for bt_gh from the primitive planes.
+// State of one point: 1/rho and q from compute_rhs's primitive planes, momenta
+// and energy from u as it is at the call, as the reference's sweeps take them.
+// The velocities are formed where the state is used, not where it is loaded
+// ahead (the products wait for the loads); they are the velocity planes' bits
+// while u is the u of those planes.
 template <typename T>
 struct BtState {
-  T ri, v[3], u5, q;
+  T ri, u[4], q;
 };
 template <typename T>
 __device__ __forceinline__ BtState<T> bt_load_state(const Fields& F, int64_t pt) {
   const int64_t NP = F.NP;
   BtState<T> s;
   s.ri = (T)F.prim[PR_RHOI * NP + pt];
-  s.v[0] = (T)F.prim[PR_US * NP + pt];
-  s.v[1] = (T)F.prim[PR_VS * NP + pt];
-  s.v[2] = (T)F.prim[PR_WS * NP + pt];
+#pragma unroll
+  for (int m = 0; m < 4; ++m) s.u[m] = (T)F.u[(m + 1) * NP + pt];
   s.q = (T)F.prim[PR_QS * NP + pt];
-  s.u5 = (T)F.u[4 * NP + pt];
   return s;
+}
+template <int DIR, typename T>
+__device__ __forceinline__ void bt_gh(const BtK<T>& k, const BtState<T>& s, BtGH<DIR, T>& o) {
+  const T v[3] = {bt_mul(s.u[0], s.ri), bt_mul(s.u[1], s.ri), bt_mul(s.u[2], s.ri)};
+  bt_gh<DIR, T>(k, s.ri, v, bt_mul(s.u[3], s.ri), s.q, o);
 }
 
 // The line solve, one thread per line (src/BT/x_solve.jl:444-488,501-1746 and
@@ -246,10 +253,10 @@ __global__ void __launch_bounds__(128) k_bt_line(Fields F, Consts K, const Work*
   T rp[5], Cp[5][5], Pcur[5][5], Pnext[5][5], Bs[5][5];
   BtGH<DIR, T> J;
   BtState<T> s = bt_load_state<T>(F, base);
-  bt_gh<DIR, T>(k, s.ri, s.v, s.u5 * s.ri, s.q, J);
+  bt_gh<DIR, T>(k, s, J);
   bt_form_p<DIR, T>(J, Pcur);
   s = bt_load_state<T>(F, base + st);
-  bt_gh<DIR, T>(k, s.ri, s.v, s.u5 * s.ri, s.q, J);
+  bt_gh<DIR, T>(k, s, J);
   bt_form_p<DIR, T>(J, Pnext);
   bt_form_b<DIR, T>(J, Bs);
 #pragma unroll
@@ -275,7 +282,7 @@ __global__ void __launch_bounds__(128) k_bt_line(Fields F, Consts K, const Work*
     }
     bt_add_px<DIR, T>(Pcur, rp, r);
     bt_add_pc<DIR, T>(Pcur, Cp, Bs, B);
-    bt_gh<DIR, T>(k, sp.ri, sp.v, sp.u5 * sp.ri, sp.q, J);
+    bt_gh<DIR, T>(k, sp, J);
     bt_form_c<DIR, T>(J, C);
 #pragma unroll
     for (int a = 0; a < 5; ++a)
@@ -414,7 +421,7 @@ __device__ __forceinline__ void bt_line12(const Fields& F, const Consts& K, cons
     double M[5][5];
     const int j = j0 + c;
     const bool end = ADJ && (j == 0 || j >= n - 1);
-    bt_gh<DIR, double>(k, s.ri, s.v, s.u5 * s.ri, s.q, J);
+    bt_gh<DIR, double>(k, s, J);
     bt_form_p<DIR, double>(J, M);
 #pragma unroll
     for (int a = 0; a < 5; ++a)

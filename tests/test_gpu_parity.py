@@ -141,6 +141,35 @@ def test_bt_line_solves_at_small_and_ragged_sizes(oracle_mod, nz, flags):
             compare(p, o, npbmz.RHS, 1e-10 if flags else FAST_REL, [z])
 
 
+MANY_WIDTHS = [5, 6, 7, 8, 9, 11, 13, 17, 5, 6, 7, 10, 12, 19, 23, 24]
+
+
+@pytest.mark.parametrize("xw,yw,nz", [([3, 8, 15], [4, 9, 14], 7), (MANY_WIDTHS, MANY_WIDTHS, 12)],
+                         ids=["few-lines", "many-lines"])
+def test_bt_sweeps_read_u_as_it_is_at_the_call(oracle_mod, xw, yw, nz):
+    """The sweeps take the momenta and the energy from u when they are called
+    (as x_solve and its copies do), 1/rho and |v|^2/2 from compute_rhs: u may
+    change between the phases."""
+    nx, ny, nzs, nbr = npbmz.zones_from_widths(xw, yw, nz)
+    geom = npbmz.Geometry(npbmz.BT, nx, ny, nzs, nbr, sum(xw), sum(yw), nz, len(xw), len(yw))
+    p, o = make_pair(oracle_mod, geom, 0.0008, 0, npbmz.CE_REFERENCE)
+    rng = np.random.default_rng(11)
+    for z in range(0, geom.nzones, 1 + geom.nzones // 10):
+        p.phase(npbmz.PHASE_RHS, z)
+        o.phase(0, z)
+        u = p.download(npbmz.U, z)
+        u[1:] *= 1.0 + 0.1 * rng.uniform(-1.0, 1.0, u[1:].shape)
+        p.upload(npbmz.U, z, u)
+        o.set(npbmz.U, z, u)
+        for ph in (npbmz.PHASE_XSOLVE, npbmz.PHASE_YSOLVE, npbmz.PHASE_ZSOLVE):
+            r = rng.normal(size=p.zone_shape(z))
+            p.upload(npbmz.RHS, z, r)
+            o.set(npbmz.RHS, z, r)
+            p.phase(ph, z)
+            o.phase(ph, z)
+            compare(p, o, npbmz.RHS, FAST_REL, [z])
+
+
 @pytest.mark.parametrize("kind", ["BT", "SP"])
 def test_default_zone_groups_equal_one_branch(kind):
     """The default groups of a graph handle (class C: six, on BT three to a
