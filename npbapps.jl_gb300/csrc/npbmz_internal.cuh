@@ -342,20 +342,6 @@ __device__ __forceinline__ double nr_rcp(double x) {
   return fma(y, e, y);
 }
 
-// The correctly rounded reciprocal: nr_rcp is within one ulp, and one further
-// FMA step from such an estimate rounds correctly unless the significand is all
-// ones (Markstein, as above), which takes the IEEE divide, as do the operands
-// nr_rcp divides for.  Six FP64 instructions; the divide takes nine.
-__device__ __forceinline__ double rcp_rn(double x) {
-  const int hi = __double2hiint(x);
-  const unsigned e = ((unsigned)hi >> 20) - 898u;  // sign clear, -125 <= exponent <= 125
-  if (__builtin_expect(e <= 250u && !((hi & 0xfffff) == 0xfffff && __double2loint(x) == -1), 1)) {
-    const double y = nr_rcp(x);
-    return fma(y, fma(-x, y, 1.0), y);
-  }
-  return 1.0 / x;
-}
-
 // Lines per sweep direction of a zone (interior transverse indices only).
 __host__ __device__ inline int zone_lines(const ZoneDev& z, int dir) {
   return dir == 0 ? (z.ny - 2) * (z.nz - 2) : (dir == 1 ? (z.nx - 2) * (z.nz - 2) : (z.nx - 2) * (z.ny - 2));

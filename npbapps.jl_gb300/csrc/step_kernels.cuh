@@ -697,11 +697,15 @@ __device__ __forceinline__ void bt_asm_b(const T n[5][5], T tmp1, const T dd[5],
     }
 }
 
-// Pivot reciprocal: correctly rounded in FP64 (the reference's division), in
-// the FMA build within one ulp; in the FP32 solves, which a double-float
-// refinement corrects, the fast reciprocal (within 2 ulp).
+// Pivot reciprocal: in FP64 the reference's division, in the FMA build within
+// one ulp; in the FP32 solves, which a double-float refinement corrects, the
+// fast reciprocal (within 2 ulp).  (A correctly rounded reciprocal by FMA steps
+// from the hardware estimate has the division's bits and is slower: its steps
+// follow one another.  Bit-exact sweeps x, y, z in us, FMA steps / division:
+// SP 128x128x16 163, 162, 98 / 157, 154, 94; BT 304x208x17 2271, 1777, 1252 /
+// 2258, 1762, 1241.)
 template <typename T>
-__device__ __forceinline__ T pivot_recip(T b) { return NPBMZ_HAS_FP32 ? nr_rcp(b) : rcp_rn(b); }
+__device__ __forceinline__ T pivot_recip(T b) { return NPBMZ_HAS_FP32 ? nr_rcp(b) : (T)1.0 / b; }
 template <>
 __device__ __forceinline__ float pivot_recip<float>(float b) { return __fdividef(1.0f, b); }
 
