@@ -237,9 +237,8 @@ __device__ __forceinline__ void bt_gh(const BtK<T>& k, const BtState<T>& s, BtGH
 // line], the eliminated rhs back into rhs.  The next point's state and rhs
 // are loaded one step ahead.
 template <int DIR, typename T>
-__global__ void __launch_bounds__(128) k_bt_line(Fields F, Consts K, const Work* __restrict__ work,
-                                                 T* __restrict__ lhsc, int64_t nlt, int add_u) {
-  const Work w = work[blockIdx.x];
+__device__ __forceinline__ void bt_line_item(const Fields& F, const Consts& K, const Work w, T* __restrict__ lhsc,
+                                             int64_t nlt, int add_u) {
   const ZoneDev Z = F.zones[w.zone];
   const int line = w.first + threadIdx.x;
   if (line >= zone_lines(Z, DIR)) return;
@@ -325,6 +324,12 @@ __global__ void __launch_bounds__(128) k_bt_line(Fields F, Consts K, const Work*
       rn[m] = r[m];
     }
   }
+}
+
+template <int DIR, typename T>
+__global__ void __launch_bounds__(128) k_bt_line(Fields F, Consts K, const Work* __restrict__ work, int nwork,
+                                                 T* __restrict__ lhsc, int64_t nlt, int add_u) {
+  for (int it = blockIdx.x; it < nwork; it += gridDim.x) bt_line_item<DIR, T>(F, K, work[it], lhsc, nlt, add_u);
 }
 
 // ---------------------------------------------------------------------------

@@ -12,6 +12,8 @@
 // (reference files cited at each kernel).
 #pragma once
 
+#include <algorithm>
+
 #include "npbmz_internal.cuh"
 
 #ifndef NPBMZ_NS
@@ -1046,10 +1048,8 @@ __device__ __forceinline__ void load_state_f64(const Fields& F, int64_t pt, doub
 // step ahead so that they overlap the elimination of point p.
 // IN_DF: b comes from the double-float planes F.rdf (hi part), not rhs.
 template <int DIR, bool IN_DF>
-__global__ void __launch_bounds__(128) k_bt_mixed_solve(Fields F, Consts K, const Work* __restrict__ work,
-                                                        float* __restrict__ scr, int64_t nlt,
-                                                        float* __restrict__ x0) {
-  const Work w = work[blockIdx.x];
+__device__ __forceinline__ void bt_mixed_item(const Fields& F, const Consts& K, const Work w, float* __restrict__ scr,
+                                              int64_t nlt, float* __restrict__ x0) {
   const ZoneDev Z = F.zones[w.zone];
   const int line = w.first + threadIdx.x;
   if (line >= zone_lines(Z, DIR)) return;
@@ -1103,6 +1103,12 @@ __global__ void __launch_bounds__(128) k_bt_mixed_solve(Fields F, Consts K, cons
       rn[m] = r[m];
     }
   }
+}
+
+template <int DIR, bool IN_DF>
+__global__ void __launch_bounds__(128) k_bt_mixed_solve(Fields F, Consts K, const Work* __restrict__ work, int nwork,
+                                                        float* __restrict__ scr, int64_t nlt, float* __restrict__ x0) {
+  for (int it = blockIdx.x; it < nwork; it += gridDim.x) bt_mixed_item<DIR, IN_DF>(F, K, work[it], scr, nlt, x0);
 }
 
 // Pass 2: r = b - T x0 in FP64, T d = r in FP32, x = x0 + d.  The residual
@@ -2634,6 +2640,23 @@ static int item_grid(const void* f, int nwork, int tpb, size_t smem, bool persis
   return nwork < per * sms ? nwork : per * sms;
 }
 
+#if NPBMZ_HAS_FP32
+// Blocks of the FP32 x sweeps that read the zone layout: 256 lines per SM at
+// once.  A line's points are contiguous there, so a warp's lines lie in 32
+// places and each 32-byte sector serves four steps of its line if it stays in
+// cache meanwhile; with all the lines that the registers allow (512) it does
+// not.  x sweep of 480x320x28, unrefined FP32, by lines per SM: 512 931 us, 384
+// 700, 256 535, 192 528 (641 at 384 by the kernel's registers before the scaled
+// Jacobians, which left room for more); both passes of the refined sweep
+// reading rhs in FP64 1309, 1173, 1153, 1158 (1152 before).
+static int x_items(int nwork, int tpb) {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return std::min(nwork, std::max(1, 256 / tpb) * sms);
+}
+#endif
+
 void launch_prim_w(bool sp, const Fields& F, const Consts& K, const Work* work, int nwork, cudaStream_t s,
                    bool persist) {
   if (nwork <= 0) return;
@@ -2688,9 +2711,10 @@ static void launch_solve_t(bool sp, int dir, const Fields& F, const Consts& K, c
   } else {
 #if NPBMZ_HAS_FP32
     (void)out;
-    if (dir == 0) k_bt_line<0, T><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u);
-    else if (dir == 1) k_bt_line<1, T><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u);
-    else k_bt_line<2, T><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u);
+    const int gx = sizeof(T) == sizeof(float) ? x_items(nwork, tpb) : nwork;
+    if (dir == 0) k_bt_line<0, T><<<gx, tpb, 0, s>>>(F, K, work, nwork, scr, nlt, add_u);
+    else if (dir == 1) k_bt_line<1, T><<<nwork, tpb, 0, s>>>(F, K, work, nwork, scr, nlt, add_u);
+    else k_bt_line<2, T><<<nwork, tpb, 0, s>>>(F, K, work, nwork, scr, nlt, add_u);
 #else
     if (dir == 0) k_bt_solve<0, T><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, out);
     else if (dir == 1) k_bt_solve<1, T><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, out);
@@ -2781,15 +2805,15 @@ void launch_solve(bool sp, int mode, int dir, const Fields& F, const Consts& K, 
     } else {
       float* x0 = reinterpret_cast<float*>(xw);
       if (dir == 0) {
-        k_bt_mixed_solve<0, false><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, x0);
+        k_bt_mixed_solve<0, false><<<x_items(nwork, tpb), tpb, 0, s>>>(F, K, work, nwork, scr, nlt, x0);
         if (resid64) k_bt_refine<0><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, x0);
         else k_bt_refine_df<0, false, false><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, x0);
       } else if (dir == 1) {
-        k_bt_mixed_solve<1, false><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, x0);
+        k_bt_mixed_solve<1, false><<<nwork, tpb, 0, s>>>(F, K, work, nwork, scr, nlt, x0);
         if (resid64) k_bt_refine<1><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, x0);
         else k_bt_refine_df<1, false, false><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, x0);
       } else {
-        k_bt_mixed_solve<2, false><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, x0);
+        k_bt_mixed_solve<2, false><<<nwork, tpb, 0, s>>>(F, K, work, nwork, scr, nlt, x0);
         if (resid64) k_bt_refine<2><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, x0);
         else k_bt_refine_df<2, false, false><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, x0);
       }
