@@ -737,19 +737,21 @@ void* line_scratch(npbmz_t* h, int dir) {
 // 55, 27; 338x118x8 (10,200 to 33,000) 106, 114, 48 / 91, 92, 62; 37x389x12 x
 // (14,300) 59 / 58; 192x104x27 (35,200, 32,000, 14,100) 107, 73, 96 / 117, 97,
 // 96; 480x320x28 (from 119,000) 586, 568, 635 / 668, 694, 708.
-bool few_lines(const npbmz_t* h, int dir) {
-  return h->problem_lines[dir] < (use_fp32(h) ? 14000 : dir == 2 ? 9000 : 12000);
+// fp32: the arithmetic of the sweep to be launched, not of the handle (the
+// adjoint's transposed sweeps are FP64 on every handle).
+bool few_lines(const npbmz_t* h, int dir, bool fp32) {
+  return h->problem_lines[dir] < (fp32 ? 14000 : dir == 2 ? 9000 : 12000);
 }
 
 int phase_solve(npbmz_t* h, int dir, int zone, int add_u, bool fused = false) {
   const Fields F = fields(h);
   const bool sp = h->kind == NPBMZ_SP;
   const int mode = use_exact(h) ? 0
-                   : !use_fp32(h) ? (!sp && few_lines(h, dir) ? 5 : 0)
+                   : !use_fp32(h) ? (!sp && few_lines(h, dir, false) ? 5 : 0)
                    : (h->flags & NPBMZ_FP32_NOREFINE) ? 1
                    : (h->flags & NPBMZ_REFINE_FP64) ? 3
                    : !(fused && h->rdf) ? 2
-                   : !sp && few_lines(h, dir) ? 6 : 4;
+                   : !sp && few_lines(h, dir, true) ? 6 : 4;
   return line_launches(h, dir, zone, [&](int lo, int hi, int tpb) {
     if (use_exact(h))
       exact::launch_solve(sp, 0, dir, F, h->K, h->wline_d[dir] + lo, hi - lo, tpb, line_scratch(h, dir),
@@ -1270,7 +1272,7 @@ int adjoint_back_step(npbmz_t* h, double* const x[3], double* ub, double* vb, do
   // the sweeps in reverse order
   for (int dir = 2; dir >= 0; --dir) {
     if (line_launches(h, dir, -1, [&](int lo, int hi, int tpb) {
-          adj_launch_solve(dir, few_lines(h, dir), F, h->K, h->wline_d[dir] + lo, hi - lo, tpb, yb, scr,
+          adj_launch_solve(dir, few_lines(h, dir, false), F, h->K, h->wline_d[dir] + lo, hi - lo, tpb, yb, scr,
                            h->nlines[dir], h->stream);
           CKL(h);
           return 0;
@@ -1597,7 +1599,7 @@ int npbmz_create(int kind, int nzones, const int* nx, const int* ny, const int* 
   // the SMs more evenly (bit-exact step of 304x208x17 6.47 ms with 64 lines per
   // block, 5.93 with 32; 480x320x28 FP64 z sweep 2.64 / 2.49)
   for (int dir = 0; dir < 3; ++dir)
-    if (!use_fp32(h) && (use_exact(h) || kind == NPBMZ_SP || !few_lines(h, dir)))
+    if (!use_fp32(h) && (use_exact(h) || kind == NPBMZ_SP || !few_lines(h, dir, false)))
       for (int& t : h->tpb_bkt[dir]) t = 32;
   if (!rc) rc = build_work_lists(h);
   if (!rc) rc = build_line_lists(h);

@@ -243,6 +243,25 @@ def test_bt_adjoint_matches_dual_numbers_on_ragged_zones(xw, yw, nz):
     assert np.all(np.abs(ad - dJ[:2]) <= DUAL_REL * np.abs(dJ[:2])), (ad, dJ[:2])
 
 
+def test_bt_transposed_sweeps_are_those_of_an_fp64_handle_on_a_mixed_one():
+    """The transposed sweeps are FP64 on every handle.  One step against a
+    target so large that u_1 - target does not depend on u_1's last bits: the
+    forcing's gradient comes from the sweeps' state and the target alone, so
+    both handles give the same bits (12,544 z lines, between the numbers from
+    which FP64 and refined FP32 sweeps take one thread per line)."""
+    g = npbmz.Geometry(npbmz.BT, *npbmz.zone_setup(npbmz.BT, 120, 120, 14, 4, 4, 1.0), 120, 120, 14, 4, 4)
+    grads = []
+    for flags in (0, npbmz.MIXED):
+        p = npbmz.Problem(g, 0.0008, flags)
+        p.setup(npbmz.CE_REFERENCE)
+        target = 2.0 ** 90 * np.random.default_rng(4).standard_normal(p.dense_total())
+        _, gf, _ = p.adjoint(1, target, checkpoint_every=1, grad_u0=False)
+        grads.append(p.flatten(gf))
+        p.close()
+    assert np.all(np.isfinite(grads[0])) and np.any(grads[0])
+    np.testing.assert_array_equal(*grads)
+
+
 def test_adjoint_rejects_bad_arguments(bt64):
     p, target, _ = bt64
     with pytest.raises(npbmz.NpbmzError, match="checkpoint_every"):
