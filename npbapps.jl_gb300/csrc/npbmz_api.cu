@@ -1597,10 +1597,16 @@ int npbmz_create(int kind, int nzones, const int* nx, const int* ny, const int* 
   if (!rc && h->rdf && fast::configure_kernels()) rc = fail(h, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(cudaGetLastError()));
   // FP64 sweeps with one thread per line: blocks of one warp, which spread over
   // the SMs more evenly (bit-exact step of 304x208x17 6.47 ms with 64 lines per
-  // block, 5.93 with 32; 480x320x28 FP64 z sweep 2.64 / 2.49)
-  for (int dir = 0; dir < 3; ++dir)
-    if (!use_fp32(h) && (use_exact(h) || kind == NPBMZ_SP || !few_lines(h, dir, false)))
+  // block, 5.93 with 32; 480x320x28 FP64 z sweep 2.64 / 2.49).  Not SP's FP64
+  // graphs with fewer than two such blocks per SM: those of two branches get in
+  // each other's way (step with two branches, 32 / 64 lines per block: 128x128x16
+  // 525 / 468 us, 160x128x16 607 / 535, 120x120x14 419 / 402; 240x240x12, 17,920
+  // lines, 725 / 792; one branch 442 / 435, 510 / 501, 384 / 383, 614 / 673).
+  for (int dir = 0; dir < 3; ++dir) {
+    const bool sp_graph = kind == NPBMZ_SP && (variant_flags & NPBMZ_GRAPH) && !use_exact(h) && lines[dir] < 304 * 32;
+    if (!use_fp32(h) && !sp_graph && (use_exact(h) || kind == NPBMZ_SP || !few_lines(h, dir, false)))
       for (int& t : h->tpb_bkt[dir]) t = 32;
+  }
   if (!rc) rc = build_work_lists(h);
   if (!rc) rc = build_line_lists(h);
   // staging offsets per layout and field
@@ -1647,23 +1653,38 @@ int npbmz_create(int kind, int nzones, const int* nx, const int* ny, const int* 
   h->launches_per_step = count_launches(h);
   *out = h;
   // Zone groups and branches of the step graph of a batched FMA-build step.
-  // Large mixed problems: six groups, since npbmz_step_inout, whose copies
-  // overlap the groups' work, gains by them (us by groups, 480x320x28 in and
-  // out every step: BT 2: 4809, 4: 4232, 6: 3899, 8: 3872, SP 4723, 4112,
-  // 3787, 3624); the resident graph runs BT's as two branches (ten steps 29.73
-  // ms, six 29.96), SP's as six (2: 27.5, 6: 26.2).  Others: two groups.  Two
-  // branches overlap FP64 phases with FP32 sweeps, which pays only where each
-  // branch still fills the chip; below that they double a chain of launches
-  // that does not.  Step us with one branch / two: mixed BT 64x64x8 147 / 183,
-  // 128x128x16 315 / 403, 304x208x17 818 / 807; SP 126 / 148, 280 / 303, 750 /
-  // 760; 480x320x14 1343 / 1298; SP FP64, bound by one pipe throughout,
-  // 64x64x8 175 / 187, 304x208x17 930 / 1069, 480x320x28 3561 / 3513; BT FP64
-  // 64x64x8 209 / 198, 304x208x17 2691 / 2951, 368x400x13 3900 / 3722.
+  // npbmz_step_inout copies by groups, each a branch of its own there; in the
+  // resident graph adjacent groups may share a branch.  Step us unless named
+  // otherwise.
+  //  - Large mixed problems: six groups, since npbmz_step_inout gains by them
+  //    (us by groups, 480x320x28 in and out every step: BT 2: 4809, 4: 4232, 6:
+  //    3899, 8: 3872, SP 4723, 4112, 3787, 3624); the resident graph runs BT's
+  //    as two branches (ten steps 29.73 ms, six 29.96), SP's as six (2: 27.5,
+  //    6: 26.2).
+  //  - SP FP64 below 0.8 M points: one group; the copies are shorter than what
+  //    two branches cost (in and out every step, one group / two: 128x128x16 584
+  //    / 593, 200x200x10 550 / 602, 240x240x12 936 / 982; 240x240x20 1498 / 1433,
+  //    304x208x17 1446 / 1318).
+  //  - Otherwise two groups.  Two branches overlap FP64 phases with FP32 sweeps,
+  //    or the chains of few long lines with each other; where the lines take one
+  //    thread each and do not fill the chip, the second branch doubles a chain
+  //    of launches for nothing.  One branch / two: mixed BT 64x64x8 147 / 183,
+  //    128x128x16 315 / 403, 304x208x17 818 / 807; mixed SP 126 / 148, 280 / 303,
+  //    750 / 760; 480x320x14 1343 / 1298; SP FP64, bound by one pipe throughout,
+  //    64x64x8 175 / 187, 304x208x17 930 / 1069, 480x320x28 3561 / 3513.  BT FP64
+  //    with twelve lanes per x and y line 64x64x8 236 / 211, 128x128x16 983 / 892,
+  //    160x128x16 1079 / 1061, 120x120x14 684 / 714; with one thread 96x160x24
+  //    1170 / 1710, 240x240x20 2875 / 3590, 304x208x17 2953 / 3187, 368x400x13 in
+  //    equal zones 3938 / 3741, 480x320x28 8523 / 8764.
   int64_t npts = 0;
   for (const ZoneDev& z : h->zh) npts += (int64_t)z.nx * z.ny * z.nz;
-  const bool large = use_fp32(h) && npts >= 2000000 && nzones >= 24;
-  const bool branches = kind == NPBMZ_BT ? !use_fp32(h) || npts >= 1000000 : npts >= 2000000;
-  const int groups = large ? 6 : 2, merge = large && kind == NPBMZ_BT ? 3 : branches ? 1 : groups;
+  const bool fp32 = use_fp32(h), bt = kind == NPBMZ_BT;
+  const bool large = fp32 && npts >= 2000000 && nzones >= 24;
+  const bool branches = !bt    ? npts >= 2000000
+                        : fp32 ? npts >= 1000000
+                               : few_lines(h, 0, false) && few_lines(h, 1, false);
+  const int groups = large ? 6 : !bt && !fp32 && npts < 800000 ? 1 : 2;
+  const int merge = large && bt ? 3 : branches ? 1 : groups;
   if ((variant_flags & NPBMZ_GRAPH) && !(variant_flags & (NPBMZ_EXACT | NPBMZ_PERZONE)) && nzones >= 8 &&
       set_groups(h, groups, merge)) {
     const std::string msg = h->err;
