@@ -254,7 +254,7 @@ struct npbmz_handle {
   // group-major, so group g owns one contiguous slice of each list
   int ngroups = 1;
   std::vector<int> zone_group;     // per zone
-  std::vector<Range> grp_pts, grp_int, grp_line[3];
+  std::vector<Range> grp_pts, grp_int;
   int step_merge = 1;              // groups per branch of the resident step graph (npbmz_step_inout: one each)
   int cur_group = -1;              // >= 0 while the phases of groups cur_group .. + cur_span - 1 are issued
   int cur_span = 1;
@@ -569,12 +569,15 @@ int build_line_lists(npbmz_t* h) {
     if (h->wline_d[dir]) { cudaFree(h->wline_d[dir]); h->wline_d[dir] = nullptr; }
     if ((int)h->zone_bucket[dir].size() != nz) assign_buckets(h, dir);
     const std::vector<int>& bk = h->zone_bucket[dir];
-    // group-major, then bucket, then the longest lines first
+    // by branch, bucket, group, then the longest lines first: one bucket of a
+    // group is a slice, and of a branch's groups together too
     std::vector<int> order(nz);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-      if (h->zone_group[a] != h->zone_group[b]) return h->zone_group[a] < h->zone_group[b];
+      const int ga = h->zone_group[a], gb = h->zone_group[b];
+      if (ga / h->step_merge != gb / h->step_merge) return ga < gb;
       if (bk[a] != bk[b]) return bk[a] < bk[b];
+      if (ga != gb) return ga < gb;
       return zone_line_len(h->zh[a], dir) > zone_line_len(h->zh[b], dir);
     });
     std::vector<Work> w;
@@ -596,7 +599,6 @@ int build_line_lists(npbmz_t* h) {
     h->nwline[dir] = (int)w.size();
     CK(h, cudaMalloc((void**)&h->wline_d[dir], std::max<size_t>(1, w.size()) * sizeof(Work)));
     CK(h, cudaMemcpy(h->wline_d[dir], w.data(), w.size() * sizeof(Work), cudaMemcpyHostToDevice));
-    h->grp_line[dir] = group_ranges(h, h->line_range[dir]);
   }
   return 0;
 }
@@ -613,16 +615,21 @@ int line_launches(npbmz_t* h, int dir, int zone, Fn fn) {
   }
   if (h->cur_group < 0 && h->cur_bucket < 0 && h->nbkt == 1)  // one shape: the whole list in one launch
     return h->nwline[dir] > 0 ? fn(0, h->nwline[dir], h->tpb_bkt[dir][0]) : 0;
-  const int g0 = h->cur_group >= 0 ? h->cur_group : 0, g1 = h->cur_group >= 0 ? h->cur_group + h->cur_span : h->ngroups;
-  if (h->cur_group >= 0 && h->cur_span > 1 && h->cur_bucket < 0 && h->nbkt == 1) {  // adjacent ranges of one shape
-    const int lo = h->gb_line[dir][g0].lo, hi = h->gb_line[dir][g1 - 1].hi;
-    return hi > lo ? fn(lo, hi, h->tpb_bkt[dir][0]) : 0;
-  }
-  for (int g = g0; g < g1; ++g)
+  // the groups issued together (a branch's, or one in npbmz_step_inout); all
+  // branches in turn outside a group
+  const int g0 = h->cur_group >= 0 ? h->cur_group : 0, span = h->cur_group >= 0 ? h->cur_span : h->step_merge;
+  const int g1 = h->cur_group >= 0 ? g0 + span : h->ngroups;
+  for (int g = g0; g < g1; g += span)
     for (int b = 0; b < h->nbkt; ++b) {
       if (h->cur_bucket >= 0 && b != h->cur_bucket) continue;
-      const Range r = h->gb_line[dir][(size_t)g * h->nbkt + b];
-      if (r.hi > r.lo && fn(r.lo, r.hi, h->tpb_bkt[dir][b])) return -1;
+      Range all{1 << 30, 0};
+      for (int q = g; q < std::min(g + span, h->ngroups); ++q) {
+        const Range r = h->gb_line[dir][(size_t)q * h->nbkt + b];
+        if (r.hi == r.lo) continue;
+        all.lo = std::min(all.lo, r.lo);
+        all.hi = std::max(all.hi, r.hi);
+      }
+      if (all.hi > all.lo && fn(all.lo, all.hi, h->tpb_bkt[dir][b])) return -1;
     }
   return 0;
 }
@@ -999,8 +1006,11 @@ int health_verdict(npbmz_t* h, const char* what) {
   return NPBMZ_ERR_STATE;
 }
 
+// Branches of the resident step graph.
+int step_branches(const npbmz_t* h) { return (h->ngroups + h->step_merge - 1) / h->step_merge; }
+
 // Kernel launches of one npbmz_step step: exch_qbc, then per batch (all
-// zones, each zone with PERZONE, each zone group in the grouped graph) the
+// zones, each zone with PERZONE, each branch of the grouped graph) the
 // primitive kernel, compute_rhs and the three sweeps (two kernels each when
 // the FP32 solves are refined).
 int count_launches(npbmz_t* h) {
@@ -1010,7 +1020,7 @@ int count_launches(npbmz_t* h) {
   const int adi = 2 + (h->pfx && !h->copy_fusion ? 1 : 0) + 3 * (refined ? 2 : 1) + (h->rdx ? 1 : 0);
   int batches = 1;
   if (h->flags & NPBMZ_PERZONE) batches = h->nzones;
-  else if ((h->flags & NPBMZ_GRAPH) && h->ngroups > 1 && !(h->flags & NPBMZ_EXACT)) batches = (h->ngroups + h->step_merge - 1) / h->step_merge;
+  else if ((h->flags & NPBMZ_GRAPH) && h->ngroups > 1 && !(h->flags & NPBMZ_EXACT)) batches = step_branches(h);
   return (h->nzones > 1 ? 1 : 0) + adi * batches;
 }
 
@@ -2078,11 +2088,11 @@ int npbmz_autotune(npbmz_t* h) {
   // 1. Lines per CTA of each sweep direction and zone-size bucket: the zones
   //    of a direction are split by line length into up to 3 buckets, and each
   //    bucket's candidates are timed on its own launches.  2. For graph
-  //    handles, the number of zone-group branches of the step graph, timed on
-  //    whole steps.  3. Persistent kernels (NPBMZ_PERSIST) on or off, timed
-  //    on whole steps.  4. The x sweep's state copies in the compute_rhs
-  //    launch or on their own (before 2 and after 3).  Timed on a snapshot of
-  //    u and rhs, restored afterwards; no choice changes the results.
+  //    handles, the number of branches of the step graph, timed on whole
+  //    steps.  3. Persistent kernels (NPBMZ_PERSIST) on or off, timed on whole
+  //    steps.  4. The x sweep's state copies in the compute_rhs launch or on
+  //    their own (before 2 and after 3).  Timed on a snapshot of u and rhs,
+  //    restored afterwards; no choice changes the results.
   const int cand[] = {32, 64, 128};
   const size_t bytes = 5 * (size_t)h->NP * sizeof(double);
   double* usave = nullptr;
@@ -2102,6 +2112,10 @@ int npbmz_autotune(npbmz_t* h) {
   };
   drop_graph(h);
   int rc = 0;
+  // what the handle came with: a candidate of every stage
+  int tpb0[3][HandleLimits::MAXB];
+  std::memcpy(tpb0, h->tpb_bkt, sizeof(tpb0));
+  const int nbkt0 = h->nbkt, groups0 = h->ngroups, merge0 = h->step_merge;
   h->nbkt = std::min(HandleLimits::MAXB, h->nzones);
   for (int dir = 0; dir < 3; ++dir) {
     assign_buckets(h, dir);
@@ -2134,8 +2148,8 @@ int npbmz_autotune(npbmz_t* h) {
       h->tpb_bkt[dir][bk] = best_tpb;
     }
   if (!rc) rc = build_line_lists(h);
-  // Whole steps decide: the bucket-tuned shapes against one bucket of 64
-  // lines per CTA, then (graph handles) the number of zone-group branches,
+  // Whole steps decide: the bucket-tuned shapes against the handle's own and
+  // one bucket of 64 lines per CTA, then (graph handles) the number of branches,
   // then persistent kernels; each candidate runs 2 + 6 steps from the saved
   // state, three times, and counts its fastest run.
   auto step_ms = [&]() -> float {
@@ -2152,24 +2166,30 @@ int npbmz_autotune(npbmz_t* h) {
     return best;
   };
   if (!rc) {
-    int tuned[3][HandleLimits::MAXB];
-    std::memcpy(tuned, h->tpb_bkt, sizeof(tuned));
-    const int tuned_nbkt = h->nbkt;
-    drop_graph(h);
-    const float t_tuned = step_ms();
-    h->nbkt = 1;
-    for (int dir = 0; dir < 3; ++dir) { assign_buckets(h, dir); h->tpb_bkt[dir][0] = 64; }
-    drop_graph(h);
-    if (build_line_lists(h)) rc = -1;
-    const float t_plain = rc ? -1.f : step_ms();
-    if (t_tuned < 0.f || t_plain < 0.f) rc = -1;
-    else if (t_tuned < t_plain) {
-      h->nbkt = tuned_nbkt;
+    struct Shapes {
+      int nbkt, tpb[3][HandleLimits::MAXB];
+    } cands[3];
+    cands[0].nbkt = h->nbkt;
+    std::memcpy(cands[0].tpb, h->tpb_bkt, sizeof(tpb0));
+    cands[1].nbkt = nbkt0;
+    std::memcpy(cands[1].tpb, tpb0, sizeof(tpb0));
+    cands[2].nbkt = 1;
+    for (auto& t : cands[2].tpb) std::fill(t, t + HandleLimits::MAXB, 64);
+    auto use = [&](const Shapes& c) -> int {
+      h->nbkt = c.nbkt;
+      std::memcpy(h->tpb_bkt, c.tpb, sizeof(tpb0));
       for (int dir = 0; dir < 3; ++dir) assign_buckets(h, dir);
-      std::memcpy(h->tpb_bkt, tuned, sizeof(tuned));
       drop_graph(h);
-      if (build_line_lists(h)) rc = -1;
+      return build_line_lists(h);
+    };
+    float best = 1e30f;
+    int pick = 0;
+    for (int c = 0; c < 3 && !rc; ++c) {
+      const float ms = use(cands[c]) ? -1.f : step_ms();
+      if (ms < 0.f) rc = -1;
+      else if (ms < best) { best = ms; pick = c; }
     }
+    if (!rc) rc = use(cands[pick]);
   }
   // the x-line-major copies in the compute_rhs launch or on their own: timed
   // before the group stage (whose choices depend on it) and again after the
@@ -2187,26 +2207,38 @@ int npbmz_autotune(npbmz_t* h) {
   };
   if (!rc) rc = tune_copy_fusion();
   if (!rc && (h->flags & NPBMZ_GRAPH) && !(h->flags & (NPBMZ_EXACT | NPBMZ_PERZONE)) && h->nzones >= 8) {
-    // zone-group branches; with more than one, the priority stream for the
-    // FP64 phases and a cap on the sweeps' resident CTAs per SM
-    const int gcand[] = {1, 2, 3, 4, 6, 8};
+    // branches of the resident graph: the handle's own, then 1 to 8 from the
+    // fewest zone groups that give them; from 0.8 M points not fewer groups than
+    // the handle came with, since npbmz_step_inout and npbmz_step_download copy
+    // by groups (480x320x28 in and out every step 4.56 ms with 2 groups, 3.67
+    // with 8; below, one group is the better there too: 64x64x8 193 us, 229 with
+    // two).  With more than one branch, the priority stream for the FP64 phases
+    // and a cap on the sweeps' resident CTAs per SM.
+    int64_t npts = 0;
+    for (const ZoneDev& z : h->zh) npts += (int64_t)z.nx * z.ny * z.nz;
+    const int least = npts >= 800000 ? groups0 : 1;
+    const int bcand[] = {1, 2, 3, 4, 6, 8};
     const int ccand[] = {0, 3, 2};
-    float best = 1e30f;
-    int best_g = h->ngroups, best_c = h->sweep_cap;
+    float best = step_ms();
+    if (best < 0.f) rc = -1;
+    int best_g = groups0, best_m = merge0, best_c = h->sweep_cap;
     bool best_p = h->fp64_prio;
-    for (int G : gcand)
-      for (int prio = 0; prio < (G > 1 ? 2 : 1) && !rc; ++prio)
-        for (int ci = 0; ci < (G > 1 ? 3 : 1) && !rc; ++ci) {
-          if (G > h->nzones || npbmz_set_step_groups(h, G)) continue;
+    for (int B : bcand) {
+      const int G = (least + B - 1) / B * B;
+      if (G > 8 || G > h->nzones) continue;
+      for (int prio = 0; prio < (B > 1 ? 2 : 1) && !rc; ++prio)
+        for (int ci = 0; ci < (B > 1 ? 3 : 1) && !rc; ++ci) {
+          if (set_groups(h, G, G / B)) { rc = -1; break; }
           h->fp64_prio = prio != 0;
           h->sweep_cap = ccand[ci];
           const float ms = step_ms();
           if (ms < 0.f) { rc = -1; break; }
-          if (ms < best) { best = ms; best_g = G; best_p = prio != 0; best_c = ccand[ci]; }
+          if (ms < best) { best = ms; best_g = G; best_m = G / B; best_p = prio != 0; best_c = ccand[ci]; }
         }
+    }
     h->fp64_prio = best_p;
     h->sweep_cap = best_c;
-    if (!rc) rc = npbmz_set_step_groups(h, best_g);
+    if (!rc) rc = set_groups(h, best_g, best_m);
   }
   if (!rc && !(h->flags & (NPBMZ_EXACT | NPBMZ_PERZONE))) {
     drop_graph(h);
@@ -2262,10 +2294,10 @@ int npbmz_describe(npbmz_t* h, char* buf, size_t n) {
   }
   tp += "]";
   snprintf(buf, n, "{\"kind\":\"%s\",\"zones\":%d,\"points\":%lld,\"flags\":%d,\"lines_per_cta\":%s,"
-           "\"zone_size_buckets\":%d,\"step_groups\":%d,\"fp64_priority\":%s,\"sweep_ctas_per_sm\":%d,"
+           "\"zone_size_buckets\":%d,\"step_groups\":%d,\"step_branches\":%d,\"fp64_priority\":%s,\"sweep_ctas_per_sm\":%d,"
            "\"persistent\":%s,\"copy_fusion\":%s,\"launches_per_step\":%d,\"device_bytes\":%lld}",
            h->kind == NPBMZ_BT ? "BT" : "SP", h->nzones, (long long)h->NP, h->flags, tp.c_str(), h->nbkt, h->ngroups,
-           h->fp64_prio ? "true" : "false", h->sweep_cap, (h->flags & NPBMZ_PERSIST) ? "true" : "false",
+           step_branches(h), h->fp64_prio ? "true" : "false", h->sweep_cap, (h->flags & NPBMZ_PERSIST) ? "true" : "false",
            h->copy_fusion ? "true" : "false", h->launches_per_step, (long long)h->device_bytes);
   return 0;
 }

@@ -710,6 +710,34 @@ def test_bt_class_b_autotuned_launch_shapes_keep_results(oracle_mod, flags):
         np.testing.assert_array_equal(a.download(npbmz.U, z), b.download(npbmz.U, z))
 
 
+@pytest.mark.parametrize("kind,cls", [("BT", "B"), ("BT", "C")])
+def test_autotuning_keeps_the_zone_groups_of_the_copies(kind, cls):
+    """The tuner picks the branches of the resident step graph; the zone groups
+    by which npbmz_step_inout copies do not get fewer than the two or, on class
+    C, six that these handles come with.  Results as on an untuned handle."""
+    import torch
+
+    geom, dt, _ = geom_class(kind, cls)
+    a, b = (npbmz.Problem(geom, dt, npbmz.MIXED | npbmz.GRAPH) for _ in range(2))
+    for p in (a, b):
+        p.setup(npbmz.CE_REFERENCE)
+    before = a.describe()
+    a.autotune()
+    after = a.describe()
+    assert before["step_branches"] == 2
+    assert after["step_groups"] >= before["step_groups"]
+    assert 1 <= after["step_branches"] <= after["step_groups"]
+    out = []
+    for p in (a, b):
+        u = torch.zeros(p.dense_total(), dtype=torch.float64).pin_memory()
+        p.transfer_raw(npbmz.U, -1, npbmz.LAYOUT_DENSE, u.data_ptr(), False)
+        p.step_inout(2, npbmz.LAYOUT_DENSE, u.data_ptr(), u.data_ptr())
+        p.step(2)
+        out.append((u.numpy(), p.flatten(p.download_all(npbmz.U))))
+    for x, y in zip(*out):
+        np.testing.assert_array_equal(x, y)
+
+
 def test_fma_build_reciprocal_error_bound():
     """The FMA build's primitive kernel takes 1/rho by Newton-Raphson
     refinement of the FP32 hardware estimate (npbmz_math_check runs the same
