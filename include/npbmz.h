@@ -302,11 +302,13 @@ int npbmz_synchronize(npbmz_t* h);
  * Synchronous.  No counterpart in the reference. */
 int npbmz_autotune(npbmz_t* h);
 
-/* The FP64 reciprocal (which = 0, the only one) that the FMA build's
- * primitive kernel uses for 1/rho instead of the IEEE divide (Newton-Raphson
- * refinement of the FP32 hardware estimate), applied on the current device
- * to x[0..n) (host) into y (host).  For the library's tests, which hold it to
- * its error bound.  No counterpart in the reference.  Synchronous. */
+/* Device arithmetic that replaces a division, applied on the current device
+ * to host operands for the library's tests.  which = 0: the FP64 reciprocal of
+ * x[0..n) that the FMA build uses for 1/rho and its pivots (Newton-Raphson
+ * refinement of the FP32 hardware estimate, within one ulp).  which = 1:
+ * LU-MZ's quotient x[0..n) / x[n..2n) by the rounded reciprocal, which has the
+ * division's bits.  Results into y[0..n).  No counterpart in the reference.
+ * Synchronous. */
 int npbmz_math_check(int which, int n, const double* x, double* y);
 
 /* Measured FP64 FMA throughput of the current device in GFLOP/s (an FMA

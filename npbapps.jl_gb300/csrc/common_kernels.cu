@@ -2,6 +2,7 @@
 // Compiled with -fmad=false: initialize / exact_rhs are bit-for-bit the
 // reference's arithmetic.
 #include "common_launch.h"
+#include "lu_types.h"
 #include "npbmz_internal.cuh"
 
 namespace npbmz {
@@ -426,12 +427,13 @@ void launch_faces(bool pack, const Fields& F, const FaceDesc* faces, int nfaces,
   else k_faces<false><<<grid, 256, 0, s>>>(F, faces, buf);
 }
 
-// The FMA build's FP64 reciprocal (nr_rcp of npbmz_internal.cuh), for
-// npbmz_math_check.
+// For npbmz_math_check: the FMA build's FP64 reciprocal (nr_rcp), or LU-MZ's
+// division x[t] / x[n + t] by the rounded reciprocal (div_y).
 __global__ void k_math_check(int which, int n, const double* __restrict__ x, double* __restrict__ y) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n || which != 0) return;
-  y[t] = nr_rcp(x[t]);
+  if (t >= n) return;
+  if (which == 0) y[t] = nr_rcp(x[t]);
+  else y[t] = npbmz_lu::div_y(x[t], x[n + t], 1.0 / x[n + t]);
 }
 
 void launch_math_check(int which, int n, const double* x, double* y, cudaStream_t s) {

@@ -34,24 +34,6 @@ __device__ inline double visc_up(double o, double a, double b) {
   return ERHS ? (o + a) + b : o + (a + b);
 }
 
-// v / t from y = 1/t rounded to nearest: the quotient estimate v y, refined by
-// its FMA residuals (P. Markstein, IBM J. Res. Dev. 34(1), 1990: one step from
-// an estimate within one ulp, with the correctly rounded reciprocal, gives the
-// correctly rounded quotient; the first step here makes the estimate so).  A
-// dependent divide costs nine FP64 instructions where this takes five, and
-// the FP64 pipe binds the sweeps.  Operands whose residual could underflow or
-// overflow take the divide.
-__device__ __forceinline__ double div_y(double v, double t, double y) {
-  const unsigned ev = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu, et = ((unsigned)__double2hiint(t) >> 20) & 0x7ffu;
-  // exponents of v in [2^-600, 2^600) and of t in [2^-300, 2^300): v, t, y, q and every residual are normal
-  if (__builtin_expect(ev - 423u < 1200u && et - 723u < 600u, 1)) {
-    double q = v * y;
-    q = fma(fma(-t, q, v), y, q);
-    return fma(fma(-t, q, v), y, q);
-  }
-  return v / t;
-}
-
 // The flux quantities of one point; returns q.
 __device__ __forceinline__ double prim_point(const double g[5], double pr[PR_COUNT]) {
   const double tmp = 1.0e+00 / g[0];

@@ -755,3 +755,51 @@ def test_fma_build_reciprocal_error_bound():
     want = 1.0 / x
     err_ulps = np.abs(y - want) / np.spacing(want)
     assert np.max(err_ulps) <= 2, (np.max(err_ulps), x[np.argmax(err_ulps)])
+
+
+def math_check(which, x, n):
+    import ctypes
+
+    dp = ctypes.POINTER(ctypes.c_double)
+    y = np.zeros(n)
+    assert npbmz.lib().npbmz_math_check(which, n, x.ctypes.data_as(dp), y.ctypes.data_as(dp)) == 0
+    return y
+
+
+@pytest.mark.parametrize("exponent", [-125, 0, 125])
+def test_fma_build_reciprocal_over_every_estimate(exponent):
+    """All 2^23 leading significands, the arguments of the FP32 hardware
+    estimate, at both ends of the exponents it is used for and between, with
+    the low 29 bits clear, half and full: within one ulp."""
+    lead = np.arange(2 ** 23, dtype=np.uint64) << np.uint64(29) | np.uint64((1023 + exponent) << 52)
+    for low in (0, 2 ** 28, 2 ** 29 - 1):
+        x = (lead | np.uint64(low)).view(np.float64)
+        want = 1.0 / x
+        assert np.max(np.abs(math_check(0, x, x.size) - want) / np.spacing(want)) <= 1.0
+
+
+def test_quotient_by_the_stored_reciprocal_has_the_division_bits():
+    """LU-MZ's division on random operands, around the exponents from which it
+    takes the divide, on all-ones and one-bit significands, and on zeros,
+    subnormal, infinite and NaN operands of both signs."""
+    rng = np.random.default_rng(23)
+
+    def draw(n, exponents):
+        return np.ldexp(rng.uniform(1.0, 2.0, n), rng.choice(exponents, n)) * rng.choice([-1.0, 1.0], n)
+
+    near = [e + d for e in (-600, -300, 300, 600) for d in (-2, -1, 0, 1)]
+    v = [draw(400000, np.arange(-20, 20)), draw(200000, np.arange(-1022, 1024)), draw(100000, near)]
+    t = [draw(400000, np.arange(-20, 20)), draw(200000, np.arange(-1022, 1024)), draw(100000, near)]
+    edge = np.array([1.0, 2.0 - 2.0 ** -52, 1.0 + 2.0 ** -52, 1.0 + 2.0 ** -51, 1.5, 4.0 / 3.0, 2.0 - 2.0 ** -51])
+    special = np.array([0.0, 5e-324, 2.0 ** -1030, 2.0 ** -1022, np.finfo(float).max, np.inf, np.nan])
+    e = np.concatenate([np.ldexp(edge, k) for k in (-601, -600, -301, -300, -1, 0, 1, 299, 300, 599, 600)] + [special])
+    e = np.concatenate([e, -e])
+    v.append(np.repeat(e, e.size))
+    t.append(np.tile(e, e.size))
+    v, t = np.concatenate(v), np.concatenate(t)
+    with np.errstate(all="ignore"):
+        want = v / t
+    got = math_check(1, np.concatenate([v, t]), v.size)
+    nan = np.isnan(want)
+    np.testing.assert_array_equal(np.isnan(got), nan)
+    np.testing.assert_array_equal(got[~nan].view(np.int64), want[~nan].view(np.int64))
