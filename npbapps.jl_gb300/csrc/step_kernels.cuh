@@ -1303,11 +1303,16 @@ __device__ __forceinline__ df64 df_from(double d) {
   return {h, __double2float_rn(d - (double)h)};
 }
 
-// The same without renormalisation (the low word may exceed half an ulp of the
-// high one by a few times): the residual's sums and products.  A product keeps
-// the operands' low words' product where both operands are themselves sums, so
-// that nothing above 2^-46 of the operands' magnitude is dropped, as in the
-// normalised forms: 4 or 5 operations instead of 7, 8 instead of 11 for a sum.
+// The same without renormalisation: the residual's sums and products.  The low
+// word of a sum is bounded by its summands, 2^-23 of the largest, not by the sum:
+// after a cancellation it may be as large as the high word.  So are the errors,
+// as those of the normalised forms are (the residual is judged by its terms'
+// size): a sum rounds its low word twice, 2^-46 of the largest summand.  A
+// product rounds its low word as much and drops the low words' product: with one
+// operand a sum, the other's low word is within 2^-23 of it (a pair, a product,
+// or none: plain FP32), which is 2^-46 again; with both operands sums nothing
+// bounds a low word by its high one, and du_mul_ss keeps their product.  That is
+// 4 or 5 operations instead of 7, 8 instead of 11 for a sum.
 // With the plain FP32 operands the residual takes 640 instructions a point
 // instead of 1040 (480x320x28 sweeps 586, 568, 635 -> 550, 527, 582 us); u's
 // error against 64 bits after 20 steps of 64x64x8 is 2.8e-15 (before 3.5e-15),

@@ -170,6 +170,33 @@ def test_bt_sweeps_read_u_as_it_is_at_the_call(oracle_mod, xw, yw, nz):
             compare(p, o, npbmz.RHS, FAST_REL, [z])
 
 
+@pytest.mark.parametrize("wiggle", [1e-3, 1e-6, 0.0])
+def test_bt_refined_solves_where_the_residual_terms_cancel(oracle_mod, wiggle):
+    """A right-hand side proportional to a nearly uniform state u: T u = u there,
+    so that x[m+1] - v x[0], the neighbours' fluxes and b - T x all cancel to
+    `wiggle` of their terms.  Lines of 15 points with dt 8e-4: the first pass is
+    within some 3e-7 of x, its correction leaves the square of that, and the
+    double-float residual 2^-45 of terms up to ten times x: 1e-12."""
+    nx, ny, nzs, nbr = npbmz.zones_from_widths([15, 9], [15, 8], 15)
+    geom = npbmz.Geometry(npbmz.BT, nx, ny, nzs, nbr, 24, 23, 15, 2, 2)
+    p, o = make_pair(oracle_mod, geom, 0.0008, npbmz.MIXED, npbmz.CE_REFERENCE)
+    rng = np.random.default_rng(8)
+    state = np.array([1.3, 2.1, -1.7, 0.9, 9.0])[:, None, None, None]
+    for z in range(geom.nzones):
+        u = state * (1.0 + wiggle * rng.uniform(-1.0, 1.0, p.zone_shape(z)))
+        p.upload(npbmz.U, z, u)
+        o.set(npbmz.U, z, u)
+        p.phase(npbmz.PHASE_RHS, z)
+        o.phase(0, z)
+        for ph in (npbmz.PHASE_XSOLVE, npbmz.PHASE_YSOLVE, npbmz.PHASE_ZSOLVE):
+            r = 0.3 * state * (1.0 + wiggle * rng.uniform(-1.0, 1.0, p.zone_shape(z)))
+            p.upload(npbmz.RHS, z, r)
+            o.set(npbmz.RHS, z, r)
+            p.phase(ph, z)
+            o.phase(ph, z)
+            compare(p, o, npbmz.RHS, 1e-12, [z])
+
+
 @pytest.mark.parametrize("kind", ["BT", "SP"])
 def test_default_zone_groups_equal_one_branch(kind):
     """The default groups of a graph handle (class C: six, on BT three to a
