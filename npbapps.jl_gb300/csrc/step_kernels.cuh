@@ -531,20 +531,23 @@ __host__ __device__ constexpr bool nnz(int a, int b) {
 }
 template <int DIR>
 __host__ __device__ constexpr bool anz(int a, int b) { return fnz<DIR>(a, b) || nnz(a, b) || a == b; }
+
+#if !NPBMZ_HAS_FP32  // the exact build's elimination; the FMA build's: bt_lines.cuh
 __host__ __device__ constexpr bool bnz(int a, int b) { return nnz(a, b) || a == b; }
 
 // fjac / njac at one point (src/BT/x_solve.jl:536-609, y_solve.jl:543-613,
 // z_solve.jl:537-618); only structural nonzeros are written.
-template <int DIR, typename T>
-__device__ __forceinline__ void bt_jac(const Consts& K, T tmp1, T u2, T u3, T u4, T u5, T q, T f[5][5], T n[5][5]) {
-  const T c1 = kv<T>(K.c1, K.f_c1), c2 = kv<T>(K.c2, K.f_c2), c3c4 = kv<T>(K.c3c4, K.f_c3c4);
-  const T c1345 = kv<T>(K.c1345, K.f_c1345), con43 = kv<T>(K.con43, K.f_con43);
-  const T tmp2 = tmp1 * tmp1;
-  const T tmp3 = tmp1 * tmp2;
+template <int DIR>
+__device__ __forceinline__ void bt_jac(const Consts& K, double tmp1, double u2, double u3, double u4, double u5,
+                                       double q, double f[5][5], double n[5][5]) {
+  const double c1 = K.c1, c2 = K.c2, c3c4 = K.c3c4;
+  const double c1345 = K.c1345, con43 = K.con43;
+  const double tmp2 = tmp1 * tmp1;
+  const double tmp3 = tmp1 * tmp2;
   if (DIR == 0) {
-    f[0][1] = (T)1.0;
+    f[0][1] = 1.0;
     f[1][0] = -(u2 * tmp2 * u2) + c2 * q;
-    f[1][1] = ((T)2.0 - c2) * (u2 * tmp1);
+    f[1][1] = (2.0 - c2) * (u2 * tmp1);
     f[1][2] = -c2 * (u3 * tmp1);
     f[1][3] = -c2 * (u4 * tmp1);
     f[1][4] = c2;
@@ -554,7 +557,7 @@ __device__ __forceinline__ void bt_jac(const Consts& K, T tmp1, T u2, T u3, T u4
     f[3][0] = -(u2 * u4) * tmp2;
     f[3][1] = u4 * tmp1;
     f[3][3] = u2 * tmp1;
-    f[4][0] = (c2 * (T)2.0 * q - c1 * (u5 * tmp1)) * (u2 * tmp1);
+    f[4][0] = (c2 * 2.0 * q - c1 * (u5 * tmp1)) * (u2 * tmp1);
     f[4][1] = c1 * u5 * tmp1 - c2 * (u2 * u2 * tmp2 + q);
     f[4][2] = -c2 * (u3 * u2) * tmp2;
     f[4][3] = -c2 * (u4 * u2) * tmp2;
@@ -572,19 +575,19 @@ __device__ __forceinline__ void bt_jac(const Consts& K, T tmp1, T u2, T u3, T u4
     n[4][3] = (c3c4 - c1345) * tmp2 * u4;
     n[4][4] = (c1345) * tmp1;
   } else if (DIR == 1) {
-    f[0][2] = (T)1.0;
+    f[0][2] = 1.0;
     f[1][0] = -(u2 * u3) * tmp2;
     f[1][1] = u3 * tmp1;
     f[1][2] = u2 * tmp1;
     f[2][0] = -(u3 * u3 * tmp2) + c2 * q;
     f[2][1] = -c2 * u2 * tmp1;
-    f[2][2] = ((T)2.0 - c2) * u3 * tmp1;
+    f[2][2] = (2.0 - c2) * u3 * tmp1;
     f[2][3] = -c2 * u4 * tmp1;
     f[2][4] = c2;
     f[3][0] = -(u3 * u4) * tmp2;
     f[3][2] = u4 * tmp1;
     f[3][3] = u3 * tmp1;
-    f[4][0] = (c2 * (T)2.0 * q - c1 * u5 * tmp1) * u3 * tmp1;
+    f[4][0] = (c2 * 2.0 * q - c1 * u5 * tmp1) * u3 * tmp1;
     f[4][1] = -c2 * u2 * u3 * tmp2;
     f[4][2] = c1 * u5 * tmp1 - c2 * (q + u3 * u3 * tmp2);
     f[4][3] = -c2 * (u3 * u4) * tmp2;
@@ -602,8 +605,8 @@ __device__ __forceinline__ void bt_jac(const Consts& K, T tmp1, T u2, T u3, T u4
     n[4][3] = (c3c4 - c1345) * tmp2 * u4;
     n[4][4] = (c1345) * tmp1;
   } else {
-    const T c3 = kv<T>(K.c3, K.f_c3), c4 = kv<T>(K.c4, K.f_c4);
-    f[0][3] = (T)1.0;
+    const double c3 = K.c3, c4 = K.c4;
+    f[0][3] = 1.0;
     f[1][0] = -(u2 * u4) * tmp2;
     f[1][1] = u4 * tmp1;
     f[1][3] = u2 * tmp1;
@@ -613,9 +616,9 @@ __device__ __forceinline__ void bt_jac(const Consts& K, T tmp1, T u2, T u3, T u4
     f[3][0] = -(u4 * u4 * tmp2) + c2 * q;
     f[3][1] = -c2 * u2 * tmp1;
     f[3][2] = -c2 * u3 * tmp1;
-    f[3][3] = ((T)2.0 - c2) * u4 * tmp1;
+    f[3][3] = (2.0 - c2) * u4 * tmp1;
     f[3][4] = c2;
-    f[4][0] = (c2 * (T)2.0 * q - c1 * (u5 * tmp1)) * (u4 * tmp1);
+    f[4][0] = (c2 * 2.0 * q - c1 * (u5 * tmp1)) * (u4 * tmp1);
     f[4][1] = -c2 * (u2 * u4) * tmp2;
     f[4][2] = -c2 * (u3 * u4) * tmp2;
     f[4][3] = c1 * (u5 * tmp1) - c2 * (q + u4 * u4 * tmp2);
@@ -637,8 +640,8 @@ __device__ __forceinline__ void bt_jac(const Consts& K, T tmp1, T u2, T u3, T u4
 
 // f <- tmp2 * f, n <- tmp1 * n: the products lhsa, lhsb and lhsc are sums of
 // (-tmp2 * f is their negative, tmp1 * 2.0 * n their double, both exactly).
-template <int DIR, typename T>
-__device__ __forceinline__ void bt_scale(T f[5][5], T n[5][5], T tmp1, T tmp2) {
+template <int DIR>
+__device__ __forceinline__ void bt_scale(double f[5][5], double n[5][5], double tmp1, double tmp2) {
 #pragma unroll
   for (int a = 0; a < 5; ++a)
 #pragma unroll
@@ -649,14 +652,15 @@ __device__ __forceinline__ void bt_scale(T f[5][5], T n[5][5], T tmp1, T tmp2) {
 }
 
 // lhsa at the point after the Jacobian point: -tmp2*f - tmp1*n - tmp1*d (diag).
-template <int DIR, typename T>
-__device__ __forceinline__ void bt_asm_a(const T f[5][5], const T n[5][5], T tmp1, const T dd[5], T A[5][5]) {
+template <int DIR>
+__device__ __forceinline__ void bt_asm_a(const double f[5][5], const double n[5][5], double tmp1, const double dd[5],
+                                         double A[5][5]) {
 #pragma unroll
   for (int a = 0; a < 5; ++a)
 #pragma unroll
     for (int b = 0; b < 5; ++b) {
       if (!anz<DIR>(a, b)) continue;
-      T t;
+      double t;
       bool have = false;
       if (fnz<DIR>(a, b)) { t = -f[a][b]; have = true; }
       if (nnz(a, b)) { t = have ? t - n[a][b] : -n[a][b]; have = true; }
@@ -666,13 +670,14 @@ __device__ __forceinline__ void bt_asm_a(const T f[5][5], const T n[5][5], T tmp
 }
 
 // lhsc at the point before the Jacobian point: tmp2*f - tmp1*n - tmp1*d (diag).
-template <int DIR, typename T>
-__device__ __forceinline__ void bt_asm_c(const T f[5][5], const T n[5][5], T tmp1, const T dd[5], T C[5][5]) {
+template <int DIR>
+__device__ __forceinline__ void bt_asm_c(const double f[5][5], const double n[5][5], double tmp1, const double dd[5],
+                                         double C[5][5]) {
 #pragma unroll
   for (int a = 0; a < 5; ++a)
 #pragma unroll
     for (int b = 0; b < 5; ++b) {
-      T t = (T)0.0;
+      double t = 0.0;
       bool have = false;
       if (fnz<DIR>(a, b)) { t = f[a][b]; have = true; }
       if (nnz(a, b)) { t = have ? t - n[a][b] : -n[a][b]; have = true; }
@@ -682,22 +687,22 @@ __device__ __forceinline__ void bt_asm_c(const T f[5][5], const T n[5][5], T tmp
 }
 
 // lhsb at the Jacobian point: 1 + tmp1*2*n + tmp1*2*d (diag), tmp1*2*n off-diag.
-template <typename T>
-__device__ __forceinline__ void bt_asm_b(const T n[5][5], T tmp1, const T dd[5], T B[5][5]) {
+__device__ __forceinline__ void bt_asm_b(const double n[5][5], double tmp1, const double dd[5], double B[5][5]) {
 #pragma unroll
   for (int a = 0; a < 5; ++a)
 #pragma unroll
     for (int b = 0; b < 5; ++b) {
       if (!bnz(a, b)) continue;
       if (a == b) {
-        T t = (T)1.0;
-        if (nnz(a, b)) t = fma((T)2.0, n[a][b], t);
-        B[a][b] = t + tmp1 * (T)2.0 * dd[a];
+        double t = 1.0;
+        if (nnz(a, b)) t = fma(2.0, n[a][b], t);
+        B[a][b] = t + tmp1 * 2.0 * dd[a];
       } else {
-        B[a][b] = (T)2.0 * n[a][b];
+        B[a][b] = 2.0 * n[a][b];
       }
     }
 }
+#endif
 
 // Pivot reciprocal: in FP64 the reference's division, in the FMA build within
 // one ulp; in the FP32 solves, which a double-float refinement corrects, the
@@ -711,6 +716,9 @@ __device__ __forceinline__ T pivot_recip(T b) { return NPBMZ_HAS_FP32 ? nr_rcp(b
 template <>
 __device__ __forceinline__ float pivot_recip<float>(float b) { return __fdividef(1.0f, b); }
 
+#if NPBMZ_HAS_FP32
+#include "bt_lines.cuh"
+#else
 // Columns of C that are nonzero in pivot row p when it is reached: the block's
 // own, and all once the row of the normal momentum (all nonzero) has been the
 // pivot; the other columns hold exact zeros, whose operations are skipped.
@@ -724,11 +732,11 @@ __host__ __device__ constexpr bool cfull(int p, int c) {
 
 // binvcrhs (src/BT/solve_subs.jl:468-723): Gauss-Jordan on B, no pivoting,
 // applied to C and r.
-template <int DIR, typename T>
-__device__ __forceinline__ void binvcrhs(T B[5][5], T C[5][5], T r[5]) {
+template <int DIR>
+__device__ __forceinline__ void binvcrhs(double B[5][5], double C[5][5], double r[5]) {
 #pragma unroll
   for (int p = 0; p < 5; ++p) {
-    const T pivot = pivot_recip<T>(B[p][p]);
+    const double pivot = pivot_recip<double>(B[p][p]);
 #pragma unroll
     for (int c = p + 1; c < 5; ++c) B[p][c] *= pivot;
 #pragma unroll
@@ -738,7 +746,7 @@ __device__ __forceinline__ void binvcrhs(T B[5][5], T C[5][5], T r[5]) {
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
       if (q == p) continue;
-      const T coeff = B[q][p];
+      const double coeff = B[q][p];
 #pragma unroll
       for (int c = p + 1; c < 5; ++c) B[q][c] -= coeff * B[p][c];
 #pragma unroll
@@ -749,25 +757,21 @@ __device__ __forceinline__ void binvcrhs(T B[5][5], T C[5][5], T r[5]) {
   }
 }
 
-template <int DIR, typename T>
-__device__ __forceinline__ void bt_load_point(const Fields& F, int64_t pt, T& ri, T& u2, T& u3, T& u4, T& u5, T& q) {
+template <int DIR>
+__device__ __forceinline__ void bt_load_point(const Fields& F, int64_t pt, double& ri, double& u2, double& u3,
+                                              double& u4, double& u5, double& q) {
   const int64_t NP = F.NP;
-  ri = (T)F.prim[PR_RHOI * NP + pt];
-  q = (T)F.prim[PR_QS * NP + pt];
-  u2 = (T)F.u[NP + pt];
-  u3 = (T)F.u[2 * NP + pt];
-  u4 = (T)F.u[3 * NP + pt];
-  u5 = (T)F.u[4 * NP + pt];
+  ri = F.prim[PR_RHOI * NP + pt];
+  q = F.prim[PR_QS * NP + pt];
+  u2 = F.u[NP + pt];
+  u3 = F.u[2 * NP + pt];
+  u4 = F.u[3 * NP + pt];
+  u5 = F.u[4 * NP + pt];
 }
 
-#if NPBMZ_HAS_FP32
-#include "bt_lines.cuh"
-#else
-// out: where the forward-eliminated rhs and the solution go (rhs itself).
-template <int DIR, typename T>
+template <int DIR>
 __global__ void __launch_bounds__(128) k_bt_solve(Fields F, Consts K, const Work* __restrict__ work,
-                                                  T* __restrict__ lhsc, int64_t nlt, int add_u,
-                                                  double* __restrict__ out) {
+                                                  double* __restrict__ lhsc, int64_t nlt, int add_u) {
   const Work w = work[blockIdx.x];
   const ZoneDev Z = F.zones[w.zone];
   const int line = w.first + threadIdx.x;
@@ -779,45 +783,42 @@ __global__ void __launch_bounds__(128) k_bt_solve(Fields F, Consts K, const Work
   const int64_t NP = F.NP;
   double* __restrict__ rhs = F.rhs;
 
-  const T tmp1 = kv<T>(DIR == 0 ? K.dttx1 : DIR == 1 ? K.dtty1 : K.dttz1, K.f_dtt1[DIR]);
-  const T tmp2 = kv<T>(DIR == 0 ? K.dttx2 : DIR == 1 ? K.dtty2 : K.dttz2, K.f_dtt2[DIR]);
-  const double d64[5] = {DIR == 0 ? K.dx1 : DIR == 1 ? K.dy1 : K.dz1, DIR == 0 ? K.dx2 : DIR == 1 ? K.dy2 : K.dz2,
-                         DIR == 0 ? K.dx3 : DIR == 1 ? K.dy3 : K.dz3, DIR == 0 ? K.dx4 : DIR == 1 ? K.dy4 : K.dz4,
-                         DIR == 0 ? K.dx5 : DIR == 1 ? K.dy5 : K.dz5};
-  T dd[5];
-#pragma unroll
-  for (int m = 0; m < 5; ++m) dd[m] = kv<T>(d64[m], K.f_d[DIR][m]);
+  const double tmp1 = DIR == 0 ? K.dttx1 : DIR == 1 ? K.dtty1 : K.dttz1;
+  const double tmp2 = DIR == 0 ? K.dttx2 : DIR == 1 ? K.dtty2 : K.dttz2;
+  const double dd[5] = {DIR == 0 ? K.dx1 : DIR == 1 ? K.dy1 : K.dz1, DIR == 0 ? K.dx2 : DIR == 1 ? K.dy2 : K.dz2,
+                        DIR == 0 ? K.dx3 : DIR == 1 ? K.dy3 : K.dz3, DIR == 0 ? K.dx4 : DIR == 1 ? K.dy4 : K.dz4,
+                        DIR == 0 ? K.dx5 : DIR == 1 ? K.dy5 : K.dz5};
 
-  T rp[5];          // r' at p-1
-  T Cp[5][5];       // C' at p-1
-  T Acur[5][5];     // lhsa at p   (structural nonzeros only)
-  T Anext[5][5];    // lhsa at p+1
-  T Bcur[5][5];     // lhsb at p   (structural nonzeros only)
-  T f[5][5], nj[5][5];
-  T ri, u2, u3, u4, u5, q;
+  double rp[5];          // r' at p-1
+  double Cp[5][5];       // C' at p-1
+  double Acur[5][5];     // lhsa at p   (structural nonzeros only)
+  double Anext[5][5];    // lhsa at p+1
+  double Bcur[5][5];     // lhsb at p   (structural nonzeros only)
+  double f[5][5], nj[5][5];
+  double ri, u2, u3, u4, u5, q;
 
 #pragma unroll
-  for (int m = 0; m < 5; ++m) rp[m] = (T)rhs[m * NP + base];
+  for (int m = 0; m < 5; ++m) rp[m] = rhs[m * NP + base];
   // Jacobian at point 0 -> lhsa at 1; at point 1 -> lhsb at 1 and lhsa at 2.
-  bt_load_point<DIR, T>(F, base, ri, u2, u3, u4, u5, q);
-  bt_jac<DIR, T>(K, ri, u2, u3, u4, u5, q, f, nj);
-  bt_scale<DIR, T>(f, nj, tmp1, tmp2);
-  bt_asm_a<DIR, T>(f, nj, tmp1, dd, Acur);
-  bt_load_point<DIR, T>(F, base + st, ri, u2, u3, u4, u5, q);
-  bt_jac<DIR, T>(K, ri, u2, u3, u4, u5, q, f, nj);
-  bt_scale<DIR, T>(f, nj, tmp1, tmp2);
-  bt_asm_b<T>(nj, tmp1, dd, Bcur);
-  if (n - 2 >= 2) bt_asm_a<DIR, T>(f, nj, tmp1, dd, Anext);
+  bt_load_point<DIR>(F, base, ri, u2, u3, u4, u5, q);
+  bt_jac<DIR>(K, ri, u2, u3, u4, u5, q, f, nj);
+  bt_scale<DIR>(f, nj, tmp1, tmp2);
+  bt_asm_a<DIR>(f, nj, tmp1, dd, Acur);
+  bt_load_point<DIR>(F, base + st, ri, u2, u3, u4, u5, q);
+  bt_jac<DIR>(K, ri, u2, u3, u4, u5, q, f, nj);
+  bt_scale<DIR>(f, nj, tmp1, tmp2);
+  bt_asm_b(nj, tmp1, dd, Bcur);
+  if (n - 2 >= 2) bt_asm_a<DIR>(f, nj, tmp1, dd, Anext);
 
   for (int p = 1; p <= n - 2; ++p) {
     const int64_t pt = base + p * st;
-    T r[5];
+    double r[5];
 #pragma unroll
-    for (int m = 0; m < 5; ++m) r[m] = (T)rhs[m * NP + pt];
+    for (int m = 0; m < 5; ++m) r[m] = rhs[m * NP + pt];
     // matvec_sub(lhsa_p, r'_{p-1}, r_p): the row sum is formed first.
 #pragma unroll
     for (int m = 0; m < 5; ++m) {
-      T s;
+      double s;
       bool have = false;
 #pragma unroll
       for (int c = 0; c < 5; ++c) {
@@ -828,12 +829,12 @@ __global__ void __launch_bounds__(128) k_bt_solve(Fields F, Consts K, const Work
       r[m] -= s;
     }
     // lhsb_p (full) = lhsb_p - lhsa_p * C'_{p-1}, one term at a time; C'_0 = 0.
-    T B[5][5];
+    double B[5][5];
 #pragma unroll
     for (int a = 0; a < 5; ++a)
 #pragma unroll
       for (int b = 0; b < 5; ++b) {
-        T t = bnz(a, b) ? Bcur[a][b] : (T)0.0;
+        double t = bnz(a, b) ? Bcur[a][b] : 0.0;
         bool have = bnz(a, b);
         if (p > 1) {
 #pragma unroll
@@ -846,19 +847,19 @@ __global__ void __launch_bounds__(128) k_bt_solve(Fields F, Consts K, const Work
         B[a][b] = t;
       }
     // Jacobian at p+1 -> lhsc_p, lhsb_{p+1}, lhsa_{p+2}
-    bt_load_point<DIR, T>(F, pt + st, ri, u2, u3, u4, u5, q);
-    bt_jac<DIR, T>(K, ri, u2, u3, u4, u5, q, f, nj);
-    bt_scale<DIR, T>(f, nj, tmp1, tmp2);
-    T C[5][5];
-    bt_asm_c<DIR, T>(f, nj, tmp1, dd, C);
+    bt_load_point<DIR>(F, pt + st, ri, u2, u3, u4, u5, q);
+    bt_jac<DIR>(K, ri, u2, u3, u4, u5, q, f, nj);
+    bt_scale<DIR>(f, nj, tmp1, tmp2);
+    double C[5][5];
+    bt_asm_c<DIR>(f, nj, tmp1, dd, C);
 #pragma unroll
     for (int a = 0; a < 5; ++a)
 #pragma unroll
       for (int b = 0; b < 5; ++b)
         if (anz<DIR>(a, b)) Acur[a][b] = Anext[a][b];
-    if (p + 1 <= n - 2) bt_asm_b<T>(nj, tmp1, dd, Bcur);
-    if (p + 2 <= n - 2) bt_asm_a<DIR, T>(f, nj, tmp1, dd, Anext);
-    binvcrhs<DIR, T>(B, C, r);
+    if (p + 1 <= n - 2) bt_asm_b(nj, tmp1, dd, Bcur);
+    if (p + 2 <= n - 2) bt_asm_a<DIR>(f, nj, tmp1, dd, Anext);
+    binvcrhs<DIR>(B, C, r);
 #pragma unroll
     for (int a = 0; a < 5; ++a)
 #pragma unroll
@@ -869,34 +870,27 @@ __global__ void __launch_bounds__(128) k_bt_solve(Fields F, Consts K, const Work
 #pragma unroll
     for (int m = 0; m < 5; ++m) {
       rp[m] = r[m];
-      out[m * NP + pt] = (double)r[m];
+      rhs[m * NP + pt] = r[m];
     }
   }
   // back substitution: r_p -= C'_p r_{p+1}, one term at a time; the boundary
   // value r_{n-1} is unchanged by the forward sweep.
-  T rn[5];
+  double rn[5];
 #pragma unroll
-  for (int m = 0; m < 5; ++m) rn[m] = (T)rhs[m * NP + base + (n - 1) * st];
-  if (out != rhs) {
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      out[m * NP + base] = rhs[m * NP + base];
-      out[m * NP + base + (n - 1) * st] = rhs[m * NP + base + (n - 1) * st];
-    }
-  }
+  for (int m = 0; m < 5; ++m) rn[m] = rhs[m * NP + base + (n - 1) * st];
   for (int p = n - 2; p >= 1; --p) {
     const int64_t pt = base + p * st;
-    T r[5];
+    double r[5];
 #pragma unroll
-    for (int m = 0; m < 5; ++m) r[m] = (p == n - 2) ? rp[m] : (T)out[m * NP + pt];
+    for (int m = 0; m < 5; ++m) r[m] = (p == n - 2) ? rp[m] : rhs[m * NP + pt];
 #pragma unroll
     for (int m = 0; m < 5; ++m)
 #pragma unroll
       for (int c = 0; c < 5; ++c) r[m] -= lhsc[((int64_t)p * 25 + m * 5 + c) * nlt + gl] * rn[c];
 #pragma unroll
     for (int m = 0; m < 5; ++m) {
-      const double v = (double)r[m];
-      out[m * NP + pt] = v;
+      const double v = r[m];
+      rhs[m * NP + pt] = v;
       if (add_u) F.u[m * NP + pt] += v;
       rn[m] = r[m];
     }
@@ -1046,8 +1040,7 @@ __device__ __forceinline__ void load_state_f64(const Fields& F, int64_t pt, doub
 
 // Pass 1: T x0 = b in FP32.  Loads of point p+2 and of b_{p+1} are issued one
 // step ahead so that they overlap the elimination of point p.
-// IN_DF: b comes from the double-float planes F.rdf (hi part), not rhs.
-template <int DIR, bool IN_DF>
+template <int DIR>
 __device__ __forceinline__ void bt_mixed_item(const Fields& F, const Consts& K, const Work w, float* __restrict__ scr,
                                               int64_t nlt, float* __restrict__ x0) {
   const ZoneDev Z = F.zones[w.zone];
@@ -1059,8 +1052,7 @@ __device__ __forceinline__ void bt_mixed_item(const Fields& F, const Consts& K, 
   const int64_t gl = Z.lineoff[DIR] + line;
   const int64_t NP = F.NP;
   const double* __restrict__ rhs = F.rhs;
-  const float* __restrict__ bdf = F.rdf;
-  auto bload = [&](int m, int64_t pt) -> float { return IN_DF ? bdf[m * NP + pt] : (float)rhs[m * NP + pt]; };
+  auto bload = [&](int m, int64_t pt) -> float { return (float)rhs[m * NP + pt]; };
   BtF32Carry<DIR> c;
   float s0[6], s1[6];
   load_state_f32(F, base, s0);
@@ -1105,10 +1097,10 @@ __device__ __forceinline__ void bt_mixed_item(const Fields& F, const Consts& K, 
   }
 }
 
-template <int DIR, bool IN_DF>
+template <int DIR>
 __global__ void __launch_bounds__(128) k_bt_mixed_solve(Fields F, Consts K, const Work* __restrict__ work, int nwork,
                                                         float* __restrict__ scr, int64_t nlt, float* __restrict__ x0) {
-  for (int it = blockIdx.x; it < nwork; it += gridDim.x) bt_mixed_item<DIR, IN_DF>(F, K, work[it], scr, nlt, x0);
+  for (int it = blockIdx.x; it < nwork; it += gridDim.x) bt_mixed_item<DIR>(F, K, work[it], scr, nlt, x0);
 }
 
 // Pass 2: r = b - T x0 in FP64, T d = r in FP32, x = x0 + d.  The residual
@@ -1416,10 +1408,7 @@ __device__ __forceinline__ void load_state_df(const Fields& F, int64_t pt, df64 
 // Refinement pass with the residual in double-float.  Point q contributes,
 // with P_q = tmp2 F_q and Q_q = tmp1 (N_q + D x_q),
 //   -P_q - Q_q to row q+1,   x_q + 2 Q_q to row q,   P_q - Q_q to row q-1.
-// IN_DF: b and the line's end values come from the double-float planes
-// F.rdf; OUT_DF: x goes back to F.rdf as the exact double-float sum x0 + d
-// instead of to rhs in FP64 (the next sweep of the same step reads it so).
-template <int DIR, bool IN_DF, bool OUT_DF>
+template <int DIR>
 __global__ void __launch_bounds__(128) k_bt_refine_df(Fields F, Consts K, const Work* __restrict__ work,
                                                       float* __restrict__ scr, int64_t nlt, int add_u,
                                                       const float* __restrict__ x0f) {
@@ -1433,14 +1422,12 @@ __global__ void __launch_bounds__(128) k_bt_refine_df(Fields F, Consts K, const 
   const int64_t gl = Z.lineoff[DIR] + line;
   const int64_t NP = F.NP;
   double* __restrict__ rhs = F.rhs;
-  float* __restrict__ bdf = F.rdf;
-
   const BtResid kr = bt_resid_consts<DIR>(K, false);
   auto load_x = [&](int q, df64 x[5]) {
     const int64_t pt = base + (int64_t)q * st;
     if (q == 0 || q == n - 1) {
 #pragma unroll
-      for (int m = 0; m < 5; ++m) x[m] = IN_DF ? df64{bdf[m * NP + pt], bdf[(5 + m) * NP + pt]} : df_from(rhs[m * NP + pt]);
+      for (int m = 0; m < 5; ++m) x[m] = df_from(rhs[m * NP + pt]);
     } else {
 #pragma unroll
       for (int m = 0; m < 5; ++m) x[m] = {x0f[m * NP + pt], 0.f};
@@ -1471,15 +1458,10 @@ __global__ void __launch_bounds__(128) k_bt_refine_df(Fields F, Consts K, const 
   // bt_f32_begin takes ri, u2, u3, u4, u5, q in that order (as sq)
   bt_f32_begin<DIR>(bt_consts<float>(K, DIR), s0, s1, c);
   df64 xn[5], sn[6];
-  // b of the next point: double-float planes (IN_DF) or FP64 rhs
-  df64 bn[5];
-  double bn64[5];
+  double bn[5];  // b of the next point
   auto load_b = [&](int64_t pt) {
 #pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      if (IN_DF) bn[m] = df64{bdf[m * NP + pt], bdf[(5 + m) * NP + pt]};
-      else bn64[m] = rhs[m * NP + pt];
-    }
+    for (int m = 0; m < 5; ++m) bn[m] = rhs[m * NP + pt];
   };
   load_x(2, xn);
   load_state_df(F, base + 2 * st, sn);
@@ -1487,12 +1469,10 @@ __global__ void __launch_bounds__(128) k_bt_refine_df(Fields F, Consts K, const 
 
   for (int p = 1; p <= n - 2; ++p) {
     double b[5];
-    df64 bd[5];
 #pragma unroll
     for (int m = 0; m < 5; ++m) {
       xq[m] = xn[m];
-      if (IN_DF) bd[m] = bn[m];
-      else b[m] = bn64[m];
+      b[m] = bn[m];
     }
 #pragma unroll
     for (int e = 0; e < 6; ++e) sq[e] = sn[e];
@@ -1506,12 +1486,7 @@ __global__ void __launch_bounds__(128) k_bt_refine_df(Fields F, Consts K, const 
 #pragma unroll
     for (int m = 0; m < 5; ++m) {
       const df64 tx = df_add(acc_c[m], df_sub(P[m], Q[m]));
-      if (IN_DF) {
-        const df64 rr = df_sub(bd[m], tx);
-        r[m] = rr.hi + rr.lo;
-      } else {
-        r[m] = __double2float_rn((b[m] - (double)tx.hi) - (double)tx.lo);
-      }
+      r[m] = __double2float_rn((b[m] - (double)tx.hi) - (double)tx.lo);
       acc_c[m] = df_add(acc_n[m], df_add(xq[m], df_scale2(Q[m])));
       acc_n[m] = df_neg(df_add(P[m], Q[m]));
     }
@@ -1531,15 +1506,9 @@ __global__ void __launch_bounds__(128) k_bt_refine_df(Fields F, Consts K, const 
       for (int cc = 0; cc < 5; ++cc) d[m] -= scr[((int64_t)p * BT_SCR + m * 5 + cc) * nlt + gl] * dn[cc];
 #pragma unroll
     for (int m = 0; m < 5; ++m) {
-      if (OUT_DF) {
-        const df64 v = df_two_sum(x0f[m * NP + pt], d[m]);
-        bdf[m * NP + pt] = v.hi;
-        bdf[(5 + m) * NP + pt] = v.lo;
-      } else {
-        const double v = (double)x0f[m * NP + pt] + (double)d[m];
-        rhs[m * NP + pt] = v;
-        if (add_u) F.u[m * NP + pt] += v;
-      }
+      const double v = (double)x0f[m * NP + pt] + (double)d[m];
+      rhs[m * NP + pt] = v;
+      if (add_u) F.u[m * NP + pt] += v;
       dn[m] = d[m];
     }
   }
@@ -2715,15 +2684,14 @@ static void launch_solve_t(bool sp, int dir, const Fields& F, const Consts& K, c
     else k_sp_solve<2, T><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, out, transform);
   } else {
 #if NPBMZ_HAS_FP32
-    (void)out;
     const int gx = sizeof(T) == sizeof(float) ? x_items(nwork, tpb) : nwork;
     if (dir == 0) k_bt_line<0, T><<<gx, tpb, 0, s>>>(F, K, work, nwork, scr, nlt, add_u);
     else if (dir == 1) k_bt_line<1, T><<<nwork, tpb, 0, s>>>(F, K, work, nwork, scr, nlt, add_u);
     else k_bt_line<2, T><<<nwork, tpb, 0, s>>>(F, K, work, nwork, scr, nlt, add_u);
 #else
-    if (dir == 0) k_bt_solve<0, T><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, out);
-    else if (dir == 1) k_bt_solve<1, T><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, out);
-    else k_bt_solve<2, T><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, out);
+    if (dir == 0) k_bt_solve<0><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u);
+    else if (dir == 1) k_bt_solve<1><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u);
+    else k_bt_solve<2><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u);
 #endif
   }
 }
@@ -2791,7 +2759,6 @@ void launch_solve(bool sp, int mode, int dir, const Fields& F, const Consts& K, 
 #undef NPBMZ_PL
     return;
   }
-  if (mode == 4) mode = 2;
   if (mode == 2 || mode == 3) {
     const bool resid64 = mode == 3;
     float* scr = reinterpret_cast<float*>(scratch);
@@ -2810,17 +2777,17 @@ void launch_solve(bool sp, int mode, int dir, const Fields& F, const Consts& K, 
     } else {
       float* x0 = reinterpret_cast<float*>(xw);
       if (dir == 0) {
-        k_bt_mixed_solve<0, false><<<x_items(nwork, tpb), tpb, 0, s>>>(F, K, work, nwork, scr, nlt, x0);
+        k_bt_mixed_solve<0><<<x_items(nwork, tpb), tpb, 0, s>>>(F, K, work, nwork, scr, nlt, x0);
         if (resid64) k_bt_refine<0><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, x0);
-        else k_bt_refine_df<0, false, false><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, x0);
+        else k_bt_refine_df<0><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, x0);
       } else if (dir == 1) {
-        k_bt_mixed_solve<1, false><<<nwork, tpb, 0, s>>>(F, K, work, nwork, scr, nlt, x0);
+        k_bt_mixed_solve<1><<<nwork, tpb, 0, s>>>(F, K, work, nwork, scr, nlt, x0);
         if (resid64) k_bt_refine<1><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, x0);
-        else k_bt_refine_df<1, false, false><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, x0);
+        else k_bt_refine_df<1><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, x0);
       } else {
-        k_bt_mixed_solve<2, false><<<nwork, tpb, 0, s>>>(F, K, work, nwork, scr, nlt, x0);
+        k_bt_mixed_solve<2><<<nwork, tpb, 0, s>>>(F, K, work, nwork, scr, nlt, x0);
         if (resid64) k_bt_refine<2><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, x0);
-        else k_bt_refine_df<2, false, false><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, x0);
+        else k_bt_refine_df<2><<<nwork, tpb, 0, s>>>(F, K, work, scr, nlt, add_u, x0);
       }
     }
     return;
