@@ -1607,14 +1607,18 @@ int npbmz_create(int kind, int nzones, const int* nx, const int* ny, const int* 
   if (!rc && h->rdf && fast::configure_kernels()) rc = fail(h, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(cudaGetLastError()));
   // FP64 sweeps with one thread per line: blocks of one warp, which spread over
   // the SMs more evenly (bit-exact step of 304x208x17 6.47 ms with 64 lines per
-  // block, 5.93 with 32; 480x320x28 FP64 z sweep 2.64 / 2.49).  Not SP's FP64
-  // graphs with fewer than two such blocks per SM: those of two branches get in
-  // each other's way (step with two branches, 32 / 64 lines per block: 128x128x16
-  // 525 / 468 us, 160x128x16 607 / 535, 120x120x14 419 / 402; 240x240x12, 17,920
-  // lines, 725 / 792; one branch 442 / 435, 510 / 501, 384 / 383, 614 / 673).
+  // block, 5.93 with 32; 480x320x28 FP64 z sweep 2.64 / 2.49).  The warps of a
+  // block go to different quarters of an SM, two blocks of one warp may meet on
+  // one.  So SP keeps 64 lines per block where the one-warp blocks would be one
+  // to two per SM (32 / 64: adjoint of 128x128x16, four steps, 14.54 / 14.41 ms,
+  // of 160x128x16 16.60 / 16.45), and its FP64 graphs also below, for their two
+  // branches (step with two branches: 128x128x16 525 / 468 us, 160x128x16 607 /
+  // 535, 120x120x14 419 / 402; 240x240x12, 17,920 lines, 725 / 792; one branch
+  // 442 / 435, 510 / 501, 384 / 383, 614 / 673).
   for (int dir = 0; dir < 3; ++dir) {
-    const bool sp_graph = kind == NPBMZ_SP && (variant_flags & NPBMZ_GRAPH) && !use_exact(h) && lines[dir] < 304 * 32;
-    if (!use_fp32(h) && !sp_graph && (use_exact(h) || kind == NPBMZ_SP || !few_lines(h, dir, false)))
+    const bool pair = kind == NPBMZ_SP && lines[dir] < 304 * 32 &&
+                      (lines[dir] >= 152 * 32 || ((variant_flags & NPBMZ_GRAPH) && !use_exact(h)));
+    if (!use_fp32(h) && !pair && (use_exact(h) || kind == NPBMZ_SP || !few_lines(h, dir, false)))
       for (int& t : h->tpb_bkt[dir]) t = 32;
   }
   if (!rc) rc = build_work_lists(h);
