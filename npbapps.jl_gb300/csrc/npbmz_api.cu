@@ -247,7 +247,8 @@ struct npbmz_handle {
   std::vector<Range> int_range;
   int* zblk_int_d = nullptr;
   bool bnd_dirty = true;          // boundary rhs must be reset to the forcing
-  Work* wline_d[3] = {nullptr, nullptr, nullptr};
+  Work* wline_d[3] = {nullptr, nullptr, nullptr};  // by branch
+  Work* wgrp_d[3] = {nullptr, nullptr, nullptr};   // by zone group, where groups share a branch
   int nwline[3] = {0, 0, 0};
   std::vector<Range> line_range[3];
   // zone groups of the pipelined step graph: every work list is ordered
@@ -258,6 +259,7 @@ struct npbmz_handle {
   int step_merge = 1;              // groups per branch of the resident step graph (npbmz_step_inout: one each)
   int cur_group = -1;              // >= 0 while the phases of groups cur_group .. + cur_span - 1 are issued
   int cur_span = 1;
+  bool by_group = false;           // npbmz_step_inout's first step: one group a branch, slices of wgrp_d
   cudaStream_t grp_stream[8] = {};
   // the x sweep's x-line-major state copies made by the compute_rhs launch
   // (k_rhs_flux_xc) instead of a kernel of their own (npbmz_set_copy_fusion)
@@ -290,7 +292,8 @@ struct npbmz_handle {
   int nbkt = 1;
   std::vector<int> zone_bucket[3];
   int tpb_bkt[3][HandleLimits::MAXB] = {{64, 64, 64}, {64, 64, 64}, {64, 64, 64}};
-  std::vector<Range> gb_line[3];   // per (group, bucket): slice of the line list
+  std::vector<Range> br_line[3];   // per (branch, bucket): slice of wline_d
+  std::vector<Range> gb_line[3];   // per (group, bucket): slice of wgrp_d (of wline_d without one)
   int cur_bucket = -1;             // >= 0: line launches of that bucket only
   int64_t problem_lines[3] = {0, 0, 0};  // of the whole problem, from its grid
   int64_t nlines[3] = {0, 0, 0};
@@ -531,13 +534,16 @@ int flush_boundary(npbmz_t* h) {
   if (h->rdx) {
     const Fields F = fields(h);
     const int saved = h->cur_group;
+    const bool by_group = h->by_group;
     h->cur_group = -1;
+    h->by_group = false;
     const int rc = line_launches(h, 0, -1, [&](int lo, int hi, int tpb) {
       fast::launch_xline_ends(F, h->wline_d[0] + lo, hi - lo, tpb, h->stream);
       CKL(h);
       return 0;
     });
     h->cur_group = saved;
+    h->by_group = by_group;
     if (rc) return -1;
   }
   h->bnd_dirty = false;
@@ -563,50 +569,59 @@ void assign_buckets(npbmz_t* h, int dir) {
   }
 }
 
+// The line work lists: by branch, bucket and then the longest lines first (they
+// start first, so that none is left at a launch's end).  Where groups share a
+// branch, npbmz_step_inout's launches, one group each, have a list by group.
 int build_line_lists(npbmz_t* h) {
-  const int nz = h->nzones;
+  const int nz = h->nzones, M = h->step_merge;
   for (int dir = 0; dir < 3; ++dir) {
-    if (h->wline_d[dir]) { cudaFree(h->wline_d[dir]); h->wline_d[dir] = nullptr; }
+    for (Work** d : {&h->wline_d[dir], &h->wgrp_d[dir]})
+      if (*d) { cudaFree(*d); *d = nullptr; }
     if ((int)h->zone_bucket[dir].size() != nz) assign_buckets(h, dir);
     const std::vector<int>& bk = h->zone_bucket[dir];
-    // by branch, bucket, group, then the longest lines first: one bucket of a
-    // group is a slice, and of a branch's groups together too
-    std::vector<int> order(nz);
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-      const int ga = h->zone_group[a], gb = h->zone_group[b];
-      if (ga / h->step_merge != gb / h->step_merge) return ga < gb;
-      if (bk[a] != bk[b]) return bk[a] < bk[b];
-      if (ga != gb) return ga < gb;
-      return zone_line_len(h->zh[a], dir) > zone_line_len(h->zh[b], dir);
-    });
-    std::vector<Work> w;
-    h->line_range[dir].assign(nz, Range());
-    h->gb_line[dir].assign((size_t)h->ngroups * h->nbkt, Range());
-    for (Range& r : h->gb_line[dir]) { r.lo = 1 << 30; r.hi = 0; }
-    for (int z : order) {
-      const int tpb = h->tpb_bkt[dir][bk[z]];
-      const int nl = zone_lines(h->zh[z], dir);
-      h->line_range[dir][z].lo = (int)w.size();
-      for (int f = 0; f < nl; f += tpb) w.push_back(Work{z, f});
-      h->line_range[dir][z].hi = (int)w.size();
-      Range& r = h->gb_line[dir][(size_t)h->zone_group[z] * h->nbkt + bk[z]];
-      r.lo = std::min(r.lo, h->line_range[dir][z].lo);
-      r.hi = std::max(r.hi, h->line_range[dir][z].hi);
-    }
-    for (Range& r : h->gb_line[dir])
-      if (r.hi < r.lo) r.lo = r.hi = 0;
-    h->nwline[dir] = (int)w.size();
-    CK(h, cudaMalloc((void**)&h->wline_d[dir], std::max<size_t>(1, w.size()) * sizeof(Work)));
-    CK(h, cudaMemcpy(h->wline_d[dir], w.data(), w.size() * sizeof(Work), cudaMemcpyHostToDevice));
+    // merge groups to a slice; zr: the zones' own slices
+    auto build = [&](int merge, Work** list, std::vector<Range>& slices, std::vector<Range>& zr) -> int {
+      auto slice = [&](int z) { return (h->zone_group[z] / merge) * h->nbkt + bk[z]; };
+      std::vector<int> order(nz);
+      std::iota(order.begin(), order.end(), 0);
+      std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+        if (slice(a) != slice(b)) return slice(a) < slice(b);
+        return zone_line_len(h->zh[a], dir) > zone_line_len(h->zh[b], dir);
+      });
+      std::vector<Work> w;
+      zr.assign(nz, Range());
+      slices.assign((size_t)((h->ngroups + merge - 1) / merge) * h->nbkt, Range());
+      for (int z : order) {
+        const int tpb = h->tpb_bkt[dir][bk[z]], nl = zone_lines(h->zh[z], dir);
+        zr[z].lo = (int)w.size();
+        for (int f = 0; f < nl; f += tpb) w.push_back(Work{z, f});
+        zr[z].hi = (int)w.size();
+        Range& r = slices[slice(z)];
+        if (r.hi == r.lo) r.lo = zr[z].lo;
+        r.hi = zr[z].hi;
+      }
+      h->nwline[dir] = (int)w.size();
+      CK(h, cudaMalloc((void**)list, std::max<size_t>(1, w.size()) * sizeof(Work)));
+      CK(h, cudaMemcpy(*list, w.data(), w.size() * sizeof(Work), cudaMemcpyHostToDevice));
+      return 0;
+    };
+    if (build(M, &h->wline_d[dir], h->br_line[dir], h->line_range[dir])) return -1;
+    std::vector<Range> zr;
+    if (M == 1) h->gb_line[dir] = h->br_line[dir];
+    else if (build(1, &h->wgrp_d[dir], h->gb_line[dir], zr)) return -1;
   }
   return 0;
 }
 
+// The list that line_launches' slices are of.
+const Work* line_list(const npbmz_t* h, int dir) {
+  return h->by_group && h->step_merge > 1 ? h->wgrp_d[dir] : h->wline_d[dir];
+}
+
 // Every launch over a line list goes through here: fn(lo, hi, tpb) for each
 // slice whose work items were built with tpb lines -- one zone, the current
-// zone group or all groups, bucket by bucket (the current bucket only when
-// one is set).
+// branch or zone group, or all branches, bucket by bucket (the current bucket
+// only when one is set).
 template <typename Fn>
 int line_launches(npbmz_t* h, int dir, int zone, Fn fn) {
   if (zone >= 0) {
@@ -615,21 +630,13 @@ int line_launches(npbmz_t* h, int dir, int zone, Fn fn) {
   }
   if (h->cur_group < 0 && h->cur_bucket < 0 && h->nbkt == 1)  // one shape: the whole list in one launch
     return h->nwline[dir] > 0 ? fn(0, h->nwline[dir], h->tpb_bkt[dir][0]) : 0;
-  // the groups issued together (a branch's, or one in npbmz_step_inout); all
-  // branches in turn outside a group
-  const int g0 = h->cur_group >= 0 ? h->cur_group : 0, span = h->cur_group >= 0 ? h->cur_span : h->step_merge;
-  const int g1 = h->cur_group >= 0 ? g0 + span : h->ngroups;
-  for (int g = g0; g < g1; g += span)
+  const std::vector<Range>& slices = h->by_group ? h->gb_line[dir] : h->br_line[dir];
+  const int merge = h->by_group ? 1 : h->step_merge, n = (int)slices.size() / h->nbkt;
+  for (int q = 0; q < n; ++q)
     for (int b = 0; b < h->nbkt; ++b) {
-      if (h->cur_bucket >= 0 && b != h->cur_bucket) continue;
-      Range all{1 << 30, 0};
-      for (int q = g; q < std::min(g + span, h->ngroups); ++q) {
-        const Range r = h->gb_line[dir][(size_t)q * h->nbkt + b];
-        if (r.hi == r.lo) continue;
-        all.lo = std::min(all.lo, r.lo);
-        all.hi = std::max(all.hi, r.hi);
-      }
-      if (all.hi > all.lo && fn(all.lo, all.hi, h->tpb_bkt[dir][b])) return -1;
+      if ((h->cur_group >= 0 && q != h->cur_group / merge) || (h->cur_bucket >= 0 && b != h->cur_bucket)) continue;
+      const Range r = slices[(size_t)q * h->nbkt + b];
+      if (r.hi > r.lo && fn(r.lo, r.hi, h->tpb_bkt[dir][b])) return -1;
     }
   return 0;
 }
@@ -687,7 +694,7 @@ int phase_prim(npbmz_t* h, int zone, bool fused = false) {
     // the x sweep of a fused step reads x-line-major copies of the state
     if (fused && h->pfx && !copy_in_rhs(h, zone, fused) &&
         line_launches(h, 0, zone, [&](int llo, int lhi, int tpb) {
-          fast::launch_xline_copy(sp, F, h->wline_d[0] + llo, lhi - llo, tpb, h->stream);
+          fast::launch_xline_copy(sp, F, line_list(h, 0) + llo, lhi - llo, tpb, h->stream);
           CKL(h);
           return 0;
         }))
@@ -713,7 +720,7 @@ int phase_rhs(npbmz_t* h, int zone, bool tx, bool norm, bool fused = false) {
   else if (copy_in_rhs(h, zone, fused)) {
     const XSlices x = x_slices(h, zone);
     fast::launch_rhs_xc(tx, norm, F, h->K, h->rc64, h->wint_d + lo, hi - lo, h->part_rhs + 5 * lo,
-                        h->wline_d[0] + x.lo, x.hi - x.lo, x.tpb, h->stream, (h->flags & NPBMZ_PERSIST) != 0);
+                        line_list(h, 0) + x.lo, x.hi - x.lo, x.tpb, h->stream, (h->flags & NPBMZ_PERSIST) != 0);
   } else fast::launch_rhs(tx, norm, F, h->K, h->wint_d + lo, hi - lo, h->part_rhs + 5 * lo, h->stream, &h->rc64,
                           (h->flags & NPBMZ_PERSIST) != 0);
   CKL(h);
@@ -761,10 +768,10 @@ int phase_solve(npbmz_t* h, int dir, int zone, int add_u, bool fused = false) {
                    : !sp && few_lines(h, dir, true) ? 6 : 4;
   return line_launches(h, dir, zone, [&](int lo, int hi, int tpb) {
     if (use_exact(h))
-      exact::launch_solve(sp, 0, dir, F, h->K, h->wline_d[dir] + lo, hi - lo, tpb, line_scratch(h, dir),
+      exact::launch_solve(sp, 0, dir, F, h->K, line_list(h, dir) + lo, hi - lo, tpb, line_scratch(h, dir),
                           h->nlines[dir], add_u, nullptr, h->stream);
     else
-      fast::launch_solve(sp, mode, dir, F, h->K, h->wline_d[dir] + lo, hi - lo, tpb, line_scratch(h, dir),
+      fast::launch_solve(sp, mode, dir, F, h->K, line_list(h, dir) + lo, hi - lo, tpb, line_scratch(h, dir),
                          h->nlines[dir], add_u, h->xw, h->stream, (h->flags & NPBMZ_PERSIST) != 0, h->sweep_cap);
     CKL(h);
     return 0;
@@ -861,6 +868,7 @@ int grouped_step(npbmz_t* h, cudaStream_t cs, bool inout) {
     if (inout) rc |= cudaStreamWaitEvent(P, h->up_ev[g], cudaEventWaitExternal) != cudaSuccess;
     if (g > 0 && P == S) rc |= cudaStreamWaitEvent(S, h->grp_ev[2 * (g - M)], 0) != cudaSuccess;
     h->stream = P;
+    h->by_group = inout;
     h->cur_group = g;
     h->cur_span = std::min(M, G - g);
     if (!rc) rc = phase_prim(h, -1, true);
@@ -875,6 +883,7 @@ int grouped_step(npbmz_t* h, cudaStream_t cs, bool inout) {
     if (!rc) rc = cudaEventRecord(h->grp_ev[2 * g + 1], S) != cudaSuccess;
   }
   h->stream = cs;
+  h->by_group = false;
   h->cur_group = -1;
   h->cur_span = 1;
   for (int g = 0; g < G && !rc; g += M) rc = cudaStreamWaitEvent(cs, h->grp_ev[2 * g + 1], 0) != cudaSuccess;
@@ -2372,7 +2381,7 @@ int npbmz_destroy(npbmz_t* h) {
   void* bufs[] = {h->zones_d, h->nbr_d, h->u, h->rhs, h->forcing, h->prim, h->uex, h->xw, h->primf, h->flux, h->fdt, h->ud, h->xd, h->fd, h->rdf, h->pfx, h->rdx, h->x0x, h->scratch, h->scratch_yz[0], h->scratch_yz[1], h->part_rhs,
                   h->part_err, h->norms_d, h->stage, h->wpts_d, h->zblk_pts_d, h->wint_d, h->zblk_int_d,
                   h->wline_d[0], h->wline_d[1],
-                  h->wline_d[2]};
+                  h->wline_d[2], h->wgrp_d[0], h->wgrp_d[1], h->wgrp_d[2]};
   for (void* b : bufs)
     if (b) cudaFree(b);
   for (int l = 0; l < 2; ++l)
