@@ -259,11 +259,13 @@ int npbmz_adjoint(npbmz_t* h, int nsteps, int checkpoint_every, const double* u_
  * so FP64-bound phases of one group run beside the FP32 sweeps of the
  * previous one.  Results are unchanged (zones are independent within a step
  * after exch_qbc).  npbmz_create gives NPBMZ_GRAPH handles with at least 8
- * zones (not NPBMZ_EXACT or NPBMZ_PERZONE) 2 groups, with NPBMZ_MIXED and from
- * 2 M points 6, by which npbmz_step_inout and npbmz_step_download copy; the
- * resident step runs them as one branch where a branch would not fill the chip
- * (mixed below 1 M points, SP below 2 M), on BT from 2 M three to a branch.
- * This call makes every group a branch.  No counterpart in the reference. */
+ * zones (not NPBMZ_EXACT or NPBMZ_PERZONE) 2 groups, by which npbmz_step_inout
+ * and npbmz_step_download copy; with NPBMZ_MIXED, from 2 M points and 24 zones,
+ * 6; FP64 SP below 0.8 M points 1.  Adjacent groups share a branch of the
+ * resident step where two branches would not gain: all of them on mixed handles
+ * below 1 M points, on SP below 2 M and on FP64 BT whose x or y lines take one
+ * thread each; three to a branch on mixed BT from 2 M.  This call makes every
+ * group a branch.  No counterpart in the reference. */
 int npbmz_set_step_groups(npbmz_t* h, int groups);
 
 /* How the zone-group branches of the step graph share the SMs.
@@ -297,8 +299,10 @@ int npbmz_synchronize(npbmz_t* h);
 /* Autotune the launch shapes (threads per block and work-item size per
  * phase and zone-size bucket), the number of zone-group branches of the step
  * graph (NPBMZ_GRAPH) and persistent kernels on or off (the NPBMZ_PERSIST bit
- * of the handle's flags) by timing candidates on the handle's own data; none
- * of them changes the results.  Leaves u, rhs and forcing as they were.
+ * of the handle's flags) by timing candidates on the handle's own data, what
+ * the handle came with among them; none of them changes the results.  From
+ * 0.8 M points the zone groups do not get fewer, since the copies of
+ * npbmz_step_inout go by them.  Leaves u, rhs and forcing as they were.
  * Synchronous.  No counterpart in the reference. */
 int npbmz_autotune(npbmz_t* h);
 

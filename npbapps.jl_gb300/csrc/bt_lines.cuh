@@ -14,9 +14,9 @@
 // on the right-hand sides.  The elimination visits the row of rho first, then
 // the two tangential momenta, the normal momentum and the energy: the rows
 // visited first have few nonzeros in C, whose zero columns are skipped until
-// they fill.  One point takes 389 FP64 instructions (531 with the blocks
-// formed entry by entry and Gauss-Jordan): five steps of 128x128x16 went from
-// 11.16 to 9.17 ms.  The FP32 sweeps of 480x320x28 (whose second pass also no
+// they fill.  One point takes 302 to 308 FP64 instructions (about 480 with the
+// blocks formed entry by entry and Gauss-Jordan): five steps of 128x128x16 went
+// from 11.16 to 9.17 ms.  The FP32 sweeps of 480x320x28 (whose second pass also no
 // longer stores C' again) went from 640, 610 and 681 to 586, 568 and 635 us.
 #pragma once
 
@@ -133,7 +133,7 @@ __device__ __forceinline__ void bt_form_b(const BtGH<DIR, T>& o, T B[5][5]) {
       if (hnz<DIR>(r, c)) B[r][c] = r == c ? fma((T)2.0, o.H[r][c], (T)1.0) : (T)2.0 * o.H[r][c];
 }
 
-// Pivot reciprocal: FP64 by Newton-Raphson from the FP32 estimate (2 ulps),
+// Pivot reciprocal: FP64 by Newton-Raphson from the FP32 estimate (one ulp),
 // FP32 the fast reciprocal (the refinement corrects the solve).
 __device__ __forceinline__ double bt_recip(double b) { return nr_rcp(b); }
 __device__ __forceinline__ float bt_recip(float b) { return __fdividef(1.0f, b); }
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(128) k_bt_line(Fields F, Consts K, const Work*
 // The same solve for launches with too few lines to give every SM quarter a
 // warp (FP64): twelve lanes per line, five lines per block of two warps.  An
 // SM quarter takes an FP64 warp instruction every 64 cycles whatever its
-// active lanes, and a line advances one point per 389 instructions of
+// active lanes, and a line advances one point per 300 or so instructions of
 // k_bt_line; here its work is spread over lanes and over both its ends.
 //   - Warp 0 eliminates each line from point 0 up to the middle, warp 1 from
 //     point n-1 down (the same line with G turned to -G).  At the seam

@@ -156,7 +156,7 @@ __device__ inline bool interior(const LuZone& Z, int i, int j, int k) {
   return i >= 2 && i <= Z.nx - 1 && j >= 2 && j <= Z.ny - 1 && k >= 2 && k <= Z.nz - 1;
 }
 
-// Bound by the FP64 pipe: about 330 FP64 instructions a point without
+// Bound by the FP64 pipe: 309 FP64 instructions a point without
 // contraction (444 with the convective fluxes formed at every neighbour, the
 // products with 2, 4 and 1/4 apart, and a divergent branch per stencil).
 // 480x320x28: 5.00 -> 2.58 ms; contracted 3.2 -> 1.98 ms.
@@ -691,7 +691,7 @@ __device__ __forceinline__ void sweep_row(const LuDev& D, const LuSweep& S, cons
 // Bound: an SM quarter takes an FP64 warp instruction every 64 cycles whatever
 // its active lanes, so the longest row's chain (45 FP64 instructions for row 4
 // without contraction) sets the time of a small hyperplane, and the sum of
-// the rows (about 160 per 32 points) that of a large one.  Rows 0 and 1, the
+// the rows (171 a point) that of a large one.  Rows 0 and 1, the
 // cheapest, run on warps 0 and 4, which share an SM quarter.
 // Both sweeps of one iteration (us, with block rows of 32 points, separate
 // loads and no overlap of the launches, and now): 64x64x8

@@ -741,10 +741,14 @@ void* line_scratch(npbmz_t* h, int dir) {
 // until the lines give every SM quarter (608) a warp; twelve lanes per line
 // take about 1.65 ns per row and line.  They meet at 9000 lines of equal
 // length (z, where all have the zones' nz points) and later where the longest
-// is well above the mean.  Thread / twelve lanes, us: 128x128x16 x (6720 lines,
-// 13 to 58 points) 748 / 340, z (14,400) 235 / 288; 120x120x14 z (12,544) 196 /
-// 247; 160x128x16 x (13,440, up to 38) 484 / 368; 176x160x20 x (20,736) 402 /
-// 542; 304x208x17 x (23,040, up to 72) 1052 / 1071.
+// is well above the mean: for x and y somewhere between the 13,440 and the 20,736
+// lines below, so 12,000 leaves twelve lanes' loss to none and some of their gain
+// unused.  Thread / twelve lanes, us: 128x128x16 x (6720 lines, 13 to 58 points)
+// 748 / 340, z (14,400) 235 / 288; 120x120x14 z (12,544) 196 / 247; 160x128x16 x
+// (13,440, up to 38) 484 / 368; 176x160x20 x (20,736) 402 / 542; 304x208x17 x
+// (23,040, up to 72) 1052 / 1071.  The adjoint's transposed sweeps follow the same
+// lines (four steps forward and back of 120x120x14 on a mixed handle: 9.98 ms with
+// twelve lanes in z, 9.75 with one thread).
 // FP32: one thread per line fills the chip at 152 SMs x 256 lines; half of
 // that, 128 lines per SM, is what two threads per line keep at once.  x, y, z
 // in us, one / two threads: 64x64x8 (1344, 1344, 3136 lines) 85, 72, 33 / 61,

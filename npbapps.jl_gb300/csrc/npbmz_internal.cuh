@@ -313,9 +313,10 @@ __device__ __forceinline__ void split_df(double v, float& hi, float& lo) {
 // of x's leading 24 bits, the operands move between the formats by bit
 // manipulation (integer pipe; a conversion instruction would take the FP64
 // pipe), and each FP64 FMA step squares the relative error -- about 2^-22 for
-// the estimate, 2^-44 after one step, within 2 ulps after the second.  Used
-// for 1/rho by the FMA build's primitive kernel, where the IEEE divide cost a
-// large share of its FP64 instructions.  Positive x inside the FP32 normal
+// the estimate, 2^-44 after one step, within one ulp after the second (tested
+// over every argument of the estimate).  Used by the FMA build for 1/rho in the
+// primitive kernel, where the IEEE divide cost a large share of the FP64
+// instructions, and for the pivots of its FP64 sweeps.  Positive x inside the FP32 normal
 // range only; anything else takes the IEEE divide.
 __device__ __forceinline__ bool f64_to_f32_bits(double x, float& xf) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);

@@ -1947,9 +1947,9 @@ __device__ __forceinline__ void bt_refine_pl_item(const Fields& F, const Consts&
           r[m] = rr.hi + rr.lo;
         }
       }
-      // the elimination runs again (its factors would be 25 more words to
-      // write and read, and the sweep is bound by memory); C' is the first
-      // pass's, so only r' is stored
+      // the elimination runs again: its factors would be 25 more words a point
+      // to write and read (480x320x28 x, y, z 640, 610, 681 -> 821, 901, 918 us);
+      // C' is the first pass's, so only r' is stored
       bt_f32_step<DIR, false>(k, r, s, c, scr_at(j, 0), nlt);
       if (j + PIPE > L) {
         // the ring does not refill this slot: r'_j stays here for the back
